@@ -405,7 +405,7 @@ def attention_leg(cfg, device, context, peak, reps=24):
     torch.cuda.synchronize(device)
     us = e0.elapsed_time(e1) * 1e3 / reps
     nbytes = 2 * context * hkv * d * 2
-    return {"kernel": "attn_decode_kernel (split-context decode attention alone)", "context": context, "launch_us": us,
+    return {"kernel": "attn_decode_mma_kernel (split-context decode attention alone)", "context": context, "launch_us": us,
             "bytes_per_launch": nbytes, "achieved": nbytes / us / 1e3, "peak": peak, "unit": "GB/s",
             "frac": nbytes / us / 1e3 / peak, "caches_rotated": n}
 

@@ -11,7 +11,7 @@
 //     by the last block to finish;
 //   * bf16(attended) * bf16(sigmoid(gate)).
 // The position is a host integer or, for CUDA-graph replay, a device scalar.
-#include "common.cuh"
+#include "attn_mma.cuh"
 
 constexpr int kAttnWarps = 8;
 constexpr int kAttnThreads = kAttnWarps * 32;
@@ -243,6 +243,251 @@ attn_decode_kernel(const AttnParams p) {
     if (tid == 0) seq_counters[kvh] = 0;
 }
 
+// ---------------------------------------------------------------- head dimension 256, tensor cores
+// The same mixer core with the inner loop on mma.sync (attn_mma.cuh): the kernel above spends its time in one
+// fp32 dot product and one warp reduction per head and position (a chain of shuffles), 64 blocks of it.  Here a
+// warp takes sixteen positions at a time, its key and value rows go from the cache straight into the fragments
+// (every element is needed by one lane), the next keys are requested before the softmax of these, and a context of
+// 8192 positions is split over 32 blocks per KV head, one of 32768 over 74 (148 blocks).  Bound by the latency of
+// that chain and of the two merges, not by the cache's bytes: B200, 16/2 heads,
+// 600 / 8192 / 32768 positions: - / 175 / 498 us with the kernel above, 21 / 24 / 44 us here (0.7 and 1.5 TB/s).
+constexpr int kAttnMmaSplitMin = 256;      // positions per split at least: two chunks per warp
+
+// One head of 256 features, feature j * 32 + lane in v[j]: norm, rounding and rotation as norm_rope_head does them.
+QD_DEVINL void norm_rope_256(float (&v)[8], const bf16* __restrict__ src, const bf16* __restrict__ gamma_w, int rotary, float theta,
+                             float eps, int position, int lane) {
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { v[j] = ld_bf16(src + j * 32 + lane); ss += v[j] * v[j]; }
+    ss = warp_sum(ss);
+    const float inv = rsqrtf(ss / 256.0f + eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = round_bf16((v[j] * inv) * (1.0f + ld_bf16(gamma_w + j * 32 + lane)));
+    const int hj = rotary / 64;            // registers per half of the rotary part (rotary a multiple of 64)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= hj) continue;
+        const float inv_freq = 1.0f / powf(theta, (float)(2 * (j * 32 + lane)) / (float)rotary);
+        const float angle = (float)position * inv_freq;
+        const float c = round_bf16(cosf(angle)), s = round_bf16(sinf(angle));
+#pragma unroll
+        for (int q = 0; q < 8; ++q)        // the partner's register number depends on hj
+            if (q == j + hj) {
+                const float lo = v[j], hi = v[q];
+                v[j] = round_bf16(lo * c + (-hi) * s);
+                v[q] = round_bf16(hi * c + lo * s);
+            }
+    }
+}
+
+QD_DEVINL uint4 ld_cache16(const uint8_t* p) {      // not the read-only path: the block itself writes one of the rows
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(kAttnThreads, 1)
+attn_decode_mma_kernel(const AttnParams p) {
+    extern __shared__ __align__(16) float mma_sm[];
+    constexpr int D = 256, stride = D + 2;
+    const int G = p.hq / p.hk;
+    const size_t z = blockIdx.z;
+    const bf16* const seq_qg = p.qg + z * (size_t)p.hq * 2 * D;
+    const bf16* const seq_v_new = p.v_new + z * (size_t)p.hk * D;
+    bf16* const k_cache = p.k_cache + (z ? (long long)z * p.cache_stride : 0);
+    bf16* const v_cache = p.v_cache + (z ? (long long)z * p.cache_stride : 0);
+    float* const partial = p.partial + z * (size_t)p.hk * p.splits * G * stride;
+    uint8_t* const q_s = reinterpret_cast<uint8_t*>(mma_sm);                       // [8][kAttnQRow]
+    float* const red = mma_sm + 8 * qd::kAttnQRow / sizeof(float);                 // [warps][G][D + 2], later [G][splits]
+    __shared__ int s_last;
+    const int kvh = blockIdx.x, split = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int position = p.position_dev ? p.position_dev[z] : p.position_host;
+    if (position < 0 || position >= p.capacity) {      // as in the kernel above: touches nothing
+        if (p.status && tid == 0) atomicOr(p.status, QD_STATUS_BAD_ARG);
+        return;
+    }
+    const int T = position + 1;
+    int active = (T + kAttnMmaSplitMin - 1) / kAttnMmaSplitMin;
+    if (active > p.splits) active = p.splits;
+    const int per = ((T + active - 1) / active + 15) & ~15;
+    const int t0 = split * per, t1 = min(T, t0 + per);
+    const bool mine = split < active && t0 < t1;
+
+    qd::AttnAcc acc;
+    acc.m = -INFINITY; acc.l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { acc.out[i][0] = 0.f; acc.out[i][1] = 0.f; acc.out[i][2] = 0.f; acc.out[i][3] = 0.f; }
+    if (mine) {
+        const size_t row_bytes = (size_t)p.hk * D * sizeof(bf16);
+        const uint8_t* kc = reinterpret_cast<const uint8_t*>(k_cache + (size_t)kvh * D);
+        const uint8_t* vc = reinterpret_cast<const uint8_t*>(v_cache + (size_t)kvh * D);
+        uint4 ka[8], kb[8];                // bytes 64 m + 16 t .. + 15 of key rows prow and 8 + prow
+        const int prow = qd::attn_key_row(g);
+        auto load_keys = [&](int first) {  // rows past the context (masked) read its last row
+            const uint8_t* r0 = kc + (size_t)min(first + prow, T - 1) * row_bytes + t * 16;
+            const uint8_t* r1 = kc + (size_t)min(first + 8 + prow, T - 1) * row_bytes + t * 16;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) { ka[m] = ld_cache16(r0 + m * 64); kb[m] = ld_cache16(r1 + m * 64); }
+        };
+        int c = t0 + warp * 16;
+        const bool owns_new = t1 == T;     // the block that writes the new row reads its rows after the barrier
+        if (!owns_new && c < t1) load_keys(c);
+        {                                  // warp = query head (heads beyond the group: zeros)
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = 0.f;
+            if (warp < G) norm_rope_256(v, seq_qg + (size_t)(kvh * G + warp) * 2 * D, p.q_norm, p.rotary, p.theta, p.eps, position, lane);
+            bf16* dst = reinterpret_cast<bf16*>(q_s + warp * qd::kAttnQRow);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) dst[j * 32 + lane] = __float2bfloat16_rn(v[j]);
+        }
+        if (owns_new && warp == kAttnWarps - 1) {
+            float v[8];
+            norm_rope_256(v, p.k_new + z * (size_t)p.hk * D + (size_t)kvh * D, p.k_norm, p.rotary, p.theta, p.eps, position, lane);
+            bf16* krow = k_cache + ((size_t)position * p.hk + kvh) * D;
+            bf16* vrow = v_cache + ((size_t)position * p.hk + kvh) * D;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                krow[j * 32 + lane] = __float2bfloat16_rn(v[j]);
+                vrow[j * 32 + lane] = seq_v_new[(size_t)kvh * D + j * 32 + lane];
+            }
+        }
+        __syncthreads();
+        if (owns_new && c < t1) load_keys(c);
+#pragma unroll 1
+        for (; c < t1; c += kAttnWarps * 16) {
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+            uint4 values[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint8_t* row = vc + (size_t)min(c + 4 * i + t, T - 1) * row_bytes + g * 64;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) values[q][i] = ld_cache16(row + q * 16);
+            }
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                qd::attn_score_step(s0, s1, lds128(q_s + g * qd::kAttnQRow + m * 64 + t * 16), ka[m], kb[m]);
+            if (c + kAttnWarps * 16 < t1) load_keys(c + kAttnWarps * 16);
+            const qd::AttnProbs pr = qd::attn_softmax(acc, s0, s1, c, t1, lane);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) qd::attn_value_step(acc, q, values[q][0], values[q][1], values[q][2], values[q][3], pr);
+        }
+        // lane (g, t): statistics of head g (the sum spread over its four lanes), out[i][c] = feature
+        // 32 g + 2 i + (c >> 1) of head 2 t + (c & 1)
+        acc.l += __shfl_xor_sync(0xffffffffu, acc.l, 1);
+        acc.l += __shfl_xor_sync(0xffffffffu, acc.l, 2);
+        if (t == 0 && g < G) {
+            float* dst = red + ((size_t)warp * G + g) * stride;
+            dst[D] = acc.m; dst[D + 1] = acc.l;
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+            const int h = 2 * t + cc;
+            if (h >= G) continue;
+            float* dst = red + ((size_t)warp * G + h) * stride + 32 * g;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                *reinterpret_cast<float2*>(dst + 2 * i) = make_float2(acc.out[i][cc], acc.out[i][2 + cc]);
+        }
+        __syncthreads();
+        // the warps of the block: thread = two features of G heads, in pairs of features
+        float* block_out = partial + (((size_t)kvh * p.splits + split) * G) * stride;
+        for (int idx = tid; idx < G * (D / 2); idx += kAttnThreads) {
+            const int h = idx / (D / 2), f = 2 * (idx % (D / 2));
+            float mm = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, red[((size_t)w * G + h) * stride + D]);
+            float n0 = 0.f, n1 = 0.f, den = 0.f;
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) {
+                const float* src = red + ((size_t)w * G + h) * stride;
+                const float wgt = src[D] == -INFINITY ? 0.f : expf(src[D] - mm);
+                const float2 v = *reinterpret_cast<const float2*>(src + f);
+                n0 += wgt * v.x; n1 += wgt * v.y; den += wgt * src[D + 1];
+            }
+            *reinterpret_cast<float2*>(block_out + (size_t)h * stride + f) = make_float2(n0, n1);
+            if (f == 0) *reinterpret_cast<float2*>(block_out + (size_t)h * stride + D) = make_float2(mm, den);
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    unsigned int* counter = p.counters + z * (size_t)p.hk + kvh;
+    if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)p.splits - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // the last block of this KV head merges the splits: their factors first, then all partial sums of a feature with
+    // independent loads
+    const int used = (T + per - 1) / per;
+    const float* base = partial + (size_t)kvh * p.splits * G * stride;
+    float* den_s = red + (size_t)G * used;
+    for (int h = warp; h < G; h += kAttnWarps) {
+        float mm = -INFINITY, den = 0.f;
+        for (int s = lane; s < used; s += 32) mm = fmaxf(mm, __ldcg(base + ((size_t)s * G + h) * stride + D));
+        mm = warp_max(mm);
+        for (int s = lane; s < used; s += 32) {
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + ((size_t)s * G + h) * stride + D));
+            const float wgt = expf(ml.x - mm);
+            red[h * used + s] = wgt;
+            den += wgt * ml.y;
+        }
+        den = warp_sum(den);
+        if (lane == 0) den_s[h] = den;
+    }
+    __syncthreads();
+    for (int idx = tid; idx < G * (D / 2); idx += kAttnThreads) {
+        const int h = idx / (D / 2), f = 2 * (idx % (D / 2));
+        float n0 = 0.f, n1 = 0.f;
+#pragma unroll 16
+        for (int s = 0; s < used; ++s) {
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(base + ((size_t)s * G + h) * stride + f));
+            const float wgt = red[h * used + s];
+            n0 += wgt * v.x; n1 += wgt * v.y;
+        }
+        const int qh = kvh * G + h;
+        const float den = den_s[h];
+        const bf16* gate = seq_qg + (size_t)qh * 2 * D + D + f;
+        const float g0 = round_bf16(sigmoid_precise(ld_bf16(gate))), g1 = round_bf16(sigmoid_precise(ld_bf16(gate + 1)));
+        *reinterpret_cast<__nv_bfloat162*>(p.out + z * (size_t)p.hq * D + (size_t)qh * D + f) =
+            __floats2bfloat162_rn(round_bf16(n0 / den) * g0, round_bf16(n1 / den) * g1);
+    }
+    if (tid == 0) *counter = 0;
+}
+
+// Either kernel for `batch` sequences.  The tensor-core one takes head dimension 256 with rows on 16-byte boundaries, a
+// rotary part of whole warps per half and partial sums on 8-byte boundaries; the splits' factors reuse the warps' area.
+static int launch_attn(const AttnParams& p, int batch, int pdl, cudaStream_t stream) {
+    const int G = p.hq / p.hk;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
+    const uintptr_t align = (uintptr_t)p.k_cache | (uintptr_t)p.v_cache;
+    const size_t merge = (size_t)kAttnWarps * G * (p.d + 2);
+    if (p.d == 256 && p.rotary % 64 == 0 && !(align & 15u) && !(p.cache_stride & 7) && !((uintptr_t)p.partial & 7u) &&
+        !((uintptr_t)p.out & 3u) && (size_t)G * (p.splits + 1) <= merge) {
+        const size_t smem = 8 * qd::kAttnQRow + sizeof(float) * merge;
+        static bool mma_configured[64];
+        if (!mma_configured[dev]) {
+            if (cudaFuncSetAttribute(attn_decode_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
+                return QD_ERR_LAUNCH;
+            mma_configured[dev] = true;
+        }
+        return qd_launch(attn_decode_mma_kernel, dim3(p.hk, p.splits, batch), dim3(kAttnThreads), smem, stream, pdl, p);
+    }
+    const size_t smem = sizeof(float) * ((size_t)G * p.d + p.d + merge);
+    if (smem > 100 * 1024) return QD_ERR_UNSUPPORTED;
+    static bool configured[64];
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
+            return QD_ERR_LAUNCH;
+        configured[dev] = true;
+    }
+    return qd_launch(attn_decode_kernel, dim3(p.hk, p.splits, batch), dim3(kAttnThreads), smem, stream, pdl, p);
+}
+
 extern "C" int qd_attn_scratch_floats(int q_heads, int kv_heads, int head_dim, int splits) {
     return kv_heads * splits * (q_heads / kv_heads) * (head_dim + 2);
 }
@@ -265,18 +510,7 @@ extern "C" int qd_attn_decode(const void* qg, const void* k_new, const void* v_n
     p.partial = scratch; p.counters = counters; p.position_dev = position_dev; p.position_host = position_host;
     p.capacity = capacity; p.hq = q_heads; p.hk = kv_heads; p.d = head_dim; p.rotary = rotary_dim;
     p.theta = theta; p.eps = eps; p.splits = splits; p.cache_stride = 0;
-    const size_t smem = sizeof(float) * ((size_t)G * head_dim + head_dim + (size_t)kAttnWarps * G * (head_dim + 2));
-    if (smem > 100 * 1024) return QD_ERR_UNSUPPORTED;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
-    static bool configured[64];
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
-            return QD_ERR_LAUNCH;
-        configured[dev] = true;
-    }
-    return qd_launch(attn_decode_kernel, dim3(kv_heads, splits), dim3(kAttnThreads), smem, (cudaStream_t)stream,
-                     pdl != 0, p);
+    return launch_attn(p, 1, pdl != 0, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------- batched form
@@ -303,18 +537,7 @@ extern "C" int qd_batch_attn_decode(const void* qg, const void* k_new, const voi
     p.partial = scratch; p.counters = counters; p.position_dev = positions; p.position_host = 0;
     p.capacity = capacity; p.hq = q_heads; p.hk = kv_heads; p.d = head_dim; p.rotary = rotary_dim;
     p.theta = theta; p.eps = eps; p.splits = splits; p.cache_stride = cache_stride;
-    const size_t smem = sizeof(float) * ((size_t)G * head_dim + head_dim + (size_t)kAttnWarps * G * (head_dim + 2));
-    if (smem > 100 * 1024) return QD_ERR_UNSUPPORTED;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
-    static bool configured[64];
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
-            return QD_ERR_LAUNCH;
-        configured[dev] = true;
-    }
-    return qd_launch(attn_decode_kernel, dim3(kv_heads, splits, batch), dim3(kAttnThreads), smem, (cudaStream_t)stream,
-                     false, p);
+    return launch_attn(p, batch, false, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------- allocation-free variant
@@ -359,14 +582,5 @@ extern "C" int qd_attn_decode_static(const void* qg, const void* k_new, const vo
     p.partial = (float*)base; p.counters = counters; p.position_dev = position_dev; p.position_host = position_host;
     p.capacity = capacity; p.hq = q_heads; p.hk = kv_heads; p.d = head_dim; p.rotary = rotary_dim;
     p.theta = theta; p.eps = eps; p.splits = splits; p.cache_stride = 0;
-    const size_t smem = sizeof(float) * ((size_t)G * head_dim + head_dim + (size_t)kAttnWarps * G * (head_dim + 2));
-    if (smem > 100 * 1024) return QD_ERR_UNSUPPORTED;
-    static bool configured[64];
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
-            return QD_ERR_LAUNCH;
-        configured[dev] = true;
-    }
-    return qd_launch(attn_decode_kernel, dim3(kv_heads, splits), dim3(kAttnThreads), smem, (cudaStream_t)stream,
-                     false, p);
+    return launch_attn(p, 1, false, (cudaStream_t)stream);
 }

@@ -308,7 +308,9 @@ def moe_block(w, x: torch.Tensor, *, config) -> torch.Tensor:
 
 
 # ----------------------------------------------------------------------------- mixers
-_ATTN_SPLITS = 32
+# Context splits at most: with 256 positions to a split at least, the tensor-core form (head dimension 256) fills 148 SMs with
+# two KV heads from 19 000 positions on; the general form walks a position at a time and pays for the merge of each split.
+_ATTN_SPLITS, _ATTN_SPLITS_MMA = 32, 74
 _scratch: dict = {}
 
 
@@ -340,14 +342,15 @@ def full_attention_block(w, x, kv_cache, position, *, config) -> torch.Tensor:
     rotary = int(d * config.partial_rotary_factor)
     assert rotary % 2 == 0 and 0 <= rotary <= d
     lib = _lib.lib()
-    floats = lib.qd_attn_scratch_floats(hq, hk, d, _ATTN_SPLITS)
+    splits = _ATTN_SPLITS_MMA if d == 256 else _ATTN_SPLITS
+    floats = lib.qd_attn_scratch_floats(hq, hk, d, splits)
     scratch, counters = _attn_scratch(x.device, floats, hk)
     gated = torch.empty(hq * d, dtype=BF16, device=x.device)
     call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(w.q_norm), ptr(w.k_norm), ptr(keys),
          ptr(values), ptr(gated), ptr(scratch), ptr(counters),
          ptr(position) if device_position else None, 0 if device_position else int(position),
          capacity, hq, hk, d, rotary, float(config.rope_theta), float(config.rms_norm_eps),
-         _ATTN_SPLITS, 0, stream_of(x))
+         splits, 0, stream_of(x))
     return _project(gated, w.o_proj)
 
 

@@ -272,6 +272,43 @@ def test_attention_long_context(K, cuda_device, capacity, position):
         assert torch.equal(k[t].cpu(), kc[t]) and torch.equal(v[t].cpu(), vc[t])
 
 
+@pytest.mark.parametrize("hq,hk,rotary", [(16, 2, 64), (3, 1, 128), (8, 8, 0), (10, 2, 256)])
+@pytest.mark.parametrize("position", [0, 1, 15, 16, 127, 128, 255, 256, 511, 4097])
+def test_attention_tensor_core_form_at_the_edges_of_its_chunks(cuda_device, hq, hk, rotary, position):
+    """Head dimension 256 with every group size class and rotary width: contexts that end on either side of a chunk of
+    sixteen, of a round of eight warps and of a split, few splits and many, rows past the position poisoned, position from
+    the host and from the device.  Bound: the operands are bf16 and exact in the oracle, sums fp32, one rounding of the
+    result and one of the gated product: 2 ulp of bf16."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    d, cap, eps, theta = 256, 4200, 1e-6, 1.0e7
+    src = synthetic.Source(77, "cpu")
+    qg, k_new, v_new = src.normal("qg", hq, 2 * d), src.normal("k", hk, d), src.normal("v", hk, d)
+    q_norm, k_norm = src.normal("qn", d, std=0.1), src.normal("kn", d, std=0.1)
+    kc, vc = src.normal("kc", cap, hk, d), src.normal("vc", cap, hk, d)
+    kc[position:], vc[position:] = float("nan"), float("nan")
+    cos, sin = O.rope_tables(position, rotary, theta)
+    q = O.apply_rope(O.rms_norm(qg[:, :d], 1 + q_norm.float(), eps), cos, sin)
+    wk, wv = kc.clone(), vc.clone()
+    wk[position], wv[position] = O.apply_rope(O.rms_norm(k_new, 1 + k_norm.float(), eps), cos, sin), v_new
+    keys, values = (t[:position + 1].double().repeat_interleave(hq // hk, 1) for t in (wk, wv))
+    p = torch.softmax(torch.einsum("hd,thd->ht", q.double(), keys) / 16.0, -1)
+    want = torch.einsum("ht,thd->hd", p, values).to(torch.bfloat16) * torch.sigmoid(qg[:, d:])
+    dev = [t.to(cuda_device) for t in (qg, k_new, v_new, q_norm, k_norm)]
+    for splits, device_position in ((1, False), (5, True), (74, False)):
+        k, v = kc.to(cuda_device), vc.to(cuda_device)
+        out = torch.empty(hq, d, dtype=torch.bfloat16, device=cuda_device)
+        scratch = torch.full((lib().qd_attn_scratch_floats(hq, hk, d, splits),), float("nan"), device=cuda_device)
+        counters = torch.zeros(hk, dtype=torch.int32, device=cuda_device)
+        at = torch.tensor(position, dtype=torch.int32, device=cuda_device)
+        for _ in range(2):                 # the counters are left ready for the next call
+            call("qd_attn_decode", *map(ptr, dev), ptr(k), ptr(v), ptr(out), ptr(scratch), ptr(counters),
+                 ptr(at) if device_position else None, 0 if device_position else position, cap, hq, hk, d, rotary, theta, eps,
+                 splits, 0, stream_of(out))
+        torch.testing.assert_close(out.cpu().float(), want.float(), rtol=2 ** -7, atol=2 ** -8 * float(want.float().abs().max()))
+        torch.testing.assert_close(k[position].cpu().float(), wk[position].float(), rtol=2 ** -7, atol=1e-2)
+        assert torch.equal(v[position].cpu(), v_new) and int(counters.sum()) == 0
+
+
 # ----------------------------------------------------- the reference's saved fixtures
 def test_reference_fixtures_through_the_operator_table(K, cuda_device, reference_fixtures):
     """The 15 saved block/step fixtures (tiny shapes, FP8 mixer projections) through
