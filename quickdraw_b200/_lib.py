@@ -85,6 +85,7 @@ HYBRID_LIBRARIES = {
     "hybrid": {
         "qd_set_chained_launches": [I],
         "qd_linear": [P, L, I, P, P, L, I, I, I, I, I, I, P, I, P, F, F, P, P],
+        "qd_linear_pieces": [P, L, P, P, L, I, I, I, I, I, I, P, I, P, P, P],
         "qd_greedy": [P, I, P, P, P, P],
         "qd_embed_norm": [P, P, I, P, P, P, P, I, I, F, I, P],
         "qd_layer_norm_rows": [P, P, P, P, P, I, I, F, I, P],

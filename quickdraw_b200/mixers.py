@@ -22,6 +22,7 @@ from .weights import (ChannelDeltaConfig, ChannelDeltaWeights, ChunkAttnConfig, 
 BF16, F32 = torch.bfloat16, torch.float32
 DTYPE_CODE = {BF16: 0, F32: 1}
 SILU, SIGMOID = 0, 1
+ROWS_FORM = 8                                                    # token rows up to which a product streams the weights
 MASK_WINDOW, MASK_CHUNK = 0, 1                                   # kinds of qd_attention_args
 NORM_NONE, NORM_ROW, NORM_HEAD = 0, 1, 2
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
@@ -42,7 +43,16 @@ def linear(x, x_column: int, ldx: int, weight, out, *, tokens: int, status, gelu
            add: bool = False, norm=None, norm_offset: float = 0.0, eps: float = 0.0) -> None:
     """out[t] = W x[t, x_column : x_column + in_features] (+ fp32 ``bias``); the first ``gelu_columns`` outputs through the exact
     GELU; ``glu``: weight rows 2i and 2i + 1 are a gate and its partner, out[i] = relu(gate) * partner; ``add``: onto
-    what ``out`` holds; ``norm`` (a few tokens only): x / rms(x) * (norm_offset + norm) in the place of x."""
+    what ``out`` holds; ``norm`` (a few tokens only): x / rms(x) * (norm_offset + norm) in the place of x.  More than
+    ``ROWS_FORM`` rows of fp32 go through the tensor cores as three bf16 pieces, where TMA takes the operands."""
+    rows, width = weight.shape
+    start = x.data_ptr() + 4 * x_column
+    if (x.dtype is F32 and tokens > ROWS_FORM and norm is None and (width | ldx | rows | out.shape[1]) % 8 == 0
+            and (start | weight.data_ptr() | out.data_ptr()) % 16 == 0):
+        planes = torch.empty(3 * tokens * width, dtype=BF16, device=x.device)
+        call_hybrid("qd_linear_pieces", column(x, x_column), ldx, ptr(weight), ptr(out), out.shape[1], DTYPE_CODE[out.dtype], tokens, rows, width,
+                    gelu_columns, int(glu), ptr(bias), int(add), ptr(planes), ptr(status), stream_of(x))
+        return
     call_hybrid("qd_linear", column(x, x_column), ldx, DTYPE_CODE[x.dtype], ptr(weight), ptr(out), out.shape[1],
                 DTYPE_CODE[out.dtype], tokens, weight.shape[0], weight.shape[1], gelu_columns, int(glu), ptr(bias), int(add), ptr(norm),
                 norm_offset, eps, ptr(status), stream_of(x))

@@ -64,6 +64,33 @@ def test_linear(M, tokens, rows, width, x_type, y_type):
     assert error(out, want) < (1e-5 if y_type == F32 else 5e-3)
 
 
+@pytest.mark.parametrize("tokens,rows,width", [(9, 8, 8), (127, 72, 256), (128, 64, 264), (129, 136, 1000), (300, 2504, 2048), (1030, 5128, 520)])
+@pytest.mark.parametrize("form", ["plain", "bias", "glu", "add"])
+def test_fp32_rows_in_pieces(M, tokens, rows, width, form):
+    """Every tile width, ragged edges, less and more than a segment of 256 inputs, all that may follow the sums, values over
+    forty binary orders.  Bound: the products are exact and each of the segments' sums is rounded; 2e-6 of the sum of
+    magnitudes is sixteen times the spacing of fp32."""
+    w = bf(rows, width, seed=2, std=width ** -0.5)
+    x = rnd(tokens, width, seed=1) * torch.exp2(torch.randint(-20, 20, (tokens, 1), generator=torch.Generator().manual_seed(3)).float())
+    x[0], x[-1, 0], x[-1, -1] = 0.0, float("inf"), float("nan")
+    bias = rnd(rows, seed=4).cuda() if form in ("bias", "glu") else None
+    out = rnd(tokens, rows // 2 if form == "glu" else rows, seed=5).cuda()
+    before, stat = out.double().cpu(), status()
+    M.linear(x.cuda(), 0, width, w.cuda(), out, tokens=tokens, status=stat, bias=bias, glu=form == "glu", add=form == "add")
+    sums, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    if bias is not None:
+        sums, scale = sums + bias.double().cpu(), scale + bias.double().abs().cpu()
+    if form == "glu":
+        gate, up = sums[:, 0::2], sums[:, 1::2]
+        scale = scale[:, 0::2] * up.abs() + gate.abs() * scale[:, 1::2] + scale[:, 0::2] * scale[:, 1::2] * 2e-6
+        sums = gate.clamp(min=0) * up
+    if form == "add":
+        sums, scale = sums + before, scale + before.abs()
+    got = out.double().cpu()
+    assert int(stat.item()) == 0 and bool(got[-1].isnan().all())
+    assert bool(((got - sums).abs()[:-1] <= 2e-6 * scale[:-1] + 1e-30).all())
+
+
 # ------------------------------------------------------------------------- residual stream
 @pytest.mark.parametrize("width", [64, 256, 320, 100, 33, 2048, 1280])
 @pytest.mark.parametrize("older,following", [(-1, True), (0, True), (1, False), (7, True)])
@@ -209,6 +236,27 @@ def test_decoding_with_long_splits(M, name, splits, dtype):
                            v=torch.empty(capacity, m.kv_heads, m.vdim, dtype=dtype, device="cuda"))
     got = drive(mixer, proj.cuda(), at, history, [60, 60, 60] + [1] * 50)
     assert error(got[180:], want()[180:]) < (5e-5 if dtype == F32 else 2e-2)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,window,tokens", [(16, 4, 32, 64, 70, 301), (18, 2, 36, 20, 500, 270), (3, 1, 128, 128, 64, 33)])
+def test_fp32_chunks_in_tiles(M, heads, kv_heads, dim, vdim, window, tokens):
+    """64 and 16 rows to a block, groups that do not divide them, column counts beside a tile's, a window that ends inside
+    a tile, and an infinite value at one token: rows that do not see it stay finite."""
+    m, bad = cases.attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, window=window, rotary_dims=dim), 40 if tokens > 100 else 20
+    w, eps, proj, at, want = attention_case(m, tokens, F32, sharp=2.0)
+    weights = WindowAttnWeights(**{k: None if v is None else v.cuda() for k, v in vars(w).items()})
+    mixer = M.WindowAttention(weights, m, eps, torch.device("cuda"))
+    new = lambda n: torch.full((min(tokens, window - 1 + tokens), kv_heads, n), float("nan"), device="cuda")
+    got = drive(mixer, proj.cuda(), at, LayerHistory(k=new(dim), v=new(vdim)), [tokens])
+    exact = want()
+    assert error(got, exact) < 5e-6
+    proj[bad, at["v"]:at["v"] + vdim] = float("inf")              # of key/value head 0
+    got = drive(mixer, proj.cuda(), at, LayerHistory(k=new(dim), v=new(vdim)), [tokens]).cpu().view(tokens, heads, vdim)
+    share, last = heads // kv_heads, min(tokens, bad + window)
+    assert not bool(got[bad:last, :share].isfinite().any())
+    unseen = torch.ones(tokens, heads, dtype=torch.bool)
+    unseen[bad:last, :share] = False
+    assert error(got[unseen], exact.view(tokens, heads, vdim)[unseen]) < 5e-6
 
 
 @pytest.mark.parametrize("inside", [True, False])
