@@ -5,19 +5,26 @@
 // mixers token by token; this is the form for prompt chunks and decode batches.
 //
 //   quantiser   x bf16 [tokens, K] -> E4M3 bytes [tokens, K] (round to nearest even, saturating)
-//   product     block = 128 tokens x 128 weight rows, eight warps of 64 x 32; both operands go
-//               through a four-stage cp.async ring in chunks of 128 inputs (rows padded to 192
-//               bytes: the 16-byte fragment loads of a quarter-warp fall on different banks) and
-//               meet on mma.sync.m16n8k32 (e4m3 x e4m3, fp32 accumulators) with the tokens as
-//               rows, so that a lane's two results are neighbouring outputs of one token.
-#include "common.cuh"
+//   product     tcgen05.mma kind::f8f6f4, both operands by tiled TMA (128-byte swizzle), persistent
+//               blocks with two accumulators in tensor memory, so that one tile's results are
+//               scaled and stored while the next is multiplied.  Tile = 128 tokens x 32 .. 256
+//               weight rows.  Bound by the operands' way from L2 (a 128 x 256 tile: 170 operations
+//               per byte): 8192 x 8192 x 2048 in 122 us = 2 240 TFLOP/s, 2047 x 2048 x 4096 in 16.5 us; on
+//               mma.sync.m16n8k32, as before, 845 us (325 TFLOP/s) and 118 us.
+#include "umma.cuh"
 
 namespace qd {
 namespace {
 
-constexpr int kF8Tile = 128, kF8Chunk = 128, kF8Row = kF8Chunk + 64, kF8Stages = 4, kF8Threads = 256;
-constexpr int kF8StageBytes = 2 * kF8Tile * kF8Row;
-constexpr size_t kF8Smem = (size_t)kF8Stages * kF8StageBytes;
+constexpr int kF8Tokens = 128, kF8Chunk = 128;      // inputs per stage: one swizzled row of 128 bytes
+template <int TN> struct F8Tile {
+    static constexpr int kABytes = kF8Tokens * kF8Chunk, kStageBytes = kABytes + TN * kF8Chunk;
+    static constexpr int kStages = TN == 256 ? 4 : TN == 128 ? 6 : 8;
+    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 4) * 8 + 16 + 1024;
+    // fp32 accumulator, E4M3 A and B (format 0), K-major, N >> 3 at 17, M >> 4 at 24
+    static constexpr uint32_t kDesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kF8Tokens >> 4) << 24);
+};
+constexpr int kF8Threads = 192;      // TMA, MMA, four warps of 32 tokens each
 
 __global__ void __launch_bounds__(256) fp8_quantize_rows_kernel(const uint4* __restrict__ x, const float* __restrict__ in_scale,
                                                                 uint2* __restrict__ q, long long n8) {
@@ -37,91 +44,141 @@ __global__ void __launch_bounds__(256) fp8_quantize_rows_kernel(const uint4* __r
     q[i] = make_uint2(out[0], out[1]);
 }
 
-QD_DEVINL void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-QD_DEVINL void f8_cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+QD_DEVINL void umma_e4m3(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+struct F8Params { const float* w_scale; const float* in_scale; bf16* y; int tokens, rows, chunks, across, tiles; };
+
+template <int TN>
 __global__ void __launch_bounds__(kF8Threads, 1)
-fp8_gemm_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ w, const float* __restrict__ w_scale,
-                const float* __restrict__ in_scale, bf16* __restrict__ y, int tokens, int rows, int K) {
+fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap) {
     chain_enter();
-    extern __shared__ __align__(128) uint8_t f8_smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int t0 = blockIdx.y * kF8Tile, r0 = blockIdx.x * kF8Tile;
-    const int m0 = (warp & 1) * 64, n0 = (warp >> 1) * 32;          // the warp's 64 tokens x 32 rows of the tile
-    const int chunks = K / kF8Chunk;
-    // rows past the ends read the last valid row and are not stored
-    auto issue = [&](int c) {
-        uint8_t* st = f8_smem + (size_t)(c % kF8Stages) * kF8StageBytes;
-#pragma unroll
-        for (int i = 0; i < 2 * kF8Tile * 8 / kF8Threads; ++i) {
-            const int piece = tid + i * kF8Threads, which = piece >> 10, row = (piece >> 3) & (kF8Tile - 1), col = piece & 7;
-            const uint8_t* src = which ? w + (size_t)min(r0 + row, rows - 1) * K : q + (size_t)min(t0 + row, tokens - 1) * K;
-            f8_cp16(st + (size_t)(which * kF8Tile + row) * kF8Row + col * 16, src + (size_t)c * kF8Chunk + col * 16);
-        }
-    };
-#pragma unroll
-    for (int c = 0; c < kF8Stages - 1; ++c) {
-        if (c < chunks) issue(c);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    using Tile = F8Tile<TN>;
+    constexpr int kStages = Tile::kStages;
+    extern __shared__ __align__(1024) uint8_t f8_smem_raw[];
+    uint8_t* smem = f8_smem_raw + ((1024u - (smem_u32(f8_smem_raw) & 1023u)) & 1023u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * Tile::kStageBytes);
+    uint64_t* empty = full + kStages;
+    uint64_t* ready = empty + kStages;         // an accumulator holds a whole tile
+    uint64_t* taken = ready + 2;               // it has been read
+    uint32_t* slot = reinterpret_cast<uint32_t*>(taken + 2);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(ready + s, 1); mbar_init(taken + s, 4); }
+        mbar_fence_init();
     }
-    float acc[4][4][4];
+    if (warp == 1) { tmem_alloc(slot, 2 * TN); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *slot;
+    const int mine = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, steps = mine * p.chunks;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int issued = 0, tile = blockIdx.x;
+            bool ok = true;
+            for (int c = 0; issued < steps; ++issued, ++c) {
+                if (c == p.chunks) { c = 0; tile += gridDim.x; }
+                const int st = issued % kStages;
+                if (issued >= kStages) ok = mbar_wait(empty + st, ((issued / kStages) - 1) & 1, nullptr);
+                if (!ok) break;
+                uint8_t* a = smem + st * Tile::kStageBytes;
+                mbar_expect_tx(full + st, Tile::kStageBytes);          // rows past a matrix's end arrive as zeros and count in full
+                tma_load_2d(a, &xmap, c * kF8Chunk, tile / p.across * kF8Tokens, full + st);
+                tma_load_2d(a + Tile::kABytes, &wmap, c * kF8Chunk, tile % p.across * TN, full + st);
+            }
+            if (!ok)            // leave no copy in flight behind
+                for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
+                    mbar_wait(full + s % kStages, (s / kStages) & 1, nullptr);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            bool ok = true;
+            int s = 0;
+            for (int k = 0; k < mine && ok; ++k) {
+                if (k >= 2) ok = mbar_wait(taken + (k & 1), ((k >> 1) - 1) & 1, nullptr);
+                if (!ok) break;
+                tc_fence_after();
+                for (int c = 0; c < p.chunks; ++c, ++s) {
+                    const int st = s % kStages;
+                    ok = mbar_wait(full + st, (s / kStages) & 1, nullptr);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + Tile::kABytes;
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[mi][ni][c] = 0.f;
+                    for (int j = 0; j < kF8Chunk / 32; ++j)
+                        umma_e4m3(tmem + (k & 1) * TN, smem_desc_sw128(a + j * 32), smem_desc_sw128(b + j * 32), Tile::kDesc, (c | j) ? 1u : 0u);
+                    umma_commit(empty + st);
+                }
+                if (ok) umma_commit(ready + (k & 1));
+            }
+        }
+    } else {
+        const int quadrant = warp & 3;
+        const float s_in = *p.in_scale, s_w = *p.w_scale;
+        const bool vectors = p.rows % 8 == 0 && ((uintptr_t)p.y & 15u) == 0;
+        bool ok = true;
+        for (int k = 0; k < mine; ++k) {
+            const int tile = blockIdx.x + k * gridDim.x;
+            const int token = tile / p.across * kF8Tokens + quadrant * 32 + lane, n0 = tile % p.across * TN;
+            ok = ok && mbar_wait(ready + (k & 1), (k >> 1) & 1, nullptr);
+            tc_fence_after();
+            bf16* out = p.y + (size_t)token * p.rows;
 #pragma unroll 1
-    for (int c = 0; c < chunks; ++c) {
-        asm volatile("cp.async.wait_group 2;" ::: "memory");       // kF8Stages - 2 younger chunks may be in flight
-        __syncthreads();                                           // chunk c is everybody's; chunk c - 1 is consumed
-        if (c + kF8Stages - 1 < chunks) issue(c + kF8Stages - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const uint8_t* xa = f8_smem + (size_t)(c % kF8Stages) * kF8StageBytes;
-        const uint8_t* wb = xa + (size_t)kF8Tile * kF8Row;
+            for (int c = 0; c < TN; c += 16) {
+                if (n0 + c >= p.rows) break;
+                uint32_t v[16];
+                if (ok) {
+                    tmem_load16(tmem + ((uint32_t)(quadrant * 32) << 16) + (k & 1) * TN + c, v);
+                    tmem_load_wait();
+                } else {        // a wait ran out (no status word here): the results say so
 #pragma unroll
-        for (int kk = 0; kk < kF8Chunk / 64; ++kk) {
-            // lane (g, t) supplies bytes 16 t .. 16 t + 15 of every 64 on both sides: two MMAs per 16-byte load
-            uint4 bw[4];
+                    for (int q = 0; q < 16; ++q) v[q] = 0x7fc00000u;
+                }
+                if (token >= p.tokens) continue;
+                uint32_t packed[8];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) bw[ni] = lds128(wb + (size_t)(n0 + 8 * ni + g) * kF8Row + kk * 64 + t * 16);
+                for (int q = 0; q < 8; ++q) {
+                    const __nv_bfloat162 two = __floats2bfloat162_rn((__uint_as_float(v[2 * q]) * s_in) * s_w, (__uint_as_float(v[2 * q + 1]) * s_in) * s_w);
+                    packed[q] = *reinterpret_cast<const uint32_t*>(&two);
+                }
+                if (vectors && n0 + c + 16 <= p.rows) {
+                    *reinterpret_cast<uint4*>(out + n0 + c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    *reinterpret_cast<uint4*>(out + n0 + c + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                } else {        // rows is even and y on a four-byte boundary
 #pragma unroll
-            for (int mi = 0; mi < 4; ++mi) {
-                const uint4 lo = lds128(xa + (size_t)(m0 + 16 * mi + g) * kF8Row + kk * 64 + t * 16);
-                const uint4 hi = lds128(xa + (size_t)(m0 + 16 * mi + g + 8) * kF8Row + kk * 64 + t * 16);
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) {
-                    mma_e4m3(acc[mi][ni], lo.x, hi.x, lo.y, hi.y, bw[ni].x, bw[ni].y);
-                    mma_e4m3(acc[mi][ni], lo.z, hi.z, lo.w, hi.w, bw[ni].z, bw[ni].w);
+                    for (int q = 0; q < 8; ++q)
+                        if (n0 + c + 2 * q < p.rows) *reinterpret_cast<uint32_t*>(out + n0 + c + 2 * q) = packed[q];
                 }
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(taken + (k & 1));
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // acc[mi][ni][0..1] = token m0 + 16 mi + g, rows n0 + 8 ni + 2 t and + 1; [2..3] = token + 8
-    const float s_in = *in_scale, s_w = *w_scale;
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int token = t0 + m0 + 16 * mi + g + 8 * half;
-            if (token >= tokens) continue;
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) {
-                const int row = r0 + n0 + 8 * ni + 2 * t;
-                if (row + 1 < rows)
-                    *reinterpret_cast<__nv_bfloat162*>(y + (size_t)token * rows + row) =
-                        __floats2bfloat162_rn((acc[mi][ni][2 * half] * s_in) * s_w, (acc[mi][ni][2 * half + 1] * s_in) * s_w);
-                else if (row < rows)
-                    y[(size_t)token * rows + row] = __float2bfloat16_rn((acc[mi][ni][2 * half] * s_in) * s_w);
-            }
-        }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 2 * TN);
+}
+
+template <int TN>
+int launch_f8(const void* q, const void* w, F8Params p, int in_features, int sms, cudaStream_t stream) {
+    using Tile = F8Tile<TN>;
+    if (cudaFuncSetAttribute(fp8_gemm_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) != cudaSuccess) return QD_ERR_LAUNCH;
+    alignas(64) CUtensorMap xmap = {}, wmap = {};
+    int rc = umma_make_map(&xmap, q, p.tokens, in_features, kF8Chunk, kF8Tokens);
+    if (rc == QD_OK) rc = umma_make_map(&wmap, w, p.rows, in_features, kF8Chunk, TN);
+    if (rc != QD_OK) return rc;
+    p.across = (p.rows + TN - 1) / TN;
+    p.tiles = p.across * ((p.tokens + kF8Tokens - 1) / kF8Tokens);
+    const unsigned grid = (unsigned)(p.tiles < sms ? p.tiles : sms);
+    qd_launch(fp8_gemm_kernel<TN>, dim3(grid), dim3(kF8Threads), Tile::kSmem, stream, true, p, xmap, wmap);
+    return qd_launch_status();
 }
 
 }  // namespace
@@ -135,7 +192,7 @@ extern "C" int qd_fp8_matmul(const void* x, const void* w, const float* w_scale,
                              int tokens, int out_features, int in_features, void* q_scratch, int convert, void* stream) {
     using namespace qd;
     QD_CHECK_ARG(x && w && w_scale && in_scale && y && q_scratch && tokens > 0 && out_features > 0 && in_features > 0);
-    if (in_features % kF8Chunk != 0 || out_features % 2 != 0 || (tokens + kF8Tile - 1) / kF8Tile > 65535) return QD_ERR_UNSUPPORTED;
+    if (in_features % kF8Chunk != 0 || out_features % 2 != 0 || (tokens + kF8Tokens - 1) / kF8Tokens > 65535) return QD_ERR_UNSUPPORTED;
     if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)q_scratch) & 15u || ((uintptr_t)y & 3u)) return QD_ERR_UNSUPPORTED;
     if (convert) {
         const long long n8 = (long long)tokens * in_features / 8;
@@ -145,14 +202,14 @@ extern "C" int qd_fp8_matmul(const void* x, const void* w, const float* w_scale,
     }
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
-    static bool configured[64];
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF8Smem) != cudaSuccess)
-            return QD_ERR_LAUNCH;
-        configured[dev] = true;
-    }
-    const dim3 grid((unsigned)((out_features + kF8Tile - 1) / kF8Tile), (unsigned)((tokens + kF8Tile - 1) / kF8Tile));
-    qd_launch(fp8_gemm_kernel, dim3(grid), dim3(kF8Threads), kF8Smem, (cudaStream_t)stream, true, 
-        (const uint8_t*)q_scratch, (const uint8_t*)w, w_scale, in_scale, (bf16*)y, tokens, out_features, in_features);
-    return qd_launch_status();
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return QD_ERR_LAUNCH;
+    const F8Params p = {w_scale, in_scale, (bf16*)y, tokens, out_features, in_features / kF8Chunk, 0, 0};
+    const long long token_tiles = (tokens + kF8Tokens - 1) / kF8Tokens;
+    const auto busy = [&](int tn) { return token_tiles * ((out_features + tn - 1) / tn) * 4 >= 3ll * sms; };
+    // the widest tile that still gives most SMs one: a wider one reads the tokens fewer times
+    if (busy(256)) return launch_f8<256>(q_scratch, w, p, in_features, sms, (cudaStream_t)stream);
+    if (busy(128)) return launch_f8<128>(q_scratch, w, p, in_features, sms, (cudaStream_t)stream);
+    if (busy(64)) return launch_f8<64>(q_scratch, w, p, in_features, sms, (cudaStream_t)stream);
+    return launch_f8<32>(q_scratch, w, p, in_features, sms, (cudaStream_t)stream);
 }

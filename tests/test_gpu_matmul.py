@@ -108,6 +108,21 @@ def test_fp8_matmul_matches_row_by_row_oracle(cuda_device, tokens, out_features,
         assert O.rel_l2(y[t].cpu(), row) < 2e-3, t
 
 
+@pytest.mark.parametrize("tokens,out_features,in_features", [(129, 34, 128), (700, 2050, 256), (900, 2050, 384), (1500, 4090, 128), (1537, 4096, 640)])
+def test_fp8_matmul_at_every_tile_width(cuda_device, tokens, out_features, in_features):
+    """Tiles of 32, 64, 128 and 256 weight rows, ragged on both sides, more tiles than SMs (two accumulators in turn), rows
+    that are not whole 16-byte pieces.  Bound: exact products, fp32 sums, one bf16 rounding."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(5)
+    draw = lambda rows: torch.randn(rows, in_features, generator=gen, device=cuda_device)
+    q, w = (draw(tokens) * 40).to(torch.float8_e4m3fn), (draw(out_features) * 40).to(torch.float8_e4m3fn)
+    scales = torch.tensor([0.01, 0.002], device=cuda_device)
+    y = torch.empty(tokens, out_features, dtype=torch.bfloat16, device=cuda_device)
+    call("qd_fp8_matmul", ptr(y), ptr(w), ptr(scales), ptr(scales[1:]), ptr(y), tokens, out_features, in_features, ptr(q), 0, stream_of(y))
+    want = q.double() @ w.double().T * (float(scales[0]) * float(scales[1]))
+    torch.testing.assert_close(y.double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+
+
 def test_two_dimensional_input_takes_the_matmul_path(cuda_device):
     from quickdraw_b200 import kernels
     src = synthetic.Source(22, "cpu")
