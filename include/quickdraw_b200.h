@@ -121,6 +121,14 @@ int qd_nvfp4_grouped_matmul(const void* x, const void* codes, const void* scales
                             int global_per_expert, int max_rows_per_expert, unsigned int* status,
                             void* stream);
 
+/* The gate and up products of the routed experts and their SwiGLU in one launch: h[r] = bf16(bf16(silu(g)) * u) of sorted
+ * row r (input row order[r] / topk), g and u its rows of the two banks.  in_features % 256 == 0, out_features % 128 == 0, at
+ * most 1024 experts, group size 16, addresses of x, h, codes and scales on 16 bytes; QD_ERR_UNSUPPORTED otherwise. */
+int qd_nvfp4_expert_swiglu(const void* x, const void* gate_codes, const void* gate_scales, const float* gate_global,
+                           const void* up_codes, const void* up_scales, const float* up_global, const int32_t* order,
+                           const int32_t* boundaries, void* h, int routes, int experts, int topk, int out_features,
+                           int in_features, int group_size, int global_per_expert, unsigned int* status, void* stream);
+
 /* The same product when an expert receives only a few rows (a short chunk, a decode batch):
  * every expert that got routes is read once, its NVFP4 rows decoded once per routes_per_pass
  * routes (8 or 32; 0 = the library's choice) and

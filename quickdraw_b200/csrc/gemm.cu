@@ -25,6 +25,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "expert_tiles.cuh"
 
 namespace {
 
@@ -516,6 +517,11 @@ extern "C" int qd_nvfp4_grouped_matmul(const void* x, const void* codes, const v
     if (group_size != 16 || in_features % kTileK != 0 || out_features % 8 != 0) return QD_ERR_UNSUPPORTED;
     const uintptr_t align = (uintptr_t)x | (uintptr_t)codes | (uintptr_t)y;
     if (align & 15u) return QD_ERR_UNSUPPORTED;
+    // Decoded weights in tensor memory wherever the sizes fit: down bank of 256 x 2048 x 512, 16 / 64 / 256 routes an expert:
+    // 68 / 98 / 295 us against 145 / 172 / 481 us of the tiles below, and never slower from two tokens on.
+    if (qd::expert_tiles_cover(experts, out_features, in_features, 256, x, codes, scales))
+        return qd::expert_tiles_matmul({x, codes, scales, global, order, boundaries, routing, (bf16*)y, routes, experts, topk, out_features,
+                                        in_features, by_token, scatter, global_per_expert, status}, (cudaStream_t)stream);
     GemmParams p = {};
     p.x = (const bf16*)x; p.codes = (const uint8_t*)codes; p.scales = (const uint8_t*)scales; p.global = global;
     p.y = (bf16*)y; p.tokens = routes; p.out_features = out_features; p.in_features = in_features; p.status = status;

@@ -41,6 +41,11 @@ class ChunkPrefill:
     ROUTES_PER_PASS = 0                                   # 8 / 32 routes per decoding of a weight tile; 0: the library chooses
     FEW_ROWS = 20                                         # mean routes per expert up to which the mma.sync form is used
 
+    TILES_FROM = 5                                        # mean routes per expert from which gate, up and SwiGLU are one launch over
+                                                          # weights decoded into tensor memory (256 experts of 512 x 2048, all three
+                                                          # banks: 4 routes 176 against 166 us of the mma.sync form, 8 routes 180
+                                                          # against 217, 16 routes 182 against 297)
+
     def __init__(self, ckpt: Checkpoint, expert_range: tuple[int, int] | None = None, group=None):
         c = ckpt.config
         self.ckpt, self.device = ckpt, ckpt.embed_tokens.device
@@ -157,6 +162,22 @@ class ChunkPrefill:
         return (routes <= self.FEW_ROWS * (self.total_experts or bank.weight.shape[0]) and bank.in_features in (512, 1024, 2048)
                 and bank.out_features % 16 == 0)
 
+    def _tiles_form(self, routes, w):
+        gate, up, down = w.experts_gate, w.experts_up, w.experts_down
+        experts = gate.weight.shape[0]
+        return (routes > self.TILES_FROM * (self.total_experts or experts) and gate.weight.shape == up.weight.shape and experts <= 1024
+                and gate.group_size == up.group_size == down.group_size == 16 and gate.in_features % 256 == 0 and gate.out_features % 128 == 0
+                and down.in_features % 256 == 0 and down.out_features % 256 == 0
+                and (gate.weight_scale_2.numel() == 1) == (up.weight_scale_2.numel() == 1))
+
+    def _expert_swiglu(self, x, gate, up, order, boundaries, routes, topk):
+        """The SwiGLU of the routed gate and up products, rows in sorted order."""
+        h = self._empty(routes, gate.out_features)
+        call("qd_nvfp4_expert_swiglu", ptr(x), ptr(gate.weight), ptr(gate.weight_scale), ptr(gate.weight_scale_2), ptr(up.weight), ptr(up.weight_scale),
+             ptr(up.weight_scale_2), ptr(order), ptr(boundaries), ptr(h), routes, gate.weight.shape[0], topk, gate.out_features, gate.in_features,
+             gate.group_size, int(gate.weight_scale_2.numel() != 1), ptr(self.status), stream_of(x))
+        return h
+
     def _expert_rows_scratch(self, in_rows, in_features):
         """The area for the f16 copy of the input rows of the few-rows form, and the input it holds."""
         if self._expert_scratch is None:
@@ -182,11 +203,11 @@ class ChunkPrefill:
         self._expert_scratch[bank.in_features] = (scratch, x)
         return out, out2
 
-    def _grouped(self, x, bank: NVFP4Linear, order, boundaries, routes, topk, *, routing=None, by_token, scatter, x_up=None):
+    def _grouped(self, x, bank: NVFP4Linear, order, boundaries, routes, topk, *, routing=None, by_token, scatter, x_up=None, tiles=False):
         # rows of experts another rank owns stay zero in the scattered (route-order) output
         out = (torch.zeros if self.sliced and scatter else torch.empty)((routes, bank.out_features), dtype=BF16, device=self.device)
         experts = bank.weight.shape[0]
-        if self._few_rows(routes, bank):
+        if not tiles and self._few_rows(routes, bank):
             # few rows per expert: weights decoded once per 8 or 32 routes on mma.sync, no 128-token tiles;
             # the f16 copy of the input rows is shared by the products of the same input (gate, up)
             scratch, source = self._expert_rows_scratch(routes // topk if by_token else routes, bank.in_features)
@@ -264,11 +285,15 @@ class ChunkPrefill:
         call("qd_seq_group_routes", ptr(ids), routes, c.num_experts, ptr(order), ptr(boundaries), stream_of(x))
         if self.sliced:      # this rank's experts: their slice of the boundaries, indices local to the bank
             boundaries = boundaries[self.expert_range[0]:self.expert_range[1] + 1]
-        gate, up = self._grouped_pair(x, w.experts_gate, w.experts_up, order, boundaries, routes, topk)
+        tiles = self._tiles_form(routes, w)
+        if tiles:
+            gate, up = self._expert_swiglu(x, w.experts_gate, w.experts_up, order, boundaries, routes, topk), None
+        else:
+            gate, up = self._grouped_pair(x, w.experts_gate, w.experts_up, order, boundaries, routes, topk)
         # the SwiGLU is formed while the rows of the down product are written as f16 (a separate kernel where
         # the 128-token tiles take the product)
         contributions = self._grouped(gate, w.experts_down, order, boundaries, routes, topk, x_up=up,
-                                      routing=weights.flatten(), by_token=False, scatter=True)
+                                      routing=weights.flatten(), by_token=False, scatter=True, tiles=tiles)
         if self.sliced:
             import torch.distributed as dist
             dist.all_reduce(contributions, group=self.group)

@@ -253,3 +253,49 @@ def test_combine_with_the_next_norm_equals_the_two_calls(cuda_device, tokens, hi
          ptr(fused_normed), ptr(fused_residual), tokens, hidden, topk, 1e-6, stream_of(out))
     assert torch.equal(fused_normed, normed) and torch.equal(fused_residual, new_residual)
 
+
+
+@pytest.mark.parametrize("counts,width,inner", [
+    ((1,), 256, 256),
+    ((0, 15, 16, 17, 0, 3), 512, 128),
+    ((80, 81, 0, 160, 161, 1, 240), 256, 256),            # items of an expert: one, two, two, three, three
+    ((5,) * 300, 256, 128),                               # more items than SMs, several to a block
+    ((33, 70, 96), 2048, 512),
+])
+def test_expert_tiles_at_the_edges_of_an_item(cuda_device, counts, width, inner):
+    """Gate, up and SwiGLU in one launch and the scattered, routed product, weights decoded into tensor memory: experts without
+    a route, one route, a whole item, one more.  Bounds: exact products, fp32 sums, one bf16 rounding of gate, up, silu and
+    the result (four of 2^-8 each: bf16 keeps eight bits); of sum, factor and result in the routed product (three)."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    from quickdraw_b200.synthetic import to_device
+    experts, routes = len(counts), sum(counts)
+    src = synthetic.Source(17, "cpu")
+    gate, up = (src.nvfp4(n, inner, width, experts, global_scale=0.05, per_expert_global=True) for n in ("gate", "up"))
+    out_bank = src.nvfp4("out", 256, width, experts, global_scale=0.5, per_expert_global=True)
+    x = src.normal("x", routes, width)
+    gen = torch.Generator().manual_seed(4)
+    order = torch.randperm(routes, generator=gen).to(torch.int32)
+    bounds = torch.tensor([0, *torch.tensor(counts).cumsum(0).tolist()], dtype=torch.int32)
+    weights = torch.rand(routes, generator=gen)
+    dev = cuda_device
+    g, u, o = (to_device(b, dev) for b in (gate, up, out_bank))
+    xd, od, bd, wd = x.to(dev), order.to(dev), bounds.to(dev), weights.to(dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    h = torch.full((routes, inner), float("nan"), dtype=torch.bfloat16, device=dev)
+    y = torch.full((routes, 256), float("nan"), dtype=torch.bfloat16, device=dev)
+    call("qd_nvfp4_expert_swiglu", ptr(xd), ptr(g.weight), ptr(g.weight_scale), ptr(g.weight_scale_2), ptr(u.weight), ptr(u.weight_scale),
+         ptr(u.weight_scale_2), ptr(od), ptr(bd), ptr(h), routes, experts, 1, inner, width, 16, 1, ptr(status), stream_of(xd))
+    call("qd_nvfp4_grouped_matmul", ptr(xd), ptr(o.weight), ptr(o.weight_scale), ptr(o.weight_scale_2), ptr(od), ptr(bd), ptr(wd), ptr(y),
+         routes, experts, 1, 256, width, 16, 0, 1, 1, routes, ptr(status), stream_of(xd))
+    assert int(status.item()) == 0
+    matrix = lambda b, e: O.dequantize_fp32(O.expert_view(b, e)).double()
+    h, y, tol = h.cpu().double(), y.cpu().double(), 2.0 ** -8
+    for e in range(experts):
+        rows = slice(int(bounds[e]), int(bounds[e + 1]))
+        if rows.start == rows.stop:
+            continue
+        xs = x[order[rows].long()].double()
+        a, b = xs @ matrix(gate, e).T, xs @ matrix(up, e).T
+        torch.testing.assert_close(h[rows], a * torch.sigmoid(a) * b, rtol=4 * tol, atol=tol * float(a.abs().max() * b.abs().max()) * 2 ** -4)
+        want = x[rows].double() @ matrix(out_bank, e).T * weights[order[rows].long()].double()[:, None]
+        torch.testing.assert_close(y[order[rows].long()], want, rtol=3.1 * tol, atol=1e-5 * float(want.abs().max()))
