@@ -25,7 +25,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
 COMMON = ("library",)
 HYBRID_SOURCES = {"hybrid": ("linear", "residual", "window_attention"), "recurrent": ("linear_recurrence",),
                   "latent": ("latent_attention",)}
-HYBRID_HEADERS = ("common.cuh", "typed.cuh", "softmax_attention.cuh")
+HYBRID_HEADERS = ("common.cuh", "typed.cuh", "softmax_attention.cuh", "flash_umma.cuh")
 TARGETS = ("nvfp4", *HYBRID_SOURCES)
 
 

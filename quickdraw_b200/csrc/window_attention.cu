@@ -7,13 +7,15 @@
 // The visible keys and values live in a ring of `capacity` rows (position p in row p mod capacity), so a
 // sequence's cache does not grow with its length.  Keys may end in columns that all heads share (k_shared).
 //
-// Prompt chunks: attn_prepare_kernel (norm, rotation, ring rows) and attn_flash_kernel (mma.sync m16n8k16;
+// Prompt chunks: attn_prepare_kernel (norm, rotation, ring rows), then flash_umma.cuh for heads of 128 value and 128 or 192 key
+// columns, attn_flash_kernel for other bf16 rows (mma.sync m16n8k16;
 // 64 or 128 packed (token, head of the group) rows per block, key tiles of 64 through two cp.async buffers,
 // only the tiles a row of the block can see; probabilities as two bf16 pieces).  attn_rows_kernel covers fp32
 // and shapes without 16-byte rows.  Decode: attn_step_kernel, one launch: norm and rotation in every
 // block, blocks = (key/value head, split of the span), the last block of a head merges.
 #include <type_traits>
 
+#include "flash_umma.cuh"
 #include "softmax_attention.cuh"
 
 namespace qd {
@@ -582,6 +584,45 @@ __global__ void __launch_bounds__(WARPS * 32) attn_flash_kernel(const __grid_con
     }
 }
 
+// Rows of a chunk through flash_umma.cuh: sink and gates on the finished result.
+struct FlashOut {
+    AttnParams p;
+    int wide;                              // gate rows on 16-byte boundaries
+    QD_DEVINL void operator()(int t, int h, int c0, const float (&o)[32], float m, float l) const {
+        const bf16* gate = as_bf16(p.gate) + (long long)t * p.ld_gate;
+        float f = 1.f / l;
+        if (p.sink_kind != QD_SINK_NONE) {
+            const float sink = p.sink_kind == QD_SINK_LEARNED ? ld_bf16(as_bf16(p.sink) + h) * kLog2e : 0.f;
+            const float top = fmaxf(m, sink), keep = exp2f(m - top);
+            f = keep / (l * keep + exp2f(sink - top));
+        }
+        if (p.gate_kind == QD_GATE_HEAD) f *= sigmoid_precise(ld_bf16(gate + h));
+        uint32_t v[16], z[16];
+        if (p.gate_kind == QD_GATE_VALUE) {
+            const bf16* own = gate + h * p.vdim + c0;
+            if (wide) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(z + 4 * i) = reinterpret_cast<const uint4*>(own)[i];
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) z[i] = (uint32_t)__bfloat16_as_ushort(own[2 * i]) | ((uint32_t)__bfloat16_as_ushort(own[2 * i + 1]) << 16);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float a = o[2 * i] * f, b = o[2 * i + 1] * f;
+            if (p.gate_kind == QD_GATE_VALUE) {
+                a *= sigmoid_precise(__uint_as_float(z[i] << 16));
+                b *= sigmoid_precise(__uint_as_float(z[i] & 0xffff0000u));
+            }
+            v[i] = pack_pair(a, b);
+        }
+        bf16* out = reinterpret_cast<bf16*>(p.out) + ((size_t)t * p.heads + h) * p.vdim + c0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(out)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+};
+
 // ------------------------------------------------------------------------------------- decode
 constexpr int kStepKeys = 64, kStepThreads = 256;
 
@@ -888,6 +929,22 @@ int launch_flash(const AttnParams& p, cudaStream_t s) {
     if (rows * p.kv_heads >= 128ll * device_sms() && flash_smem<DV>(p, 8) <= kMaxSmem) return launch_flash_rows<DV, 8>(p, rows, s);
     return launch_flash_rows<DV, 4>(p, rows, s);
 }
+// Heads of 128 value columns and 128 or 192 key columns: never slower there, from nine tokens on (25 us each way) to 2048
+// (window 1024, 16/4 heads: 243 -> 58 us; 16 heads with 64 shared key columns: 293 -> 75 us).
+bool umma_covers(const AttnParams& p) {
+    return p.vdim == 128 && (p.dim + p.shared_dim == 128 || p.dim + p.shared_dim == 192) && aligned16(p.out) &&
+           p.ld_k < (1ll << 31) && p.ld_v < (1ll << 31) && p.ld_shared < (1ll << 31) &&
+           (long long)p.tokens * (p.heads / p.kv_heads) <= 65535ll * 256;
+}
+int launch_umma(const AttnParams& a, cudaStream_t s) {
+    flash::In p = {};
+    p.q = (const bf16*)a.q_rows; p.k = (const bf16*)a.k_cache; p.v = (const bf16*)a.v_cache; p.common = (const bf16*)a.k_shared; p.position_ptr = a.position_ptr;
+    p.slopes = a.slopes; p.ld_k = a.ld_k; p.ld_v = a.ld_v; p.ld_common = a.ld_shared; p.scale = a.scale * kLog2e; p.position = a.position;
+    p.tokens = a.tokens; p.heads = a.heads; p.kv_heads = a.kv_heads; p.dim = a.dim; p.capacity = a.capacity; p.span = a.span;
+    p.chunked = a.mask == QD_MASK_CHUNK;
+    const FlashOut out = {a, a.ld_gate % 8 == 0 && aligned16(a.gate)};
+    return a.dim + a.shared_dim == 128 ? flash::launch<128, 128, 2, true>(p, out, s) : flash::launch<192, 128, 2, true>(p, out, s);
+}
 template <int ROWS>
 int launch_tiles(const AttnParams& p, long long rows, cudaStream_t s) {
     const size_t smem = 4 * tiles_floats(ROWS, p.dim + p.shared_dim, p.vdim);
@@ -915,6 +972,7 @@ int chunk(const AttnParams& p, cudaStream_t s) {
     const bool rows16 = sizeof(T) == 2 && p.dim % 8 == 0 && p.vdim % 8 == 0 && p.shared_dim % 8 == 0 && p.ld_k % 8 == 0 && p.ld_v % 8 == 0 &&
                         p.ld_shared % 8 == 0 && aligned16(p.q_rows) && aligned16(p.k_cache) && aligned16(p.v_cache) && aligned16(p.k_shared) &&
                         ((uintptr_t)p.out & 3u) == 0;
+    if (rows16 && umma_covers(p)) return launch_umma(p, s);
     if (rows16 && p.vdim <= 256 && flash_smem<256>(p, 4) <= kMaxSmem) {
         if (p.vdim <= 32) return launch_flash<32>(p, s);
         if (p.vdim <= 64) return launch_flash<64>(p, s);

@@ -1,0 +1,91 @@
+"""Attention of a prompt chunk on tcgen05 (flash_umma.cuh) against plain 64-bit attention on the same rows."""
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def plain(q, keys, values, scale, visible, bias=None, sink=None):
+    """q [T, H, d]; keys [S, G, d] and values [S, G, dv] by position; visible [T, S]; bias [H, T, S]; sink [H]."""
+    share = q.shape[1] // keys.shape[1]
+    k, v = keys.double().repeat_interleave(share, 1), values.double().repeat_interleave(share, 1)
+    s = torch.einsum("thd,shd->hts", q.double(), k) * scale
+    if bias is not None:
+        s = s + bias
+    s = s.masked_fill(~visible, -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink.double()[:, None, None].expand(-1, s.shape[1], 1)], -1)
+    p = torch.softmax(s, -1)[..., :keys.shape[0]]
+    return torch.einsum("hts,shd->thd", p, v)
+
+
+def close(got, want, rounds):
+    """Per row: exact products and fp32 sums; ``rounds`` bf16 roundings (2^-8 each) of probabilities, result and factors."""
+    worst = (got.double() - want).abs().amax(-1) / want.abs().amax(-1)
+    assert float(worst.max()) < rounds * 2.0 ** -8, float(worst.max())
+
+
+@pytest.mark.parametrize("tokens,position,heads,kv_heads", [
+    (2, 0, 16, 2), (16, 0, 16, 2), (17, 63, 16, 2), (65, 0, 16, 2), (200, 1000, 16, 2), (130, 3, 6, 2), (300, 0, 2, 2), (129, 64, 4, 1), (2048, 37, 16, 2)])
+def test_gated_attention_of_a_chunk(cuda_device, tokens, position, heads, kv_heads):
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape, std=1.0: (torch.randn(shape, generator=gen, device=cuda_device) * std).to(BF16)
+    capacity = position + tokens + 3
+    keys, values = new(capacity, kv_heads, 256, std=2.0), new(capacity, kv_heads, 256)
+    keys[position + tokens:], values[position + tokens:] = float("nan"), float("nan")          # not written yet
+    qg, k, v = new(tokens, heads * 512), new(tokens, kv_heads * 256), new(tokens, kv_heads * 256)
+    norm = torch.zeros(256, dtype=BF16, device=cuda_device)
+    q, out = torch.empty(tokens, heads, 256, dtype=BF16, device=cuda_device), torch.empty(tokens, heads, 256, dtype=BF16, device=cuda_device)
+    call("qd_seq_attention", ptr(qg), ptr(k), ptr(v), ptr(norm), ptr(norm), ptr(keys), ptr(values), ptr(q), ptr(out), tokens, position, capacity,
+         heads, kv_heads, 256, 64, 1e6, 1e-6, stream_of(q))
+    end = position + tokens
+    at = torch.arange(position, end, device=cuda_device)
+    visible = torch.arange(end, device=cuda_device)[None] <= at[:, None]
+    want = plain(q, keys[:end], values[:end], 0.0625, visible) * torch.sigmoid(qg.view(tokens, heads, 2, 256)[:, :, 1].double())
+    close(out, want, 4)
+
+
+@pytest.mark.parametrize("tokens,position,heads,kv_heads,shared,span,capacity,chunked,slopes,sink,gate", [
+    (300, 0, 16, 4, 0, 1024, 300, False, False, 1, 1),          # windowed, learned sinks, a gate per head
+    (700, 100, 8, 2, 0, 100, 900, False, False, 1, 1),          # ... a short window: leading tiles that later rows do not see
+    (513, 2000, 8, 8, 64, 256, 1024, False, False, 0, 2),       # shared key columns, a gate per column, the ring wraps
+    (400, 700, 16, 4, 0, 256, 1024, True, True, 2, 0),          # chunks, distance penalty, a zero sink
+    (129, 0, 3, 1, 0, 64, 256, True, True, 2, 0),               # heads that do not divide a row tile
+    (1200, 5, 4, 4, 64, 5000, 1300, False, False, 0, 2),
+])
+def test_bounded_attention_of_a_chunk(cuda_device, tokens, position, heads, kv_heads, shared, span, capacity, chunked, slopes, sink, gate):
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call_hybrid, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape, std=1.0: (torch.randn(shape, generator=gen, device=cuda_device) * std).to(BF16)
+    first, end = max(0, position - span + 1), position + tokens
+    keys, values, common = new(end, kv_heads, 128, std=2.0), new(end, kv_heads, 128), new(end, shared)
+    ring = lambda t: torch.full((capacity, *t.shape[1:]), float("nan"), dtype=BF16, device=cuda_device)
+    kr, vr, cr = ring(keys), ring(values), ring(common)
+    for j in range(max(first, end - capacity), end):
+        kr[j % capacity], vr[j % capacity], cr[j % capacity] = keys[j], values[j], common[j]
+    q, gates = new(tokens, heads, 128 + shared), new(tokens, heads * (128 if gate == 2 else 1))
+    slope = torch.rand(heads, generator=gen, device=cuda_device) * 0.05
+    sinks, out = new(heads), torch.empty(tokens, heads, 128, dtype=BF16, device=cuda_device)
+    scale = (128 + shared) ** -0.5
+    args = AttentionArgs(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, shared_dim=shared, scale=scale, ld_k=kv_heads * 128, ld_v=kv_heads * 128,
+                         ld_shared=shared, k_cache=ptr(kr), v_cache=ptr(vr), k_shared=ptr(cr) if shared else None, q_rows=ptr(q), out=ptr(out),
+                         gate=ptr(gates), ld_gate=gates.shape[1], gate_kind=gate, sink=ptr(sinks), sink_kind=sink,
+                         slopes=ptr(slope) if slopes else None, mask=int(chunked), span=min(span, capacity), capacity=capacity, position=position,
+                         tokens=tokens, dtype=0)
+    call_hybrid("qd_attention", byref(args), stream_of(q))
+    at, j = torch.arange(position, end, device=cuda_device)[:, None], torch.arange(end, device=cuda_device)[None]
+    visible = (j <= at) & (j >= (at - at % span if chunked else at - span + 1))
+    bias = -slope.double()[:, None, None] * (at - j) if slopes else None
+    with_shared = torch.cat([keys, common[:, None].expand(-1, kv_heads, -1)], -1)
+    extra = {0: None, 1: sinks, 2: torch.zeros(heads, device=cuda_device)}[sink]
+    want = plain(q, with_shared, values, scale, visible, bias, extra)
+    if gate:
+        want = want * torch.sigmoid(gates.double().view(tokens, heads, -1))
+    close(out, want, 1.5)
