@@ -275,6 +275,9 @@ int qd_nvfp4_dequantize(const void* codes, const void* scales, float global, flo
 /* F.linear on bf16 with a bf16 result (router, shared-expert gate, DeltaNet a/b, bf16 LM
  * head) — quickdraw/models/qwen.py:129-130,173,192. */
 int qd_bf16_gemv(const void* x, const void* w, void* y, int rows, int width, void* stream);
+/* Two matrices of the same input (rows1 may be 0). */
+int qd_bf16_gemv2(const void* x, const void* w0, void* y0, int rows0, const void* w1, void* y1, int rows1, int width,
+                  void* stream);
 
 /* fp8_gemv(x, proj) — quickdraw/kernel/triton/matvec.py:102-115, qwen.py:25-33. */
 int qd_fp8_gemv(const void* x, const void* w, const float* w_scale, const float* in_scale, void* y,

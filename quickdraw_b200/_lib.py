@@ -27,6 +27,7 @@ SIGNATURES = {
     "qd_nvfp4_gate_up": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "qd_nvfp4_dequantize": [P, P, F, P, L, I, I, I, P],
     "qd_bf16_gemv": [P, P, P, I, I, P],
+    "qd_bf16_gemv2": [P, P, P, I, P, P, I, I, P],
     "qd_fp8_gemv": [P, P, P, P, P, I, I, I, P],
     "qd_fp8_matmul": [P, P, P, P, P, I, I, I, P, I, P],
     "qd_route_topk": [P, I, I, I, P, P, P],
@@ -182,8 +183,8 @@ def exported_symbols() -> list[str]:
 
 
 def ptr(t: torch.Tensor | None):
-    """Device address of a tensor (or NULL)."""
-    return None if t is None else c_void_p(t.data_ptr())
+    """Device address of a tensor (or NULL), as the int that a pointer argument takes."""
+    return None if t is None else t.data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -194,7 +195,7 @@ def stream_of(t: torch.Tensor):
     launches: the raw-handle query (a fraction of a microsecond) instead of building a
     ``torch.cuda.Stream`` object per launch (several microseconds) is 3 ms of host time per chunk."""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(t.device.index if t.device.index is not None else torch.cuda.current_device()))
+        return _raw_stream(t.get_device())
     return c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
@@ -204,7 +205,9 @@ def check(code: int, name: str) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(lib(), name)(*args), name)
+    code = getattr(_lib or lib(), name)(*args)
+    if code:
+        check(code, name)
 
 
 def call_hybrid(name: str, *args) -> None:

@@ -224,24 +224,60 @@ extern "C" int qd_nvfp4_dequantize(const void* codes, const void* scales, float 
 // ------------------------------------------------------------------------ bf16 gemv
 // y = bf16(W x) with fp32 accumulation; router, shared-expert gate, DeltaNet a/b and the
 // bf16 LM head of the synthetic model (quickdraw/models/qwen.py:129-130,173,192).
-__global__ void bf16_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                 bf16* __restrict__ y, int rows, int width) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// A warp per row.  PIECES: rows in 16-byte pieces, a lane's first eight (2048 inputs) requested together: the few small
+// matrices of a token wait for one trip to memory (2 us), where two bytes at a time took 4 to 6.  Up to two matrices of the
+// same input share a launch.
+template <bool PIECES>
+__global__ void __launch_bounds__(256) bf16_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w0, bf16* __restrict__ y0, int rows0,
+                                                        const bf16* __restrict__ w1, bf16* __restrict__ y1, int rows1, int width) {
+    int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= rows) return;
-    const bf16* row = w + (size_t)warp * width;
+    if (r >= rows0 + rows1) return;
+    const bool second = r >= rows0;
+    if (second) r -= rows0;
+    const bf16* row = (second ? w1 : w0) + (size_t)r * width;
     float acc = 0.f;
-    for (int i = lane; i < width; i += 32) acc += ld_bf16(row + i) * ld_bf16(x + i);
+    if (PIECES) {
+        const uint4* wr = reinterpret_cast<const uint4*>(row);
+        const uint4* xr = reinterpret_cast<const uint4*>(x);
+        const int pieces = width / 8;
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
+        const auto add = [&](const uint4& a, const uint4& b) {
+            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) part[q] = fmaf(__uint_as_float(aw[q] & 0xffff0000u), __uint_as_float(bw[q] & 0xffff0000u),
+                                                       fmaf(__uint_as_float(aw[q] << 16), __uint_as_float(bw[q] << 16), part[q]));
+        };
+        int i = lane;
+        for (; i + 7 * 32 < pieces; i += 8 * 32) {
+            uint4 a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) a[u] = __ldg(wr + i + 32 * u);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) b[u] = xr[i + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) add(a[u], b[u]);
+        }
+        for (; i < pieces; i += 32) add(__ldg(wr + i), xr[i]);
+        acc = (part[0] + part[1]) + (part[2] + part[3]);
+    } else {
+        for (int i = lane; i < width; i += 32) acc += ld_bf16(row + i) * ld_bf16(x + i);
+    }
     acc = warp_sum(acc);
-    if (lane == 0) y[warp] = __float2bfloat16_rn(acc);
+    if (lane == 0) (second ? y1 : y0)[r] = __float2bfloat16_rn(acc);
 }
 
-extern "C" int qd_bf16_gemv(const void* x, const void* w, void* y, int rows, int width, void* stream) {
-    QD_CHECK_ARG(x && w && y && rows >= 0 && width > 0);
-    if (rows == 0) return QD_OK;
-    bf16_gemv_kernel<<<(rows + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
-        (const bf16*)x, (const bf16*)w, (bf16*)y, rows, width);
+extern "C" int qd_bf16_gemv2(const void* x, const void* w0, void* y0, int rows0, const void* w1, void* y1, int rows1, int width, void* stream) {
+    QD_CHECK_ARG(x && w0 && y0 && rows0 >= 0 && rows1 >= 0 && width > 0 && (rows1 == 0 || (w1 && y1)));
+    if (rows0 + rows1 == 0) return QD_OK;
+    const bool pieces = width % 8 == 0 && !(((uintptr_t)x | (uintptr_t)w0 | (uintptr_t)w1) & 15u);
+    const auto kernel = pieces ? bf16_gemv_kernel<true> : bf16_gemv_kernel<false>;
+    kernel<<<(unsigned)(((long long)rows0 + rows1 + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)w0, (bf16*)y0, rows0, (const bf16*)w1,
+                                                                                (bf16*)y1, rows1, width);
     return qd_launch_status();
+}
+extern "C" int qd_bf16_gemv(const void* x, const void* w, void* y, int rows, int width, void* stream) {
+    return qd_bf16_gemv2(x, w, y, rows, nullptr, nullptr, 0, width, stream);
 }
 
 // ------------------------------------------------------------------------- fp8 gemv

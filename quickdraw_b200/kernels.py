@@ -28,14 +28,20 @@ def _is_cuda_bf16(x):
 
 
 def _check_fp4(x, proj: NVFP4Linear):
+    """The contract of a packed operand, a tensor attribute read once; (out_features, in_features).  A call of the operator
+    table is as long as its host side, and this was half of it."""
+    weight, scale, scale_2, group = proj.weight, proj.weight_scale, proj.weight_scale_2, proj.group_size
     assert _is_cuda_bf16(x), "activations must be contiguous bf16 on a CUDA device"
-    assert x.shape[-1] == proj.in_features
-    assert proj.weight.dtype == torch.uint8 and proj.weight.is_contiguous()
-    assert proj.weight_scale.dtype == torch.float8_e4m3fn and proj.weight_scale.is_contiguous()
-    assert proj.weight_scale_2.dtype == torch.float32
-    assert proj.group_size % 2 == 0 and proj.in_features % proj.group_size == 0
-    assert proj.weight_scale.shape == (*proj.weight.shape[:-1], proj.in_features // proj.group_size)
-    assert x.device == proj.weight.device == proj.weight_scale.device == proj.weight_scale_2.device
+    *lead, rows, half = weight.shape
+    width = 2 * half
+    assert x.shape[-1] == width
+    assert weight.dtype is torch.uint8 and weight.is_contiguous()
+    assert scale.dtype is torch.float8_e4m3fn and scale.is_contiguous()
+    assert scale_2.dtype is torch.float32
+    assert group % 2 == 0 and width % group == 0
+    assert scale.shape == (*lead, rows, width // group)
+    assert x.get_device() == weight.get_device() == scale.get_device() == scale_2.get_device()
+    return rows, width
 
 
 # ------------------------------------------------------------------------------- norm
@@ -70,13 +76,27 @@ def _scalar_f32(value, device):
     return torch.tensor([float(value)], dtype=torch.float32, device=device)
 
 
+def _check_bf16(x, weight):
+    assert _is_cuda_bf16(x) and x.ndim == 1 and _is_cuda_bf16(weight) and weight.ndim == 2
+    rows, width = weight.shape
+    assert width == x.numel() and weight.get_device() == x.get_device()
+    return rows, width
+
+
 def bf16_gemv(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """bf16 [in] times bf16 [out, in] -> bf16 [out], fp32 accumulation."""
-    assert _is_cuda_bf16(x) and x.ndim == 1 and _is_cuda_bf16(weight) and weight.ndim == 2
-    assert weight.shape[1] == x.numel() and weight.device == x.device
-    out = torch.empty(weight.shape[0], dtype=BF16, device=x.device)
-    call("qd_bf16_gemv", ptr(x), ptr(weight), ptr(out), weight.shape[0], weight.shape[1], stream_of(x))
+    rows, width = _check_bf16(x, weight)
+    out = x.new_empty(rows)
+    call("qd_bf16_gemv", ptr(x), ptr(weight), ptr(out), rows, width, stream_of(x))
     return out
+
+
+def _bf16_gemv_pair(x, weight0, weight1):
+    """Two small matrices of the same input in one launch."""
+    (rows0, width), (rows1, _) = _check_bf16(x, weight0), _check_bf16(x, weight1)
+    out0, out1 = x.new_empty(rows0), x.new_empty(rows1)
+    call("qd_bf16_gemv2", ptr(x), ptr(weight0), ptr(out0), rows0, ptr(weight1), ptr(out1), rows1, width, stream_of(x))
+    return out0, out1
 
 
 def nvfp4_gemv(x: torch.Tensor, proj, *, routing_weight=None, force_generic: bool = False) -> torch.Tensor:
@@ -88,14 +108,14 @@ def nvfp4_gemv(x: torch.Tensor, proj, *, routing_weight=None, force_generic: boo
     if x.ndim == 2:            # a chunk of tokens (prefill): the tensor-core path
         assert routing_weight is None
         return matmul(x, proj)
-    assert x.ndim == 1 and proj.weight.ndim == 2
-    _check_fp4(x, proj)
-    assert proj.weight_scale_2.numel() == 1
+    weight, scale_2 = proj.weight, proj.weight_scale_2
+    assert x.ndim == 1 and weight.ndim == 2
+    rows, width = _check_fp4(x, proj)
+    assert scale_2.numel() == 1
     routing = None if routing_weight is None else _scalar_f32(routing_weight, x.device)
-    out = torch.empty(proj.out_features, dtype=BF16, device=x.device)
-    call("qd_nvfp4_gemv", ptr(x), ptr(proj.weight), ptr(proj.weight_scale), ptr(proj.weight_scale_2),
-         ptr(routing), ptr(out), proj.out_features, proj.in_features, proj.group_size,
-         int(force_generic), stream_of(x))
+    out = x.new_empty(rows)
+    call("qd_nvfp4_gemv", ptr(x), ptr(weight), ptr(proj.weight_scale), ptr(scale_2), ptr(routing), ptr(out), rows, width,
+         proj.group_size, int(force_generic), stream_of(x))
     return out
 
 
@@ -208,7 +228,12 @@ def expert_gemv(x, proj: NVFP4Linear, ids, weights=None, *, force_generic: bool 
 
 def gate_up(x, gate: NVFP4Linear, up: NVFP4Linear, ids=None, *, force_generic: bool = False):
     """bf16(silu(bf16 gate.x)) * bf16(up.x) for one projection pair or selected experts."""
-    _check_fp4(x, gate)
+    return _gate_up(x, gate, up, ids, force_generic)
+
+
+def _gate_up(x, gate, up, ids=None, force_generic=False, out=None):
+    """``out``: contiguous rows for the result, as many as there are slots."""
+    rows, width = _check_fp4(x, gate)
     _check_fp4(x, up)
     assert x.ndim == 1 and up.weight.shape == gate.weight.shape and up.group_size == gate.group_size
     assert up.weight_scale_2.shape == gate.weight_scale_2.shape
@@ -220,10 +245,11 @@ def gate_up(x, gate: NVFP4Linear, up: NVFP4Linear, ids=None, *, force_generic: b
     else:
         assert gate.weight_scale_2.numel() == 1
     slots = ids.numel() if bank else 1
-    out = torch.empty((slots, gate.out_features) if bank else (gate.out_features,), dtype=BF16, device=x.device)
+    if out is None:
+        out = x.new_empty((slots, rows) if bank else (rows,))
     call("qd_nvfp4_gate_up", ptr(x), ptr(gate.weight), ptr(gate.weight_scale), ptr(gate.weight_scale_2),
          ptr(up.weight), ptr(up.weight_scale), ptr(up.weight_scale_2), ptr(ids), ptr(out),
-         gate.out_features, gate.in_features, gate.group_size, slots,
+         rows, width, gate.group_size, slots,
          int(bank and gate.weight_scale_2.numel() != 1), int(force_generic), stream_of(x))
     return out
 
@@ -285,12 +311,14 @@ def moe_block(w, x: torch.Tensor, *, config) -> torch.Tensor:
     assert _is_cuda_bf16(x) and x.ndim == 1
     k = config.num_experts_per_tok
     assert 1 <= k <= config.num_experts
-    ids, weights = route(bf16_gemv(x, w.router), k)
-    strength = bf16_gemv(x, w.shared_expert_gate)
+    logits, strength = _bf16_gemv_pair(x, w.router, w.shared_expert_gate)
+    ids, weights = route(logits, k)
     inter = w.experts_gate.out_features
-    hidden = torch.empty((k + 1, inter), dtype=BF16, device=x.device)
-    hidden[:k] = gate_up(x, w.experts_gate, w.experts_up, ids)
-    hidden[k] = gate_up(x, w.shared_gate, w.shared_up)
+    assert w.shared_gate.out_features == inter
+    hidden = x.new_empty((k + 1, inter))
+    routed, shared_row = hidden.split_with_sizes((k, 1))
+    _gate_up(x, w.experts_gate, w.experts_up, ids, out=routed)
+    _gate_up(x, w.shared_gate, w.shared_up, out=shared_row)
     out = torch.empty_like(x)
     per_expert = int(w.experts_down.weight_scale_2.numel() != 1)
     if inter == 512 and k <= 8 and w.shared_down.in_features == 512:
@@ -314,8 +342,8 @@ _ATTN_SPLITS, _ATTN_SPLITS_MMA = 32, 74
 _scratch: dict = {}
 
 
-def _attn_scratch(device, floats: int, kv_heads: int):
-    key = (device, floats, kv_heads, torch.cuda.current_stream(device).cuda_stream)
+def _attn_scratch(device, floats: int, kv_heads: int, stream):
+    key = (device, floats, kv_heads, stream)
     if key not in _scratch:
         _scratch[key] = (torch.empty(floats, dtype=torch.float32, device=device),
                          torch.zeros(kv_heads, dtype=torch.int32, device=device))
@@ -344,13 +372,14 @@ def full_attention_block(w, x, kv_cache, position, *, config) -> torch.Tensor:
     lib = _lib.lib()
     splits = _ATTN_SPLITS_MMA if d == 256 else _ATTN_SPLITS
     floats = lib.qd_attn_scratch_floats(hq, hk, d, splits)
-    scratch, counters = _attn_scratch(x.device, floats, hk)
-    gated = torch.empty(hq * d, dtype=BF16, device=x.device)
+    stream = stream_of(x)
+    scratch, counters = _attn_scratch(x.device, floats, hk, stream)
+    gated = x.new_empty(hq * d)
     call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(w.q_norm), ptr(w.k_norm), ptr(keys),
          ptr(values), ptr(gated), ptr(scratch), ptr(counters),
          ptr(position) if device_position else None, 0 if device_position else int(position),
          capacity, hq, hk, d, rotary, float(config.rope_theta), float(config.rms_norm_eps),
-         splits, 0, stream_of(x))
+         splits, 0, stream)
     return _project(gated, w.o_proj)
 
 
@@ -365,8 +394,7 @@ def gated_delta_net_block(w, x, rec_state, conv_state, position, *, config) -> t
     assert hv % hk == 0
     mixed = _project(x, w.in_proj_qkv)
     z = _project(x, w.in_proj_z)
-    a = bf16_gemv(x, w.in_proj_a)
-    b = bf16_gemv(x, w.in_proj_b)
+    a, b = _bf16_gemv_pair(x, w.in_proj_a, w.in_proj_b)
     channels, width = mixed.numel(), config.linear_conv_kernel_dim
     assert conv_state.shape == (channels, width - 1) and rec_state.shape == (hv, dk, dv)
     taps = w.conv1d.reshape(channels, width)
@@ -374,7 +402,7 @@ def gated_delta_net_block(w, x, rec_state, conv_state, position, *, config) -> t
     conv = torch.empty_like(mixed)
     s = stream_of(x)
     call("qd_gdn_conv", ptr(mixed), ptr(taps), ptr(conv_state), ptr(conv), channels, width, s)
-    core = torch.empty(hv * dv, dtype=BF16, device=x.device)
+    core = x.new_empty(hv * dv)
     call("qd_gdn_recurrence", ptr(conv), ptr(a), ptr(b), ptr(w.A_log), ptr(w.dt_bias), ptr(rec_state),
          ptr(core), hk, hv, dk, dv, 0, s)
     gated = torch.empty_like(core)
