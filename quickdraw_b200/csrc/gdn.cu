@@ -8,6 +8,7 @@
 // bf16, the sum is fp32, SiLU, bf16; the history shifts left by one.
 __global__ void gdn_conv_kernel(const bf16* __restrict__ mixed, const bf16* __restrict__ taps,
                                 bf16* __restrict__ state, bf16* __restrict__ out, int channels, int width) {
+    chain_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     bf16* hist = state + (size_t)c * (width - 1);
@@ -27,9 +28,8 @@ __global__ void gdn_conv_kernel(const bf16* __restrict__ mixed, const bf16* __re
 extern "C" int qd_gdn_conv(const void* mixed, const void* taps, void* conv_state, void* out,
                            int channels, int width, void* stream) {
     QD_CHECK_ARG(mixed && taps && out && channels > 0 && width >= 1 && (width == 1 || conv_state));
-    gdn_conv_kernel<<<(channels + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-        (const bf16*)mixed, (const bf16*)taps, (bf16*)conv_state, (bf16*)out, channels, width);
-    return qd_launch_status();
+    return qd_launch(gdn_conv_kernel, dim3((channels + 127) / 128), dim3(128), 0, (cudaStream_t)stream, 3, (const bf16*)mixed, (const bf16*)taps,
+                     (bf16*)conv_state, (bf16*)out, channels, width);
 }
 
 // ------------------------------------------------------------------------- recurrence

@@ -9,6 +9,7 @@
 template <typename T>
 __global__ void rms_norm_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
                                 T* __restrict__ out, int width, float eps) {
+    chain_enter();
     __shared__ float partial[32];
     const T* row = x + (size_t)blockIdx.x * width;
     T* dst = out + (size_t)blockIdx.x * width;
@@ -33,12 +34,8 @@ extern "C" int qd_rms_norm(const void* x, const float* gamma, void* out, int row
     if (rows == 0) return QD_OK;
     const int threads = width >= 1024 ? 256 : 128;
     if (is_fp32)
-        rms_norm_kernel<float><<<rows, threads, 0, (cudaStream_t)stream>>>(
-            (const float*)x, gamma, (float*)out, width, eps);
-    else
-        rms_norm_kernel<bf16><<<rows, threads, 0, (cudaStream_t)stream>>>(
-            (const bf16*)x, gamma, (bf16*)out, width, eps);
-    return qd_launch_status();
+        return qd_launch(rms_norm_kernel<float>, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, 3, (const float*)x, gamma, (float*)out, width, eps);
+    return qd_launch(rms_norm_kernel<bf16>, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, 3, (const bf16*)x, gamma, (bf16*)out, width, eps);
 }
 
 // Fused residual update of the step (quickdraw/models/qwen.py:214-217): total = x + r in
@@ -46,6 +43,7 @@ extern "C" int qd_rms_norm(const void* x, const float* gamma, void* out, int row
 __global__ void add_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
                                 const float* __restrict__ gamma, bf16* __restrict__ normed,
                                 bf16* __restrict__ residual_out, int width, float eps) {
+    chain_enter();
     __shared__ float partial[32];
     float ss = 0.f;
     for (int i = threadIdx.x; i < width; i += blockDim.x) {
@@ -70,9 +68,8 @@ extern "C" int qd_add_rms_norm(const void* x, const void* residual, const float*
                                void* stream) {
     QD_CHECK_ARG(x && gamma && normed && residual_out && width > 0);
     QD_CHECK_ARG(residual_out != residual && residual_out != x);
-    add_norm_kernel<<<1, 512, 0, (cudaStream_t)stream>>>(
-        (const bf16*)x, (const bf16*)residual, gamma, (bf16*)normed, (bf16*)residual_out, width, eps);
-    return qd_launch_status();
+    return qd_launch(add_norm_kernel, dim3(1), dim3(512), 0, (cudaStream_t)stream, 3, (const bf16*)x, (const bf16*)residual, gamma, (bf16*)normed,
+                     (bf16*)residual_out, width, eps);
 }
 
 // ------------------------------------------------------------------- NVFP4 matvec
@@ -230,6 +227,7 @@ extern "C" int qd_nvfp4_dequantize(const void* codes, const void* scales, float 
 template <bool PIECES>
 __global__ void __launch_bounds__(256) bf16_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w0, bf16* __restrict__ y0, int rows0,
                                                         const bf16* __restrict__ w1, bf16* __restrict__ y1, int rows1, int width) {
+    chain_enter();
     int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (r >= rows0 + rows1) return;
@@ -271,10 +269,12 @@ extern "C" int qd_bf16_gemv2(const void* x, const void* w0, void* y0, int rows0,
     QD_CHECK_ARG(x && w0 && y0 && rows0 >= 0 && rows1 >= 0 && width > 0 && (rows1 == 0 || (w1 && y1)));
     if (rows0 + rows1 == 0) return QD_OK;
     const bool pieces = width % 8 == 0 && !(((uintptr_t)x | (uintptr_t)w0 | (uintptr_t)w1) & 15u);
-    const auto kernel = pieces ? bf16_gemv_kernel<true> : bf16_gemv_kernel<false>;
-    kernel<<<(unsigned)(((long long)rows0 + rows1 + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)w0, (bf16*)y0, rows0, (const bf16*)w1,
-                                                                                (bf16*)y1, rows1, width);
-    return qd_launch_status();
+    const dim3 grid((unsigned)(((long long)rows0 + rows1 + 7) / 8));
+    if (pieces)
+        return qd_launch(bf16_gemv_kernel<true>, grid, dim3(256), 0, (cudaStream_t)stream, 3, (const bf16*)x, (const bf16*)w0, (bf16*)y0, rows0,
+                         (const bf16*)w1, (bf16*)y1, rows1, width);
+    return qd_launch(bf16_gemv_kernel<false>, grid, dim3(256), 0, (cudaStream_t)stream, 3, (const bf16*)x, (const bf16*)w0, (bf16*)y0, rows0,
+                     (const bf16*)w1, (bf16*)y1, rows1, width);
 }
 extern "C" int qd_bf16_gemv(const void* x, const void* w, void* y, int rows, int width, void* stream) {
     return qd_bf16_gemv2(x, w, y, rows, nullptr, nullptr, 0, width, stream);
@@ -369,6 +369,7 @@ QD_DEVINL void route_warp(const bf16* __restrict__ logits_bf16, const float* __r
 
 __global__ void route_kernel(const bf16* logits_bf16, const float* logits_f32, int experts, int topk,
                              int32_t* ids, float* weights) {
+    chain_enter();
     route_warp(logits_bf16, logits_f32, experts, topk, ids, weights, threadIdx.x);
 }
 
@@ -376,10 +377,8 @@ extern "C" int qd_route_topk(const void* logits, int logits_fp32, int experts, i
                              float* weights, void* stream) {
     QD_CHECK_ARG(logits && ids && weights && experts >= 1 && experts <= 1024 && topk >= 1 &&
                  topk <= experts && topk <= 32);
-    route_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(
-        logits_fp32 ? nullptr : (const bf16*)logits, logits_fp32 ? (const float*)logits : nullptr,
-        experts, topk, ids, weights);
-    return qd_launch_status();
+    return qd_launch(route_kernel, dim3(1), dim3(32), 0, (cudaStream_t)stream, 3, logits_fp32 ? nullptr : (const bf16*)logits,
+                     logits_fp32 ? (const float*)logits : nullptr, experts, topk, ids, weights);
 }
 
 // --------------------------------------------------------------------- MoE combine

@@ -394,7 +394,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
 }
 
 template <int KC, bool WITH_BF16>
-int launch_variant(const StreamParams& p, int grid, cudaStream_t stream, bool pdl) {
+int launch_variant(const StreamParams& p, int grid, cudaStream_t stream, int pdl) {
     constexpr int K = KC * 1024;
     const size_t smem = (size_t)kStreamStages * kStreamStageBytes + K * 4 + (size_t)kStreamStages * kRowPartialFloats * 4 +
                         2 * kStreamConvRows * kStreamConvWidth * 2 + 3 * kStreamStages * 8 + 64 * 4 * 2 + 64;
@@ -422,7 +422,7 @@ int stream_sm_count() {
     return counts[dev];
 }
 
-int stream_launch(const StreamParams& p_in, int grid, cudaStream_t stream, bool pdl) {
+int stream_launch(const StreamParams& p_in, int grid, cudaStream_t stream, int pdl) {
     StreamParams p = p_in;
     if (grid <= 0) grid = stream_sm_count();
     if (grid > 1024) grid = 1024;
@@ -484,5 +484,5 @@ int qd_stream_matvec_try(const Fp4Args& a, cudaStream_t stream) {
         sg.w_stride = (long long)a.rows * (a.in_features / 2);
         sg.s_stride = (long long)a.rows * (a.in_features / 16);
     }
-    return stream_launch(p, 0, stream, false);
+    return stream_launch(p, 0, stream, 3);
 }

@@ -79,7 +79,7 @@ struct StreamParams {
 };
 
 // grid <= 0 picks the default number of blocks per SM.  Returns a QD_* code.
-int stream_launch(const StreamParams& p, int grid, cudaStream_t stream, bool pdl);
+int stream_launch(const StreamParams& p, int grid, cudaStream_t stream, int pdl);
 int stream_sm_count();
 
 }  // namespace qd

@@ -72,6 +72,7 @@ struct Bars {
 __global__ void __launch_bounds__(kThreads, 1)
 nvfp4_umma_matvec_kernel(const __grid_constant__ UmmaParams p, const __grid_constant__ CUtensorMap code_map,
                          const __grid_constant__ CUtensorMap scale_map) {
+    chain_enter();                // before the tensor memory: a block that waits for its predecessor must not hold what that one needs
     extern __shared__ __align__(1024) uint8_t umma_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(umma_smem_raw) + 1023) & ~uintptr_t(1023));
     const int K = p.k, chunks = K / 256, halves = K / 2048;   // 256-input chunks; 128-byte groups of a scale row
@@ -269,6 +270,5 @@ int qd_umma_matvec_try(const Fp4Args& a, cudaStream_t stream) {
             return QD_ERR_LAUNCH;
         configured[dev] = true;
     }
-    nvfp4_umma_matvec_kernel<<<grid, kThreads, smem, stream>>>(p, code_map, scale_map);
-    return qd_launch_status();
+    return qd_launch(nvfp4_umma_matvec_kernel, dim3(grid), dim3(kThreads), smem, stream, 3, p, code_map, scale_map);
 }

@@ -21,6 +21,7 @@ from ._lib import call, ptr, stream_of
 from .weights import FP8Linear, NVFP4Linear
 
 BF16 = torch.bfloat16
+CHAINED = 3            # launched behind its predecessor in the stream as a programmatic dependent, outside of captures
 
 
 def _is_cuda_bf16(x):
@@ -326,7 +327,7 @@ def moe_block(w, x: torch.Tensor, *, config) -> torch.Tensor:
         call("qd_moe_down_combine", ptr(hidden), ptr(ids), ptr(weights), ptr(w.experts_down.weight),
              ptr(w.experts_down.weight_scale), ptr(w.experts_down.weight_scale_2),
              ptr(w.shared_down.weight), ptr(w.shared_down.weight_scale), ptr(w.shared_down.weight_scale_2),
-             ptr(strength), ptr(out), None, None, x.numel(), inter, k, per_expert, lo, hi, 0, stream_of(x))
+             ptr(strength), ptr(out), None, None, x.numel(), inter, k, per_expert, lo, hi, CHAINED, stream_of(x))
         return out
     contributions = expert_gemv(hidden[:k].contiguous(), w.experts_down, ids, weights)
     shared = nvfp4_gemv(hidden[k].contiguous(), w.shared_down)
@@ -379,7 +380,7 @@ def full_attention_block(w, x, kv_cache, position, *, config) -> torch.Tensor:
          ptr(values), ptr(gated), ptr(scratch), ptr(counters),
          ptr(position) if device_position else None, 0 if device_position else int(position),
          capacity, hq, hk, d, rotary, float(config.rope_theta), float(config.rms_norm_eps),
-         splits, 0, stream)
+         splits, CHAINED, stream)
     return _project(gated, w.o_proj)
 
 

@@ -344,3 +344,18 @@ def test_reference_fixtures_through_the_operator_table(K, cuda_device, reference
         compare(actual, data["expected"], data["rtol"], data["atol"])
         for arg in state_args.get(fn, ()):
             compare(kwargs[arg], data["after"][arg], data["rtol"], data["atol"])
+
+
+@pytest.mark.parametrize("rows0,rows1,width", [(1, 1, 8), (32, 32, 2048), (256, 1, 2048), (7, 3, 2056), (5, 9, 2047), (9, 0, 4104)])
+def test_bf16_matrices_of_one_input_share_a_launch(cuda_device, rows0, rows1, width):
+    """Whole batches of 16-byte pieces, remainders and odd widths; bound: fp32 sums, one bf16 rounding (2^-8)."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(rows0)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).bfloat16()
+    x, w0, w1 = new(width), new(rows0, width), new(rows1, width)
+    y0, y1 = x.new_empty(rows0), x.new_empty(rows1)
+    call("qd_bf16_gemv2", ptr(x), ptr(w0), ptr(y0), rows0, ptr(w1) if rows1 else None, ptr(y1) if rows1 else None, rows1, width, stream_of(x))
+    for w, y in ((w0, y0), (w1, y1)):
+        if w.shape[0]:
+            want = w.double() @ x.double()
+            torch.testing.assert_close(y.double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
