@@ -89,6 +89,10 @@ int qd_linear_recurrence(const float* q, const float* k, const float* g, const f
     float* kq, float* state, float* out, int tokens, int heads, int kv_heads, int dim, int vdim, int delta, void*
     stream);
 
+/* The same with delta = 0 in segments of `span` tokens side by side.  scratch: heads * dim * (vdim + 1) floats a segment. */
+int qd_gla_segments(const float* q, const float* k, const float* g, const float* v, float* state, float* out, int tokens, int
+    heads, int kv_heads, int dim, int vdim, int span, float* scratch, void* stream);
+
 /* out[t, h] = x[t, h] / rms(x[t, h]) * w * act(gate[t, h]), act 0 = SiLU, 1 = sigmoid; w [vdim] shared by the heads. */
 int qd_head_norm_gate(const float* x, const void* w, const void* gate, long long ld_gate, void* out, int tokens, int
     heads, int vdim, float eps, int act, int dtype, void* stream);

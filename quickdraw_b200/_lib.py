@@ -101,6 +101,7 @@ HYBRID_LIBRARIES = {
         "qd_gla_prepare": [P, P, P, L, P, P, F, P, P, P, P, I, I, I, I, I, P],
         "qd_channel_delta_prepare": [P, P, P, P, L, P, P, P, P, P, P, P, I, P, I, P, P, P, P, P, P, I, I, I, I, I, I, P],
         "qd_linear_recurrence": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
+        "qd_gla_segments": [P, P, P, P, P, P, I, I, I, I, I, I, P, P],
         "qd_head_norm_gate": [P, P, P, L, P, I, I, I, F, I, I, P],
         "qd_gla_step": [P, P, P, P, P, P, I, F, P, P, F, P, P, I, I, I, I, P],
         "qd_channel_delta_step": [P, P, P, P, P, P, P, I, P, P, P, P, P, I, P, I, P, P, I, P, F, P, P, I, I, I, I, I, P],

@@ -8,7 +8,10 @@
 // registers.  A warp owns eight value columns; a lane a group of key rows and a few columns, held as row
 // pairs for the packed fp32 FMA.  Both read-outs of the delta rule use the decayed state before the
 // write, o = (gS)^T q + (k . q) u, so that the second one hides in the first one's shuffles.
-// Latency-bound: one warp per scheduler, a dependent chain per token.
+// Latency-bound: one warp per scheduler, a dependent chain per token.  Without the delta rule the state behind a segment of tokens is
+// the product of its decays times the state in front of it plus what it adds itself, so a long chunk goes in segments side by
+// side: what each adds (no read-out), the states in front of them, then the walk of each.  2048 tokens of 16 heads of 128:
+// 437 -> 235 us.
 // Decode: recurrence_step_kernel does everything between the projections and the output projection in
 // one launch: low-rank decay (and output gate), convolution, unit norms, recurrence, per-head RMS norm,
 // gate.  A cluster of blocks shares a head (32 value columns each) and adds its sums of squares over
@@ -219,7 +222,13 @@ struct RecurrenceParams {
     const float* scales;          // delta rule: per token and key/value head the factors that make k and q unit vectors (q's / sqrt(dim)), k . q of the unit vectors
     float* state; float* out;
     int tokens, heads, kv_heads, dim, vdim, vectors;
+    // a chunk in segments of `span` tokens (blockIdx.z): states [segment][heads][dim][vdim], products of decays [segment][heads][dim]
+    float* segment_states; float* segment_decays;
+    int span, segments;
 };
+// WHOLE: the chunk from the state.  LOCAL: a segment from zero, its last state and the product of its decays.  REST: a segment
+// from the state in front of it.
+enum { WHOLE, LOCAL, REST };
 
 // floats of one staged token: q, k, decay - 1 (padded to `row`), v columns, step size and the three scales
 constexpr int rec_token_floats(int row) { return 3 * row + kRecCols + 4; }
@@ -279,9 +288,10 @@ template <int N> QD_DEVINL void load_columns(const float* p, float (&v)[N]) {
 // more rounds) instead of a butterfly per column.
 template <int KL, int CC> constexpr int rec_threads() { return kRecCols / (32 / KL * CC) * 32; }
 
-template <int KL, int CC, int J, bool DELTA, bool GATHER>
+template <int KL, int CC, int J, bool DELTA, bool GATHER, int PASS = WHOLE>
 __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kernel(const __grid_constant__ RecurrenceParams p) {
     chain_enter();
+    const int first = PASS == WHOLE ? 0 : blockIdx.z * p.span, tokens = PASS == WHOLE ? p.tokens : min(p.span, p.tokens - first);
     extern __shared__ __align__(16) float tiles[];
     constexpr int kRow = 4 * KL * J, kToken = rec_token_floats(kRow), kThreads = rec_threads<KL, CC>();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kl = lane % KL, cl = lane / KL;
@@ -289,6 +299,13 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
     const int local = (warp * (32 / KL) + cl) * CC, col = c0 + local;
     const int dim = p.dim, vdim = p.vdim;
     float* state = p.state + (size_t)head * dim * vdim;
+    if (PASS != WHOLE) state = p.segment_states + ((size_t)blockIdx.z * p.heads + head) * dim * vdim;
+    // The segment's decays multiplied up, this lane's rows, by one warp and in 64 bits: the rounding of a slow decay, the same at
+    // every token, would add up (3e-5 of the state after 3000 tokens instead of 1e-6).
+    const bool multiplies = PASS == LOCAL && blockIdx.y == 0 && warp == 0;
+    double product[J][4];
+#pragma unroll
+    for (int j = 0; j < J; ++j) product[j][0] = product[j][1] = product[j][2] = product[j][3] = 1.0;
 
     for (int i = tid; i < 2 * kRecTile * kToken; i += kThreads) tiles[i] = 0.f;      // padding rows stay zero
     u64 s[J][2][CC];
@@ -299,7 +316,7 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
 #pragma unroll
             for (int c = 0; c < CC; ++c) {
                 const int r = j * 4 * KL + kl * 4 + h * 2;
-                const bool ok = col + c < vdim;
+                const bool ok = PASS != LOCAL && col + c < vdim;
                 s[j][h][c] = pack2(ok && r < dim ? state[(size_t)r * vdim + col + c] : 0.f,
                                    ok && r + 1 < dim ? state[(size_t)(r + 1) * vdim + col + c] : 0.f);
             }
@@ -309,7 +326,7 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
     const int cols = min(kRecCols, vdim - c0), unit = p.vectors ? 4 : 1;
     const int kp = dim / unit, per = 3 * kp + cols / unit;
     auto stage = [&](int tile) {
-        const int t0 = tile * kRecTile, count = min(kRecTile, p.tokens - t0);
+        const int count = min(kRecTile, tokens - tile * kRecTile), t0 = first + tile * kRecTile;
         float* base = tiles + (tile & 1) * kRecTile * kToken;
         for (int piece = tid; piece < per; piece += kThreads) {
             const int which = piece / kp, e = (which < 3 ? piece - which * kp : piece - 3 * kp) * unit;
@@ -338,12 +355,12 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
         for (int j = 0; j < J; ++j) {
             f.g[j] = *reinterpret_cast<const ulonglong2*>(token + 2 * kRow + j * 4 * KL + kl * 4);
             f.k[j] = *reinterpret_cast<const ulonglong2*>(token + kRow + j * 4 * KL + kl * 4);
-            f.q[j] = *reinterpret_cast<const ulonglong2*>(token + j * 4 * KL + kl * 4);
+            if (PASS != LOCAL) f.q[j] = *reinterpret_cast<const ulonglong2*>(token + j * 4 * KL + kl * 4);
         }
         load_columns<CC>(token + 3 * kRow + local, f.v);
     };
-    float* out = p.out + (size_t)head * vdim;
     const size_t out_stride = (size_t)p.heads * vdim;
+    float* out = p.out + first * out_stride + (size_t)head * vdim;
     // one token; o: the read-outs of this lane's rows
     auto advance = [&](const RecVectors<J, CC>& f, const float* token, float* o) {
         u64 oa[CC], ob[CC];
@@ -393,6 +410,21 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
                 }
                 o[c] = fmaf(w.z, (lo2(oa[c]) + hi2(oa[c])) + (lo2(ob[c]) + hi2(ob[c])), kl == 0 ? u * w.w : 0.f);
             }
+        } else if (PASS == LOCAL) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                if (multiplies) {
+                    const float g[4] = {lo2(f.g[j].x), hi2(f.g[j].x), lo2(f.g[j].y), hi2(f.g[j].y)};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) product[j][i] = fma(product[j][i], (double)g[i], product[j][i]);
+                }
+#pragma unroll
+                for (int c = 0; c < CC; ++c) {
+                    const u64 vv = pack2(f.v[c], f.v[c]);
+                    s[j][0][c] = fma2(f.k[j].x, vv, fma2(s[j][0][c], f.g[j].x, s[j][0][c]));
+                    s[j][1][c] = fma2(f.k[j].y, vv, fma2(s[j][1][c], f.g[j].y, s[j][1][c]));
+                }
+            }
         } else {
 #pragma unroll
             for (int c = 0; c < CC; ++c) {
@@ -409,13 +441,13 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
         }
     };
 
-    const int ntiles = (p.tokens + kRecTile - 1) / kRecTile;
+    const int ntiles = (tokens + kRecTile - 1) / kRecTile;
     stage(0);
     for (int tile = 0; tile < ntiles; ++tile) {
         if (tile + 1 < ntiles) { stage(tile + 1); copies_wait<1>(); } else { copies_wait<0>(); }
         __syncthreads();
         const float* token = tiles + (tile & 1) * kRecTile * kToken;
-        const int count = min(kRecTile, p.tokens - tile * kRecTile);
+        const int count = min(kRecTile, tokens - tile * kRecTile);
         RecVectors<J, CC> even, odd;                     // the next token's vectors are read while this one is reduced
         fetch(token, even);
         for (int tt = 0; tt < count; tt += 4, token += 4 * kToken) {
@@ -430,12 +462,25 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
             if (tt + 2 < count) advance(even, token + 2 * kToken, o + 2 * CC);
             if (tt + 4 < count) fetch(token + 4 * kToken, even);
             if (tt + 3 < count) advance(odd, token + 3 * kToken, o + 3 * CC);
+            if (PASS == LOCAL) continue;
             const float mine = scatter_sum<KL, 4 * CC>(o, kl);
             const int value = kl / (KL / (4 * CC)), t = value / CC, c = value % CC;
             if (kl % (KL / (4 * CC)) == 0 && tt + t < count && col + c < vdim) out[t * out_stride + col + c] = mine;
             out += 4 * out_stride;
         }
         __syncthreads();                 // the buffer may be refilled
+    }
+    if (PASS == REST) {
+        if ((int)blockIdx.z + 1 < p.segments) return;
+        state = p.state + (size_t)head * dim * vdim;
+    }
+    if (multiplies && cl == 0) {
+        float* decays = p.segment_decays + ((size_t)blockIdx.z * p.heads + head) * dim;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (j * 4 * KL + kl * 4 + i < dim) decays[j * 4 * KL + kl * 4 + i] = (float)product[j][i];
     }
 #pragma unroll
     for (int j = 0; j < J; ++j)
@@ -453,12 +498,12 @@ __global__ void __launch_bounds__(rec_threads<KL, CC>()) linear_recurrence_kerne
 
 // Launched ordinarily: started as a dependent while the kernel before it still fills the SMs, the blocks
 // gather on the few SMs that free up first (1.1 ms instead of 0.58 and 0.45 ms at 2048 tokens).
-template <int KL, int CC, int J, bool DELTA, bool GATHER>
+template <int KL, int CC, int J, bool DELTA, bool GATHER, int PASS = WHOLE>
 int launch_recurrence(const RecurrenceParams& p, cudaStream_t stream) {
     const size_t smem = 2ull * kRecTile * rec_token_floats(4 * KL * J) * 4;
-    if (!allow_smem(linear_recurrence_kernel<KL, CC, J, DELTA, GATHER>, smem)) return QD_ERR_LAUNCH;
-    return qd_launch(linear_recurrence_kernel<KL, CC, J, DELTA, GATHER>, dim3(p.heads, (p.vdim + kRecCols - 1) / kRecCols),
-                     dim3(rec_threads<KL, CC>()), smem, stream, 0, p);
+    if (!allow_smem(linear_recurrence_kernel<KL, CC, J, DELTA, GATHER, PASS>, smem)) return QD_ERR_LAUNCH;
+    return qd_launch(linear_recurrence_kernel<KL, CC, J, DELTA, GATHER, PASS>,
+                     dim3(p.heads, (p.vdim + kRecCols - 1) / kRecCols, PASS == WHOLE ? 1 : p.segments), dim3(rec_threads<KL, CC>()), smem, stream, 0, p);
 }
 // Layouts by measurement (2048 tokens, 32 heads of 128): the delta rule 584 us with sixteen lanes and four
 // columns (630 with 8 x 2, 642 with 16 x 2, 679 with 32 x 4), gated linear attention 393 us with 32 x 8.
@@ -469,11 +514,27 @@ int delta_recurrence(const RecurrenceParams& p, cudaStream_t stream) {
     if (p.dim <= 256) return launch_recurrence<16, 4, 4, true, false>(p, stream);
     return QD_ERR_UNSUPPORTED;
 }
+template <int PASS = WHOLE>
 int gla_recurrence(const RecurrenceParams& p, cudaStream_t stream) {
-    if (p.dim <= 64) return launch_recurrence<16, 4, 1, false, false>(p, stream);
-    if (p.dim <= 128) return launch_recurrence<32, 8, 1, false, false>(p, stream);
-    if (p.dim <= 256) return launch_recurrence<32, 8, 2, false, false>(p, stream);
+    if (p.dim <= 64) return launch_recurrence<16, 4, 1, false, false, PASS>(p, stream);
+    if (p.dim <= 128) return launch_recurrence<32, 8, 1, false, false, PASS>(p, stream);
+    if (p.dim <= 256) return launch_recurrence<32, 8, 2, false, false, PASS>(p, stream);
     return QD_ERR_UNSUPPORTED;
+}
+
+// The state in front of every segment in the place of the segment's own: S' = diag(product of decays) S + (own state).
+__global__ void __launch_bounds__(256) segment_states_kernel(const float* __restrict__ state, float* __restrict__ states,
+                                                             const float* __restrict__ decays, long long elements, int vdim, int segments) {
+    chain_enter();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, rows = elements / vdim;
+    if (i >= elements) return;
+    const long long row = i / vdim;
+    float s = state[i];
+    for (int z = 0; z < segments; ++z) {
+        const float own = states[z * elements + i];
+        states[z * elements + i] = s;
+        s = fmaf(decays[z * rows + row], s, own);
+    }
 }
 
 // ------------------------------------------------------------------------ per-head norm, gate
@@ -790,6 +851,23 @@ extern "C" int qd_linear_recurrence(const float* q, const float* k, const float*
     const int vectors = dim % 4 == 0 && vdim % 4 == 0 && qd::aligned16(q) && qd::aligned16(k) && qd::aligned16(g) && qd::aligned16(v);
     const qd::RecurrenceParams p = {q, k, g, v, beta, scales, state, out, tokens, heads, kv_heads, dim, vdim, vectors};
     return delta ? qd::delta_recurrence(p, (cudaStream_t)stream) : qd::gla_recurrence(p, (cudaStream_t)stream);
+}
+
+extern "C" int qd_gla_segments(const float* q, const float* k, const float* g, const float* v, float* state, float* out, int tokens, int heads,
+                               int kv_heads, int dim, int vdim, int span, float* scratch, void* stream) {
+    QD_CHECK_ARG(q && k && g && v && state && out && scratch && tokens > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && vdim > 0);
+    QD_CHECK_ARG(span > 0 && (tokens + span - 1) / span <= 65535);
+    const int vectors = dim % 4 == 0 && vdim % 4 == 0 && qd::aligned16(q) && qd::aligned16(k) && qd::aligned16(g) && qd::aligned16(v);
+    const long long elements = (long long)heads * dim * vdim;
+    qd::RecurrenceParams p = {q, k, g, v, nullptr, nullptr, state, out, tokens, heads, kv_heads, dim, vdim, vectors};
+    p.span = span; p.segments = (tokens + span - 1) / span;
+    p.segment_states = scratch; p.segment_decays = scratch + p.segments * elements;
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = qd::gla_recurrence<qd::LOCAL>(p, s);
+    if (rc == QD_OK)
+        rc = qd_launch(qd::segment_states_kernel, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, s, 0, (const float*)state, p.segment_states,
+                       (const float*)p.segment_decays, elements, vdim, p.segments);
+    return rc == QD_OK ? qd::gla_recurrence<qd::REST>(p, s) : rc;
 }
 
 extern "C" int qd_head_norm_gate(const float* x, const void* w, const void* gate, long long ld_gate, void* out, int tokens, int heads,

@@ -490,3 +490,32 @@ def test_sizes_of_a_real_layer(cuda_device):
     steps = run_portions(engine_of(ckpt, F32), tokens, [1] * 140)
     half = run_portions(engine_of(ckpt, BF16, chunk=140), tokens, [140])
     assert error(steps, exact.cpu()) < 1e-4 and error(half, exact.cpu()) < 6e-2
+
+
+@pytest.mark.parametrize("tokens,heads,dim,vdim,span", [(1, 2, 128, 128, 16), (48, 3, 128, 128, 16), (333, 2, 128, 96, 48), (100, 1, 64, 40, 16),
+                                                        (130, 2, 200, 64, 64), (129, 2, 30, 33, 32), (700, 2, 128, 128, 176)])
+def test_gated_linear_attention_in_segments(cuda_device, tokens, heads, dim, vdim, span):
+    """Segments side by side against the walk of the whole chunk and 64 bits: as close to 64 bits as the walk is (sums of as many
+    terms; half as much again for the order), tokens that do not fill the last segment, rows that are not whole pieces."""
+    from quickdraw_b200._lib import call_hybrid, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device)
+    q, k, v = new(tokens, heads, dim), new(tokens, heads, dim), new(tokens, heads, vdim)
+    g = -torch.rand(tokens, heads, dim, generator=gen, device=cuda_device) ** 6       # decays less one: most channels remember long
+    state = new(heads, dim, vdim)
+    runs = []
+    for segments in (False, True):
+        s, out = state.clone(), torch.empty_like(v)
+        if segments:
+            scratch = torch.full((-(-tokens // span) * heads * dim * (vdim + 1),), float("nan"), device=cuda_device)
+            call_hybrid("qd_gla_segments", ptr(q), ptr(k), ptr(g), ptr(v), ptr(s), ptr(out), tokens, heads, heads, dim, vdim, span, ptr(scratch), stream_of(q))
+        else:
+            call_hybrid("qd_linear_recurrence", ptr(q), ptr(k), ptr(g), ptr(v), None, None, ptr(s), ptr(out), tokens, heads, heads, dim, vdim, 0, stream_of(q))
+        runs.append((out.double(), s.double()))
+    s, want = state.double(), []
+    for t in range(tokens):
+        s = s * (1 + g[t].double())[..., None] + k[t].double()[..., None] * v[t].double()[:, None]
+        want.append(torch.einsum("hd,hdv->hv", q[t].double(), s))
+    error = lambda got, exact: float((got - exact).norm() / exact.norm())
+    for walk, parts, exact in zip(*runs, (torch.stack(want), s)):
+        assert error(parts, exact) <= 1.5 * error(walk, exact) + 1e-7, (error(walk, exact), error(parts, exact))
