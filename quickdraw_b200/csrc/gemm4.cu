@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(kThreads4, TN == 128 ? 2 : 1)
 nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ CUtensorMap x_codes,
                        const __grid_constant__ CUtensorMap x_scales, const __grid_constant__ CUtensorMap w_codes,
                        const __grid_constant__ CUtensorMap w_scales) {
+    chain_enter();                // before the tensor memory: a block that waits for its predecessor must not hold what that one needs
     extern __shared__ __align__(1024) uint8_t gemm4_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm4_smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int kStages4 = stages_of(TN), kStage4Bytes = stage_bytes(TN), kHalves = TN / 128;
@@ -184,17 +185,32 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
 }
 
 // ---- activation quantiser --------------------------------------------------------------
-// Largest magnitude of the chunk (bf16 magnitudes order like their bit patterns).
-__global__ void act_amax_kernel(const uint4* __restrict__ x, long long n8, unsigned int* __restrict__ amax_bits) {
-    uint32_t m = 0u;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
-        const uint4 v = x[i];
-        m = max(m, max(max(v.x & 0x7fffu, (v.x >> 16) & 0x7fffu), max(v.y & 0x7fffu, (v.y >> 16) & 0x7fffu)));
-        m = max(m, max(max(v.z & 0x7fffu, (v.z >> 16) & 0x7fffu), max(v.w & 0x7fffu, (v.w >> 16) & 0x7fffu)));
+// Largest magnitude of the chunk (bf16 magnitudes order like their bit patterns).  Four pieces of a thread in flight and one atomic
+// a block: 8192 x 2048 in 11.8 us, 13.8 with one piece and an atomic a warp.
+__global__ void __launch_bounds__(256) act_amax_kernel(const uint4* __restrict__ x, long long n8, unsigned int* __restrict__ amax_bits) {
+    __shared__ uint32_t warps[8];
+    const long long step = (long long)gridDim.x * blockDim.x;
+    uint32_t m = 0u;                                  // a pair of magnitudes
+    const auto take = [&](const uint4& v) {
+        m = __vmaxu2(m, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+    };
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * step < n8; i += 4 * step) {
+        const uint4 a = x[i], b = x[i + step], c = x[i + 2 * step], d = x[i + 3 * step];
+        take(a); take(b); take(c); take(d);
     }
+    for (; i < n8; i += step) take(x[i]);
+    m = max(m & 0xffffu, m >> 16);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(amax_bits, m);
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < 8 ? warps[threadIdx.x] : 0u;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (threadIdx.x == 0 && m) atomicMax(amax_bits, m);
+    }
 }
 
 // Eight values -> eight E2M1 codes, round to nearest even, saturating; value 2i in the low
@@ -223,6 +239,7 @@ QD_DEVINL uint32_t e4m3_of(float v) {                 // round to nearest even, 
 // nearest even; a block whose scale rounds to zero gets zero codes.
 __global__ void act_quantize_kernel(const bf16* __restrict__ x, long long blocks, const unsigned int* __restrict__ amax_bits,
                                     uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, float* __restrict__ global) {
+    chain_enter();
     const float amax = __uint_as_float(*amax_bits << 16);
     const float g = amax > 0.f ? amax / (6.f * 448.f) : 1.f;
     if (blockIdx.x == 0 && threadIdx.x == 0) *global = g;
@@ -273,9 +290,9 @@ extern "C" int qd_nvfp4_quantize_act(const void* x, int tokens, int in_features,
     const int grid = (int)std::min<long long>((n / 8 + 255) / 256, 148 * 8);
     act_amax_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(x), n / 8, amax_scratch);
     const long long blocks = n / 16;
-    act_quantize_kernel<<<(unsigned)((blocks + 255) / 256), 256, 0, s>>>(reinterpret_cast<const bf16*>(x), blocks, amax_scratch,
-                                                                     reinterpret_cast<uint8_t*>(codes), reinterpret_cast<uint8_t*>(scales), global);
-    return qd_launch_status();
+    if (qd_launch_status() != QD_OK) return QD_ERR_LAUNCH;
+    return qd_launch(act_quantize_kernel, dim3((unsigned)((blocks + 255) / 256)), dim3(256), 0, s, 3, reinterpret_cast<const bf16*>(x), blocks,
+                     (const unsigned int*)amax_scratch, reinterpret_cast<uint8_t*>(codes), reinterpret_cast<uint8_t*>(scales), global);
 }
 
 extern "C" int qd_nvfp4_matmul_w4a4(const void* x_codes, const void* x_scales, const float* x_global, const void* w_codes,
@@ -302,15 +319,15 @@ extern "C" int qd_nvfp4_matmul_w4a4(const void* x_codes, const void* x_scales, c
     const long long token_tiles = (tokens + kTile - 1) / kTile;
     const bool wide = wide_tiles >= 0 ? wide_tiles != 0 : (out_features % 256 == 0 && token_tiles * (out_features / 256) >= 2ll * sms);
     static bool configured[2][64];
-    auto launch = [&](auto kernel, int tn) -> int {
-        const size_t smem = (size_t)stages_of(tn) * stage_bytes(tn) + sizeof(Bars4) + 64 + 1024;
-        if (!configured[tn == 256][dev]) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return QD_ERR_LAUNCH;
-            configured[tn == 256][dev] = true;
-        }
-        const dim3 grid((unsigned)(out_features / tn), (unsigned)token_tiles);
-        kernel<<<grid, kThreads4, smem, (cudaStream_t)stream>>>(p, xc, xs, wc, ws);
-        return qd_launch_status();
-    };
-    return wide ? launch(nvfp4_gemm_w4a4_kernel<256>, 256) : launch(nvfp4_gemm_w4a4_kernel<128>, 128);
+    const size_t smem = wide ? (size_t)stages_of(256) * stage_bytes(256) + sizeof(Bars4) + 64 + 1024
+                             : (size_t)stages_of(128) * stage_bytes(128) + sizeof(Bars4) + 64 + 1024;
+    if (!configured[wide][dev]) {
+        if ((wide ? cudaFuncSetAttribute(nvfp4_gemm_w4a4_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                  : cudaFuncSetAttribute(nvfp4_gemm_w4a4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return QD_ERR_LAUNCH;
+        configured[wide][dev] = true;
+    }
+    const dim3 grid((unsigned)(out_features / (wide ? 256 : 128)), (unsigned)token_tiles);
+    if (wide) return qd_launch(nvfp4_gemm_w4a4_kernel<256>, grid, dim3(kThreads4), smem, (cudaStream_t)stream, 3, p, xc, xs, wc, ws);
+    return qd_launch(nvfp4_gemm_w4a4_kernel<128>, grid, dim3(kThreads4), smem, (cudaStream_t)stream, 3, p, xc, xs, wc, ws);
 }
