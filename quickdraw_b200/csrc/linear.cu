@@ -2,7 +2,7 @@
 // same launch: a bias, the exact GELU on the leading columns (the up projection of a feed-forward whose
 // launch also carries other rows), a gated linear unit over neighbouring weight rows, the addition to
 // what y already holds (a residual stream).  What may precede it for few token rows: the RMS norm of x.
-// Three forms behind one entry point,:
+// Four forms, the last one behind an entry point of its own:
 //   linear_umma_kernel  many token rows, bf16 x: tcgen05.mma kind::f16, both operands by tiled TMA
 //                       (128-byte swizzle), accumulators in tensor memory.  Tensor-bound.
 //   linear_rows_kernel  up to eight token rows: a warp streams whole weight rows (16-byte loads, the
