@@ -181,6 +181,10 @@ QD_DEVINL void grid_launch_dependents() { asm volatile("griddepcontrol.launch_de
 // the next kernel of the stream may be scheduled behind this one's blocks, then the kernel waits until
 // the one before it has finished and its writes are visible.  Before this call a kernel must not touch
 // anything another kernel of the stream writes; in an ordinary launch both instructions do nothing.
+// Some kernels fetch weights or a state before their own wait, and starts are handed on: each kernel of a chain
+// may start while several in front of it run.  So a kernel whose result may be such a weight or state (codes of the activation
+// quantiser, a matrix, a convolution history) does not use this call but grid_dependency_wait() alone: its dependents start
+// when its last block has ended.
 QD_DEVINL void chain_enter() { grid_launch_dependents(); grid_dependency_wait(); }
 
 QD_DEVINL uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }

@@ -8,7 +8,7 @@
 // bf16, the sum is fp32, SiLU, bf16; the history shifts left by one.
 __global__ void gdn_conv_kernel(const bf16* __restrict__ mixed, const bf16* __restrict__ taps,
                                 bf16* __restrict__ state, bf16* __restrict__ out, int channels, int width) {
-    chain_enter();
+    grid_dependency_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     bf16* hist = state + (size_t)c * (width - 1);

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kThreads4, TN == 128 ? 2 : 1)
 nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ CUtensorMap x_codes,
                        const __grid_constant__ CUtensorMap x_scales, const __grid_constant__ CUtensorMap w_codes,
                        const __grid_constant__ CUtensorMap w_scales) {
-    chain_enter();                // before the tensor memory: a block that waits for its predecessor must not hold what that one needs
+    grid_dependency_wait();       // before the tensor memory: a block that waits for its predecessor must not hold what that one needs
     extern __shared__ __align__(1024) uint8_t gemm4_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm4_smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int kStages4 = stages_of(TN), kStage4Bytes = stage_bytes(TN), kHalves = TN / 128;
@@ -236,10 +236,11 @@ QD_DEVINL uint32_t e4m3_of(float v) {                 // round to nearest even, 
 
 // One thread per block of sixteen inputs: tensor scale g = amax / (6 * 448) (1 for a zero chunk),
 // block scale s = e4m3(block amax / (6 g)), codes = e2m1(x / (s g)), everything round to
-// nearest even; a block whose scale rounds to zero gets zero codes.
+// nearest even; a block whose scale rounds to zero gets zero codes.  The result has the layout of a weight, which some
+// products fetch before they wait for the kernel in front of them: nobody is released before the stores are visible.
 __global__ void act_quantize_kernel(const bf16* __restrict__ x, long long blocks, const unsigned int* __restrict__ amax_bits,
                                     uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, float* __restrict__ global) {
-    chain_enter();
+    grid_dependency_wait();
     const float amax = __uint_as_float(*amax_bits << 16);
     const float g = amax > 0.f ? amax / (6.f * 448.f) : 1.f;
     if (blockIdx.x == 0 && threadIdx.x == 0) *global = g;
@@ -261,6 +262,7 @@ __global__ void act_quantize_kernel(const bf16* __restrict__ x, long long blocks
     for (int i = 0; i < 16; ++i) v[i] *= inv;
     reinterpret_cast<uint2*>(codes)[b] = make_uint2(e2m1x8(v, 0), e2m1x8(v, 8));
     scales[b] = (uint8_t)sbits;
+    __threadfence();
 }
 
 int scale_map_of(CUtensorMap* map, const void* base, long long rows, long long row_bytes) {

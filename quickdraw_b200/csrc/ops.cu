@@ -9,7 +9,7 @@
 template <typename T>
 __global__ void rms_norm_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
                                 T* __restrict__ out, int width, float eps) {
-    chain_enter();
+    grid_dependency_wait();
     __shared__ float partial[32];
     const T* row = x + (size_t)blockIdx.x * width;
     T* dst = out + (size_t)blockIdx.x * width;

@@ -59,7 +59,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
 
     if (warp == CW) {
         // ------------------------------------------------------------------ producer
-        if (p.ids_in) grid_dependency_wait();      // bank entries depend on the routing
+        if (p.ids_in || p.wait_first) grid_dependency_wait();      // bank entries depend on the routing
         if (lane == 0) {
             int it = 0;
             unsigned seg_start = 0;
@@ -470,6 +470,7 @@ int qd_stream_matvec_try(const Fp4Args& a, cudaStream_t stream) {
     p.x = a.x;
     p.nseg = a.slots;
     p.expert_lo = 0; p.expert_hi = 0x7fffffff;
+    p.wait_first = 1;
     if (a.ids) { p.ids_in = a.ids; p.topk = a.slots; }
     for (int s = 0; s < a.slots; ++s) {
         StreamSeg& sg = p.seg[s];

@@ -75,6 +75,9 @@ struct StreamParams {
     // EP_ARGMAX
     float* best_val; int* best_idx; unsigned int* counter; long long* token_out;
     unsigned int* status;
+    // The weights, too, may be what a kernel in front writes: no copy starts before the wait.  (The decode step's are the
+    // checkpoint's, and their copies run ahead of it.)
+    int wait_first;
     unsigned int quota, remainder;   // filled by stream_launch: total cost = quota * grid + remainder
 };
 

@@ -359,3 +359,39 @@ def test_bf16_matrices_of_one_input_share_a_launch(cuda_device, rows0, rows1, wi
         if w.shape[0]:
             want = w.double() @ x.double()
             torch.testing.assert_close(y.double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("rows", [1024, 333])                # a row count for the FP4 tensor core and one for the streaming kernel
+@pytest.mark.parametrize("use", ["gate_up", "gemv", "gemv_streamed", "matmul_rows"])
+def test_weights_written_right_in_front_of_their_use(K, cuda_device, use, rows):
+    """Codes and scales that kernels of the same stream write, used at once, in buffers that held other matrices before: the
+    same bits as behind a synchronisation."""
+    if use == "matmul_rows":
+        rows = 1024
+    gen = torch.Generator(device=cuda_device).manual_seed(rows)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).bfloat16()
+    a, b = new(4096, 4096), new(4096, 4096)
+    x, chunk = new(2048), new(8, 2048)
+
+    def product(gate, up):
+        if use == "gate_up":
+            return K.gate_up(x, gate, up)
+        if use == "matmul_rows":
+            return K.matmul_rows(chunk, up)[0]
+        return K.nvfp4_gemv(x, up, force_generic=2 if use == "gemv_streamed" else False)
+
+    got, projections = [], []
+    for i in range(24):
+        matrices = new(2, rows, 2048) * 2.0 ** (i % 5)
+        torch.cuda.synchronize()
+        if i % 3 == 0:
+            torch.matmul(a, b)                                  # some hundred microseconds that everything below is queued behind
+        projections.append([NVFP4Linear(*K.quantize_act(m)) for m in matrices])
+        got.append(product(*projections[-1]))
+        if i >= 8:                                              # their memory goes to a later matrix
+            projections[i - 8] = [NVFP4Linear(p.weight.clone(), p.weight_scale.clone(), p.weight_scale_2.clone()) for p in projections[i - 8]]
+    torch.cuda.synchronize()
+    for pair, y in zip(projections, got):
+        want = product(*pair)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)

@@ -321,3 +321,38 @@ def test_every_kernel_launched_as_a_programmatic_dependent_waits_for_its_predece
             dependents += 1
     assert dependents >= 30
 
+
+
+def test_operator_table_kernels_read_nothing_before_their_wait():
+    """Source check: what the operator table launches as a programmatic dependent (mode 3) may follow a kernel that writes any of
+    its operands, weights included, so no operand is read in front of the wait; and the kernels whose results may be weights
+    or states that others fetch ahead of their own wait release nobody before they end."""
+    sources = {path.name: path.read_text() for path in (ROOT / "quickdraw_b200" / "csrc").glob("*.cu*")}
+    everything = "\n".join(sources.values())
+
+    def kernel(name):                    # (parameters, body)
+        match = re.search(r"__global__[^{;]*?\b" + name + r"\s*\(([^{;]*)\)\s*\{", everything, flags=re.S)
+        depth, at = 1, match.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(everything[at], 0)
+            at += 1
+        return match.group(1), re.sub(r"//[^\n]*", "", everything[match.end():at - 1])
+
+    names = set(re.findall(r"qd_launch\((?:qd::)?(\w+)(?:<\w+>)?, (?:[^;]*?), 3, ", everything))
+    names |= {"attn_decode_kernel", "attn_decode_mma_kernel", "moe_down_kernel"}          # the mode is an argument of their entry points
+    assert names >= {"rms_norm_kernel", "add_norm_kernel", "bf16_gemv_kernel", "route_kernel", "act_quantize_kernel", "gdn_conv_kernel",
+                     "nvfp4_umma_matvec_kernel", "nvfp4_gemm_w4a4_kernel"}
+    waits = r"chain_enter\(\);|grid_dependency_wait\(\);"
+    for name in names:
+        parameters, body = kernel(name)
+        front = body[:re.search(waits, body).start()]
+        pointers = re.findall(r"\*\s*(?:const\s+)?(?:__restrict__\s+)?(\w+)", parameters)
+        reads = [p for p in pointers if re.search(r"\b" + p + r"\s*\[|[=(,+]\s*\*" + p + r"\b", front)]
+        assert not reads and not re.search(r"\bp\.\w+\s*\[|\*\s*p\.\w+\s*[;)]|\bld_\w+\(|\bload\w*\(|__ldc?g\(|bulk_load|cp16|copy16", front), (name, reads)
+    _, body = kernel("stream_kernel")    # fetches weights ahead of the wait in the decode step, not here
+    assert body.index("if (p.ids_in || p.wait_first) grid_dependency_wait();") < body.index("bulk_load(")
+    entry = sources["stream.cu"][sources["stream.cu"].index("int qd_stream_matvec_try("):]
+    assert entry.index("p.prologue = PRO_NONE;") < entry.index("p.wait_first = 1;") < entry.index("return stream_launch(p, 0, stream, 3);")
+    for name in ("act_quantize_kernel", "nvfp4_gemm_w4a4_kernel", "rms_norm_kernel", "gdn_conv_kernel"):
+        body = kernel(name)[1]
+        assert "chain_enter" not in body and "grid_launch_dependents" not in body, name
