@@ -126,7 +126,7 @@ fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUte
         for (int k = 0; k < mine; ++k) {
             const int tile = blockIdx.x + k * gridDim.x;
             const int token = tile / p.across * kF8Tokens + quadrant * 32 + lane, n0 = tile % p.across * TN;
-            ok = ok && mbar_wait(ready + (k & 1), (k >> 1) & 1, nullptr);
+            ok = __all_sync(0xffffffffu, ok && mbar_wait(ready + (k & 1), (k >> 1) & 1, nullptr));
             tc_fence_after();
             bf16* out = p.y + (size_t)token * p.rows;
 #pragma unroll 1
@@ -140,21 +140,23 @@ fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUte
 #pragma unroll
                     for (int q = 0; q < 16; ++q) v[q] = 0x7fc00000u;
                 }
-                if (token >= p.tokens) continue;
-                uint32_t packed[8];
+                if (token < p.tokens) {
+                    uint32_t packed[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const __nv_bfloat162 two = __floats2bfloat162_rn((__uint_as_float(v[2 * q]) * s_in) * s_w, (__uint_as_float(v[2 * q + 1]) * s_in) * s_w);
-                    packed[q] = *reinterpret_cast<const uint32_t*>(&two);
-                }
-                if (vectors && n0 + c + 16 <= p.rows) {
-                    *reinterpret_cast<uint4*>(out + n0 + c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    *reinterpret_cast<uint4*>(out + n0 + c + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                } else {        // rows is even and y on a four-byte boundary
+                    for (int q = 0; q < 8; ++q) {
+                        const __nv_bfloat162 two = __floats2bfloat162_rn((__uint_as_float(v[2 * q]) * s_in) * s_w, (__uint_as_float(v[2 * q + 1]) * s_in) * s_w);
+                        packed[q] = *reinterpret_cast<const uint32_t*>(&two);
+                    }
+                    if (vectors && n0 + c + 16 <= p.rows) {
+                        *reinterpret_cast<uint4*>(out + n0 + c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                        *reinterpret_cast<uint4*>(out + n0 + c + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                    } else {        // rows is even and y on a four-byte boundary
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (n0 + c + 2 * q < p.rows) *reinterpret_cast<uint32_t*>(out + n0 + c + 2 * q) = packed[q];
+                        for (int q = 0; q < 8; ++q)
+                            if (n0 + c + 2 * q < p.rows) *reinterpret_cast<uint32_t*>(out + n0 + c + 2 * q) = packed[q];
+                    }
                 }
+                __syncwarp();       // the next read of tensor memory is the whole warp's
             }
             tc_fence_before();
             __syncwarp();

@@ -482,7 +482,7 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
         for (int i = 0; i < kHalf; ++i) acc[i] = 0.f;
         bool ok = true;
         for (int seg = 0; seg < segments && ok; ++seg) {
-            ok = mbar_wait(ready + (seg & 1), (seg >> 1) & 1, p.status);
+            ok = __all_sync(0xffffffffu, mbar_wait(ready + (seg & 1), (seg >> 1) & 1, p.status));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t from = tmem + ((uint32_t)(quadrant * 32) << 16) + (seg & 1) * TN + half * kHalf;

@@ -356,3 +356,16 @@ def test_operator_table_kernels_read_nothing_before_their_wait():
     for name in ("act_quantize_kernel", "nvfp4_gemm_w4a4_kernel", "rms_norm_kernel", "gdn_conv_kernel"):
         body = kernel(name)[1]
         assert "chain_enter" not in body and "grid_launch_dependents" not in body, name
+
+
+def test_tensor_memory_is_read_by_whole_warps():
+    """Source check of the tcgen05 products of fp32 rows and of static FP8: the collective reads follow a wait whose result the warp
+    shares, and no lane leaves an iteration (a token past the last one) on its own."""
+    csrc = ROOT / "quickdraw_b200" / "csrc"
+    for name, kernel, read in (("fp8_gemm.cu", "fp8_gemm_kernel", "tmem_load16("), ("linear.cu", "linear_pieces_kernel", "tmem_ld32(")):
+        text = (csrc / name).read_text()
+        body = text[re.search(r"\b" + kernel + r"\(const", text).start():]
+        epilogue = body[body.rindex("const int ", 0, body.index(read)):body.index("__syncthreads();", body.index(read))]
+        before = body[:body.index(read)]
+        assert re.search(r"ok = __all_sync\(0xffffffffu, (?:ok && )?mbar_wait\(ready", before[before.rindex("} else {\n        const int "):]), name
+        assert "continue;" not in epilogue, name
