@@ -189,6 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
         const int slot_first = key_first % p.capacity, ld_own = (int)(values ? p.ld_v : p.ld_k), ld_common = (int)p.ld_common;
         const bf16* own = values ? p.v + g * DV : p.k + g * p.dim;
         bool ok = true;
+        int issued = -1;                                                     // the last tile whose copies this warp has started
         const auto fill = [&](auto pieces, int tile) {
             constexpr int kPieces = decltype(pieces)::value, kBatch = 8;
             static_assert(kRowsEach * kPieces % (32 * kBatch) == 0, "");
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
         for (int tile = stage; tile < tiles && ok; tile += 2) {
             ok = __all_sync(0xffffffffu, mbar_wait(empty, ((tile >> 1) & 1) ^ 1, nullptr));
             if (!ok) break;
+            issued = tile;
             // Boxes where the tile is whole: row by row an SM copies 18 bytes a clock, by TMA what L2 gives.
             const int slot = (int)((slot_first + (long long)tile * kKeys) % p.capacity);
             if (p.boxes && key_first + (tile + 1) * kKeys - 1 <= pos_last && slot + kKeys <= p.capacity) {
@@ -239,8 +241,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(full);
         }
-        const int last = (tiles - 1 - stage) & ~1;                           // of this stage, plus the stage: no copy outlives the block
-        if (ok && last >= 0) mbar_wait(full, (last >> 1) & 1, nullptr);
+        if (issued >= 0) mbar_wait(full, (issued >> 1) & 1, nullptr);        // no copy outlives the block, also where a wait ran out
     } else if (warp == kMma) {
         const bool leader = elected();
         const uint32_t qa = smem_u32(smem), ka = smem_u32(ks), va = smem_u32(vs);

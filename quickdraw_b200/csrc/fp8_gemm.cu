@@ -20,7 +20,7 @@ constexpr int kF8Tokens = 128, kF8Chunk = 128;      // inputs per stage: one swi
 template <int TN> struct F8Tile {
     static constexpr int kABytes = kF8Tokens * kF8Chunk, kStageBytes = kABytes + TN * kF8Chunk;
     static constexpr int kStages = TN == 256 ? 4 : TN == 128 ? 6 : 8;
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 4) * 8 + 16 + 1024;
+    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 5) * 8 + 16 + 1024;
     // fp32 accumulator, E4M3 A and B (format 0), K-major, N >> 3 at 17, M >> 4 at 24
     static constexpr uint32_t kDesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kF8Tokens >> 4) << 24);
 };
@@ -64,11 +64,13 @@ fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUte
     uint64_t* empty = full + kStages;
     uint64_t* ready = empty + kStages;         // an accumulator holds a whole tile
     uint64_t* taken = ready + 2;               // it has been read
-    uint32_t* slot = reinterpret_cast<uint32_t*>(taken + 2);
+    uint64_t* drained = taken + 2;             // every MMA has ended
+    uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(ready + s, 1); mbar_init(taken + s, 4); }
+        mbar_init(drained, 1);
         mbar_fence_init();
     }
     if (warp == 1) { tmem_alloc(slot, 2 * TN); tmem_relinquish(); }
@@ -117,6 +119,8 @@ fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUte
                 }
                 if (ok) umma_commit(ready + (k & 1));
             }
+            umma_commit(drained);             // tensor memory is given back only behind the last MMA, also where a wait ran out
+            mbar_wait(drained, 0, nullptr);
         }
     } else {
         const int quadrant = warp & 3;

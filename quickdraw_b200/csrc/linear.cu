@@ -400,7 +400,7 @@ template <int TN> struct PieceTile {
     static constexpr int kABytes = 128 * 128, kBBytes = TN * 128, kStageBytes = 3 * kABytes + kBBytes;
     static constexpr int kStages = TN == 256 ? 2 : 3;
     static constexpr int kThreads = 320;
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 4) * 8 + 16 + 1024;
+    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 5) * 8 + 16 + 1024;
 };
 
 template <typename TY, int TN>
@@ -416,7 +416,8 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
     uint64_t* empty = full + kStages;
     uint64_t* ready = empty + kStages;         // an accumulator holds a whole segment
     uint64_t* taken = ready + 2;               // it has been read
-    uint32_t* slot = reinterpret_cast<uint32_t*>(taken + 2);
+    uint64_t* drained = taken + 2;             // every MMA has ended
+    uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t0 = blockIdx.x * 128, n0 = blockIdx.y * TN;
     const int steps = (p.width + kStepK - 1) / kStepK, segments = (p.width + kSegment - 1) / kSegment;
@@ -427,6 +428,7 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(ready + s, 1); mbar_init(taken + s, 8); }
+        mbar_init(drained, 1);
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -474,6 +476,8 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
                 umma_commit_to(empty + st);
                 if (inside == kPerSegment - 1 || s == steps - 1) umma_commit_to(ready + (seg & 1));
             }
+            umma_commit_to(drained);          // tensor memory is given back only behind the last MMA, also where a wait ran out
+            mbar_wait(drained, 0, p.status);
         }
     } else {
         const int half = (warp - 2) >> 2, quadrant = warp & 3;

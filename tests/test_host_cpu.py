@@ -369,3 +369,17 @@ def test_tensor_memory_is_read_by_whole_warps():
         before = body[:body.index(read)]
         assert re.search(r"ok = __all_sync\(0xffffffffu, (?:ok && )?mbar_wait\(ready", before[before.rindex("} else {\n        const int "):]), name
         assert "continue;" not in epilogue, name
+
+
+def test_a_wait_that_ran_out_leaves_nothing_in_flight():
+    """Source check of the tcgen05 kernels with several warps of bounded waits: tensor memory is given back behind a commit of all
+    MMAs, which no earlier result guards, and the attention's loaders wait for the copies they have started in any case."""
+    csrc = ROOT / "quickdraw_b200" / "csrc"
+    for name, kernel in (("fp8_gemm.cu", "fp8_gemm_kernel"), ("linear.cu", "linear_pieces_kernel"), ("flash_umma.cuh", "flash_umma_kernel"),
+                         ("expert_tiles.cu", "expert_tiles_kernel")):
+        text = (csrc / name).read_text()
+        body = text[re.search(r"\b" + kernel + r"\(const", text).start():]
+        body = body[:min(body.index(word) for word in ("tmem_dealloc", "tcgen05.dealloc") if word in body)]
+        assert re.search(r"commit\w*\(&?(?:bars->)?drained\);[^\n]*\n\s*mbar_wait\(&?(?:bars->)?drained, 0", body), name
+    loaders = (csrc / "flash_umma.cuh").read_text()
+    assert re.search(r"\n        if \(issued >= 0\) mbar_wait\(full, \(issued >> 1\) & 1, nullptr\);", loaders)
