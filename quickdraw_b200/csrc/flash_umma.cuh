@@ -3,7 +3,7 @@
 //
 // A block owns TILES x 128 packed (token, head of the group) rows of one key/value head and walks the positions they see in
 // tiles of 64.  Per tile and 128 rows: S = Q K^T (both from shared memory), a thread per row takes the softmax in registers,
-// P goes over S as bf16 (TWO: as two bf16 pieces, sixteen bits), O += P V.  The result is rescaled only when a row's maximum
+// P goes over S as two bf16 pieces (sixteen bits), O += P V.  The result is rescaled only when a row's maximum
 // has grown by more than 2^8 since the last time (P stays below 2^8 and the sum in fp32, so the quotient is the same to
 // rounding): after the first tiles a warp hardly ever reads O before the end.
 //   warps 0 .. 4 TILES - 1   softmax, one row a thread; then the epilogue
@@ -13,11 +13,14 @@
 // Values are read as they lie (rows of a key, the result's columns innermost): a B operand with the columns as the major
 // dimension.  Every wait is bounded; a block whose wait ran out writes NaN.
 //
-// Measured (2048 tokens, with the launch gap; before: mma.sync, eight or sixteen rows a warp).  Head dimension 256, 16/2 heads, one
-// piece: behind 0 / 2000 / 30000 positions 126 / 210 / 1347 us (478 / 1017 / 7949).  128 columns, two pieces, window 1024: 16/4
-// heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 2500 clocks at head dimension 256: 1280 of
+// Measured (2048 tokens, with the launch gap; before: mma.sync, eight or sixteen rows a warp).  Head dimension 256, 16/2 heads:
+// behind 0 / 2000 / 30000 positions 128 / 223 / 1595 us (478 / 1017 / 7949).  128 columns, window 1024: 16/4
+// heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 3000 clocks at head dimension 256: 1800 of
 // MMAs (those of S are bound by shared memory, 48 clocks for 64 columns), 1100 of keys and values at 64 bytes a clock, and the
-// hand-over of S and P; copied with cp.async alone it took 3700.
+// hand-over of S and P.
+// One piece, eight bits, takes 120 / 199 / 1290 us there, but since the largest P is not one here (the reference lags behind the
+// maximum) its rounding reaches the result: 2.04e-3 from 64 bits with sharp scores, where the result's own rounding is 1.65e-3
+// and mma.sync with the exact maximum had 1.72e-3.  Two pieces: 1.65e-3.
 #pragma once
 #include <cuda.h>
 
@@ -139,7 +142,7 @@ struct Bars {
 
 // Out: called per row and 32 columns as out(token, head, c0, o, m, l) with the unnormalised columns c0 .. c0 + 31 and the row's
 // softmax state (log2 of the reference, the sum relative to it); l NaN marks a failed wait.
-template <int QD, int DV, int TILES, bool TWO, typename Out>
+template <int QD, int DV, int TILES, typename Out>
 __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_constant__ In p, const __grid_constant__ Maps maps, const __grid_constant__ Out out) {
     chain_enter();
     using S = Shape<QD, DV, TILES>;
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
                         for (int j = 0; j < kKeys / 16; ++j) {
                             const uint64_t desc = desc_mn(b + j * 2048, kKeys * 128);
                             mma_ts(d, a + j * 8, desc, idesc(DV, 1), (i | j) ? 1u : 0u);
-                            if (TWO) mma_ts(d, a + 32 + j * 8, desc, idesc(DV, 1), 1u);
+                            mma_ts(d, a + 32 + j * 8, desc, idesc(DV, 1), 1u);
                         }
                         commit(&bars->o_done[t][i & 1]);
                         if (t == TILES - 1) commit(bars->v_empty + (i & 1));
@@ -376,13 +379,11 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
 #pragma unroll
             for (int c = 0; c < 32; ++c) hi[c] = pair(s[c >> 4][(2 * c) & 31], s[c >> 4][(2 * c + 1) & 31]);
             store32(s_at + b * kKeys, hi);
-            if (TWO) {
-                uint32_t lo[32];
+            uint32_t lo[32];
 #pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    lo[c] = pair(s[c >> 4][(2 * c) & 31] - __uint_as_float(hi[c] << 16), s[c >> 4][(2 * c + 1) & 31] - __uint_as_float(hi[c] & 0xffff0000u));
-                store32(s_at + b * kKeys + 32, lo);
-            }
+            for (int c = 0; c < 32; ++c)
+                lo[c] = pair(s[c >> 4][(2 * c) & 31] - __uint_as_float(hi[c] << 16), s[c >> 4][(2 * c + 1) & 31] - __uint_as_float(hi[c] & 0xffff0000u));
+            store32(s_at + b * kKeys + 32, lo);
             stored();
             fence_before();
             __syncwarp();
@@ -420,7 +421,7 @@ inline bool map_of(CUtensorMap* map, const void* base, long long columns, long l
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int QD, int DV, int TILES, bool TWO, typename Out>
+template <int QD, int DV, int TILES, typename Out>
 int launch(In p, const Out& out, cudaStream_t stream) {
     alignas(64) Maps maps = {};
     p.boxes = p.dim % 64 == 0 && p.capacity >= kKeys && map_of(&maps.k, p.k, (long long)p.kv_heads * p.dim, p.ld_k, p.capacity) &&
@@ -431,13 +432,13 @@ int launch(In p, const Out& out, cudaStream_t stream) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
     static bool configured[64];
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(flash_umma_kernel<QD, DV, TILES, TWO, Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(flash_umma_kernel<QD, DV, TILES, Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return QD_ERR_LAUNCH;
         configured[dev] = true;
     }
     const long long rows = (long long)p.tokens * (p.heads / p.kv_heads);
     const dim3 grid(p.kv_heads, (unsigned)((rows + 128 * TILES - 1) / (128 * TILES)));
-    return qd_launch(flash_umma_kernel<QD, DV, TILES, TWO, Out>, grid, dim3(kThreads), smem, stream, 1, p, maps, out);
+    return qd_launch(flash_umma_kernel<QD, DV, TILES, Out>, grid, dim3(kThreads), smem, stream, 1, p, maps, out);
 }
 
 }  // namespace flash

@@ -47,5 +47,5 @@ int seq_flash_attention(const bf16* q, const bf16* qg, const bf16* k_cache, cons
     p.scale = 0.0625f * 1.4426950408889634f;                 // 1 / sqrt(256)
     p.position = position0; p.tokens = tokens; p.heads = q_heads; p.kv_heads = kv_heads; p.dim = 256; p.capacity = capacity;
     const GatedOut store = {qg, out, q_heads, (((uintptr_t)out | (uintptr_t)qg) & 15u) == 0};
-    return qd::flash::launch<256, 256, 1, false>(p, store, stream);
+    return qd::flash::launch<256, 256, 1>(p, store, stream);
 }

@@ -943,7 +943,7 @@ int launch_umma(const AttnParams& a, cudaStream_t s) {
     p.tokens = a.tokens; p.heads = a.heads; p.kv_heads = a.kv_heads; p.dim = a.dim; p.capacity = a.capacity; p.span = a.span;
     p.chunked = a.mask == QD_MASK_CHUNK;
     const FlashOut out = {a, a.ld_gate % 8 == 0 && aligned16(a.gate)};
-    return a.dim + a.shared_dim == 128 ? flash::launch<128, 128, 2, true>(p, out, s) : flash::launch<192, 128, 2, true>(p, out, s);
+    return a.dim + a.shared_dim == 128 ? flash::launch<128, 128, 2>(p, out, s) : flash::launch<192, 128, 2>(p, out, s);
 }
 template <int ROWS>
 int launch_tiles(const AttnParams& p, long long rows, cudaStream_t s) {

@@ -89,3 +89,23 @@ def test_bounded_attention_of_a_chunk(cuda_device, tokens, position, heads, kv_h
     if gate:
         want = want * torch.sigmoid(gates.double().view(tokens, heads, -1))
     close(out, want, 1.5)
+
+
+@pytest.mark.parametrize("tokens,position", [(64, 0), (511, 0), (200, 3000)])
+def test_chunk_attention_rounds_its_result_only(cuda_device, tokens, position):
+    """Sharp scores, gates of one: with probabilities of sixteen bits the distance to 64 bits is that of one bf16 rounding
+    of the result (their own part is 2^-18 of it, below a hundredth); eight bits add a quarter."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).to(BF16)
+    end = position + tokens
+    keys, values, qg = new(end, 2, 256), new(end, 2, 256), new(tokens, 16, 2, 256)
+    qg[:, :, 1] = 30.0
+    k, v, norm, q_norm = new(tokens, 512), new(tokens, 512), torch.zeros(256, dtype=BF16, device=cuda_device), torch.full((256,), 3.0, dtype=BF16, device=cuda_device)
+    q, out = torch.empty(tokens, 16, 256, dtype=BF16, device=cuda_device), torch.empty(tokens, 16, 256, dtype=BF16, device=cuda_device)
+    call("qd_seq_attention", ptr(qg), ptr(k), ptr(v), ptr(q_norm), ptr(norm), ptr(keys), ptr(values), ptr(q), ptr(out), tokens, position, end,
+         16, 2, 256, 64, 1e6, 1e-6, stream_of(q))
+    at = torch.arange(position, end, device=cuda_device)
+    want = plain(q, keys, values, 0.0625, torch.arange(end, device=cuda_device)[None] <= at[:, None])
+    error = lambda t: float((t.double() - want).norm() / want.norm())
+    assert error(out) < 1.01 * error(want.to(BF16)), (error(out), error(want.to(BF16)))
