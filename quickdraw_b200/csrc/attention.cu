@@ -248,7 +248,9 @@ attn_decode_kernel(const AttnParams p) {
 // fp32 dot product and one warp reduction per head and position (a chain of shuffles), 64 blocks of it.  Here a
 // warp takes sixteen positions at a time, its key and value rows go from the cache straight into the fragments
 // (every element is needed by one lane), the next keys are requested before the softmax of these, and a context of
-// 8192 positions is split over 32 blocks per KV head, one of 32768 over 74 (148 blocks).  Bound by the latency of
+// 8192 positions is split over 32 blocks per KV head, one of 32768 over 74 (148 blocks).  The probabilities enter as three
+// bf16 pieces, the fp32 values of the kernel above (with two, sixteen bits, eight times as many results are rounded to the other
+// neighbour: 1.6e-3 of them instead of 2e-4).  Bound by the latency of
 // that chain and of the two merges, not by the cache's bytes: B200, 16/2 heads,
 // 600 / 8192 / 32768 positions: - / 175 / 498 us with the kernel above, 21 / 24 / 44 us here (0.7 and 1.5 TB/s).
 constexpr int kAttnMmaSplitMin = 256;      // positions per split at least: two chunks per warp
@@ -374,7 +376,7 @@ attn_decode_mma_kernel(const AttnParams p) {
             if (c + kAttnWarps * 16 < t1) load_keys(c + kAttnWarps * 16);
             const qd::AttnProbs pr = qd::attn_softmax(acc, s0, s1, c, t1, lane);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) qd::attn_value_step(acc, q, values[q][0], values[q][1], values[q][2], values[q][3], pr);
+            for (int q = 0; q < 4; ++q) qd::attn_value_step<true>(acc, q, values[q][0], values[q][1], values[q][2], values[q][3], pr);
         }
         // lane (g, t): statistics of head g (the sum spread over its four lanes), out[i][c] = feature
         // 32 g + 2 i + (c >> 1) of head 2 t + (c & 1)

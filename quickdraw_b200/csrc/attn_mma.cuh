@@ -43,9 +43,9 @@ QD_DEVINL void attn_score_step(float (&s0)[4], float (&s1)[4], const uint4& q4, 
     mma_bf16(s1, q4.z, 0u, q4.w, 0u, k1.z, k1.w);
 }
 
-// Probabilities of a chunk as the B operand of the value product, split into two bf16 pieces
-// (sixteen bits of mantissa).
-struct AttnProbs { uint32_t hi0, hi1, lo0, lo1; };
+// Probabilities of a chunk as the B operand of the value product, split into bf16 pieces: the first two hold
+// sixteen bits of mantissa, all three the fp32 value.
+struct AttnProbs { uint32_t hi0, hi1, lo0, lo1, rest0, rest1; };
 
 // Running softmax over the chunk's scores; rescales the accumulator.  first: context position of
 // row 0 of the chunk; t1: end of the range (rows at or past it are masked).
@@ -70,8 +70,11 @@ QD_DEVINL AttnProbs attn_softmax(AttnAcc& acc, const float (&s0)[4], const float
     acc.m = m_new;
     AttnProbs pr;
     pr.hi0 = pack_bf16x2(p[0], p[1]); pr.hi1 = pack_bf16x2(p[2], p[3]);
-    pr.lo0 = pack_bf16x2(p[0] - __uint_as_float(pr.hi0 << 16), p[1] - __uint_as_float(pr.hi0 & 0xffff0000u));
-    pr.lo1 = pack_bf16x2(p[2] - __uint_as_float(pr.hi1 << 16), p[3] - __uint_as_float(pr.hi1 & 0xffff0000u));
+    p[0] -= __uint_as_float(pr.hi0 << 16); p[1] -= __uint_as_float(pr.hi0 & 0xffff0000u);
+    p[2] -= __uint_as_float(pr.hi1 << 16); p[3] -= __uint_as_float(pr.hi1 & 0xffff0000u);
+    pr.lo0 = pack_bf16x2(p[0], p[1]); pr.lo1 = pack_bf16x2(p[2], p[3]);
+    pr.rest0 = pack_bf16x2(p[0] - __uint_as_float(pr.lo0 << 16), p[1] - __uint_as_float(pr.lo0 & 0xffff0000u));
+    pr.rest1 = pack_bf16x2(p[2] - __uint_as_float(pr.lo1 << 16), p[3] - __uint_as_float(pr.lo1 & 0xffff0000u));
     const float a_even = __shfl_sync(0xffffffffu, alpha, 8 * t), a_odd = __shfl_sync(0xffffffffu, alpha, 8 * t + 4);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -80,7 +83,8 @@ QD_DEVINL AttnProbs attn_softmax(AttnAcc& acc, const float (&s0)[4], const float
     return pr;
 }
 
-// Values: bytes 64 g + 16 q .. + 15 of the value rows t, 4 + t, 8 + t, 12 + t of the chunk.
+// Values: bytes 64 g + 16 q .. + 15 of the value rows t, 4 + t, 8 + t, 12 + t of the chunk.  WHOLE: with the third piece.
+template <bool WHOLE = false>
 QD_DEVINL void attn_value_step(AttnAcc& acc, int q, const uint4& r0, const uint4& r1, const uint4& r2, const uint4& r3,
                                const AttnProbs& pr) {
     const uint32_t w0[4] = {r0.x, r0.y, r0.z, r0.w}, w1[4] = {r1.x, r1.y, r1.z, r1.w};
@@ -91,6 +95,7 @@ QD_DEVINL void attn_value_step(AttnAcc& acc, int q, const uint4& r0, const uint4
         const uint32_t a2 = __byte_perm(w2[e], w3[e], 0x5410), a3 = __byte_perm(w2[e], w3[e], 0x7632);
         mma_bf16(acc.out[q * 4 + e], a0, a1, a2, a3, pr.hi0, pr.hi1);
         mma_bf16(acc.out[q * 4 + e], a0, a1, a2, a3, pr.lo0, pr.lo1);
+        if (WHOLE) mma_bf16(acc.out[q * 4 + e], a0, a1, a2, a3, pr.rest0, pr.rest1);
     }
 }
 

@@ -395,3 +395,27 @@ def test_weights_written_right_in_front_of_their_use(K, cuda_device, use, rows):
         want = product(*pair)
         torch.cuda.synchronize()
         assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("position", [999, 8191])
+def test_decode_attention_keeps_its_probabilities_whole(cuda_device, position):
+    """Head dimension 256, gates of one: fp32 probabilities and sums (2^-22 of the result) round 2^-22 / 2^-9 twice over, 2.4e-4, of
+    the results to the other bf16 neighbour; probabilities of sixteen bits about 2e-3 of them."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    differ = total = 0
+    for seed in range(12):
+        gen = torch.Generator(device=cuda_device).manual_seed(seed)
+        new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).bfloat16()
+        keys, values = new(position + 1, 2, 256), new(position + 1, 2, 256)
+        qg, k_new, v_new, norm = new(16, 2, 256), new(2, 256), new(2, 256), torch.zeros(256, dtype=torch.bfloat16, device=cuda_device)
+        qg[:, 1] = 30.0
+        out, counters = new(16, 256), torch.zeros(2, dtype=torch.int32, device=cuda_device)
+        scratch = torch.empty(lib().qd_attn_scratch_floats(16, 2, 256, 74), device=cuda_device)
+        call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(norm), ptr(norm), ptr(keys), ptr(values), ptr(out), ptr(scratch), ptr(counters),
+             None, position, position + 1, 16, 2, 256, 0, 1e6, 1e-6, 74, 0, stream_of(out))
+        q = qg[:, 0].float()
+        q = (q * torch.rsqrt(q.square().sum(-1, keepdim=True) / 256 + 1e-6)).bfloat16().double()
+        k, v = (t.double().repeat_interleave(8, 1) for t in (keys, values))
+        want = torch.einsum("ht,thd->hd", torch.softmax(torch.einsum("hd,thd->ht", q, k) / 16, -1), v)
+        differ, total = differ + int((out != want.bfloat16()).sum()), total + out.numel()
+    assert differ < total * 2 ** -10, differ / total
