@@ -366,9 +366,10 @@ attn_decode_mma_kernel(const AttnParams p) {
             uint4 values[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint8_t* row = vc + (size_t)min(c + 4 * i + t, T - 1) * row_bytes + g * 64;
+                const bool seen = c + 4 * i + t < t1;      // zeros behind the context: nothing else gives zero times a probability of zero
+                const uint8_t* row = vc + (size_t)(c + 4 * i + t) * row_bytes + g * 64;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) values[q][i] = ld_cache16(row + q * 16);
+                for (int q = 0; q < 4; ++q) values[q][i] = seen ? ld_cache16(row + q * 16) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
             for (int m = 0; m < 8; ++m)

@@ -419,3 +419,21 @@ def test_decode_attention_keeps_its_probabilities_whole(cuda_device, position):
         want = torch.einsum("ht,thd->hd", torch.softmax(torch.einsum("hd,thd->ht", q, k) / 16, -1), v)
         differ, total = differ + int((out != want.bfloat16()).sum()), total + out.numel()
     assert differ < total * 2 ** -10, differ / total
+
+
+@pytest.mark.parametrize("position", [0, 20, 300])
+def test_an_infinite_value_of_the_new_token_stays_infinite(cuda_device, position):
+    """The last chunk of sixteen positions is not full: what its empty places multiply must not be the last row again."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(position)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).bfloat16()
+    keys, values, qg, k_new, v_new = new(position + 1, 2, 256), new(position + 1, 2, 256), new(16, 512), new(2, 256), new(2, 256)
+    v_new[0, 7], v_new[1, 100] = float("inf"), float("-inf")
+    norm, out, counters = torch.zeros(256, dtype=torch.bfloat16, device=cuda_device), new(16, 256), torch.zeros(2, dtype=torch.int32, device=cuda_device)
+    scratch = torch.empty(lib().qd_attn_scratch_floats(16, 2, 256, 74), device=cuda_device)
+    call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(norm), ptr(norm), ptr(keys), ptr(values), ptr(out), ptr(scratch), ptr(counters),
+         None, position, position + 1, 16, 2, 256, 64, 1e6, 1e-6, 74, 0, stream_of(out))
+    infinite = torch.zeros(16, 256, dtype=torch.bool, device=cuda_device)
+    infinite[:8, 7] = infinite[8:, 100] = True
+    assert bool((out[:8, 7] == float("inf")).all()) and bool((out[8:, 100] == float("-inf")).all())
+    assert bool(out[~infinite].isfinite().all())
