@@ -412,6 +412,22 @@ attn_decode_mma_kernel(const AttnParams p) {
                 const float2 v = *reinterpret_cast<const float2*>(src + f);
                 n0 += wgt * v.x; n1 += wgt * v.y; den += wgt * src[D + 1];
             }
+            // A value that is not finite makes NaN of its products with the pieces of a probability (some are zero); what it gives
+            // with the whole probability is summed again, which is slow and next to never needed.
+            if (den < INFINITY && !(fabsf(n0) < INFINITY && fabsf(n1) < INFINITY)) {
+                const bf16* query = reinterpret_cast<const bf16*>(q_s + h * qd::kAttnQRow);
+                n0 = n1 = 0.f;
+#pragma unroll 1
+                for (int pos = t0; pos < t1; ++pos) {
+                    const bf16* key = reinterpret_cast<const bf16*>(kc + (size_t)pos * row_bytes);
+                    const bf16* value = reinterpret_cast<const bf16*>(vc + (size_t)pos * row_bytes) + f;
+                    float score = 0.f;
+#pragma unroll 1
+                    for (int d = 0; d < D; ++d) score = fmaf(ld_bf16(query + d), ld_bf16(key + d), score);
+                    const float w = expf(score * 0.0625f - mm);
+                    n0 = fmaf(w, ld_bf16(value), n0); n1 = fmaf(w, ld_bf16(value + 1), n1);
+                }
+            }
             *reinterpret_cast<float2*>(block_out + (size_t)h * stride + f) = make_float2(n0, n1);
             if (f == 0) *reinterpret_cast<float2*>(block_out + (size_t)h * stride + D) = make_float2(mm, den);
         }
