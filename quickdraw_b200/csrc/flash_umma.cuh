@@ -14,7 +14,7 @@
 // dimension.  Every wait is bounded; a block whose wait ran out writes NaN.
 //
 // Measured (2048 tokens, with the launch gap; before: mma.sync, eight or sixteen rows a warp).  Head dimension 256, 16/2 heads:
-// behind 0 / 2000 / 30000 positions 128 / 223 / 1595 us (478 / 1017 / 7949).  128 columns, window 1024: 16/4
+// behind 0 / 2000 / 30000 positions 129 / 225 / 1611 us (478 / 1017 / 7949).  128 columns, window 1024: 16/4
 // heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 3000 clocks at head dimension 256: 1800 of
 // MMAs (those of S are bound by shared memory, 48 clocks for 64 columns), 1100 of keys and values at 64 bytes a clock, and the
 // hand-over of S and P.
@@ -139,6 +139,39 @@ template <int TILES>
 struct Bars {
     uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[TILES][3], p_full[TILES][3], o_done[TILES][2], q_full, drained;
 };
+
+// Columns `column` .. + 31 of the rows of the warp's lanes `rows` once more, summed in fp32 over the keys that a row sees and no
+// others; a lane's row, `m` and `l` are as for Out.  For results that are not finite although their rows' probabilities are: a value
+// that is not finite makes NaN of its products with the zeros of the keys that a row does not see, and with pieces of a
+// probability that are zero.
+template <int QD, int DV, typename Out>
+__device__ __noinline__ void plain_columns(const In& p, const Out& out, unsigned rows, int row, float m, float l, int column) {
+    const int lane = threadIdx.x & 31, share = p.heads / p.kv_heads, g = blockIdx.x;
+    for (; rows; rows &= rows - 1) {
+        const int from = __ffs(rows) - 1, r = __shfl_sync(0xffffffffu, row, from), head = g * share + r % share;
+        const float reference = __shfl_sync(0xffffffffu, m, from);
+        const int pos = (p.position_ptr ? *p.position_ptr : p.position) + r / share;
+        const bf16* q = p.q + ((size_t)(r / share) * p.heads + head) * QD;
+        const float slope = p.slopes ? p.slopes[head] * 1.4426950408889634f : 0.f;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int j = lowest(p, pos); j <= pos; ++j) {
+            const long long slot = j % p.capacity;
+            const bf16* own = p.k + slot * p.ld_k + g * p.dim;
+            float score = 0.f;
+#pragma unroll 1
+            for (int d = lane; d < QD; d += 32)
+                score = fmaf(ld_bf16(q + d), ld_bf16(d < p.dim ? own + d : p.common + slot * p.ld_common + (d - p.dim)), score);
+            const float w = exp2f(fmaf(warp_sum(score), p.scale, slope * (float)(j - pos)) - reference);
+            sum = fmaf(w, ld_bf16(p.v + slot * p.ld_v + g * DV + column + lane), sum);
+        }
+        float o[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = __shfl_sync(0xffffffffu, sum, e);
+        if (lane == from) out(row / share, head, column, o, m, l);
+        __syncwarp();
+    }
+}
 
 // Out: called per row and 32 columns as out(token, head, c0, o, m, l) with the unnormalised columns c0 .. c0 + 31 and the row's
 // softmax state (log2 of the reference, the sum relative to it); l NaN marks a failed wait.
@@ -397,7 +430,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
             float o[32];
             load32(o_at + c, o);
             loaded(o);
+            bool odd = false;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) odd |= !(fabsf(o[e]) < INFINITY);
             if (row < total) out(row / share, head, c, o, m, l);
+            const unsigned rows = __ballot_sync(0xffffffffu, odd && row < total && l < INFINITY);      // (and the whole warp goes on)
+            if (rows) plain_columns<QD, DV>(p, out, rows, row, m, l, c);
         }
     }
     fence_before();

@@ -109,3 +109,52 @@ def test_chunk_attention_rounds_its_result_only(cuda_device, tokens, position):
     want = plain(q, keys, values, 0.0625, torch.arange(end, device=cuda_device)[None] <= at[:, None])
     error = lambda t: float((t.double() - want).norm() / want.norm())
     assert error(out) < 1.01 * error(want.to(BF16)), (error(out), error(want.to(BF16)))
+
+
+@pytest.mark.parametrize("tokens,position,heads,kv_heads,span,capacity", [
+    (200, 30, 16, 2, 0, 240),           # the gated form, head dimension 256
+    (300, 100, 8, 2, 64, 512),          # a window: masked keys on both sides, whole tiles and partial ones
+    (150, 900, 4, 4, 100, 256),         # ... whose ring wraps
+])
+def test_values_that_are_not_finite_reach_those_who_see_them(cuda_device, tokens, position, heads, kv_heads, span, capacity):
+    """An infinity and a NaN among a chunk's values: rows that do not see their tokens are what they were, the others are infinite or
+    NaN in that column alone."""
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call, call_hybrid, ptr, stream_of
+    dim, end = 128 if span else 256, position + tokens
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).to(BF16)
+    keys, values, q, qg = new(end, kv_heads, dim), new(end, kv_heads, dim), new(tokens, heads, dim), new(tokens, heads, 2, dim)
+
+    def attend(values):
+        out = torch.empty(tokens, heads, dim, dtype=BF16, device=cuda_device)
+        kr, vr = (torch.zeros(capacity, kv_heads, dim, dtype=BF16, device=cuda_device) for _ in range(2))
+        for j in range(max(0, end - capacity), end):
+            kr[j % capacity], vr[j % capacity] = keys[j], values[j]
+        if span:
+            args = AttentionArgs(heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, shared_dim=0, scale=dim ** -0.5, ld_k=kv_heads * dim,
+                                 ld_v=kv_heads * dim, k_cache=ptr(kr), v_cache=ptr(vr), q_rows=ptr(q), out=ptr(out), gate=ptr(q), ld_gate=8, gate_kind=0,
+                                 sink_kind=0, mask=0, span=span, capacity=capacity, position=position, tokens=tokens, dtype=0)
+            call_hybrid("qd_attention", byref(args), stream_of(q))
+        else:
+            norm, rows = torch.zeros(dim, dtype=BF16, device=cuda_device), torch.empty_like(q)
+            fresh = [t[position:].reshape(tokens, -1).contiguous() for t in (keys, values)]
+            call("qd_seq_attention", ptr(qg), *map(ptr, fresh), ptr(norm), ptr(norm), ptr(kr), ptr(vr), ptr(rows), ptr(out), tokens, position,
+                 capacity, heads, kv_heads, dim, 64, 1e6, 1e-6, stream_of(q))
+        return out
+
+    plainly, share = attend(values), heads // kv_heads
+    bad = [(position + 20, 0, 5, float("inf")), (position + tokens - 10, kv_heads - 1, dim - 1, float("nan")), (position + 83, 0, 70, float("-inf"))]
+    want = plainly.clone()
+    for j, g, column, value in bad:
+        values[j, g, column] = value
+        last = min(tokens, j - position + span) if span else tokens
+        want[j - position:last, g * share:(g + 1) * share, column] = value
+    got = attend(values)
+    finite = want.isfinite()
+    # (Sums done again in fp32 may round to the other neighbour, which is a bf16 spacing, at most 2^-7; the gated form rounds twice, the
+    # attended value and its product with the gate: two spacings.  And 2^-17 of the sum of magnitudes.)
+    torch.testing.assert_close(got[finite], want[finite], rtol=2 ** -7 if span else 2 ** -6, atol=2 ** -17 * float(values[values.isfinite()].abs().max()))
+    assert torch.equal(got.isnan(), want.isnan())
+    assert bool((got[~finite & ~want.isnan()] == want[~finite & ~want.isnan()]).all())
