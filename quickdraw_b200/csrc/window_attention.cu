@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const __grid_constant__
                         const float4 v = load4(vs + (size_t)(j + jj) * vdim + tx * 4 + 64 * c);
 #pragma unroll
                         for (int i = 0; i < RM; ++i) {
-                            if (decltype(guarded)::value && w[i][jj] == 0.f) continue;
+                            if (decltype(guarded)::value && (j0 + j + jj > pos_of[i] || j0 + j + jj < lo_of[i])) continue;
                             acc[i][c][0] = fmaf(w[i][jj], v.x, acc[i][c][0]); acc[i][c][1] = fmaf(w[i][jj], v.y, acc[i][c][1]);
                             acc[i][c][2] = fmaf(w[i][jj], v.z, acc[i][c][2]); acc[i][c][3] = fmaf(w[i][jj], v.w, acc[i][c][3]);
                         }

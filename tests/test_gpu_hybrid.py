@@ -519,3 +519,21 @@ def test_gated_linear_attention_in_segments(cuda_device, tokens, heads, dim, vdi
     error = lambda got, exact: float((got - exact).norm() / exact.norm())
     for walk, parts, exact in zip(*runs, (torch.stack(want), s)):
         assert error(parts, exact) <= 1.5 * error(walk, exact) + 1e-7, (error(walk, exact), error(parts, exact))
+
+
+def test_fp32_chunks_keep_the_product_of_a_vanished_probability(cuda_device):
+    """A key that a row sees and whose probability underflows to zero: zero times its infinite value is NaN, as in the sums of a
+    warp per row; rows that do not see it stay finite."""
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call_hybrid, ptr, stream_of
+    tokens, bad, span = 90, 10, 50
+    keys, values, q = (torch.zeros(tokens, 1, 128, device=cuda_device) for _ in range(3))
+    q[:, :, 0], keys[bad, 0, 0], values[bad, 0, 3], out = 1.0, -4000.0, float("inf"), torch.empty_like(q)
+    args = AttentionArgs(heads=1, kv_heads=1, dim=128, vdim=128, shared_dim=0, scale=1.0, ld_k=128, ld_v=128, k_cache=ptr(keys), v_cache=ptr(values),
+                         q_rows=ptr(q), out=ptr(out), gate=None, ld_gate=4, gate_kind=0, sink_kind=0, mask=0, span=span, capacity=tokens, position=0,
+                         tokens=tokens, dtype=1)
+    call_hybrid("qd_attention", byref(args), stream_of(q))
+    want = torch.zeros(tokens, 1, 128, device=cuda_device)
+    want[bad:bad + span, :, 3] = float("nan")
+    assert torch.equal(out.isnan(), want.isnan()) and not bool(out.nan_to_num().any())
