@@ -32,9 +32,8 @@ int qd_linear(const void* x, long long ldx, int x_dtype, const void* w, void* y,
     float eps, unsigned int* status, void* stream);
 
 /* The same for many rows of fp32 x on the tensor cores: x is cut into three bf16 pieces that add up to it exactly, and
- * sums longer than 256 inputs are added in fp32 registers.  planes: 3 * tokens * width bf16 of scratch.  width, ldx, rows
- * and ldy multiples of eight, every address on a 16-byte boundary (QD_ERR_UNSUPPORTED otherwise).  An infinite weight
- * gives NaN where a piece of x is zero. */
+ * the sums of 64 inputs each are added in fp32 registers.  planes: 3 * tokens * width bf16 of scratch.  width, ldx, rows
+ * and ldy multiples of eight, every address on a 16-byte boundary (QD_ERR_UNSUPPORTED otherwise). */
 int qd_linear_pieces(const float* x, long long ldx, const void* w, void* y, long long ldy, int y_dtype, int tokens, int
     rows, int width, int gelu_cols, int glu, const float* bias, int add, void* planes, unsigned int* status, void* stream);
 

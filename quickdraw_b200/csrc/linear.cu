@@ -221,7 +221,13 @@ QD_DEVINL void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-struct LinearParams { void* y; long long ldy; int tokens, rows, width; Finish f; unsigned int* status; };
+struct LinearParams {
+    void* y; long long ldy;
+    int tokens, rows, width;
+    Finish f;
+    unsigned int* status;
+    const float* x; long long ldx; const bf16* w;      // (fp32 rows in pieces: for sums that are not finite)
+};
 
 // Eight neighbouring sums of a token, the first of them output n: what follows them, and the store.  bias: of these outputs,
 // in shared memory (read where there is one).
@@ -403,6 +409,26 @@ template <int TN> struct PieceTile {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 5) * 8 + 16 + 1024;
 };
 
+// The sums of outputs n .. n + 7 of token t, product by product.  An infinite weight makes NaN of its products with the pieces of x
+// that are zero (those of 1.0 are: one infinity, two zeros times infinity), so sums that are not finite are formed again.
+struct Eight { float v[8]; };
+__device__ __noinline__ Eight plain_sums(const LinearParams& p, int t, int n) {
+    Eight r;
+    const float* x = p.x + t * p.ldx;
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+        const bf16* w = p.w + (long long)(n + q) * p.width;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < p.width && sum == sum; k += 4) {          // (NaN stays NaN; width is a multiple of eight)
+            const float4 a = load4(x + k), b = load4(w + k);
+            sum = fmaf(a.x, b.x, sum); sum = fmaf(a.y, b.y, sum); sum = fmaf(a.z, b.z, sum); sum = fmaf(a.w, b.w, sum);
+        }
+        r.v[q] = sum;
+    }
+    return r;
+}
+
 template <typename TY, int TN>
 __global__ void __launch_bounds__(PieceTile<TN>::kThreads, 1)
 linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap) {
@@ -511,6 +537,15 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
                     float f[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) f[q] = acc[c + q];
+                    bool odd = false;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) odd |= !(fabsf(f[q]) < INFINITY);
+                    if (odd) {
+                        const Eight plain = plain_sums(p, t, n);
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (!(fabsf(f[q]) < INFINITY)) f[q] = plain.v[q];
+                    }
                     finish8(p, f, row, n, bias + half * kHalf + c);
                 }
             }
@@ -711,7 +746,7 @@ extern "C" int qd_linear_pieces(const float* x, long long ldx, const void* w, vo
     QD_CHECK_ARG(ldy >= (glu ? rows / 2 : rows) && (!glu || (rows % 2 == 0 && gelu_cols == 0 && !add)));
     if (width % 8 || ldx % 8 || rows % 8 || ldy % 8 || !qd::aligned16(x) || !qd::aligned16(w) || !qd::aligned16(y) || !qd::aligned16(planes))
         return QD_ERR_UNSUPPORTED;
-    const qd::LinearParams p = {y, ldy, tokens, rows, width, {bias, gelu_cols, glu, add}, status};
+    const qd::LinearParams p = {y, ldy, tokens, rows, width, {bias, gelu_cols, glu, add}, status, x, ldx, (const bf16*)w};
     if (y_dtype == QD_F32) return qd::pieces_dispatch<float>(x, ldx, w, p, (bf16*)planes, (cudaStream_t)stream);
     if (y_dtype == QD_BF16) return qd::pieces_dispatch<bf16>(x, ldx, w, p, (bf16*)planes, (cudaStream_t)stream);
     return QD_ERR_UNSUPPORTED;

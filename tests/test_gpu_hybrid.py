@@ -537,3 +537,18 @@ def test_fp32_chunks_keep_the_product_of_a_vanished_probability(cuda_device):
     want = torch.zeros(tokens, 1, 128, device=cuda_device)
     want[bad:bad + span, :, 3] = float("nan")
     assert torch.equal(out.isnan(), want.isnan()) and not bool(out.nan_to_num().any())
+
+
+@pytest.mark.parametrize("tokens,rows,width", [(9, 64, 64), (200, 136, 520)])
+@pytest.mark.parametrize("add", [False, True])
+def test_fp32_rows_with_infinite_weights(M, tokens, rows, width, add):
+    """Infinite and NaN weights under x whose lower pieces are zero (whole numbers) and not: plain products and sums, an infinity
+    where there is one and NaN where two meet or a zero of x meets one."""
+    w, x, stat = bf(rows, width, seed=2), rnd(tokens, width, seed=1), status()
+    x[:4] = x[:4].round()
+    x[1, 5], x[2] = 0.0, 1.0
+    w[3, 5], w[17, 8], w[17, 60], w[40, 9] = float("inf"), float("-inf"), float("-inf"), float("nan")
+    out = rnd(tokens, rows, seed=5).cuda()
+    want = (torch.zeros_like(out) if not add else out).double().cpu() + sum(x[:, None, k].double() * w[None, :, k].double() for k in range(width))
+    M.linear(x.cuda(), 0, width, w.cuda(), out, tokens=tokens, status=stat, add=add)
+    torch.testing.assert_close(out.cpu().double(), want, rtol=1e-5, atol=1e-4, equal_nan=True)
