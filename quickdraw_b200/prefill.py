@@ -168,7 +168,8 @@ class ChunkPrefill:
         return (routes > self.TILES_FROM * (self.total_experts or experts) and gate.weight.shape == up.weight.shape and experts <= 1024
                 and gate.group_size == up.group_size == down.group_size == 16 and gate.in_features % 256 == 0 and gate.out_features % 128 == 0
                 and down.in_features % 256 == 0 and down.out_features % 256 == 0
-                and (gate.weight_scale_2.numel() == 1) == (up.weight_scale_2.numel() == 1))
+                and (gate.weight_scale_2.numel() == 1) == (up.weight_scale_2.numel() == 1)
+                and all(t.data_ptr() % 16 == 0 for bank in (gate, up, down) for t in (bank.weight, bank.weight_scale)))
 
     def _expert_swiglu(self, x, gate, up, order, boundaries, routes, topk):
         """The SwiGLU of the routed gate and up products, rows in sorted order."""

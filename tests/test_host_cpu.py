@@ -383,3 +383,26 @@ def test_a_wait_that_ran_out_leaves_nothing_in_flight():
         assert re.search(r"commit\w*\(&?(?:bars->)?drained\);[^\n]*\n\s*mbar_wait\(&?(?:bars->)?drained, 0", body), name
     loaders = (csrc / "flash_umma.cuh").read_text()
     assert re.search(r"\n        if \(issued >= 0\) mbar_wait\(full, \(issued >> 1\) & 1, nullptr\);", loaders)
+
+
+def test_banks_off_a_16_byte_boundary_keep_the_form_that_takes_them():
+    """The launch of gate, up and SwiGLU refuses such addresses, the grouped product does not: a chunk goes the second way then."""
+    from types import SimpleNamespace
+
+    from quickdraw_b200.prefill import ChunkPrefill
+    from quickdraw_b200.weights import NVFP4Linear
+    prefill = ChunkPrefill.__new__(ChunkPrefill)
+    prefill.total_experts = 64
+
+    def bank(rows, width, shift="", by=8):
+        def part(name, *shape):
+            count = torch.Size(shape).numel()
+            flat = torch.zeros(count + by, dtype=torch.uint8)
+            return (flat[by:] if name == shift else flat[:count]).view(shape)
+        return NVFP4Linear(part("codes", 64, rows, width // 2), part("scales", 64, rows, width // 16), torch.ones(()))
+
+    plain = {"experts_gate": bank(512, 256), "experts_up": bank(512, 256), "experts_down": bank(256, 512)}
+    assert prefill._tiles_form(64 * 64, SimpleNamespace(**plain))
+    for name, b in plain.items():
+        for shift in ("codes", "scales"):
+            assert not prefill._tiles_form(64 * 64, SimpleNamespace(**{**plain, name: bank(b.out_features, b.in_features, shift)})), (name, shift)
