@@ -39,12 +39,9 @@ class ChunkPrefill:
     CHUNKED_FROM = 64                                     # tokens from which the DeltaNet recurrence takes the chunked form
     FEW_TOKENS = 32                                       # token rows up to which a dense product takes the mma.sync form
     ROUTES_PER_PASS = 0                                   # 8 / 32 routes per decoding of a weight tile; 0: the library chooses
-    FEW_ROWS = 20                                         # mean routes per expert up to which the mma.sync form is used
-
-    TILES_FROM = 5                                        # mean routes per expert from which gate, up and SwiGLU are one launch over
-                                                          # weights decoded into tensor memory (256 experts of 512 x 2048, all three
-                                                          # banks: 4 routes 176 against 166 us of the mma.sync form, 8 routes 180
-                                                          # against 217, 16 routes 182 against 297)
+    FEW_ROWS = 20                                         # mean routes per expert up to which the mma.sync form is used, for banks
+                                                          # and counts that _tiles_form does not take
+    TILES_FROM, SMALL_BANK = 5, 2 ** 25                   # see _tiles_form
 
     def __init__(self, ckpt: Checkpoint, expert_range: tuple[int, int] | None = None, group=None):
         c = ckpt.config
@@ -163,9 +160,16 @@ class ChunkPrefill:
                 and bank.out_features % 16 == 0)
 
     def _tiles_form(self, routes, w):
+        """Whether gate, up and SwiGLU of the routed experts are one launch over weights decoded into tensor memory.  That form takes
+        the same 20 to 25 us for any small bank and reads each weight once; the mma.sync form grows with the weights times the
+        passes of eight routes.  All three products, mma.sync against tensor memory, mean routes an expert: 256 experts of 2048 x
+        512 4 routes 166 / 176 us, 8 routes 217 / 180; 64 of 2048 x 512 6 routes 56.8 / 57.2, 8 routes 63 / 57; 32 of 2048 x 512 6
+        routes 35.2 / 35.8, 8 routes 38.4 / 35.8; 16 of 2048 x 512 12 routes 26.7 / 33.1; 16 of 1024 x 512 8 routes 19.5 / 23.9, 20
+        routes 24.7 / 26.4.  Above 20 routes the alternative is 128-token tiles, slower everywhere (16 of 1024 x 512 24 routes 42 / 28)."""
         gate, up, down = w.experts_gate, w.experts_up, w.experts_down
-        experts = gate.weight.shape[0]
-        return (routes > self.TILES_FROM * (self.total_experts or experts) and gate.weight.shape == up.weight.shape and experts <= 1024
+        experts, weights = gate.weight.shape[0], 2 * gate.weight.numel()
+        above = self.FEW_ROWS if weights < self.SMALL_BANK else self.TILES_FROM + 2 * self.SMALL_BANK / weights
+        return (routes > above * (self.total_experts or experts) and gate.weight.shape == up.weight.shape and experts <= 1024
                 and gate.group_size == up.group_size == down.group_size == 16 and gate.in_features % 256 == 0 and gate.out_features % 128 == 0
                 and down.in_features % 256 == 0 and down.out_features % 256 == 0
                 and (gate.weight_scale_2.numel() == 1) == (up.weight_scale_2.numel() == 1)

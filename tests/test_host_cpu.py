@@ -406,3 +406,20 @@ def test_banks_off_a_16_byte_boundary_keep_the_form_that_takes_them():
     for name, b in plain.items():
         for shift in ("codes", "scales"):
             assert not prefill._tiles_form(64 * 64, SimpleNamespace(**{**plain, name: bank(b.out_features, b.in_features, shift)})), (name, shift)
+
+
+def test_small_expert_banks_keep_the_few_rows_form():
+    """Where the launch of gate, up and SwiGLU was measured to be the slower one, and where it was the faster."""
+    from types import SimpleNamespace
+
+    from quickdraw_b200.prefill import ChunkPrefill
+    from quickdraw_b200.weights import NVFP4Linear
+    prefill = ChunkPrefill.__new__(ChunkPrefill)
+    for experts, hidden, inner, slower, faster in ((16, 1024, 512, (6, 12, 20), (21, 200)), (16, 2048, 512, (8, 12), (24,)), (32, 2048, 512, (4, 6), (8, 40)),
+                                                   (64, 2048, 512, (4, 6), (8, 20)), (256, 2048, 512, (4,), (6, 8, 64))):
+        bank = lambda rows, width: NVFP4Linear(torch.empty(experts, rows, width // 2, dtype=torch.uint8),
+                                               torch.empty(experts, rows, width // 16, dtype=torch.uint8), torch.ones(()))
+        w = SimpleNamespace(experts_gate=bank(inner, hidden), experts_up=bank(inner, hidden), experts_down=bank(hidden, inner))
+        prefill.total_experts = experts
+        assert not any(prefill._tiles_form(n * experts, w) for n in slower), (experts, hidden)
+        assert all(prefill._tiles_form(n * experts, w) for n in faster), (experts, hidden)
