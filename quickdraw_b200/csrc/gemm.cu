@@ -500,6 +500,25 @@ extern "C" int qd_nvfp4_matmul(const void* x, const void* codes, const void* sca
     return launch_gemm<true, 256>(p, row_tiles, row_tiles, (cudaStream_t)stream);
 }
 
+// Whether a grouped product is faster with its weights decoded into tensor memory (expert_tiles.cu) than in the tiles above, where
+// both take it; `mean` routes an expert.  Measured (tiles above | tensor memory, us): 256 experts of 2048 x 512, mean 16 / 64 / 256:
+// 145 | 68, 172 | 98, 481 | 295; 64 of 2048 x 512 mean 4 / 64 / 512: 35 | 21, 46 | 30, 175 | 148; 8 of 4096 x 4096 mean 8 / 1024: 79 | 40,
+// 572 | 356; 16 of 1024 x 512 mean 12 / 64 / 256: 10.2 | 9.9, 13.6 | 13.1, 25 | 19.  Two exceptions:
+//   - a bank that its few items, 256 weight rows each, leave most SMs without, unless there are many routes: 8 of 1024 x 512 mean 24 / 64 / 96:
+//     8.9 | 10.8, 11.0 | 12.9, 10.3 | 11.9, mean 256: 22 | 13; 4 of 1024 x 512 mean 64 / 160: 8.6 | 12.5, 11.7 | 12.5;
+//   - items of at most 80 routes that fill the SMs once and a bit more: 160 items, mean 160: 8 of 2048 x 2048 32 | 38, 32 of 512 x 2048
+//     35 | 39.5, 16 of 1024 x 512 15.6 | 18.0; 128 and 256 items (mean 96 and 256): 26 | 22 and 63 | 38, 29 | 25 and 58 | 40.
+static bool tiles_pay(int routes, int experts, int out_features, int in_features) {
+    if ((long long)experts * out_features * in_features <= 1ll << 22 && routes <= 1280) return false;
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 148;
+    const double mean = (double)routes / experts;
+    const double items = (mean + 40) / 80 * experts * (out_features / 256);         // the parts of an expert: its routes spread around the mean
+    return mean <= 64 || items <= sms || items > 1.25 * sms;
+}
+
 // grouped_matmul(x, bank, grouping, routing=None) — quickdraw/kernel/triton/moe.py:99-151: the
 // routes (token, slot) of a chunk sorted by expert; every expert's rows go through that
 // expert's matrix.  by_token: input row = order[r] / topk (gate, up), else the sorted row r
@@ -517,9 +536,7 @@ extern "C" int qd_nvfp4_grouped_matmul(const void* x, const void* codes, const v
     if (group_size != 16 || in_features % kTileK != 0 || out_features % 8 != 0) return QD_ERR_UNSUPPORTED;
     const uintptr_t align = (uintptr_t)x | (uintptr_t)codes | (uintptr_t)y;
     if (align & 15u) return QD_ERR_UNSUPPORTED;
-    // Decoded weights in tensor memory wherever the sizes fit: down bank of 256 x 2048 x 512, 16 / 64 / 256 routes an expert:
-    // 68 / 98 / 295 us against 145 / 172 / 481 us of the tiles below, and never slower from two tokens on.
-    if (qd::expert_tiles_cover(experts, out_features, in_features, 256, x, codes, scales))
+    if (qd::expert_tiles_cover(experts, out_features, in_features, 256, x, codes, scales) && tiles_pay(routes, experts, out_features, in_features))
         return qd::expert_tiles_matmul({x, codes, scales, global, order, boundaries, routing, (bf16*)y, routes, experts, topk, out_features,
                                         in_features, by_token, scatter, global_per_expert, status}, (cudaStream_t)stream);
     GemmParams p = {};

@@ -85,7 +85,7 @@ def test_fp8_mixer_blocks_of_a_chunk_match_the_oracle(cuda_device):
 @pytest.mark.parametrize("experts,topk,tokens,width,rows,few_rows", [
     (8, 3, 21, 512, 264, 0),       # few tiles: 64-row weight tiles
     (40, 2, 30, 256, 256, 0),      # 128-row weight tiles
-    (64, 2, 40, 256, 768, 0),      # every SM busy: 256-row (or balanced 128-row) weight tiles
+    (64, 2, 40, 256, 768, 0),      # weights decoded into tensor memory
     (8, 3, 21, 512, 272, 32),      # the few-rows form: up to eight routes per expert, a ragged last weight tile
     (4, 2, 50, 2048, 512, 32),     # ... 25 routes per expert: four groups of eight, the last one with a single route
     (40, 8, 3, 512, 2048, 32),     # ... most experts without a route
@@ -299,3 +299,45 @@ def test_expert_tiles_at_the_edges_of_an_item(cuda_device, counts, width, inner)
         torch.testing.assert_close(h[rows], a * torch.sigmoid(a) * b, rtol=4 * tol, atol=tol * float(a.abs().max() * b.abs().max()) * 2 ** -4)
         want = x[rows].double() @ matrix(out_bank, e).T * weights[order[rows].long()].double()[:, None]
         torch.testing.assert_close(y[order[rows].long()], want, rtol=3.1 * tol, atol=1e-5 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("counts,width,rows", [
+    # sizes that the form with weights in tensor memory refuses, a weight tile of ...
+    ((5, 0, 9), 320, 264),                                # 64 rows, 128-token tiles
+    ((2, 0) * 30, 320, 384),                              # 128 rows
+    ((3,) * 64, 320, 776),                                # 256 rows
+    ((130, 0, 70, 257), 320, 264),                        # 64 rows, 256-token tiles
+    ((100, 300, 1), 320, 3080),                           # 128 rows
+    ((70,) * 10, 320, 3848),                              # 256 rows
+    # sizes that it takes: a small bank and a few SMs more than once over go to the tiles, the others do not
+    ((80, 81, 3), 256, 512), ((160,) * 8, 512, 2048),
+    ((1,) + (0,) * 19, 1024, 512), ((80, 81, 0, 160, 161, 1, 240), 2048, 512), ((33, 70, 96), 2048, 1024),
+])
+def test_grouped_product_in_every_tile_shape(cuda_device, counts, width, rows):
+    """Bounds: exact products, fp32 sums, one bf16 rounding of the result (2^-8); of sum, factor and result in the routed
+    product (three)."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    from quickdraw_b200.synthetic import to_device
+    experts, routes = len(counts), sum(counts)
+    src = synthetic.Source(23, "cpu")
+    bank = src.nvfp4("bank", rows, width, experts, global_scale=0.5, per_expert_global=True)
+    b, x = to_device(bank, cuda_device), src.normal("x", routes, width).to(cuda_device)
+    gen = torch.Generator().manual_seed(routes)
+    order = torch.randperm(routes, generator=gen).to(torch.int32).to(cuda_device)
+    weights = torch.rand(routes, generator=gen).to(cuda_device)
+    edges = [0, *torch.tensor(counts).cumsum(0).tolist()]
+    bounds, status = torch.tensor(edges, dtype=torch.int32, device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    plain, routed = (torch.full((routes, rows), float("nan"), dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    for y, factor, by_token, scatter in ((plain, None, 1, 0), (routed, weights, 0, 1)):
+        call("qd_nvfp4_grouped_matmul", ptr(x), ptr(b.weight), ptr(b.weight_scale), ptr(b.weight_scale_2), ptr(order), ptr(bounds), ptr(factor), ptr(y),
+             routes, experts, 1, rows, width, 16, by_token, scatter, 1, max(counts), ptr(status), stream_of(x))
+    assert int(status.item()) == 0
+    for e in range(experts):
+        here = slice(edges[e], edges[e + 1])
+        if not counts[e]:
+            continue
+        matrix, at = O.dequantize_fp32(O.expert_view(bank, e)).to(cuda_device).double(), order[here].long()
+        want = x[at].double() @ matrix.T
+        torch.testing.assert_close(plain[here].double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+        want = x[here].double() @ matrix.T * weights[at].double()[:, None]
+        torch.testing.assert_close(routed[at].double(), want, rtol=3.1 * 2 ** -8, atol=1e-5 * float(want.abs().max()))
