@@ -84,13 +84,13 @@ def ring_segments(first: int, count: int, capacity: int) -> list[tuple[int, int]
     return [(row, head)] + ([(0, count - head)] if count > head else [])
 
 
-def gla_span(tokens: int, blocks: int) -> int:
+def gla_span(tokens: int, blocks: int, sms: int) -> int:
     """Tokens of a segment of gated linear attention, 0: the chunk as a whole.  The whole chunk keeps ``blocks`` SMs busy and a
     segment is walked twice, so there is nothing to gain once they are half of the SMs; three blocks to an SM take all there
     is, and segments below 80 tokens cost more states than they save (heads of 128: 16 heads 400 / 777 / 2048 tokens 92 / 170 /
     437 -> 73 / 111 / 235 us, 4 heads 2048 tokens 427 -> 93 us; 32 heads 438 -> 413, not taken)."""
-    count = min(tokens // 80, 3 * 148 // blocks)
-    return -(-tokens // count // 16) * 16 if count >= 3 and 2 * blocks <= 148 else 0
+    count = min(tokens // 80, 3 * sms // blocks)
+    return -(-tokens // count // 16) * 16 if count >= 3 and 2 * blocks <= sms else 0
 
 
 def step_covers(m) -> bool:
@@ -250,7 +250,7 @@ class LinearRecurrence:
     def _walk(self, q, k, decay, v, beta, scales, history, gate, gate_column: int, act: int, dtype):
         m, tokens = self.m, q.shape[0]
         raw = torch.empty((tokens, self.out_columns), dtype=F32, device=q.device)
-        span = 0 if beta is not None else gla_span(tokens, m.heads * -(-m.vdim // 32))
+        span = 0 if beta is not None else gla_span(tokens, m.heads * -(-m.vdim // 32), self.sms)
         if span:
             scratch = torch.empty(-(-tokens // span) * m.heads * m.dim * (m.vdim + 1), dtype=F32, device=q.device)
             call_hybrid("qd_gla_segments", ptr(q), ptr(k), ptr(decay), ptr(v), ptr(history.rec), ptr(raw), tokens, m.heads, self.kv_heads, m.dim, m.vdim,
@@ -267,6 +267,7 @@ class LinearRecurrence:
 class GatedLinearAttention(LinearRecurrence):
     def __init__(self, weights: GLAWeights, m: GLAConfig, eps: float, device):
         super().__init__(weights, m, eps, m.heads)
+        self.sms = torch.cuda.get_device_properties(device).multi_processor_count
         self.projections = {"q": weights.q, "k": weights.k, "v": weights.v, "g": weights.g, "a1": weights.a1}
 
     def chunk(self, proj, at, history: LayerHistory, position, status):

@@ -298,3 +298,13 @@ def test_replay_refuses_a_number_format_the_design_does_not_have(monkeypatch, tm
     (tmp_path / "config.json").write_text(json.dumps({"text_config": {}}))
     monkeypatch.setattr(sys, "argv", ["trace_run", "--model", str(tmp_path), "--dtype", "float32", "--out", str(tmp_path)])
     assert replay.main() == 3
+
+
+def test_segments_of_gated_linear_attention_follow_the_device():
+    """A chunk goes in segments where its blocks leave half of the SMs idle, at most three blocks to an SM: of the device at hand."""
+    assert mixers.gla_span(2048, 64, 148) == 352 and mixers.gla_span(2048, 64, 100) == 0 and mixers.gla_span(2048, 16, 148) == 96
+    assert mixers.gla_span(2048, 16, 64) == 176 and mixers.gla_span(239, 16, 148) == 0 and mixers.gla_span(240, 16, 148) == 80
+    for tokens in range(240, 700, 7):
+        for blocks in (1, 7, 33, 74):
+            span = mixers.gla_span(tokens, blocks, 148)
+            assert span == 0 or (span % 16 == 0 and -(-tokens // span) * blocks <= 3 * 148)
