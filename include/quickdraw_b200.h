@@ -328,7 +328,9 @@ int qd_gdn_gated_norm(const void* o, const void* z, const void* gamma, void* out
  * [capacity, kv_heads, head_dim]; out [q_heads*head_dim].  position_dev (int32 device scalar)
  * overrides position_host when not NULL.  scratch: qd_attn_scratch_floats() floats;
  * counters: kv_heads zeroed uint32 (the kernel leaves them zero).  head_dim <= 256,
- * q_heads / kv_heads <= 8. */
+ * q_heads / kv_heads <= 8.  pdl: 0 an ordinary launch, 3 a programmatic dependent of the kernel before it in the
+ * stream but an ordinary launch while the stream is captured, any other value a dependent always; dependents
+ * become ordinary launches where qd_set_chained_launches(0) holds. */
 int qd_attn_scratch_floats(int q_heads, int kv_heads, int head_dim, int splits);
 int qd_attn_decode(const void* qg, const void* k_new, const void* v_new, const void* q_norm,
                    const void* k_norm, void* k_cache, void* v_cache, void* out, float* scratch,
@@ -360,7 +362,7 @@ int qd_attn_decode_static(const void* qg, const void* k_new, const void* v_new, 
  * shared down + _reduce in one launch).  hidden [topk+1, 512] (last row: shared expert).
  * Either `out` (combined bf16 [hidden_size]) or, for expert parallelism, `routed_out`
  * (fp32 partial sum over the experts in [expert_lo, expert_hi), bank pointers local to that
- * range) with `shared_out` (gated shared row); qd_moe_finish adds them after the all-reduce. */
+ * range) with `shared_out` (gated shared row); qd_moe_finish adds them after the all-reduce.  pdl as in qd_attn_decode. */
 int qd_moe_down_combine(const void* hidden, const int32_t* ids, const float* weights,
                         const void* down_codes, const void* down_scales, const float* down_global,
                         const void* shared_codes, const void* shared_scales, const float* shared_global,

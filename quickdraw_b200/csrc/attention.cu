@@ -529,7 +529,7 @@ extern "C" int qd_attn_decode(const void* qg, const void* k_new, const void* v_n
     p.partial = scratch; p.counters = counters; p.position_dev = position_dev; p.position_host = position_host;
     p.capacity = capacity; p.hq = q_heads; p.hk = kv_heads; p.d = head_dim; p.rotary = rotary_dim;
     p.theta = theta; p.eps = eps; p.splits = splits; p.cache_stride = 0;
-    return launch_attn(p, 1, pdl, (cudaStream_t)stream);
+    return launch_attn(p, 1, launch_mode(pdl), (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------- batched form

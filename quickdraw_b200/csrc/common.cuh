@@ -200,6 +200,8 @@ inline int& qd_chain_switch() { static int on = 1; return on; }
 // the stream.  pdl: 0 = ordinary launch, 1 = dependent unless chained launches are switched off,
 // 2 = always dependent (a kernel that fetches weights before its wait), 3 = as 1 but ordinary while the stream is captured
 // (the operator table: 17 launches of a layer's blocks 182 -> 170 us, where a graph's programmatic edges cost more than they give).
+// The pdl argument of an entry point: 0, 3, and any other value for 1.
+static inline int launch_mode(int pdl) { return pdl == 3 ? 3 : pdl != 0; }
 template <typename... KArgs, typename... Args>
 static inline int qd_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                             cudaStream_t stream, int pdl, Args... args) {

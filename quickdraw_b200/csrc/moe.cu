@@ -202,7 +202,7 @@ extern "C" int qd_moe_down_combine(const void* hidden, const int32_t* ids, const
             return QD_ERR_LAUNCH;
         configured[device] = true;
     }
-    return qd_launch(moe_down_kernel, dim3(grid), dim3(kDownThreads), smem, (cudaStream_t)stream, pdl, p);
+    return qd_launch(moe_down_kernel, dim3(grid), dim3(kDownThreads), smem, (cudaStream_t)stream, launch_mode(pdl), p);
 }
 
 extern "C" int qd_moe_finish(const float* routed, const void* shared, void* out, int n, int pdl, void* stream) {

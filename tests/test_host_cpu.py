@@ -423,3 +423,14 @@ def test_small_expert_banks_keep_the_few_rows_form():
         prefill.total_experts = experts
         assert not any(prefill._tiles_form(n * experts, w) for n in slower), (experts, hidden)
         assert all(prefill._tiles_form(n * experts, w) for n in faster), (experts, hidden)
+
+
+def test_launch_modes_of_the_entry_points():
+    """Any value but 0 asked for a dependent launch before the third mode existed, and still does: no other value of a caller
+    reaches the launch helper's modes of its own."""
+    csrc = ROOT / "quickdraw_b200" / "csrc"
+    assert "{ return pdl == 3 ? 3 : pdl != 0; }" in (csrc / "common.cuh").read_text()
+    for name in ("attention.cu", "moe.cu", "gdn.cu", "step.cu", "ops.cu"):
+        text = (csrc / name).read_text()
+        for entry in re.finditer(r'extern "C" int qd_\w+\([^)]*\bint pdl\b[^)]*\) \{(.*?)\n\}', text, flags=re.S):
+            assert re.search(r"pdl != 0|launch_mode\(pdl\)", entry.group(1)) and not re.search(r"[ (]pdl[,)] *(?!!)", entry.group(1).replace("launch_mode(pdl)", "")), name
