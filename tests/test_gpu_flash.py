@@ -158,3 +158,38 @@ def test_values_that_are_not_finite_reach_those_who_see_them(cuda_device, tokens
     torch.testing.assert_close(got[finite], want[finite], rtol=2 ** -7 if span else 2 ** -6, atol=2 ** -17 * float(values[values.isfinite()].abs().max()))
     assert torch.equal(got.isnan(), want.isnan())
     assert bool((got[~finite & ~want.isnan()] == want[~finite & ~want.isnan()]).all())
+
+
+@pytest.mark.parametrize("dim,shared,heads,kv_heads,wider,tokens,position,span,capacity", [
+    (96, 32, 8, 2, 0, 90, 10, 50, 256),           # shared columns inside a box of 64: rows copied one by one
+    (136, 56, 4, 4, 8, 70, 0, 300, 300),          # ... and rows wider than their heads
+    (64, 128, 6, 2, 64, 200, 100, 70, 320),       # shared columns in boxes of their own
+    (128, 0, 8, 2, 24, 300, 500, 128, 512),       # wider rows through boxes
+    (128, 64, 4, 1, 0, 20, 33, 20, 40),           # a ring below a tile
+    (192, 0, 2, 2, 0, 33, 7, 64, 100),
+])
+def test_forms_of_rows_that_a_chunk_may_have(cuda_device, dim, shared, heads, kv_heads, wider, tokens, position, span, capacity):
+    """Every split of the key columns between a head's own and shared ones, strides, rings: what the dispatch takes to tcgen05."""
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call_hybrid, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(dim)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).to(BF16)
+    end = position + tokens
+    keys, values, common, q = new(end, kv_heads, dim), new(end, kv_heads, 128), new(end, shared), new(tokens, heads, dim + shared)
+    rings = []
+    for rows in (keys, values, common):
+        flat = rows.reshape(end, -1)
+        ring = torch.full((capacity, flat.shape[1] + wider), float("nan"), dtype=BF16, device=cuda_device)
+        for j in range(max(0, end - capacity), end):
+            ring[j % capacity, :flat.shape[1]] = flat[j]
+        rings.append(ring)
+    out = torch.empty(tokens, heads, 128, dtype=BF16, device=cuda_device)
+    scale = (dim + shared) ** -0.5
+    args = AttentionArgs(heads=heads, kv_heads=kv_heads, dim=dim, vdim=128, shared_dim=shared, scale=scale, ld_k=rings[0].shape[1], ld_v=rings[1].shape[1],
+                         ld_shared=rings[2].shape[1], k_cache=ptr(rings[0]), v_cache=ptr(rings[1]), k_shared=ptr(rings[2]) if shared else None,
+                         q_rows=ptr(q), out=ptr(out), gate=None, ld_gate=8, gate_kind=0, sink_kind=0, mask=0, span=span, capacity=capacity,
+                         position=position, tokens=tokens, dtype=0)
+    call_hybrid("qd_attention", byref(args), stream_of(q))
+    at, j = torch.arange(position, end, device=cuda_device)[:, None], torch.arange(end, device=cuda_device)[None]
+    close(out, plain(q, torch.cat([keys, common[:, None].expand(-1, kv_heads, -1)], -1), values, scale, (j <= at) & (j > at - span)), 1.5)
