@@ -434,3 +434,11 @@ def test_launch_modes_of_the_entry_points():
         text = (csrc / name).read_text()
         for entry in re.finditer(r'extern "C" int qd_\w+\([^)]*\bint pdl\b[^)]*\) \{(.*?)\n\}', text, flags=re.S):
             assert re.search(r"pdl != 0|launch_mode\(pdl\)", entry.group(1)) and not re.search(r"[ (]pdl[,)] *(?!!)", entry.group(1).replace("launch_mode(pdl)", "")), name
+
+
+def test_splits_of_the_decode_attention_follow_the_form_that_is_taken():
+    from quickdraw_b200.kernels import _attn_splits
+    cache = torch.zeros(4 * 2 * 256 + 4, dtype=torch.bfloat16)
+    whole, shifted = cache[:2048].view(4, 2, 256), cache[4:2052].view(4, 2, 256)
+    assert [_attn_splits(256, r, whole, whole) for r in (0, 64, 256, 32, 96)] == [74, 74, 74, 32, 32]
+    assert _attn_splits(128, 64, whole, whole) == 32 and _attn_splits(256, 64, whole, shifted) == 32
