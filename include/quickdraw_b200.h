@@ -286,7 +286,7 @@ int qd_fp8_gemv(const void* x, const void* w, const float* w_scale, const float*
  * prompt chunks go through fp8_gemv row by row): activations quantised once to E4M3 bytes
  * (q_scratch: tokens * in_features bytes, 16-byte aligned; convert = 0 reuses what the previous call
  * left there, for projections that share input and input scale), E4M3 x E4M3 products on
- * mma.sync.m16n8k32, fp32 sum, y = bf16((sum * in_scale) * w_scale).  in_features % 128 == 0,
+ * tcgen05.mma kind::f8f6f4, fp32 sum, y = bf16((sum * in_scale) * w_scale).  in_features % 128 == 0,
  * out_features even, else QD_ERR_UNSUPPORTED. */
 int qd_fp8_matmul(const void* x, const void* w, const float* w_scale, const float* in_scale, void* y,
                   int tokens, int out_features, int in_features, void* q_scratch, int convert, void* stream);

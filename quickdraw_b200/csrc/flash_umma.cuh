@@ -5,7 +5,8 @@
 // tiles of 64.  Per tile and 128 rows: S = Q K^T (both from shared memory), a thread per row takes the softmax in registers,
 // P goes over S as two bf16 pieces (sixteen bits), O += P V.  The result is rescaled only when a row's maximum
 // has grown by more than 2^8 since the last time (P stays below 2^8 and the sum in fp32, so the quotient is the same to
-// rounding): after the first tiles a warp hardly ever reads O before the end.
+// rounding): after the first tiles a warp hardly ever reads O before the end.  (Conditional rescaling is published with
+// FlashAttention-4.)
 //   warps 0 .. 4 TILES - 1   softmax, one row a thread; then the epilogue
 //   warp 4 TILES             issues the MMAs: S of tile i + 1 before O of tile i, so that the softmax and the products overlap
 //   the rest                 keys and values into the 128-byte swizzled layout, two stages of each: by tiled TMA where a tile's 64

@@ -364,7 +364,8 @@ linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant
 
 // ------------------------------------------------------------------ fp32 rows on the tensor cores
 // x = h + m + l with three bf16 pieces of eight significant bits each, cut off and not rounded, so that the three together
-// are x to the last bit (and a piece cannot overflow).  The weights are bf16, every product of a piece and a weight is exact
+// are x to the last bit (below 2^-110, to 2^-133; and a piece cannot overflow).  Splitting fp32 into three bf16 values is
+// published (Henry, Tang and Heinecke, 2019).  The weights are bf16, every product of a piece and a weight is exact
 // in fp32, and what is left to rounding is the order of the sums.  The tensor core adds into its accumulator without
 // rounding to nearest, which over a long sum pulls the result towards zero; so an accumulator takes kSegment inputs at most
 // and the segments are added in registers, rounded to nearest: two accumulators, one filled while the other is read.

@@ -10,8 +10,8 @@
 // Prompt chunks: attn_prepare_kernel (norm, rotation, ring rows), then flash_umma.cuh for heads of 128 value and 128 or 192 key
 // columns, attn_flash_kernel for other bf16 rows (mma.sync m16n8k16;
 // 64 or 128 packed (token, head of the group) rows per block, key tiles of 64 through two cp.async buffers,
-// only the tiles a row of the block can see; probabilities as two bf16 pieces).  attn_rows_kernel covers fp32
-// and shapes without 16-byte rows.  Decode: attn_step_kernel, one launch: norm and rotation in every
+// only the tiles a row of the block can see; probabilities as two bf16 pieces).  attn_tiles_kernel takes fp32 rows of whole
+// 16-byte pieces, attn_rows_kernel everything else.  Decode: attn_step_kernel, one launch: norm and rotation in every
 // block, blocks = (key/value head, split of the span), the last block of a head merges.
 #include <type_traits>
 

@@ -218,7 +218,8 @@ class ChunkPrefill:
             scratch, source = self._expert_rows_scratch(routes // topk if by_token else routes, bank.in_features)
             fresh = x_up is not None or source is not x
             # 512 inputs (the down product) and eight or more routes per expert: 32 routes per decoding of a tile
-            # (measured at 16 routes per expert: 91 against 105 us; the 2048-input products: 245 against 201 us)
+            # (measured at 16 routes per expert: 91 against 105 us; the 2048-input products: 245 against 201 us); reached with
+            # banks that _tiles_form does not take
             per_pass = self.ROUTES_PER_PASS or (32 if bank.in_features == 512 and routes >= 8 * (self.total_experts or experts) else 0)
             call("qd_nvfp4_expert_rows", ptr(x), ptr(x_up), ptr(bank.weight), ptr(bank.weight_scale), ptr(bank.weight_scale_2),
                  ptr(order), ptr(boundaries), ptr(routing), ptr(out), routes, experts, topk, bank.out_features,
@@ -266,8 +267,8 @@ class ChunkPrefill:
         qg, k, v = self._matmul_many(x, [w.q_proj, w.k_proj, w.v_proj])
         q_scratch = self._empty(tokens, c.num_attention_heads * c.head_dim)
         out = torch.empty_like(q_scratch)
-        # q/k norm + RoPE + cache rows, then causal attention on the tensor cores: every cache tile
-        # is read once per sixteen tokens
+        # q/k norm + RoPE + cache rows, then causal attention on the tensor cores: every cache tile is read once per 128 rows of
+        # (token, head of the group), sixteen tokens of the published model
         call("qd_seq_attention", ptr(qg), ptr(k), ptr(v), ptr(w.q_norm), ptr(w.k_norm), ptr(state.kv_k[index]),
              ptr(state.kv_v[index]), ptr(q_scratch), ptr(out), tokens, position0, state.kv_k.shape[1],
              c.num_attention_heads, c.num_key_value_heads, c.head_dim, int(c.head_dim * c.partial_rotary_factor),

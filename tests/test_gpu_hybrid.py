@@ -64,11 +64,12 @@ def test_linear(M, tokens, rows, width, x_type, y_type):
     assert error(out, want) < (1e-5 if y_type == F32 else 5e-3)
 
 
-@pytest.mark.parametrize("tokens,rows,width", [(9, 8, 8), (127, 72, 256), (128, 64, 264), (129, 136, 1000), (300, 2504, 2048), (1030, 5128, 520)])
+@pytest.mark.parametrize("tokens,rows,width", [(9, 8, 8), (127, 72, 256), (128, 64, 264), (129, 136, 1000), (300, 2504, 2048), (1030, 5128, 520),
+                                               (20, 64, 56), (65, 72, 64), (130, 64, 72), (33, 136, 128), (70, 64, 136), (40, 64, 192)])
 @pytest.mark.parametrize("form", ["plain", "bias", "glu", "add"])
 def test_fp32_rows_in_pieces(M, tokens, rows, width, form):
-    """Every tile width, ragged edges, less and more than a segment of 256 inputs, all that may follow the sums, values over
-    forty binary orders.  Bound: the products are exact and each of the segments' sums is rounded; 2e-6 of the sum of
+    """Every tile width, ragged edges, less, just as much and more than one, two and three segments of 64 inputs (two accumulators
+    in turn), all that may follow the sums, values over forty binary orders.  Bound: the products are exact and each of the segments' sums is rounded; 2e-6 of the sum of
     magnitudes is sixteen times the spacing of fp32."""
     w = bf(rows, width, seed=2, std=width ** -0.5)
     x = rnd(tokens, width, seed=1) * torch.exp2(torch.randint(-20, 20, (tokens, 1), generator=torch.Generator().manual_seed(3)).float())
