@@ -7,7 +7,7 @@
 // has grown by more than 2^8 since the last time (P stays below 2^8 and the sum in fp32, so the quotient is the same to
 // rounding): after the first tiles a warp hardly ever reads O before the end.  (Conditional rescaling is published with
 // FlashAttention-4.)
-//   warps 0 .. 4 TILES - 1   softmax, one row a thread; then the epilogue
+//   warps 0 .. 4 TILES - 1   softmax, one row a thread; then the epilogue, for one row tile together with the loading warps
 //   warp 4 TILES             issues the MMAs: S of tile i + 1 before O of tile i, so that the softmax and the products overlap
 //   the rest                 keys and values into the 128-byte swizzled layout, two stages of each: by tiled TMA where a tile's 64
 //                            rows lie together, else (the last tile, the ring's end) row by row with cp.async, zeros past the end
@@ -15,11 +15,11 @@
 // dimension.  Every wait is bounded; a block whose wait ran out writes NaN.
 //
 // Measured (2048 tokens, with the launch gap; before: mma.sync, eight or sixteen rows a warp).  Head dimension 256, 16/2 heads:
-// behind 0 / 2000 / 30000 positions 129 / 225 / 1611 us (478 / 1017 / 7949).  128 columns, window 1024: 16/4
-// heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 3000 clocks at head dimension 256: 1800 of
+// behind 0 / 2000 / 30000 positions 108 / 203 / 1582 us (478 / 1017 / 7949), 128 tokens behind 0 / 500
+// positions 26 / 37 us (50 / 112).  128 columns, window 1024: 16/4 heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 3000 clocks at head dimension 256: 1800 of
 // MMAs (those of S are bound by shared memory, 48 clocks for 64 columns), 1100 of keys and values at 64 bytes a clock, and the
 // hand-over of S and P.
-// One piece, eight bits, takes 120 / 199 / 1290 us there, but since the largest P is not one here (the reference lags behind the
+// One piece, eight bits, took 120 / 199 / 1290 us there where two took 129 / 225 / 1611 (before the epilogue was shared), but since the largest P is not one here (the reference lags behind the
 // maximum) its rounding reaches the result: 2.04e-3 from 64 bits with sharp scores, where the result's own rounding is 1.65e-3
 // and mma.sync with the exact maximum had 1.72e-3.  Two pieces: 1.65e-3.
 #pragma once
@@ -132,13 +132,17 @@ struct Shape {
     static constexpr int kScores = TILES == 1 ? 3 : 2;                                  // score buffers of a row tile
     static constexpr int kTileCols = DV + kScores * kKeys;
     static constexpr int kQBytes = TILES * 128 * QD * 2, kKBytes = kKeys * QD * 2, kVBytes = kKeys * DV * 2;
-    static constexpr size_t kSmem = kQBytes + 2 * (kKBytes + kVBytes) + 512 + 1024;
+    // A block of one row tile has eight loading warps that are free at its end: a row's columns are shared by three warps then.  (Alone
+    // a softmax warp takes 1.4 us for 32 columns, most of it the gates: 16 tokens behind 500 positions 46 us, 35 shared.)
+    static constexpr int kSharers = TILES == 1 ? 1 + kLoaders / 4 : 1;
+    static constexpr int kStatsBytes = TILES == 1 ? 128 * 8 : 0;
+    static constexpr size_t kSmem = kQBytes + 2 * (kKBytes + kVBytes) + 512 + kStatsBytes + 1024;
     static_assert(TILES * kTileCols <= 512 && QD % 64 == 0 && DV % 64 == 0 && DV <= 256 && kLoaders % 4 == 0 && kSmem <= 227 * 1024, "");
 };
 
 template <int TILES>
 struct Bars {
-    uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[TILES][3], p_full[TILES][3], o_done[TILES][2], q_full, drained;
+    uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[TILES][3], p_full[TILES][3], o_done[TILES][2], q_full, stats_full, drained;
 };
 
 // Columns `column` .. + 31 of the rows of the warp's lanes `rows` once more, summed in fp32 over the keys that a row sees and no
@@ -187,6 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
     Bars<TILES>* bars = reinterpret_cast<Bars<TILES>*>(vs + 2 * S::kVBytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
     static_assert(sizeof(Bars<TILES>) + 8 <= 512, "");
+    float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + 512);        // of the rows, for those who share the epilogue
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int kMma = 4 * TILES, kRows = 128 * TILES;
     const int share = p.heads / p.kv_heads, g = blockIdx.x, total = p.tokens * share;
@@ -204,6 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
         for (int t = 0; t < TILES; ++t)
             for (int s = 0; s < 3; ++s) { mbar_init(&bars->s_full[t][s], 1); mbar_init(&bars->p_full[t][s], 4); }
         mbar_init(&bars->q_full, 4 * TILES);
+        mbar_init(&bars->stats_full, 4);
         mbar_init(&bars->drained, 1);
         mbar_fence_init();
     }
@@ -215,6 +221,22 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
     __syncthreads();
     fence_after();
     constexpr uint32_t tmem = 0;               // all 512 columns, so the allocation starts at column 0
+    // the result of a row of tile t, 32 columns of every kSharers * 32, from the first-th 32 on
+    const auto finish = [&](int t, int row, float m, float l, int first) {
+        const uint32_t o_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + t * S::kTileCols;
+#pragma unroll 1
+        for (int c = first * 32; c < DV; c += S::kSharers * 32) {
+            float o[32];
+            load32(o_at + c, o);
+            loaded(o);
+            bool odd = false;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) odd |= !(fabsf(o[e]) < INFINITY);
+            if (row < total) out(row / share, g * share + row % share, c, o, m, l);
+            const unsigned rows = __ballot_sync(0xffffffffu, odd && row < total && l < INFINITY);      // (and the whole warp goes on)
+            if (rows) plain_columns<QD, DV>(p, out, rows, row, m, l, c);
+        }
+    };
 
     if (warp > kMma) {
         // ---- keys and values: warps of (matrix, stage) take every second tile
@@ -279,6 +301,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
             if (lane == 0) mbar_arrive(full);
         }
         if (issued >= 0) mbar_wait(full, (issued >> 1) & 1, nullptr);        // no copy outlives the block, also where a wait ran out
+        if constexpr (S::kSharers > 1) {
+            __syncwarp();
+            const int r = (warp & 3) * 32 + lane;
+            // behind the statistics the last product has ended: its barrier is in its last phase
+            const bool done = __all_sync(0xffffffffu, mbar_wait(&bars->stats_full, 0, nullptr) &&
+                                                      mbar_wait(&bars->o_done[0][(tiles - 1) & 1], ((tiles - 1) >> 1) & 1, nullptr));
+            const float2 ml = done ? stats[r] : make_float2(0.f, NAN);
+            fence_after();
+            finish(0, r0 + r, ml.x, ml.y, 1 + (w >> 2));
+        }
     } else if (warp == kMma) {
         const bool leader = elected();
         const uint32_t qa = smem_u32(smem), ka = smem_u32(ks), va = smem_u32(vs);
@@ -426,18 +458,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t][(tiles - 1) & 1], ((tiles - 1) >> 1) & 1, nullptr));
         fence_after();
         if (!ok) l = NAN;
-#pragma unroll 1
-        for (int c = 0; c < DV; c += 32) {
-            float o[32];
-            load32(o_at + c, o);
-            loaded(o);
-            bool odd = false;
-#pragma unroll
-            for (int e = 0; e < 32; ++e) odd |= !(fabsf(o[e]) < INFINITY);
-            if (row < total) out(row / share, head, c, o, m, l);
-            const unsigned rows = __ballot_sync(0xffffffffu, odd && row < total && l < INFINITY);      // (and the whole warp goes on)
-            if (rows) plain_columns<QD, DV>(p, out, rows, row, m, l, c);
+        if constexpr (S::kSharers > 1) {
+            stats[tid] = make_float2(m, l);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->stats_full);
         }
+        finish(t, row, m, l, 0);
     }
     fence_before();
     __syncthreads();

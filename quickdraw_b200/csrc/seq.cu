@@ -1364,9 +1364,10 @@ extern "C" int qd_seq_attention(const void* qg, const void* k_new, const void* v
         (bf16*)k_cache, (bf16*)v_cache, (bf16*)q_scratch, position0, q_heads, kv_heads, head_dim, rotary_dim, theta, eps,
         nullptr, 0, capacity);
     if (qd_launch_status() != QD_OK) return QD_ERR_LAUNCH;
-    // Tensor cores but for the first few positions of a sequence, where the walk of a position at a time is over sooner: 16 tokens at
-    // position 0 17 against 37 us, 23 at position 20 28 against 38, 24 at position 40 34 against 38 (and 44 of eight heads a warp).
-    if (head_dim == 256 && tokens >= 2 && (tokens >= 24 || position0 + tokens > 48)) {
+    // Tensor cores but for the first few positions of a sequence, where the walk of a position at a time is over sooner (both with the
+    // preparation, 16/2 heads): 24 tokens at position 0 16 against 23 us, 33 21 against 24, 64 35 against 24; 23 at position 20 23 against
+    // 23.5, 33 27 against 24; 2 at position 20 14 against 20, at 47 24 against 20.
+    if (head_dim == 256 && tokens >= 2 && position0 + tokens > 40) {
         return seq_flash_attention((const bf16*)q_scratch, (const bf16*)qg, (const bf16*)k_cache, (const bf16*)v_cache, (bf16*)out, tokens, position0,
                                    capacity, q_heads, kv_heads, (cudaStream_t)stream);
     }

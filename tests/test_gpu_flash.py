@@ -30,6 +30,7 @@ def close(got, want, rounds):
 
 
 @pytest.mark.parametrize("tokens,position,heads,kv_heads", [
+    (40, 0, 16, 2), (41, 0, 16, 2), (20, 20, 8, 8), (21, 20, 8, 8), (2, 39, 16, 2),               # both sides of the line between the forms
     (2, 0, 16, 2), (16, 0, 16, 2), (17, 63, 16, 2), (65, 0, 16, 2), (200, 1000, 16, 2), (130, 3, 6, 2), (300, 0, 2, 2), (129, 64, 4, 1), (2048, 37, 16, 2)])
 def test_gated_attention_of_a_chunk(cuda_device, tokens, position, heads, kv_heads):
     from quickdraw_b200._lib import call, ptr, stream_of
