@@ -1032,12 +1032,19 @@ seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts
     int id[kAhead];
     const auto fetch = [&](int r0) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) { const int r = r0 + 32 * u + lane; id[u] = r < end ? __ldg(ids + r) : -1; }
+        for (int u = 0; u < kAhead; ++u) {
+            if (r0 + 32 * u >= end) break;               // (a slice of a short chunk is 32 routes, often of one warp only)
+            const int r = r0 + 32 * u + lane;
+            id[u] = r < end ? __ldg(ids + r) : -1;
+        }
     };
     for (int r0 = begin; r0 < end; r0 += 32 * kAhead) {
         fetch(r0);
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) if (id[u] >= 0) atomicAdd(mine + id[u], 1);
+        for (int u = 0; u < kAhead; ++u) {
+            if (r0 + 32 * u >= end) break;
+            if (id[u] >= 0) atomicAdd(mine + id[u], 1);
+        }
     }
     __syncthreads();
     // totals per expert, their exclusive scan, then every warp's first position per expert
@@ -1076,9 +1083,13 @@ seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts
         if (end - begin > 32 * kAhead) fetch(r0);        // (a single batch is still there)
         unsigned same[kAhead];
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) same[u] = __match_any_sync(0xffffffffu, id[u]);
+        for (int u = 0; u < kAhead; ++u) {
+            if (r0 + 32 * u >= end) break;
+            same[u] = __match_any_sync(0xffffffffu, id[u]);
+        }
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
+            if (r0 + 32 * u >= end) break;
             const int e = id[u];
             int at = 0;
             if (e >= 0) at = mine[e] + __popc(same[u] & ((1u << lane) - 1u));
