@@ -84,13 +84,16 @@ def ring_segments(first: int, count: int, capacity: int) -> list[tuple[int, int]
     return [(row, head)] + ([(0, count - head)] if count > head else [])
 
 
-def gla_span(tokens: int, blocks: int, sms: int) -> int:
+def gla_span(tokens: int, blocks: int, sms: int, dim: int = 128) -> int:
     """Tokens of a segment of gated linear attention, 0: the chunk as a whole.  The whole chunk keeps ``blocks`` SMs busy and a
     segment is walked twice, so there is nothing to gain once they are half of the SMs; three blocks to an SM take all there
     is, and segments below 80 tokens cost more states than they save (heads of 128: 16 heads 400 / 777 / 2048 tokens 92 / 170 /
-    437 -> 73 / 111 / 235 us, 4 heads 2048 tokens 427 -> 93 us; 32 heads 438 -> 413, not taken)."""
-    count = min(tokens // 80, 3 * sms // blocks)
-    return -(-tokens // count // 16) * 16 if count >= 3 and 2 * blocks <= sms else 0
+    437 -> 73 / 111 / 235 us, 4 heads 2048 tokens 427 -> 93 us; 32 heads 438 -> 413, not taken).  Above 128 key rows two blocks fill an SM,
+    and three segments that do not fit at once are no gain (heads of 256 x 256, 8 heads: 240 tokens walk 91, three segments 104; 400
+    tokens 142, four 125, five 155; 700 tokens 238, four 175, six 209; 4 heads 240 tokens 91, three 72)."""
+    count = min(tokens // 80, (3 if dim <= 128 else 2) * sms // blocks)
+    gains = count >= 3 and (dim <= 128 or count >= 4 or count * blocks <= sms)
+    return -(-tokens // count // 16) * 16 if gains and 2 * blocks <= sms else 0
 
 
 def step_covers(m) -> bool:
@@ -250,7 +253,7 @@ class LinearRecurrence:
     def _walk(self, q, k, decay, v, beta, scales, history, gate, gate_column: int, act: int, dtype):
         m, tokens = self.m, q.shape[0]
         raw = torch.empty((tokens, self.out_columns), dtype=F32, device=q.device)
-        span = 0 if beta is not None else gla_span(tokens, m.heads * -(-m.vdim // 32), self.sms)
+        span = 0 if beta is not None else gla_span(tokens, m.heads * -(-m.vdim // 32), self.sms, m.dim)
         if span:
             scratch = torch.empty(-(-tokens // span) * m.heads * m.dim * (m.vdim + 1), dtype=F32, device=q.device)
             call_hybrid("qd_gla_segments", ptr(q), ptr(k), ptr(decay), ptr(v), ptr(history.rec), ptr(raw), tokens, m.heads, self.kv_heads, m.dim, m.vdim,

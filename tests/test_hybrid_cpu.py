@@ -304,6 +304,7 @@ def test_segments_of_gated_linear_attention_follow_the_device():
     """A chunk goes in segments where its blocks leave half of the SMs idle, at most three blocks to an SM: of the device at hand."""
     assert mixers.gla_span(2048, 64, 148) == 352 and mixers.gla_span(2048, 64, 100) == 0 and mixers.gla_span(2048, 16, 148) == 96
     assert mixers.gla_span(2048, 16, 64) == 176 and mixers.gla_span(239, 16, 148) == 0 and mixers.gla_span(240, 16, 148) == 80
+    assert [mixers.gla_span(t, 64, 148, 256) for t in (240, 300, 400, 700)] == [0, 0, 112, 176] and mixers.gla_span(240, 32, 148, 256) == 80
     for tokens in range(240, 700, 7):
         for blocks in (1, 7, 33, 74):
             span = mixers.gla_span(tokens, blocks, 148)
