@@ -23,6 +23,10 @@ BF16, F32 = torch.bfloat16, torch.float32
 DTYPE_CODE = {BF16: 0, F32: 1}
 SILU, SIGMOID = 0, 1
 ROWS_FORM = 8                                                    # token rows up to which a product streams the weights
+# fp32 rows go to the tensor cores from this width or this many products on: their two launches and the planes between them take 11.4 us
+# of host time, the FMA tiles 6.7 and 0.09 an input (64 x 64 8.5 against 11.3 us, 64 x 96 11.0 / 11.3, 64 x 128 13.8 / 11.4; 2048
+# outputs of 16 inputs, 777 / 2048 tokens 8.1 / 14.6 against 11.4 / 11.6; of 64 inputs, 128 / 300 tokens 8.7 / 14.8 against 11.3)
+PIECES_WIDTH, PIECES_PRODUCTS = 96, 2 ** 25
 MASK_WINDOW, MASK_CHUNK = 0, 1                                   # kinds of qd_attention_args
 NORM_NONE, NORM_ROW, NORM_HEAD = 0, 1, 2
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
@@ -44,10 +48,10 @@ def linear(x, x_column: int, ldx: int, weight, out, *, tokens: int, status, gelu
     """out[t] = W x[t, x_column : x_column + in_features] (+ fp32 ``bias``); the first ``gelu_columns`` outputs through the exact
     GELU; ``glu``: weight rows 2i and 2i + 1 are a gate and its partner, out[i] = relu(gate) * partner; ``add``: onto
     what ``out`` holds; ``norm`` (a few tokens only): x / rms(x) * (norm_offset + norm) in the place of x.  More than
-    ``ROWS_FORM`` rows of fp32 go through the tensor cores as three bf16 pieces, where TMA takes the operands."""
+    ``ROWS_FORM`` rows of fp32 go through the tensor cores as three bf16 pieces, where TMA takes the operands and there is enough to do."""
     rows, width = weight.shape
     start = x.data_ptr() + 4 * x_column
-    if (x.dtype is F32 and tokens > ROWS_FORM and norm is None and (width | ldx | rows | out.shape[1]) % 8 == 0
+    if (x.dtype is F32 and tokens > ROWS_FORM and norm is None and (width >= PIECES_WIDTH or tokens * rows * width >= PIECES_PRODUCTS) and (width | ldx | rows | out.shape[1]) % 8 == 0
             and (start | weight.data_ptr() | out.data_ptr()) % 16 == 0):
         planes = torch.empty(3 * tokens * width, dtype=BF16, device=x.device)
         call_hybrid("qd_linear_pieces", column(x, x_column), ldx, ptr(weight), ptr(out), out.shape[1], DTYPE_CODE[out.dtype], tokens, rows, width,

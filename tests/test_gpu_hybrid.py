@@ -67,10 +67,11 @@ def test_linear(M, tokens, rows, width, x_type, y_type):
 @pytest.mark.parametrize("tokens,rows,width", [(9, 8, 8), (127, 72, 256), (128, 64, 264), (129, 136, 1000), (300, 2504, 2048), (1030, 5128, 520),
                                                (20, 64, 56), (65, 72, 64), (130, 64, 72), (33, 136, 128), (70, 64, 136), (40, 64, 192)])
 @pytest.mark.parametrize("form", ["plain", "bias", "glu", "add"])
-def test_fp32_rows_in_pieces(M, tokens, rows, width, form):
+def test_fp32_rows_in_pieces(M, monkeypatch, tokens, rows, width, form):
     """Every tile width, ragged edges, less, just as much and more than one, two and three segments of 64 inputs (two accumulators
     in turn), all that may follow the sums, values over forty binary orders.  Bound: the products are exact and each of the segments' sums is rounded; 2e-6 of the sum of
     magnitudes is sixteen times the spacing of fp32."""
+    monkeypatch.setattr(M, "PIECES_WIDTH", 8)                     # (small ones would go to the FMA tiles)
     w = bf(rows, width, seed=2, std=width ** -0.5)
     x = rnd(tokens, width, seed=1) * torch.exp2(torch.randint(-20, 20, (tokens, 1), generator=torch.Generator().manual_seed(3)).float())
     x[0], x[-1, 0], x[-1, -1] = 0.0, float("inf"), float("nan")
@@ -542,9 +543,10 @@ def test_fp32_chunks_keep_the_product_of_a_vanished_probability(cuda_device):
 
 @pytest.mark.parametrize("tokens,rows,width", [(9, 64, 64), (200, 136, 520)])
 @pytest.mark.parametrize("add", [False, True])
-def test_fp32_rows_with_infinite_weights(M, tokens, rows, width, add):
+def test_fp32_rows_with_infinite_weights(M, monkeypatch, tokens, rows, width, add):
     """Infinite and NaN weights under x whose lower pieces are zero (whole numbers) and not: plain products and sums, an infinity
     where there is one and NaN where two meet or a zero of x meets one."""
+    monkeypatch.setattr(M, "PIECES_WIDTH", 8)
     w, x, stat = bf(rows, width, seed=2), rnd(tokens, width, seed=1), status()
     x[:4] = x[:4].round()
     x[1, 5], x[2] = 0.0, 1.0

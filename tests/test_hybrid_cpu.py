@@ -309,3 +309,13 @@ def test_segments_of_gated_linear_attention_follow_the_device():
         for blocks in (1, 7, 33, 74):
             span = mixers.gla_span(tokens, blocks, 148)
             assert span == 0 or (span % 16 == 0 and -(-tokens // span) * blocks <= 3 * 148)
+
+
+def test_small_fp32_products_keep_the_fma_tiles(recorder):
+    """Where two launches and the planes between them take longer than the product on the FMA pipe."""
+    for tokens, rows, width, pieces in ((9, 64, 64, False), (777, 2048, 16, False), (2048, 2048, 16, True), (128, 2048, 64, False), (300, 2048, 64, True),
+                                        (9, 64, 96, True), (16, 512, 512, True), (8, 2048, 2048, False)):
+        x, w, out = torch.zeros(tokens, width), torch.zeros(rows, width, dtype=torch.bfloat16), torch.empty(tokens, rows)
+        recorder.clear()
+        mixers.linear(x, 0, width, w, out, tokens=tokens, status=torch.zeros(1, dtype=torch.int32))
+        assert [name for name, _ in recorder] == ["qd_linear_pieces" if pieces else "qd_linear"], (tokens, rows, width)
