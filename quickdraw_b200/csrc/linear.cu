@@ -531,6 +531,20 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
         const int t = t0 + quadrant * 32 + lane;
         if (ok && t < p.tokens) {
             TY* row = reinterpret_cast<TY*>(p.y) + (long long)t * p.ldy;
+            float finite = 0.f;                    // NaN if a sum is not
+#pragma unroll
+            for (int i = 0; i < kHalf; ++i) finite = fmaf(acc[i], 0.f, finite);
+            if (finite != finite) {
+#pragma unroll
+                for (int c = 0; c < kHalf; c += 8) {
+                    const int n = n0 + half * kHalf + c;
+                    if (n >= p.rows) break;
+                    const Eight plain = plain_sums(p, t, n);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (!(fabsf(acc[c + q]) < INFINITY)) acc[c + q] = plain.v[q];
+                }
+            }
 #pragma unroll
             for (int c = 0; c < kHalf; c += 8) {
                 const int n = n0 + half * kHalf + c;
@@ -538,15 +552,6 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
                     float f[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) f[q] = acc[c + q];
-                    bool odd = false;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) odd |= !(fabsf(f[q]) < INFINITY);
-                    if (odd) {
-                        const Eight plain = plain_sums(p, t, n);
-#pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            if (!(fabsf(f[q]) < INFINITY)) f[q] = plain.v[q];
-                    }
                     finish8(p, f, row, n, bias + half * kHalf + c);
                 }
             }

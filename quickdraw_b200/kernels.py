@@ -343,11 +343,10 @@ _ATTN_SPLITS, _ATTN_SPLITS_MMA = 32, 74
 _scratch: dict = {}
 
 
-def _attn_splits(head_dim: int, rotary: int, keys, values) -> int:
+def _attn_splits(head_dim: int, rotary: int, addresses: int) -> int:
     """By the form that the library takes: the general one, which also has head dimension 256 where the rotary part is not whole warps
     or the caches are off a 16-byte boundary, is slower with more splits (4000 / 8192 positions 124 / 178 us with 32, 156 / 192 with 74)."""
-    mma = head_dim == 256 and rotary % 64 == 0 and (keys.data_ptr() | values.data_ptr()) % 16 == 0
-    return _ATTN_SPLITS_MMA if mma else _ATTN_SPLITS
+    return _ATTN_SPLITS_MMA if head_dim == 256 and rotary % 64 == 0 and addresses % 16 == 0 else _ATTN_SPLITS
 
 
 def _attn_scratch(device, floats: int, kv_heads: int, stream):
@@ -378,13 +377,13 @@ def full_attention_block(w, x, kv_cache, position, *, config) -> torch.Tensor:
     rotary = int(d * config.partial_rotary_factor)
     assert rotary % 2 == 0 and 0 <= rotary <= d
     lib = _lib.lib()
-    splits = _attn_splits(d, rotary, keys, values)
+    key_rows, value_rows = ptr(keys), ptr(values)
+    splits = _attn_splits(d, rotary, key_rows | value_rows)
     floats = lib.qd_attn_scratch_floats(hq, hk, d, splits)
     stream = stream_of(x)
     scratch, counters = _attn_scratch(x.device, floats, hk, stream)
     gated = x.new_empty(hq * d)
-    call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(w.q_norm), ptr(w.k_norm), ptr(keys),
-         ptr(values), ptr(gated), ptr(scratch), ptr(counters),
+    call("qd_attn_decode", ptr(qg), ptr(k_new), ptr(v_new), ptr(w.q_norm), ptr(w.k_norm), key_rows, value_rows, ptr(gated), ptr(scratch), ptr(counters),
          ptr(position) if device_position else None, 0 if device_position else int(position),
          capacity, hq, hk, d, rotary, float(config.rope_theta), float(config.rms_norm_eps),
          splits, CHAINED, stream)

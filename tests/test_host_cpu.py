@@ -438,7 +438,5 @@ def test_launch_modes_of_the_entry_points():
 
 def test_splits_of_the_decode_attention_follow_the_form_that_is_taken():
     from quickdraw_b200.kernels import _attn_splits
-    cache = torch.zeros(4 * 2 * 256 + 4, dtype=torch.bfloat16)
-    whole, shifted = cache[:2048].view(4, 2, 256), cache[4:2052].view(4, 2, 256)
-    assert [_attn_splits(256, r, whole, whole) for r in (0, 64, 256, 32, 96)] == [74, 74, 74, 32, 32]
-    assert _attn_splits(128, 64, whole, whole) == 32 and _attn_splits(256, 64, whole, shifted) == 32
+    assert [_attn_splits(256, r, 4096) for r in (0, 64, 256, 32, 96)] == [74, 74, 74, 32, 32]
+    assert _attn_splits(128, 64, 4096) == 32 and _attn_splits(256, 64, 4096 | 4104) == 32
