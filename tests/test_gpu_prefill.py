@@ -216,6 +216,39 @@ def test_chunked_recurrence_matches_token_by_token(cuda_device, value_dim, token
     assert float(rows.max()) < 3e-2, float(rows.max())
 
 
+@pytest.mark.parametrize("tokens,hk,hv,value_dim,offset", [(1, 2, 4, 128, 0), (16, 1, 1, 32, 0), (63, 2, 2, 64, 4), (65, 1, 3, 96, 0),
+                                                           (128, 2, 4, 128, 4), (193, 1, 4, 32, 0), (300, 2, 6, 64, 0)])
+def test_chunked_recurrence_against_64_bits(cuda_device, tokens, hk, hv, value_dim, offset):
+    """Ends of chunks and of 16-token blocks, one to four value heads to a key head, rows that start 8 bytes off a 16-byte boundary.
+    Operands are two bf16 pieces (2^-16 of their size): 1e-4 leaves the state a factor of six for sums of many of them; the result is
+    rounded to bf16 (1.66e-3 alone)."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    key_dim, f64 = 128, torch.float64
+    channels = 2 * hk * key_dim + hv * value_dim
+    src = synthetic.Source(23, "cpu")
+    flat = torch.empty(tokens * channels + 8, dtype=torch.bfloat16, device=cuda_device)
+    conv = flat[offset:offset + tokens * channels].view(tokens, channels)
+    conv.copy_(src.normal("conv", tokens, channels))
+    place = torch.empty(tokens * hv * value_dim + 8, dtype=torch.bfloat16, device=cuda_device)
+    out = place[offset // 2:offset // 2 + tokens * hv * value_dim].view(tokens, hv, value_dim)
+    a, b = src.normal("a", tokens, hv).to(cuda_device), src.normal("b", tokens, hv).to(cuda_device)
+    a_log, dt_bias = src.normal("alog", hv, std=0.5).to(cuda_device), src.normal("dt", hv).to(cuda_device)
+    rec = src.normal("rec0", hv, key_dim, value_dim, std=0.1).float().to(cuda_device)
+    state = rec.double()
+    scratch = torch.empty(lib().qd_seq_gdn_chunk_scratch_bytes(tokens, hv), dtype=torch.uint8, device=cuda_device)
+    call("qd_seq_gdn_recurrence_chunked", ptr(conv), ptr(a), ptr(b), ptr(a_log), ptr(dt_bias), ptr(rec), ptr(out), tokens, hk, hv,
+         key_dim, value_dim, ptr(scratch), stream_of(conv))
+    q, k, v = conv.to(f64).split([hk * key_dim, hk * key_dim, hv * value_dim], -1)
+    unit = lambda x: (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(hv // hk, 1)
+    q, k, v = unit(q.unflatten(-1, (hk, key_dim))) / key_dim ** 0.5, unit(k.unflatten(-1, (hk, key_dim))), v.unflatten(-1, (hv, value_dim))
+    beta, decay = torch.sigmoid(b.to(f64)), torch.exp(-a_log.to(f64).exp() * torch.nn.functional.softplus(a.to(f64) + dt_bias.to(f64)))
+    want = torch.empty_like(v)
+    for t in range(tokens):
+        want[t] = O.delta_rule(q[t], k[t], v[t], beta[t], decay[t], state)
+    assert float((rec.double() - state).norm() / state.norm()) < 1e-4
+    assert float((out.double() - want).norm() / want.norm()) < 1.8e-3
+
+
 @pytest.mark.parametrize("routes,experts", [(4088, 256), (24, 16), (5000, 7), (1, 3)])
 def test_group_routes_is_the_stable_sort_by_expert(cuda_device, routes, experts):
     from quickdraw_b200._lib import call, ptr, stream_of
