@@ -29,6 +29,7 @@ from dataclasses import dataclass
 import torch
 
 from .registry import design_of, design_of_directory
+from .state import upload
 from .weights import Checkpoint, DokulixCheckpoint, FezopelCheckpoint
 
 
@@ -158,7 +159,7 @@ class Engine:
         places among the tokens) a list of the logits at those places."""
         start, count = self.state.position, len(token_ids)
         asked = [count - 1] if want is None else want
-        tokens = torch.tensor(token_ids, dtype=torch.long, device=self.device)
+        tokens = upload(token_ids, torch.long, self.device)
         found: list[torch.Tensor] = []
         done = 0
         while done < count:
@@ -197,7 +198,7 @@ class Engine:
         among them, in the order given.  ``reset`` starts a request."""
         config = self.ckpt.config
         assert 0 < len(token_ids) and self.state.position + len(token_ids) <= self.max_context, "context capacity reached"
-        assert all(0 <= t < config.vocab_size for t in token_ids), "token id outside the vocabulary"
+        assert 0 <= min(token_ids) and max(token_ids) < config.vocab_size, "token id outside the vocabulary"
         assert all(0 <= w < len(token_ids) for w in want), "a wanted place lies outside the tokens"
         self._fold()
         self.pending_token = None
@@ -210,12 +211,11 @@ class Engine:
     def _note(self, ids: list[int]) -> None:
         """Record tokens processed at the positions after ``history`` and what that did to the
         cache: a row is rewritten with the same content exactly when the whole prefix is the same."""
-        for token in ids:
-            at = len(self.history)
-            if not (at < len(self._kv_tokens) and self._kv_tokens[at] == token):
-                del self._kv_tokens[at:]
-                self._kv_tokens.append(token)
-            self.history.append(token)
+        known = self._kv_tokens[len(self.history):len(self.history) + len(ids)]
+        same = len(known) if known == ids[:len(known)] else next(i for i, token in enumerate(known) if token != ids[i])
+        if same < len(ids):
+            self._kv_tokens[len(self.history) + same:] = ids[same:]
+        self.history += ids
 
     def _fold(self) -> None:
         """Bring ``history`` up to date with the decode steps taken (their tokens stay on the

@@ -21,7 +21,7 @@ import torch
 
 from ._lib import call_hybrid, ptr, stream_of
 from .mixers import BF16, DTYPE_CODE, F32, MIXERS, column, linear, stack_rows
-from .state import HybridState
+from .state import HybridState, upload
 from .weights import DokulixCheckpoint, FezopelCheckpoint
 
 GREEDY_BLOCKS = 128
@@ -68,7 +68,7 @@ class HybridModel:
         stream = self._layers(token_ids, position0, state, token_ids.numel(), bool(want) or record is not None, record)
         if not want:
             return None
-        rows = torch.tensor(list(want), dtype=torch.int32, device=self.device)
+        rows = upload(list(want), torch.int32, self.device)
         assert 0 <= min(want) and max(want) < token_ids.numel()
         return self._head(stream, rows)
 

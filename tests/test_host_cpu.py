@@ -440,3 +440,21 @@ def test_splits_of_the_decode_attention_follow_the_form_that_is_taken():
     from quickdraw_b200.kernels import _attn_splits
     assert [_attn_splits(256, r, 4096) for r in (0, 64, 256, 32, 96)] == [74, 74, 74, 32, 32]
     assert _attn_splits(128, 64, 4096) == 32 and _attn_splits(256, 64, 4096 | 4104) == 32
+
+
+@pytest.mark.parametrize("rows,before,ids", [([], 0, [1, 2]), ([1, 2, 3], 0, [1, 2]), ([1, 2, 3], 1, [2, 3, 4]), ([1, 2, 3, 4], 1, [2, 9, 4]),
+                                             ([1, 2, 3], 0, [7]), ([1, 2], 2, [3]), ([1, 2, 3], 1, [])])
+def test_cache_rows_follow_the_tokens_one_by_one(rows, before, ids):
+    """What a run of tokens does to the record of the cache's rows is what its tokens do one after the other."""
+    from types import SimpleNamespace
+    from quickdraw_b200.engine import Engine
+    want, history = list(rows), list(rows[:before])
+    for token in ids:
+        at = len(history)
+        if not (at < len(want) and want[at] == token):
+            del want[at:]
+            want.append(token)
+        history.append(token)
+    engine = SimpleNamespace(history=list(rows[:before]), _kv_tokens=list(rows))
+    Engine._note(engine, ids)
+    assert engine._kv_tokens == want and engine.history == history
