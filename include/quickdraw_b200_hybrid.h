@@ -92,6 +92,13 @@ int qd_linear_recurrence(const float* q, const float* k, const float* g, const f
 int qd_gla_segments(const float* q, const float* k, const float* g, const float* v, float* state, float* out, int tokens, int
     heads, int kv_heads, int dim, int vdim, int span, float* scratch, void* stream);
 
+/* Both on the tensor cores, sixteen tokens at a time (operands in three bf16 pieces).  dim 128, vdim a multiple of 16, addresses of q, k,
+ * g, v and scratch on 16-byte boundaries; QD_ERR_UNSUPPORTED otherwise.  scratch: qd_channel_chunk_scratch_bytes bytes. */
+int qd_channel_recurrence_chunked(const float* q, const float* k, const float* g, const float* v, const float* beta, const
+    float* scales, float* state, float* out, int tokens, int heads, int kv_heads, int dim, int vdim, int delta, void* scratch,
+    unsigned int* status, void* stream);
+long long qd_channel_chunk_scratch_bytes(int tokens, int heads);
+
 /* out[t, h] = x[t, h] / rms(x[t, h]) * w * act(gate[t, h]), act 0 = SiLU, 1 = sigmoid; w [vdim] shared by the heads. */
 int qd_head_norm_gate(const float* x, const void* w, const void* gate, long long ld_gate, void* out, int tokens, int
     heads, int vdim, float eps, int act, int dtype, void* stream);

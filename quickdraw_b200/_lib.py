@@ -102,6 +102,8 @@ HYBRID_LIBRARIES = {
         "qd_channel_delta_prepare": [P, P, P, P, L, P, P, P, P, P, P, P, I, P, I, P, P, P, P, P, P, I, I, I, I, I, I, P],
         "qd_linear_recurrence": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
         "qd_gla_segments": [P, P, P, P, P, P, I, I, I, I, I, I, P, P],
+        "qd_channel_chunk_scratch_bytes": [I, I],
+        "qd_channel_recurrence_chunked": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, P, P, P],
         "qd_head_norm_gate": [P, P, P, L, P, I, I, I, F, I, I, P],
         "qd_gla_step": [P, P, P, P, P, P, I, F, P, P, F, P, P, I, I, I, I, P],
         "qd_channel_delta_step": [P, P, P, P, P, P, P, I, P, P, P, P, P, I, P, I, P, P, I, P, F, P, P, I, I, I, I, I, P],
@@ -113,7 +115,7 @@ HYBRID_LIBRARIES = {
         "qd_latent_step": [P, P],
     },
 }
-HYBRID_LONG_RESULTS = {"qd_attention_step_floats", "qd_latent_step_floats"}
+HYBRID_LONG_RESULTS = {"qd_attention_step_floats", "qd_latent_step_floats", "qd_channel_chunk_scratch_bytes"}
 HYBRID_OWNER = {name: target for target, names in HYBRID_LIBRARIES.items() for name in names}
 
 

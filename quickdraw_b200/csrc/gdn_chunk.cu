@@ -23,7 +23,7 @@
 // tf32 (11 bits) and every product went through shared memory in 16 x 16 warp tiles behind five barriers a chunk.  16 key and 32 value heads of
 // 128, both kernels, before and now: 64 tokens 25 -> 15 us, 511 68 -> 37, 2048 259 -> 99, 8192 1016 -> 353 us; error of the state against 64 bits
 // after 2048 tokens 3.5e-4 -> 7e-6.  A chunk of the recurrence takes 2.4 us, of which the MMAs of a walking warp are 1.3 (316 at eight clocks).
-#include "common.cuh"
+#include "pieces_mma.cuh"
 
 namespace qd {
 namespace {
@@ -50,54 +50,6 @@ QD_DEVINL float log_decay(float a, float a_log, float bias) { return -expf(a_log
 
 QD_DEVINL int block_of(int row, int col) { return row * (row + 1) / 2 + col; }
 
-// x0, x1 as two bf16 pieces each (cut off, then the rest rounded), packed as MMA operands take them.
-QD_DEVINL void split_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
-    const uint32_t b0 = __float_as_uint(x0), b1 = __float_as_uint(x1);
-    hi = __byte_perm(b0, b1, 0x7632);
-    const __nv_bfloat162 rest = __floats2bfloat162_rn(x0 - __uint_as_float(b0 & 0xffff0000u), x1 - __uint_as_float(b1 & 0xffff0000u));
-    lo = *reinterpret_cast<const uint32_t*>(&rest);
-}
-// Accumulators of two neighbouring n-tiles (16 rows x 16 columns) as the A operand of the next product, in two pieces.
-QD_DEVINL void split_tiles(const float (&l)[4], const float (&r)[4], uint4& hi, uint4& lo) {
-    split_pair(l[0], l[1], hi.x, lo.x);
-    split_pair(l[2], l[3], hi.y, lo.y);
-    split_pair(r[0], r[1], hi.z, lo.z);
-    split_pair(r[2], r[3], hi.w, lo.w);
-}
-QD_DEVINL void mma_bf16(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
-}
-QD_DEVINL uint4 ldsm(uint32_t addr) {
-    uint4 v;
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-QD_DEVINL uint4 ldsm_t(uint32_t addr) {
-    uint4 v;
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-QD_DEVINL uint32_t transposed(uint32_t v) {        // an 8 x 8 matrix of 16-bit values across the warp
-    uint32_t r;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
-
-// Sixteen bytes global -> shared in the background; zeros where there is no token.  wide: the source is 16-byte aligned (else 8).
-QD_DEVINL void copy16(uint32_t dst, const void* src, bool there, bool wide) {
-    const uint32_t bytes = there ? 16u : 0u;
-    if (wide) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes / 2) : "memory");
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + 8), "l"((const char*)src + 8), "r"(bytes / 2) : "memory");
-    }
-}
-QD_DEVINL void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int LEFT> QD_DEVINL void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
-
 // A chunk's rows of one head of keys or queries -> [64][128] bf16 in shared memory, 16-byte pieces p of row r at p ^ (r & 7).
 template <int THREADS>
 QD_DEVINL void copy_rows(uint32_t dst, const bf16* first, int t_base, int tokens, int channels, int tid, bool wide) {
@@ -108,7 +60,6 @@ QD_DEVINL void copy_rows(uint32_t dst, const bf16* first, int t_base, int tokens
         copy16(dst + r * 256 + ((piece ^ (r & 7)) << 4), first + (size_t)tok * channels + piece * 8, t_base + r < tokens, wide);
     }
 }
-QD_DEVINL void named_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 // ------------------------------------------------------------------------------- prepare
 // Eight warps; warps 0 - 3 and 4 - 7 invert the matrices of one value head each.

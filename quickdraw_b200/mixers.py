@@ -100,6 +100,20 @@ def gla_span(tokens: int, blocks: int, sms: int, dim: int = 128) -> int:
     return -(-tokens // count // 16) * 16 if gains and 2 * blocks <= sms else 0
 
 
+def chunked_recurrence(m, tokens: int, delta: bool, sms: int) -> bool:
+    """Whether a chunk's recurrence goes to the tensor cores, sixteen tokens at a time, instead of a token at a time.  Gated linear
+    attention always gains (heads of 128: 16 heads 9 / 100 / 2048 tokens 10.6 / 29 / 224 -> 8.1 / 19 / 126 us) but where long segments of very few heads
+    share the SMs (4 heads 777 / 1200 / 2048 tokens 47 / 61 / 91 against 44 / 65 / 109; 16 heads of 16 value columns, 777 tokens 44 against 51).  The
+    delta rule gains once its prepare launch pays (16 heads 9 / 24 / 48 tokens 10.6 / 14.6 / 20.9 against 10.7 / 14.0 / 15.8), later where two slices
+    of columns share a block (32 heads 48 / 64 / 80 tokens 20.8 / 25.0 / 29.1 against 23.4 / 25.3 / 27.0; 2048 tokens 583 -> 272)."""
+    if m.dim != 128 or m.vdim % 16:
+        return False
+    if delta:
+        return tokens >= (24 if m.heads * m.vdim // 16 <= sms else 80)
+    blocks = m.heads * -(-m.vdim // 32)
+    return not gla_span(tokens, blocks, sms, m.dim) or (m.vdim % 32 == 0 and (tokens <= 1000 or blocks > 16))
+
+
 def step_covers(m) -> bool:
     """Whether the one-launch decode form of a recurrence takes these sizes (a cluster of at most eight blocks of 32 value columns)."""
     return m.vdim <= 256
@@ -243,8 +257,9 @@ class LatentAttention:
 class LinearRecurrence:
     """What the two recurrences share: the fp32 operands of a chunk, the walk over its tokens, the per-head norm and gate."""
 
-    def __init__(self, weights, m, eps: float, kv_heads: int):
+    def __init__(self, weights, m, eps: float, kv_heads: int, device):
         self.w, self.m, self.eps, self.kv_heads = weights, m, eps, kv_heads
+        self.sms = torch.cuda.get_device_properties(device).multi_processor_count
         self.out_columns = m.heads * m.vdim
 
     def _operands(self, proj, at, status):
@@ -254,17 +269,23 @@ class LinearRecurrence:
         linear(proj, at["a1"], proj.shape[1], self.w.a2, decay, tokens=tokens, status=status)      # logits; decays in place later
         return (new(tokens, self.kv_heads * m.dim), new(tokens, self.kv_heads * m.dim), decay, new(tokens, m.heads * m.vdim))
 
-    def _walk(self, q, k, decay, v, beta, scales, history, gate, gate_column: int, act: int, dtype):
+    def _walk(self, q, k, decay, v, beta, scales, history, gate, gate_column: int, act: int, dtype, status):
         m, tokens = self.m, q.shape[0]
         raw = torch.empty((tokens, self.out_columns), dtype=F32, device=q.device)
-        span = 0 if beta is not None else gla_span(tokens, m.heads * -(-m.vdim // 32), self.sms, m.dim)
-        if span:
+        delta = beta is not None
+        chunked = chunked_recurrence(m, tokens, delta, self.sms)
+        span = 0 if delta or chunked else gla_span(tokens, m.heads * -(-m.vdim // 32), self.sms, m.dim)
+        if chunked:
+            scratch = torch.empty(size_hybrid("qd_channel_chunk_scratch_bytes", tokens, m.heads), dtype=torch.uint8, device=q.device)
+            call_hybrid("qd_channel_recurrence_chunked", ptr(q), ptr(k), ptr(decay), ptr(v), ptr(beta), ptr(scales), ptr(history.rec), ptr(raw), tokens,
+                        m.heads, self.kv_heads, m.dim, m.vdim, int(delta), ptr(scratch), ptr(status), stream_of(q))
+        elif span:
             scratch = torch.empty(-(-tokens // span) * m.heads * m.dim * (m.vdim + 1), dtype=F32, device=q.device)
             call_hybrid("qd_gla_segments", ptr(q), ptr(k), ptr(decay), ptr(v), ptr(history.rec), ptr(raw), tokens, m.heads, self.kv_heads, m.dim, m.vdim,
                         span, ptr(scratch), stream_of(q))
         else:
             call_hybrid("qd_linear_recurrence", ptr(q), ptr(k), ptr(decay), ptr(v), ptr(beta), ptr(scales), ptr(history.rec), ptr(raw), tokens,
-                        m.heads, self.kv_heads, m.dim, m.vdim, int(beta is not None), stream_of(q))
+                        m.heads, self.kv_heads, m.dim, m.vdim, int(delta), stream_of(q))
         out = torch.empty((tokens, self.out_columns), dtype=dtype, device=q.device)
         call_hybrid("qd_head_norm_gate", ptr(raw), ptr(self.w.norm), column(gate, gate_column), gate.shape[1], ptr(out), tokens, m.heads,
                     m.vdim, self.eps, act, DTYPE_CODE[dtype], stream_of(q))
@@ -273,8 +294,7 @@ class LinearRecurrence:
 
 class GatedLinearAttention(LinearRecurrence):
     def __init__(self, weights: GLAWeights, m: GLAConfig, eps: float, device):
-        super().__init__(weights, m, eps, m.heads)
-        self.sms = torch.cuda.get_device_properties(device).multi_processor_count
+        super().__init__(weights, m, eps, m.heads, device)
         self.projections = {"q": weights.q, "k": weights.k, "v": weights.v, "g": weights.g, "a1": weights.a1}
 
     def chunk(self, proj, at, history: LayerHistory, position, status):
@@ -282,7 +302,7 @@ class GatedLinearAttention(LinearRecurrence):
         q, k, decay, v = self._operands(proj, at, status)
         call_hybrid("qd_gla_prepare", *[column(proj, at[n]) for n in "qkv"], proj.shape[1], ptr(decay), ptr(self.w.a2_b), m.tau, ptr(q),
                     ptr(k), ptr(decay), ptr(v), tokens, m.heads, m.dim, m.vdim, DTYPE_CODE[proj.dtype], stream_of(proj))
-        return self._walk(q, k, decay, v, None, None, history, proj, at["g"], SILU, proj.dtype)
+        return self._walk(q, k, decay, v, None, None, history, proj, at["g"], SILU, proj.dtype, status)
 
     def step(self, proj, at, history: LayerHistory, position, status):
         m = self.m
@@ -297,7 +317,7 @@ class GatedLinearAttention(LinearRecurrence):
 
 class ChannelDelta(LinearRecurrence):
     def __init__(self, weights: ChannelDeltaWeights, m: ChannelDeltaConfig, eps: float, device):
-        super().__init__(weights, m, eps, m.kv_heads)
+        super().__init__(weights, m, eps, m.kv_heads, device)
         self.projections = {"q": weights.q, "k": weights.k, "v": weights.v, "b": weights.b, "a1": weights.a1, "g1": weights.g1}
 
     def _convolution(self, history):
@@ -314,7 +334,7 @@ class ChannelDelta(LinearRecurrence):
                     m.heads, m.kv_heads, m.dim, m.vdim, DTYPE_CODE[proj.dtype], stream_of(proj))
         gate = torch.empty((tokens, self.out_columns), dtype=proj.dtype, device=dev)
         linear(proj, at["g1"], proj.shape[1], self.w.g2, gate, tokens=tokens, status=status)
-        return self._walk(q, k, decay, v, beta, scales, history, gate, 0, SIGMOID, proj.dtype)
+        return self._walk(q, k, decay, v, beta, scales, history, gate, 0, SIGMOID, proj.dtype, status)
 
     def step(self, proj, at, history: LayerHistory, position, status):
         m = self.m

@@ -555,3 +555,64 @@ def test_fp32_rows_with_infinite_weights(M, monkeypatch, tokens, rows, width, ad
     want = (torch.zeros_like(out) if not add else out).double().cpu() + sum(x[:, None, k].double() * w[None, :, k].double() for k in range(width))
     M.linear(x.cuda(), 0, width, w.cuda(), out, tokens=tokens, status=stat, add=add)
     torch.testing.assert_close(out.cpu().double(), want, rtol=1e-5, atol=1e-4, equal_nan=True)
+
+
+# ------------------------------------------------------------------- recurrences sixteen tokens at a time
+def recurrence_inputs(tokens, heads, kv_heads, vdim, delta, seed=3):
+    """q, k, decay - 1, v, step sizes, scales, state of a recurrence with fast and slow decays, and results and last state in 64 bits."""
+    q, k, v = rnd(tokens, kv_heads, 128, seed=seed), rnd(tokens, kv_heads, 128, seed=seed + 1), rnd(tokens, heads, vdim, seed=seed + 2)
+    fade = torch.nn.functional.softplus(rnd(tokens, heads, 128, seed=seed + 3) + 3.0 * rnd(heads, 128, seed=seed + 4) - 2.0)
+    g, state, beta, scales = torch.expm1(-fade), rnd(heads, 128, vdim, seed=seed + 5, std=0.3), None, None
+    if delta:
+        beta = torch.sigmoid(rnd(tokens, heads, seed=seed + 6))
+        ks, qs = torch.rsqrt(k.square().sum(-1) + 1e-6), torch.rsqrt(q.square().sum(-1) + 1e-6) * 128 ** -0.5
+        scales = torch.stack([ks, qs, (q * k).sum(-1) * ks * qs], -1).contiguous()
+    s, out, share = state.to(F64), torch.empty(tokens, heads, vdim, dtype=F64), heads // kv_heads
+    for t in range(tokens):
+        kt, qt = k[t].to(F64), q[t].to(F64)
+        if delta:
+            kt, qt = kt * scales[t, :, :1].to(F64), qt * scales[t, :, 1:2].to(F64)
+        kt, qt, u = kt.repeat_interleave(share, 0), qt.repeat_interleave(share, 0), v[t].to(F64)
+        s = s + s * g[t].to(F64)[..., None]
+        if delta:
+            u = beta[t].to(F64)[:, None] * (u - (kt[:, None] @ s)[:, 0])
+        s = s + kt[..., None] * u[:, None]
+        out[t] = (qt[:, None] @ s)[:, 0]
+    return (q, k, g, v, beta, scales, state), out, s
+
+
+def run_chunked(inputs, tokens, heads, kv_heads, vdim, delta):
+    from quickdraw_b200._lib import call_hybrid, ptr, size_hybrid, stream_of
+    q, k, g, v, beta, scales, state = (None if x is None else x.cuda() for x in inputs)
+    out, stat = torch.full((tokens, heads, vdim), float("nan"), device="cuda"), status()
+    scratch = torch.empty(size_hybrid("qd_channel_chunk_scratch_bytes", tokens, heads), dtype=torch.uint8, device="cuda")
+    call_hybrid("qd_channel_recurrence_chunked", ptr(q), ptr(k), ptr(g), ptr(v), ptr(beta), ptr(scales), ptr(state), ptr(out), tokens, heads,
+                kv_heads, 128, vdim, int(delta), ptr(scratch), ptr(stat), stream_of(q))
+    assert int(stat) == 0
+    return out.cpu(), state.cpu()
+
+
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("tokens,heads,kv_heads,vdim", [(1, 2, 2, 16), (15, 2, 1, 48), (16, 1, 1, 128), (17, 3, 1, 32), (33, 4, 2, 80), (112, 2, 2, 256),
+                                                        (47, 40, 20, 64), (640, 64, 32, 16)])
+def test_recurrence_in_chunks(delta, tokens, heads, kv_heads, vdim):
+    """Ends of chunks, one and two slices of columns to a block, more chunks than the scratch area takes at once (640 tokens of 64
+    heads), against 64 bits.  A token's arithmetic is fp32 (6e-8 a rounding, some ten of them on the way of a value): 1e-6."""
+    kv_heads = kv_heads if delta else heads
+    inputs, want, last = recurrence_inputs(tokens, heads, kv_heads, vdim, delta)
+    out, state = run_chunked(inputs, tokens, heads, kv_heads, vdim, delta)
+    assert error(out, want) < 1e-6 and error(state, last) < 1e-6
+
+
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_recurrence_in_chunks_keeps_to_the_past(delta, bad):
+    """A value that is not finite reaches its column from its token on and nothing else."""
+    tokens, heads, vdim = 40, 2, 32
+    inputs, want, _ = recurrence_inputs(tokens, heads, heads, vdim, delta)
+    inputs[3][21, 1, 5] = bad
+    out, _ = run_chunked(inputs, tokens, heads, heads, vdim, delta)
+    reached = torch.zeros(tokens, heads, vdim, dtype=torch.bool)
+    reached[21:, 1, 5] = True
+    assert not torch.isfinite(out[reached]).any()
+    assert error(out[~reached], want[~reached]) < 1e-6

@@ -319,3 +319,14 @@ def test_small_fp32_products_keep_the_fma_tiles(recorder):
         recorder.clear()
         mixers.linear(x, 0, width, w, out, tokens=tokens, status=torch.zeros(1, dtype=torch.int32))
         assert [name for name, _ in recorder] == ["qd_linear_pieces" if pieces else "qd_linear"], (tokens, rows, width)
+
+
+def test_which_recurrences_go_in_chunks():
+    """The lines that were measured: heads of 128 keys, value columns in slices of sixteen, enough tokens, and not where segments are faster."""
+    from types import SimpleNamespace
+    from quickdraw_b200.mixers import chunked_recurrence
+    takes = lambda tokens, delta, heads=16, dim=128, vdim=128: chunked_recurrence(SimpleNamespace(heads=heads, dim=dim, vdim=vdim), tokens, delta, 148)
+    assert takes(2, False) and takes(2048, False) and takes(2048, False, heads=8) and takes(1000, False, heads=4)
+    assert not takes(1001, False, heads=4) and not takes(777, False, vdim=16) and takes(128, False, vdim=16)
+    assert takes(24, True) and not takes(23, True) and takes(80, True, heads=32) and not takes(79, True, heads=32)
+    assert not takes(512, True, dim=96) and not takes(512, False, dim=256) and not takes(512, True, vdim=24)
