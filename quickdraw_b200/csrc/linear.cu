@@ -2,7 +2,8 @@
 // same launch: a bias, the exact GELU on the leading columns (the up projection of a feed-forward whose
 // launch also carries other rows), a gated linear unit over neighbouring weight rows, the addition to
 // what y already holds (a residual stream).  What may precede it for few token rows: the RMS norm of x.
-// Four forms, the last one behind an entry point of its own:
+// Five forms, the last one behind an entry point of its own:
+//   linear_pair_kernel  bf16 x and enough tiles of 256 tokens by 256 outputs: pairs of SMs (linear_pair.cuh)
 //   linear_umma_kernel  many token rows, bf16 x: tcgen05.mma kind::f16, both operands by tiled TMA
 //                       (128-byte swizzle), accumulators in tensor memory.  Tensor-bound.
 //   linear_rows_kernel  up to eight token rows: a warp streams whole weight rows (16-byte loads, the
@@ -183,14 +184,14 @@ linear_tile_kernel(const TX* __restrict__ x, long long ldx, const bf16* __restri
 // ------------------------------------------------------------------------------- tensor cores
 constexpr int kStepK = 64;                     // inputs per stage: one 128-byte swizzled row
 
-// Tile of HALVES x 128 tokens by TN weight rows; warp 0 issues the TMA loads, warp 1 the MMAs, four warps
-// per token half read the accumulators back (a warp may read the tensor-memory lanes 32 (warp mod 4) ..).
-template <int HALVES, int TN> struct UmmaTile {
-    static constexpr int kABytes = HALVES * 128 * 128, kBBytes = TN * 128, kStageBytes = kABytes + kBBytes;
-    static constexpr int kStages = HALVES == 2 ? 3 : (TN == 256 ? 4 : 3);
-    static constexpr int kCols = HALVES * TN;
-    static constexpr int kThreads = 64 + HALVES * 128;
-    static constexpr int kBlocksPerSm = (HALVES == 1 && TN <= 128) ? 2 : 1;
+// Tile of 128 tokens by TN weight rows; warp 0 issues the TMA loads, warp 1 the MMAs, four warps
+// read the accumulators back (a warp may read the tensor-memory lanes 32 (warp mod 4) ..).
+template <int TN> struct UmmaTile {
+    static constexpr int kABytes = 128 * 128, kBBytes = TN * 128, kStageBytes = kABytes + kBBytes;
+    static constexpr int kStages = TN == 256 ? 4 : 3;
+    static constexpr int kCols = TN;
+    static constexpr int kThreads = 192;
+    static constexpr int kBlocksPerSm = TN <= 128 ? 2 : 1;
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
 };
 
@@ -254,12 +255,12 @@ QD_DEVINL void finish8(const LinearParams& p, float (&f)[8], TY* row, int n, con
     store4(row + n + 4, make_float4(f[4], f[5], f[6], f[7]));
 }
 
-template <typename TY, int HALVES, int TN>
-__global__ void __launch_bounds__(UmmaTile<HALVES, TN>::kThreads, UmmaTile<HALVES, TN>::kBlocksPerSm)
+template <typename TY, int TN>
+__global__ void __launch_bounds__(UmmaTile<TN>::kThreads, UmmaTile<TN>::kBlocksPerSm)
 linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant__ CUtensorMap xmap,
                    const __grid_constant__ CUtensorMap wmap) {
     chain_enter();
-    using Tile = UmmaTile<HALVES, TN>;
+    using Tile = UmmaTile<TN>;
     constexpr int kStages = Tile::kStages;
     // fp32 accumulator (bits [4,6) = 1), bf16 A and B (bits [7,10), [10,13) = 1), K-major, N >> 3 at 17, M >> 4 at 24
     constexpr uint32_t kDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -271,12 +272,11 @@ linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     uint32_t* slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* failed = reinterpret_cast<volatile int*>(slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int t0 = blockIdx.x * HALVES * 128, n0 = blockIdx.y * TN;
+    const int t0 = blockIdx.x * 128, n0 = blockIdx.y * TN;
     const int steps = (p.width + kStepK - 1) / kStepK;
     __shared__ __align__(16) float bias[TN];
     if (p.f.bias)
         for (int i = tid; i < TN; i += Tile::kThreads) bias[i] = n0 + i < p.rows ? p.f.bias[n0 + i] : 0.f;
-    const int halves = (HALVES == 2 && p.tokens - t0 > 128) ? 2 : 1;       // a half without tokens is not multiplied
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
@@ -319,28 +319,25 @@ linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + Tile::kABytes;
-#pragma unroll 1
-                for (int h = 0; h < halves; ++h)
 #pragma unroll
-                    for (int j = 0; j < kStepK / 16; ++j)
-                        umma_f16(tmem + h * TN, desc_sw128(a + h * 128 * 128 + j * 32), desc_sw128(b + j * 32), kDesc, (s | j) ? 1u : 0u);
+                for (int j = 0; j < kStepK / 16; ++j) umma_f16(tmem, desc_sw128(a + j * 32), desc_sw128(b + j * 32), kDesc, (s | j) ? 1u : 0u);
                 umma_commit_to(empty + st);
             }
             if (ok) umma_commit_to(done);
             else *failed = 1;
         }
     } else {
-        const int half = (warp - 2) >> 2, quadrant = warp & 3;
+        const int quadrant = warp & 3;
         const bool ok = mbar_wait(done, 0, p.status) && !*failed;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok && half < halves) {
-            const int t = t0 + half * 128 + quadrant * 32 + lane;
+        if (ok) {
+            const int t = t0 + quadrant * 32 + lane;
             TY* row = reinterpret_cast<TY*>(p.y) + (long long)t * p.ldy;
 #pragma unroll 1
             for (int c = 0; c < TN; c += 32) {
                 if (n0 + c >= p.rows) break;
                 uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(quadrant * 32) << 16) + half * TN + c, v);
+                tmem_ld32(tmem + ((uint32_t)(quadrant * 32) << 16) + c, v);
                 if (t < p.tokens) {
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
@@ -361,6 +358,14 @@ linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Tile::kCols) : "memory");
 }
+
+}  // namespace
+}  // namespace qd
+
+#include "linear_pair.cuh"
+
+namespace qd {
+namespace {
 
 // ------------------------------------------------------------------ fp32 rows on the tensor cores
 // x = h + m + l with three bf16 pieces of eight significant bits each, cut off and not rounded, so that the three together
@@ -590,27 +595,42 @@ int tile_map(CUtensorMap* map, const void* base, long long rows, long long width
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? QD_OK : QD_ERR_LAUNCH;
 }
 
-template <typename TY, int HALVES, int TN>
+template <typename TY, int TN>
 int launch_umma(const void* x, long long ldx, const void* w, const LinearParams& p, cudaStream_t stream) {
-    using Tile = UmmaTile<HALVES, TN>;
-    if (!allow_smem(linear_umma_kernel<TY, HALVES, TN>, Tile::kSmem)) return QD_ERR_LAUNCH;
+    using Tile = UmmaTile<TN>;
+    if (!allow_smem(linear_umma_kernel<TY, TN>, Tile::kSmem)) return QD_ERR_LAUNCH;
     alignas(64) CUtensorMap xmap = {}, wmap = {};
-    int rc = tile_map(&xmap, x, p.tokens, p.width, ldx, HALVES * 128);
+    int rc = tile_map(&xmap, x, p.tokens, p.width, ldx, 128);
     if (rc == QD_OK) rc = tile_map(&wmap, w, p.rows, p.width, p.width, TN);
     if (rc != QD_OK) return rc;
-    const dim3 grid((p.tokens + HALVES * 128 - 1) / (HALVES * 128), (p.rows + TN - 1) / TN);
-    return qd_launch(linear_umma_kernel<TY, HALVES, TN>, grid, dim3(Tile::kThreads), Tile::kSmem, stream, 1, p, xmap, wmap);
+    const dim3 grid((p.tokens + 128 - 1) / (128), (p.rows + TN - 1) / TN);
+    return qd_launch(linear_umma_kernel<TY, TN>, grid, dim3(Tile::kThreads), Tile::kSmem, stream, 1, p, xmap, wmap);
+}
+
+template <typename TY>
+int launch_pair(const void* x, long long ldx, const void* w, const LinearParams& p, cudaStream_t stream) {
+    using Tile = PairTile;
+    if (!allow_smem(linear_pair_kernel<TY>, Tile::kSmem)) return QD_ERR_LAUNCH;
+    alignas(64) CUtensorMap xmap = {}, wmap = {};
+    int rc = tile_map(&xmap, x, p.tokens, p.width, ldx, Tile::kRows / 2);
+    if (rc == QD_OK) rc = tile_map(&wmap, w, p.rows, p.width, p.width, Tile::kRows / 2);
+    if (rc != QD_OK) return rc;
+    const long long tiles = (long long)((p.tokens + Tile::kRows - 1) / Tile::kRows) * ((p.rows + Tile::kRows - 1) / Tile::kRows), pairs = device_sms() / 2;
+    return qd_launch(linear_pair_kernel<TY>, dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))), dim3(Tile::kThreads), Tile::kSmem, stream,
+                     1, p, xmap, wmap);
 }
 
 template <typename TY>
 int umma_dispatch(const void* x, long long ldx, const void* w, const LinearParams& p, cudaStream_t stream) {
     const long long sms = device_sms();
     const auto tiles = [&](int tm, int tn) { return (long long)((p.tokens + tm - 1) / tm) * ((p.rows + tn - 1) / tn); };
+    // half of the pairs with a tile, and both blocks of a pair with tokens (34 / 48 / 64 tiles 17.3 / 17.9 / 18.4 us against 18.2 / 21.1 / 19.9 in the
+    // tiles below, of 2048 inputs; 32 tiles 16.7 against 15.5, 64 tiles of 128 tokens 19.0 against 17.3)
+    if (p.tokens > 128 && tiles(256, 256) * 4 >= sms) return launch_pair<TY>(x, ldx, w, p, stream);
     // the largest tile that still gives most SMs one (a larger tile reads each operand fewer times)
-    if (tiles(256, 256) * 4 >= sms * 3) return launch_umma<TY, 2, 256>(x, ldx, w, p, stream);
-    if (tiles(128, 256) * 4 >= sms * 3) return launch_umma<TY, 1, 256>(x, ldx, w, p, stream);
-    if (tiles(128, 128) * 4 >= sms * 3) return launch_umma<TY, 1, 128>(x, ldx, w, p, stream);
-    return launch_umma<TY, 1, 64>(x, ldx, w, p, stream);
+    if (tiles(128, 256) * 4 >= sms * 3) return launch_umma<TY, 256>(x, ldx, w, p, stream);
+    if (tiles(128, 128) * 4 >= sms * 3) return launch_umma<TY, 128>(x, ldx, w, p, stream);
+    return launch_umma<TY, 64>(x, ldx, w, p, stream);
 }
 
 template <typename TX, typename TY, int R>

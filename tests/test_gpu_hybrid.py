@@ -45,6 +45,35 @@ SHAPES = [(1, 200, 256), (2, 33, 1032), (3, 8, 4104), (7, 5000, 64), (8, 77, 24)
           (64, 24, 2056), (1100, 4104, 136), (40, 37, 50), (5, 19, 7), (70, 128, 9), (2600, 4160, 40)]
 
 
+@pytest.mark.parametrize("tokens,rows,width,y_type,finish", [
+    (129, 9472, 64, BF16, ""), (257, 4872, 200, BF16, "bias gelu"), (300, 9480, 72, BF16, "glu bias"), (255, 9480, 64, F32, "glu"), (1537, 1800, 40, F32, "gelu"),
+    (700, 3336, 136, BF16, "add bias"), (2049, 1288, 1032, F32, "add"), (4000, 4000, 128, BF16, "")])
+def test_linear_on_pairs(M, tokens, rows, width, y_type, finish):
+    """Tiles that end inside a block's half, one tile for each pair of SMs and several, everything that may follow the sums, and a
+    neighbour on the right of the outputs that stays."""
+    assert tokens > 128 and -(-tokens // 256) * -(-rows // 256) >= 37
+    x, w = bf(tokens, width, seed=1), bf(rows, width, seed=2, std=width ** -0.5)
+    cols, glu, gelu = rows // 2 if "glu" in finish else rows, "glu" in finish, rows // 3 if "gelu" in finish else 0
+    bias = rnd(rows, seed=3) if "bias" in finish else None
+    ldy = cols + 8 + -cols % 8
+    before = rnd(tokens, ldy, seed=4).to(y_type)
+    out, stat, want = before.cuda(), status(), x.double() @ w.double().T
+    if bias is not None:
+        want = want + bias.double()
+    want[:, :gelu] = O.gelu_erf(want[:, :gelu])
+    if glu:
+        want = torch.relu(want[:, 0::2]) * want[:, 1::2]
+    if "add" in finish:
+        want = want + before[:, :cols].double()
+    from quickdraw_b200._lib import call_hybrid, ptr, stream_of
+    x, w, bias = x.cuda(), w.cuda(), None if bias is None else bias.cuda()
+    call_hybrid("qd_linear", ptr(x), width, 0, ptr(w), ptr(out), ldy, M.DTYPE_CODE[y_type], tokens, rows, width, gelu, int(glu), ptr(bias),
+                int("add" in finish), None, 0.0, 0.0, ptr(stat), stream_of(x))
+    assert int(stat) == 0
+    assert error(out[:, :cols], want) < (2e-6 if y_type == F32 else 3e-3)      # sums in fp32; one rounding to bf16 (1.7e-3)
+    assert torch.equal(out[:, cols:].cpu(), before[:, cols:])
+
+
 @pytest.mark.parametrize("tokens,rows,width", SHAPES)
 @pytest.mark.parametrize("x_type,y_type", [(BF16, BF16), (BF16, F32), (F32, F32)])
 def test_linear(M, tokens, rows, width, x_type, y_type):
