@@ -2,10 +2,11 @@
 // same launch: a bias, the exact GELU on the leading columns (the up projection of a feed-forward whose
 // launch also carries other rows), a gated linear unit over neighbouring weight rows, the addition to
 // what y already holds (a residual stream).  What may precede it for few token rows: the RMS norm of x.
-// Five forms, the last one behind an entry point of its own:
+// Six forms, the last one behind an entry point of its own:
 //   linear_pair_kernel  bf16 x and enough tiles of 256 tokens by 256 outputs: pairs of SMs (linear_pair.cuh)
 //   linear_umma_kernel  many token rows, bf16 x: tcgen05.mma kind::f16, both operands by tiled TMA
 //                       (128-byte swizzle), accumulators in tensor memory.  Tensor-bound.
+//   linear_stream_kernel  one token, fewer than 32 weight rows an SM: two buffers of a row's pieces in registers.  HBM-bound, and by its start and end.
 //   linear_rows_kernel  up to eight token rows: a warp streams whole weight rows (16-byte loads, the
 //                       first inputs of each row - up to 4096 - requested before the wait for the
 //                       preceding kernel), the token rows in shared memory as fp32.  HBM-bound.
@@ -131,6 +132,92 @@ linear_rows_kernel(const TX* __restrict__ x, long long ldx, const bf16* __restri
             for (int r = 0; r < NR; ++r)
                 if (n0 + r < rows) put(y + t * ldy + n0 + r, finished(f, v[r], n0 + r), f.add);
         }
+    }
+}
+
+// One token.  A warp takes NR whole rows, P pieces of 256 inputs of each at a time, in two buffers: one that has been used is
+// filled again while the other is multiplied.  Both are requested before the wait for the preceding kernel; x lies in
+// shared memory as a whole.  Before, the form below was used for one token as well: rows of up to 2048 inputs left half of its registers
+// empty and needed two waves of blocks, longer ones were read in rounds.  Inside a graph, weights from HBM, inputs -> outputs: 2048 -> 4160 8.7 -> 4.3 us
+// (floor 2.6), 2048 -> 2048 4.4 -> 3.1, 1536 -> 3072 7.2 -> 2.8, 8192 -> 2048 10.8 -> 9.1 (5.2).  One buffer of the same size in half of the
+// registers spills or reads in rounds (7.3 us for the first); eight warps an SM with a ring of pieces a lane wait for its oldest load on all.
+constexpr int kStreamWidth = 24576;
+template <typename TX, typename TY, int NR, int P>
+__global__ void __launch_bounds__(256, 2)
+linear_stream_kernel(const TX* __restrict__ x, const bf16* __restrict__ w, TY* __restrict__ y, int rows, int width, const Finish f,
+                     const InputNorm norm) {
+    extern __shared__ __align__(16) float xs[];        // the row, zeros up to a multiple of 256 P
+    __shared__ float squares[8];
+    constexpr int kBatch = 256 * P;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (blockIdx.x * 8 + warp) * NR, padded = (width + kBatch - 1) / kBatch * kBatch;
+    uint4 wv[2][NR][P];
+    auto request = [&](uint4 (&to)[NR][P], int k0) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const int k = k0 + (i * 32 + lane) * 8;
+                to[r][i] = (n0 + r < rows && k < width) ? __ldg(reinterpret_cast<const uint4*>(w + (size_t)(n0 + r) * width + k)) : make_uint4(0u, 0u, 0u, 0u);
+            }
+    };
+    grid_launch_dependents();
+#pragma unroll
+    for (int b = 0; b < 2; ++b) request(wv[b], b * kBatch);
+    grid_dependency_wait();
+    float ss = 0.f;
+    for (int k = threadIdx.x * 4; k < padded; k += 1024) {
+        float4 v = k < width ? load4(x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (norm.weight && k < width) {
+            const float4 g = load4(norm.weight + k);
+            ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+            v.x *= norm.offset + g.x; v.y *= norm.offset + g.y; v.z *= norm.offset + g.z; v.w *= norm.offset + g.w;
+        }
+        *reinterpret_cast<float4*>(xs + k) = v;
+    }
+    if (norm.weight) {
+        ss = warp_sum(ss);
+        if (lane == 0) squares[warp] = ss;
+    }
+    __syncthreads();
+    float acc[NR][2];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) acc[r][0] = acc[r][1] = 0.f;
+    for (int k0 = 0; k0 < width; k0 += 2 * kBatch)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            if (b && k0 + b * kBatch >= width) break;
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const float* xk = xs + k0 + b * kBatch + (i * 32 + lane) * 8;
+                const float4 u = *reinterpret_cast<const float4*>(xk), v = *reinterpret_cast<const float4*>(xk + 4);
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    float wf[8];
+                    unpack8(wv[b][r][i], wf);
+                    acc[r][0] = fmaf(wf[0], u.x, fmaf(wf[1], u.y, fmaf(wf[2], u.z, fmaf(wf[3], u.w, acc[r][0]))));
+                    acc[r][1] = fmaf(wf[4], v.x, fmaf(wf[5], v.y, fmaf(wf[6], v.z, fmaf(wf[7], v.w, acc[r][1]))));
+                }
+            }
+            if (k0 + (2 + b) * kBatch < width) request(wv[b], k0 + (2 + b) * kBatch);
+        }
+    float factor = 1.f;                                // the same for every row: applied to the sums
+    if (norm.weight) {
+        float total = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) total += squares[i];
+        factor = 1.0f / sqrtf(total / (float)width + norm.eps);
+    }
+    float v[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) v[r] = warp_sum(acc[r][0] + acc[r][1]) * factor;
+    if (lane) return;
+    if (NR == 2 && f.glu) {
+        if (n0 < rows) put(y + n0 / 2, fmaxf(finished(f, v[0], n0), 0.f) * finished(f, v[NR - 1], n0 + 1), f.add);
+    } else {
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+            if (n0 + r < rows) put(y + n0 + r, finished(f, v[r], n0 + r), f.add);
     }
 }
 
@@ -644,11 +731,28 @@ int launch_rows(const void* x, long long ldx, const void* w, void* y, long long 
                      (const TX*)x, ldx, (const bf16*)w, (TY*)y, ldy, tokens, rows, width, f, norm);
 }
 
+template <typename TX, typename TY, int NR, int P>
+int launch_stream(const void* x, const void* w, void* y, int rows, int width, const Finish& f, const InputNorm& norm,
+                  cudaStream_t stream) {
+    const size_t smem = (size_t)(width + 256 * P - 1) / (256 * P) * P * 1024;
+    if (!allow_smem(linear_stream_kernel<TX, TY, NR, P>, smem)) return QD_ERR_LAUNCH;
+    return qd_launch(linear_stream_kernel<TX, TY, NR, P>, dim3((rows + 8 * NR - 1) / (8 * NR)), dim3(256), smem, stream, 2, (const TX*)x,
+                     (const bf16*)w, (TY*)y, rows, width, f, norm);
+}
+
 template <typename TX, typename TY>
 int dispatch(const void* x, long long ldx, const void* w, void* y, long long ldy, int tokens, int rows, int width,
              const Finish& f, const InputNorm& norm, unsigned int* status, cudaStream_t stream) {
     const bool vectors = width % 8 == 0 && ldx % 8 == 0 && aligned16(x) && aligned16(w);
     if (vectors && tokens <= 8 && (!norm.weight || ((uintptr_t)norm.weight & 7u) == 0)) {
+        // One token, below the size from which the form for several tokens keeps the SMs full with small blocks (inputs -> outputs, weights
+        // from HBM: 2048 -> 6144 5.9 us there and 6.4 here, 2048 -> 8192 6.6 / 7.2).  Up to sixteen rows an SM a row to a warp (2048 -> 2048 3.1 us, two
+        // rows 3.4), from there on, for narrow rows and for pairs two (2048 -> 3072 2.8, one row 4.7; 1024 -> 2080 2.4 / 2.8).
+        const int sms = device_sms();
+        if (tokens == 1 && width <= kStreamWidth && rows < 32 * sms) {
+            if (!f.glu && rows <= 16 * sms && width > 1024) return launch_stream<TX, TY, 1, 8>(x, w, y, rows, width, f, norm, stream);
+            return launch_stream<TX, TY, 2, 4>(x, w, y, rows, width, f, norm, stream);
+        }
         if (tokens == 1) return launch_rows<TX, TY, 1>(x, ldx, w, y, ldy, tokens, rows, width, f, norm, stream);
         if (tokens == 2) return launch_rows<TX, TY, 2>(x, ldx, w, y, ldy, tokens, rows, width, f, norm, stream);
         if (tokens <= 4) return launch_rows<TX, TY, 4>(x, ldx, w, y, ldy, tokens, rows, width, f, norm, stream);

@@ -74,6 +74,32 @@ def test_linear_on_pairs(M, tokens, rows, width, y_type, finish):
     assert torch.equal(out[:, cols:].cpu(), before[:, cols:])
 
 
+@pytest.mark.parametrize("rows,width,finish", [(9, 8, ""), (2369, 1032, "bias"), (2368, 1024, "add"), (1000, 2048, "gelu norm"), (2360, 6152, "norm add"), (4735, 520, ""),
+                                               (4734, 4104, "glu norm"), (30, 24576, "glu"), (17, 24584, "norm"), (4736, 64, "")])
+@pytest.mark.parametrize("x_type", [BF16, F32])
+def test_linear_of_one_token(M, rows, width, finish, x_type):
+    """Rows that end inside a piece, a batch and a pair of batches, one and two rows to a warp, both sides of the lines between the forms."""
+    x, w = rnd(1, width, seed=1).to(x_type), bf(rows, width, seed=2, std=width ** -0.5)
+    glu, gelu, add = "glu" in finish, rows // 3 if "gelu" in finish else 0, "add" in finish
+    bias, norm = rnd(rows, seed=3) if "bias" in finish else None, bf(width, seed=5) if "norm" in finish else None
+    out = rnd(1, rows // 2 if glu else rows, seed=4)
+    want = x.double()
+    if norm is not None:
+        want = want * torch.rsqrt(want.square().mean() + 1e-6) * (1.0 + norm.double())
+    want = want @ w.double().T
+    if bias is not None:
+        want = want + bias.double()
+    want[:, :gelu] = O.gelu_erf(want[:, :gelu])
+    if glu:
+        want = torch.relu(want[:, 0::2]) * want[:, 1::2]
+    if add:
+        want = want + out.double()
+    got, stat = out.cuda(), status()
+    M.linear(x.cuda(), 0, width, w.cuda(), got, tokens=1, status=stat, gelu_columns=gelu, glu=glu, bias=None if bias is None else bias.cuda(), add=add,
+             norm=None if norm is None else norm.cuda(), norm_offset=1.0, eps=1e-6)
+    assert int(stat) == 0 and error(got, want) < 2e-6
+
+
 @pytest.mark.parametrize("tokens,rows,width", SHAPES)
 @pytest.mark.parametrize("x_type,y_type", [(BF16, BF16), (BF16, F32), (F32, F32)])
 def test_linear(M, tokens, rows, width, x_type, y_type):
