@@ -8,17 +8,17 @@
 // rounding): after the first tiles a warp hardly ever reads O before the end.  (Conditional rescaling is published with
 // FlashAttention-4.)
 //   warps 0 .. 4 TILES - 1   softmax, one row a thread; then the epilogue, for one row tile together with the loading warps
-//   warp 4 TILES             issues the MMAs: S of tile i + 1 before O of tile i, so that the softmax and the products overlap
+//   warps 4 TILES .. 5 TILES - 1   issue the MMAs of a row tile each: S of key tile i + 1 before O of tile i, so that softmax and products overlap
 //   the rest                 keys and values into the 128-byte swizzled layout, two stages of each: by tiled TMA where a tile's 64
 //                            rows lie together, else (the last tile, the ring's end) row by row with cp.async, zeros past the end
 // Values are read as they lie (rows of a key, the result's columns innermost): a B operand with the columns as the major
 // dimension.  Every wait is bounded; a block whose wait ran out writes NaN.
 //
 // Measured (2048 tokens, with the launch gap; before: mma.sync, eight or sixteen rows a warp).  Head dimension 256, 16/2 heads:
-// behind 0 / 2000 / 30000 positions 108 / 203 / 1582 us (478 / 1017 / 7949), 128 tokens behind 0 / 500
-// positions 26 / 37 us (50 / 112).  128 columns, window 1024: 16/4 heads 58 us (243), 16 heads with 64 shared key columns 75 us (293).  A key tile takes 3000 clocks at head dimension 256: 1800 of
-// MMAs (those of S are bound by shared memory, 48 clocks for 64 columns), 1100 of keys and values at 64 bytes a clock, and the
-// hand-over of S and P.
+// behind 0 / 2048 / 6144 positions 106 / 193 / 365 us (2000 positions by mma.sync 1017), 128 and 16 tokens behind 500 positions 36 and 33 us.  128 columns, window
+// 1024: 16/4 heads 48 us (243), 16 heads with 64 shared key columns 64 us (293).  With one warp issuing for both row tiles, and a descriptor built
+// for every MMA, these were 110 / 207 / 402, 38 and 35, 55 and 73: that warp took 4200 clocks for a key tile, 90 an MMA.  Now a key tile takes
+// 2300 clocks at 192 + 128 columns, of which the tensor core has 2180 (a product of S is bound by shared memory: 48 clocks for 64 columns).
 // One piece, eight bits, took 120 / 199 / 1290 us there where two took 129 / 225 / 1611 (before the epilogue was shared), but since the largest P is not one here (the reference lags behind the
 // maximum) its rounding reaches the result: 2.04e-3 from 64 bits with sharp scores, where the result's own rounding is 1.65e-3
 // and mma.sync with the exact maximum had 1.72e-3.  Two pieces: 1.65e-3.
@@ -32,7 +32,7 @@
 namespace qd {
 namespace flash {
 
-constexpr int kKeys = 64, kThreads = 13 * 32;
+constexpr int kKeys = 64;
 
 struct In {
     const bf16* q;                         // [tokens, heads, QD]
@@ -53,23 +53,24 @@ QD_DEVINL int lowest(const In& p, int position) {
     return max(0, position - p.span + 1);
 }
 
-QD_DEVINL uint64_t desc_k(uint32_t addr) {          // K-major, 128-byte swizzle
-    return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// MN-major, 128-byte swizzle: 64 columns innermost, eight rows of K to a 1024-byte group; `apart` bytes to the next 64 columns
-QD_DEVINL uint64_t desc_mn(uint32_t addr, uint32_t apart) {
-    return (uint64_t)((addr >> 4) & 0x3fffu) | ((uint64_t)(apart >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
+// Shared-memory descriptors, lower words; the upper one is the same for all: 1024 bytes between groups of eight rows, 128-byte swizzle.
+// The products walk by adding to them (16-byte units): a descriptor built anew for every MMA made the issuing warp the bound (90 clocks an MMA).
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (1u << 30);
+QD_DEVINL uint32_t desc_k(uint32_t addr) { return ((addr >> 4) & 0x3fffu) | (1u << 16); }          // K-major
+// MN-major: 64 columns innermost; `apart` bytes to the next 64 columns
+QD_DEVINL uint32_t desc_mn(uint32_t addr, uint32_t apart) { return ((addr >> 4) & 0x3fffu) | ((apart >> 4) << 16); }
 constexpr uint32_t idesc(int n, int b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
-QD_DEVINL void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t i, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d), "l"(a), "l"(b), "r"(i), "r"(accumulate) : "memory");
+QD_DEVINL void mma_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t i, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b), "r"(i), "r"(kDescHigh), "r"(accumulate) : "memory");
 }
-QD_DEVINL void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t i, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(d), "r"(a), "l"(b), "r"(i), "r"(accumulate) : "memory");
+QD_DEVINL void mma_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t i, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b), "r"(i), "r"(kDescHigh), "r"(accumulate) : "memory");
 }
 QD_DEVINL void commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -128,7 +129,8 @@ QD_DEVINL uint32_t pair(float lo, float hi) {
 
 template <int QD, int DV, int TILES>
 struct Shape {
-    static constexpr int kLoaders = 13 - 1 - 4 * TILES, kPerStage = kLoaders / 4;        // loader warps; of one stage of keys or values
+    static constexpr int kLoaders = 12 - 4 * TILES, kPerStage = kLoaders / 4;            // loader warps; of one stage of keys or values
+    static constexpr int kThreads = 32 * (5 * TILES + kLoaders);
     static constexpr int kScores = TILES == 1 ? 3 : 2;                                  // score buffers of a row tile
     static constexpr int kTileCols = DV + kScores * kKeys;
     static constexpr int kQBytes = TILES * 128 * QD * 2, kKBytes = kKeys * QD * 2, kVBytes = kKeys * DV * 2;
@@ -181,7 +183,7 @@ __device__ __noinline__ void plain_columns(const In& p, const Out& out, unsigned
 // Out: called per row and 32 columns as out(token, head, c0, o, m, l) with the unnormalised columns c0 .. c0 + 31 and the row's
 // softmax state (log2 of the reference, the sum relative to it); l NaN marks a failed wait.
 template <int QD, int DV, int TILES, typename Out>
-__global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_constant__ In p, const __grid_constant__ Maps maps, const __grid_constant__ Out out) {
+__global__ void __launch_bounds__(Shape<QD, DV, TILES>::kThreads, 1) flash_umma_kernel(const __grid_constant__ In p, const __grid_constant__ Maps maps, const __grid_constant__ Out out) {
     chain_enter();
     using S = Shape<QD, DV, TILES>;
     extern __shared__ __align__(16) uint8_t flash_raw[];        // (the largest alignment of a file holds for all its kernels)
@@ -203,14 +205,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(bars->k_full + s, S::kPerStage); mbar_init(bars->v_full + s, S::kPerStage);
-            mbar_init(bars->k_empty + s, 1); mbar_init(bars->v_empty + s, 1);
+            mbar_init(bars->k_empty + s, TILES); mbar_init(bars->v_empty + s, TILES);
             for (int t = 0; t < TILES; ++t) mbar_init(&bars->o_done[t][s], 1);
         }
         for (int t = 0; t < TILES; ++t)
             for (int s = 0; s < 3; ++s) { mbar_init(&bars->s_full[t][s], 1); mbar_init(&bars->p_full[t][s], 4); }
         mbar_init(&bars->q_full, 4 * TILES);
         mbar_init(&bars->stats_full, 4);
-        mbar_init(&bars->drained, 1);
+        mbar_init(&bars->drained, TILES);
         mbar_fence_init();
     }
     if (warp == kMma) {
@@ -238,9 +240,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
         }
     };
 
-    if (warp > kMma) {
+    if (warp >= kMma + TILES) {
         // ---- keys and values: warps of (matrix, stage) take every second tile
-        const int w = warp - kMma - 1, part = w >> 2, stage = w & 1, values = (w >> 1) & 1;
+        const int w = warp - kMma - TILES, part = w >> 2, stage = w & 1, values = (w >> 1) & 1;
         constexpr int kRowsEach = kKeys / S::kPerStage;
         const uint32_t dst = smem_u32(values ? vs + stage * S::kVBytes : ks + stage * S::kKBytes);
         uint64_t* full = (values ? bars->v_full : bars->k_full) + stage;
@@ -311,57 +313,51 @@ __global__ void __launch_bounds__(kThreads, 1) flash_umma_kernel(const __grid_co
             fence_after();
             finish(0, r0 + r, ml.x, ml.y, 1 + (w >> 2));
         }
-    } else if (warp == kMma) {
+    } else if (warp >= kMma) {
+        const int t = warp - kMma;
         const bool leader = elected();
-        const uint32_t qa = smem_u32(smem), ka = smem_u32(ks), va = smem_u32(vs);
+        const uint32_t qa = desc_k(smem_u32(smem) + t * (128 * QD * 2)), ka = desc_k(smem_u32(ks)), va = desc_mn(smem_u32(vs), kKeys * 128);
+        const uint32_t o_at = tmem + t * S::kTileCols;
         bool ok = true;
-        const auto scores = [&](int t, int i) {                              // S of row tile t, key tile i
-            const uint32_t d = tmem + t * S::kTileCols + DV + (i % S::kScores) * kKeys, a = qa + t * (128 * QD * 2), b = ka + (i & 1) * S::kKBytes;
+        const auto scores = [&](int i) {                                     // S of key tile i
+            const uint32_t d = o_at + DV + (i % S::kScores) * kKeys, b = ka + (i & 1) * (S::kKBytes >> 4);
 #pragma unroll
             for (int j = 0; j < QD / 16; ++j)
-                mma_ss(d, desc_k(a + (j >> 2) * 16384 + (j & 3) * 32), desc_k(b + (j >> 2) * (kKeys * 128) + (j & 3) * 32), idesc(kKeys, 0), j ? 1u : 0u);
+                mma_ss(d, qa + (j >> 2) * (16384 >> 4) + (j & 3) * 2, b + (j >> 2) * (kKeys * 128 >> 4) + (j & 3) * 2, idesc(kKeys, 0), j ? 1u : 0u);
             commit(&bars->s_full[t][i % S::kScores]);
+            commit(bars->k_empty + (i & 1));
         };
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->q_full, 0, nullptr) && mbar_wait(bars->k_full, 0, nullptr));
         if (ok) {
             fence_after();
-            if (leader) {
-                for (int t = 0; t < TILES; ++t) scores(t, 0);
-                commit(bars->k_empty);
-            }
+            if (leader) scores(0);
             __syncwarp();
         }
         for (int i = 0; i < tiles && ok; ++i) {
-            if (i + 1 < tiles) ok = __all_sync(0xffffffffu, mbar_wait(bars->k_full + ((i + 1) & 1), ((i + 1) >> 1) & 1, nullptr));
+            if (i + 1 < tiles) {
+                const int before = i + 1 - S::kScores;                        // the probabilities that lie where these scores go are read
+                ok = __all_sync(0xffffffffu, mbar_wait(bars->k_full + ((i + 1) & 1), ((i + 1) >> 1) & 1, nullptr) &&
+                                                 (before < 0 || mbar_wait(&bars->o_done[t][before & 1], (before >> 1) & 1, nullptr)));
+                fence_after();
+                if (ok && leader) scores(i + 1);
+                __syncwarp();
+            }
+            if (ok)
+                ok = __all_sync(0xffffffffu, mbar_wait(bars->v_full + (i & 1), (i >> 1) & 1, nullptr) &&
+                                                 mbar_wait(&bars->p_full[t][i % S::kScores], (i / S::kScores) & 1, nullptr));
+            if (ok) {
+                fence_after();
+                if (leader) {
+                    const uint32_t a = o_at + DV + (i % S::kScores) * kKeys, b = va + (i & 1) * (S::kVBytes >> 4);
 #pragma unroll
-            for (int t = 0; t < TILES; ++t) {
-                if (ok && i + 1 < tiles) {
-                    const int before = i + 1 - S::kScores;                    // the probabilities that lie where these scores go are read
-                    if (before >= 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t][before & 1], (before >> 1) & 1, nullptr));
-                    fence_after();
-                    if (ok && leader) {
-                        scores(t, i + 1);
-                        if (t == TILES - 1) commit(bars->k_empty + ((i + 1) & 1));
+                    for (int j = 0; j < kKeys / 16; ++j) {
+                        mma_ts(o_at, a + j * 8, b + j * (2048 >> 4), idesc(DV, 1), (i | j) ? 1u : 0u);
+                        mma_ts(o_at, a + 32 + j * 8, b + j * (2048 >> 4), idesc(DV, 1), 1u);
                     }
-                    __syncwarp();
+                    commit(&bars->o_done[t][i & 1]);
+                    commit(bars->v_empty + (i & 1));
                 }
-                if (ok && t == 0) ok = __all_sync(0xffffffffu, mbar_wait(bars->v_full + (i & 1), (i >> 1) & 1, nullptr));
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->p_full[t][i % S::kScores], (i / S::kScores) & 1, nullptr));
-                if (ok) {
-                    fence_after();
-                    if (leader) {
-                        const uint32_t d = tmem + t * S::kTileCols, a = d + DV + (i % S::kScores) * kKeys, b = va + (i & 1) * S::kVBytes;
-#pragma unroll
-                        for (int j = 0; j < kKeys / 16; ++j) {
-                            const uint64_t desc = desc_mn(b + j * 2048, kKeys * 128);
-                            mma_ts(d, a + j * 8, desc, idesc(DV, 1), (i | j) ? 1u : 0u);
-                            mma_ts(d, a + 32 + j * 8, desc, idesc(DV, 1), 1u);
-                        }
-                        commit(&bars->o_done[t][i & 1]);
-                        if (t == TILES - 1) commit(bars->v_empty + (i & 1));
-                    }
-                    __syncwarp();
-                }
+                __syncwarp();
             }
         }
         if (leader) commit(&bars->drained);                 // tensor memory is given back only behind the last MMA
@@ -503,7 +499,7 @@ int launch(In p, const Out& out, cudaStream_t stream) {
     }
     const long long rows = (long long)p.tokens * (p.heads / p.kv_heads);
     const dim3 grid(p.kv_heads, (unsigned)((rows + 128 * TILES - 1) / (128 * TILES)));
-    return qd_launch(flash_umma_kernel<QD, DV, TILES, Out>, grid, dim3(kThreads), smem, stream, 1, p, maps, out);
+    return qd_launch(flash_umma_kernel<QD, DV, TILES, Out>, grid, dim3(Shape<QD, DV, TILES>::kThreads), smem, stream, 1, p, maps, out);
 }
 
 }  // namespace flash
