@@ -13,36 +13,34 @@
 // are moved into tensor memory, the accumulator lives in tensor memory.  The result differs from
 // the W4A16 product by the activation rounding only; the exact path stays qd_nvfp4_matmul.
 //
-// Tile: 128 tokens x 128 weight rows per block, K in stages of 256 inputs (a 128-byte row of
+// Small products, nvfp4_gemm_w4a4_kernel: 128 tokens x 128 weight rows per block, K in stages of 256 inputs (a 128-byte row of
 // codes, sixteen scales).  Two blocks share an SM (3 stages of 36 KB and 256 columns of tensor
 // memory each), so one block's epilogue overlaps the other's K loop.
 //   warp 0      TMA: per stage four boxes (codes and scales of both operands)
 //   warp 1      allocates tensor memory, issues 4 MMAs of 128 x 128 x 64 per stage
 //   warps 2..5  move the stage's block scales shared memory -> tensor memory (every warp fills
 //               its own 32-lane quarter), then run the epilogue: one token per lane
+// Large ones, w4a4_pair_kernel: 256 x 256 tiles on pairs of SMs, see there.
 // Every wait is bounded; a wait that runs out sets the status word and the block leaves.
 #include <algorithm>
 
+#include "pair.cuh"
 #include "umma.cuh"
 
 namespace qd {
 namespace {
 
-constexpr int kTile = 128;                    // tokens per block (tensor-memory lanes)
-// Weight rows per block = columns of one MMA: template parameter TN.  128: 3 stages of 36 KB and
-// 256 tensor-memory columns, two blocks per SM.  256: 4 stages of 54 KB, all 512 columns, one block
-// per SM; a block-scaled MMA takes the same 152 clocks for 256 columns as for 128.
-constexpr int stages_of(int tn) { return tn == 128 ? 3 : 4; }
+constexpr int kTile = 128;                    // tokens and weight rows per block
+constexpr int kStages4 = 3;
 constexpr int kCodeBytes = kTile * 128;       // 128 rows x 256 inputs
 constexpr int kScaleBytes = kTile * 16;       // 128 rows x 16 scales
-constexpr int stage_bytes(int tn) { return (1 + tn / 128) * (kCodeBytes + kScaleBytes); }      // 36 / 54 KB
+constexpr int kStage4Bytes = 2 * (kCodeBytes + kScaleBytes);
 constexpr int kThreads4 = 6 * 32;
-constexpr uint32_t tmem_cols(int tn) { return tn == 128 ? 256u : 512u; }
-constexpr uint32_t kColAcc = 0;
+constexpr uint32_t kCols4 = 256, kColAcc = 0, kColSf = 128;
 // scale columns of a stage: 16 for the 128 tokens (four per 64-input step: rows l, l + 32, l + 64,
-// l + 96 of lane l), then four per step and 128 weight rows
-constexpr uint32_t sf_cols(int tn) { return 16u + 16u * (tn / 128); }
-constexpr uint32_t desc_of(int tn) { return (1u << 7) | (1u << 10) | (((uint32_t)tn >> 3) << 17) | ((128u >> 4) << 24); }
+// l + 96 of lane l), then as many for the weight rows
+constexpr uint32_t kSfCols = 32;
+constexpr uint32_t desc_of(int m, int n) { return (1u << 7) | (1u << 10) | (((uint32_t)n >> 3) << 17) | (((uint32_t)m >> 4) << 24); }
 
 struct Gemm4Params {
     const float* x_global; const float* w_global; bf16* y;
@@ -50,22 +48,30 @@ struct Gemm4Params {
     unsigned int* status;
 };
 
-struct Bars4 { uint64_t full[4], empty[4], sf_ready[4], done; };
+struct Bars4 { uint64_t full[kStages4], empty[kStages4], sf_ready[kStages4], done; };
 
-template <int TN>
-__global__ void __launch_bounds__(kThreads4, TN == 128 ? 2 : 1)
+// the scale words of rows l, l + 32, l + 64, l + 96 of lane l (rows of sixteen bytes from `from` on): four columns per 64-input step
+QD_DEVINL void scales_of_128(uint32_t to, const uint8_t* from, int lane) {
+    uint32_t w[16];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const uint4 v = *reinterpret_cast<const uint4*>(from + (lane + 32 * g) * 16);
+        w[0 + g] = v.x; w[4 + g] = v.y; w[8 + g] = v.z; w[12 + g] = v.w;
+    }
+    tmem_store16(to, w);
+}
+
+__global__ void __launch_bounds__(kThreads4, 2)
 nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ CUtensorMap x_codes,
                        const __grid_constant__ CUtensorMap x_scales, const __grid_constant__ CUtensorMap w_codes,
                        const __grid_constant__ CUtensorMap w_scales) {
     grid_dependency_wait();       // before the tensor memory: a block that waits for its predecessor must not hold what that one needs
     extern __shared__ __align__(1024) uint8_t gemm4_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm4_smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int kStages4 = stages_of(TN), kStage4Bytes = stage_bytes(TN), kHalves = TN / 128;
-    constexpr uint32_t kCols4 = tmem_cols(TN), kColSf = TN, kSfCols = sf_cols(TN);
     Bars4* bars = reinterpret_cast<Bars4*>(smem + kStages4 * kStage4Bytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int t0 = blockIdx.y * kTile, n0 = blockIdx.x * TN;
+    const int t0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
     const int chunks = p.in_features / 256;
 
     if (tid == 0) {
@@ -89,15 +95,12 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
                 // rows past the end of a matrix arrive as zeros; a box always counts in full
                 mbar_expect_tx(bars->full + st, kStage4Bytes);
                 uint8_t* base = stage(st);
-                // codes: tokens, then the weight rows (128 at a time); scales in the same order
-                uint8_t* sc = base + (1 + kHalves) * kCodeBytes;
+                // codes: tokens, then the weight rows; scales in the same order
+                uint8_t* sc = base + 2 * kCodeBytes;
                 tma_load_2d(base, &x_codes, c * 128, t0, bars->full + st);
                 tma_load_2d(sc, &x_scales, c * 16, t0, bars->full + st);
-#pragma unroll
-                for (int h = 0; h < kHalves; ++h) {
-                    tma_load_2d(base + (1 + h) * kCodeBytes, &w_codes, c * 128, n0 + h * 128, bars->full + st);
-                    tma_load_2d(sc + (1 + h) * kScaleBytes, &w_scales, c * 16, n0 + h * 128, bars->full + st);
-                }
+                tma_load_2d(base + kCodeBytes, &w_codes, c * 128, n0, bars->full + st);
+                tma_load_2d(sc + kScaleBytes, &w_scales, c * 16, n0, bars->full + st);
             }
         }
     } else if (warp == 1) {
@@ -113,7 +116,7 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
                 const uint32_t sfa = tmem + kColSf + st * kSfCols, sfb = sfa + 16;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)       // a 64-input step: 32 bytes further in both operands
-                    umma_nvfp4_lo(tmem + kColAcc, a_lo + 2 * j, b_lo + 2 * j, desc_of(TN), sfa + j * 4, sfb + j * 4 * kHalves,
+                    umma_nvfp4_lo(tmem + kColAcc, a_lo + 2 * j, b_lo + 2 * j, desc_of(128, 128), sfa + j * 4, sfb + j * 4,
                                   (c | j) ? 1u : 0u);
                 umma_commit(bars->empty + st);    // the stage (and its scale columns) is free once these MMAs are done
             }
@@ -127,29 +130,9 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
         for (int c = 0; c < chunks && ok; ++c) {
             const int st = c % kStages4;
             if (!mbar_wait(bars->full + st, (c / kStages4) & 1, p.status)) { ok = false; break; }
-            const uint8_t* sc = stage(st) + (1 + kHalves) * kCodeBytes;
-            {   // the tokens' scales: four columns per 64-input step
-                uint32_t w[16];
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(sc + (lane + 32 * g) * 16);
-                    w[0 + g] = v.x; w[4 + g] = v.y; w[8 + g] = v.z; w[12 + g] = v.w;
-                }
-                tmem_store16(quarter + kColSf + st * kSfCols, w);
-            }
-            // the weight rows' scales: 4 * kHalves columns per step (row l + 32 g of lane l in column g)
-#pragma unroll
-            for (int pair = 0; pair < kHalves; ++pair) {      // steps 2 pair, 2 pair + 1 (256 rows) or all four (128 rows)
-                uint32_t w[16];
-#pragma unroll
-                for (int g = 0; g < 4 * kHalves; ++g) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(sc + kScaleBytes + (lane + 32 * g) * 16);
-                    const uint32_t word[4] = {v.x, v.y, v.z, v.w};
-                    if (kHalves == 1) { w[0 + g] = word[0]; w[4 + g] = word[1]; w[8 + g] = word[2]; w[12 + g] = word[3]; }
-                    else { w[g] = word[2 * pair]; w[8 + g] = word[2 * pair + 1]; }
-                }
-                tmem_store16(quarter + kColSf + st * kSfCols + 16 + pair * 16, w);
-            }
+            const uint8_t* sc = stage(st) + 2 * kCodeBytes;
+            scales_of_128(quarter + kColSf + st * kSfCols, sc, lane);
+            scales_of_128(quarter + kColSf + st * kSfCols + 16, sc + kScaleBytes, lane);
             tmem_store_wait();
             tc_fence_before();
             __syncwarp();
@@ -162,7 +145,7 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
             const int token = t0 + (warp & 3) * 32 + lane;
             bf16* out = p.y + (size_t)token * p.out_features + n0;
 #pragma unroll 1
-            for (int col = 0; col < TN; col += 16) {
+            for (int col = 0; col < kTile; col += 16) {
                 uint32_t v[16];
                 tmem_load16(quarter + kColAcc + col, v);
                 tmem_load_wait();
@@ -182,6 +165,184 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, kCols4);
+}
+
+// ---- large products
+// Tiles of 256 tokens x 256 weight rows on a pair of SMs that stays for many of them (tcgen05 cta_group::2): each block holds the codes of
+// half of the tokens and half of the weight rows, the scales of its tokens and of all the weight rows, and 256 columns of sums.  With one
+// 128 x 256 tile to a block, operands came from L2 at 54 KB a stage and block, where an SM gets some 40 bytes a clock (the MMAs would need 89), and
+// the prologue and an epilogue of scattered 16-byte stores lay open.  Here it is 38 KB, loads run on through the end of a tile, and the
+// sums wait only for a pass of eight warps from tensor memory into registers (tensor memory holds no second set beside the scales).
+//   warp 0      TMA: codes count at the first block, scales in their own
+//   warp 1      of the first block: 4 MMAs of 256 x 256 x 64 per stage
+//   warps 2-13  scales to tensor memory, as above, every third stage each four; the weight rows' in eight columns per 64-input step
+//   the last 8  sums, 32 tokens x 128 outputs each, as bf16 through shared memory in whole 128-byte lines
+// What bounded both forms was the way of the scales, some 1000 clocks a stage for its four warps from the wait to the hand-over: 8192 x 8192 x
+// 2048 127 us before, here 141 with one group of four warps, 111 with two, 102 with three, then the operands from L2 (1100 clocks a
+// stage).  2048 x 8192 x 2048 37 -> 33 us.
+struct Pair4 {
+    static constexpr int kStages = 5, kStageBytes = 2 * kCodeBytes + 3 * kScaleBytes, kEpilogueWarps = 8, kStagingBytes = 32 * 128;
+    static constexpr int kScaleGroups = 3, kFirst = 2 + 4 * kScaleGroups, kThreads = 32 * (kFirst + kEpilogueWarps);
+    static constexpr uint32_t kColSf = 256, kSfCols = 48;
+    struct Bars { uint64_t full[kStages], scales[kStages], sf_ready[kStages], empty[kStages], ready, taken; };
+    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + sizeof(Bars) + 64 + 1024;
+    static_assert(kColSf + kStages * kSfCols <= 512 && kStageBytes % 1024 == 0 && kSmem <= 227 * 1024, "");
+};
+QD_DEVINL void pair_umma_nvfp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %7, 0;\n\t"
+                 "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+                 "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], da, db, %4, [%5], [%6], p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHiSw128), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair4::kThreads, 1)
+w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ CUtensorMap x_codes, const __grid_constant__ CUtensorMap x_scales,
+                 const __grid_constant__ CUtensorMap w_codes, const __grid_constant__ CUtensorMap w_scales) {
+    grid_dependency_wait();       // before the tensor memory, as above
+    extern __shared__ __align__(1024) uint8_t gemm4_smem_raw[];
+    using T = Pair4;
+    constexpr int kStages = T::kStages;
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm4_smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* staging = smem + kStages * T::kStageBytes;
+    T::Bars* bars = reinterpret_cast<T::Bars*>(staging + T::kEpilogueWarps * T::kStagingBytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, chunks = p.in_features / 256;
+    const int across = (p.tokens + 255) / 256, tiles = across * ((p.out_features + 255) / 256);
+
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(bars->full + s, 1); mbar_init(bars->scales + s, 1); mbar_init(bars->sf_ready + s, 2 * 4); mbar_init(bars->empty + s, 1);
+        }
+        mbar_init(&bars->ready, 1);
+        mbar_init(&bars->taken, 2 * T::kEpilogueWarps);
+        mbar_fence_init();
+    }
+    if (warp == 1) pair_tmem_alloc(tmem_slot, 512);
+    tc_fence_before();
+    cluster_sync();               // the barriers of both blocks are there
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    // A wait that runs out ends a role; everybody meets at the end, by when all copies and MMAs have long ended (the limit is 0.2 s).
+    if (warp == 0) {
+        if (lane == 0) {
+            bool ok = true;
+            int it = 0;
+            for (int tile = pair; tile < tiles && ok; tile += pairs) {
+                const int t0 = (tile % across) * 256 + rank * 128, n0 = (tile / across) * 256;
+                for (int c = 0; c < chunks; ++c, ++it) {
+                    const int st = it % kStages;
+                    ok = mbar_wait(bars->empty + st, ((it / kStages) & 1) ^ 1, p.status);
+                    if (!ok) break;
+                    uint8_t* base = smem + st * T::kStageBytes;
+                    uint8_t* sc = base + 2 * kCodeBytes;
+                    const uint32_t bar = of_first_block(bars->full + st);
+                    if (rank == 0) mbar_expect_tx(bars->full + st, 4 * kCodeBytes);
+                    pair_tma_tile(base, &x_codes, c * 128, t0, bar);
+                    pair_tma_tile(base + kCodeBytes, &w_codes, c * 128, n0 + rank * 128, bar);
+                    mbar_expect_tx(bars->scales + st, 3 * kScaleBytes);
+                    tma_load_2d(sc, &x_scales, c * 16, t0, bars->scales + st);
+                    tma_load_2d(sc + kScaleBytes, &w_scales, c * 16, n0, bars->scales + st);
+                    tma_load_2d(sc + 2 * kScaleBytes, &w_scales, c * 16, n0 + 128, bars->scales + st);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            bool ok = true;
+            int it = 0, i = 0;
+            for (int tile = pair; tile < tiles && ok; tile += pairs, ++i) {
+                if (i) ok = mbar_wait(&bars->taken, (i - 1) & 1, p.status);
+                for (int c = 0; c < chunks && ok; ++c, ++it) {
+                    const int st = it % kStages;
+                    ok = mbar_wait(bars->full + st, (it / kStages) & 1, p.status) && mbar_wait(bars->sf_ready + st, (it / kStages) & 1, p.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a_lo = desc_lo_sw128(smem_u32(smem + st * T::kStageBytes)), b_lo = a_lo + (kCodeBytes >> 4);
+                    const uint32_t sfa = tmem + T::kColSf + st * T::kSfCols, sfb = sfa + 16;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        pair_umma_nvfp4(tmem, a_lo + 2 * j, b_lo + 2 * j, desc_of(256, 256), sfa + j * 4, sfb + j * 8, (c | j) ? 1u : 0u);
+                    pair_commit(bars->empty + st);
+                }
+                if (ok) pair_commit(&bars->ready);
+            }
+        }
+    } else if (warp < T::kFirst) {
+        const uint32_t quarter = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T::kColSf;
+        const int group = (warp - 2) >> 2, steps = pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0;
+        bool ok = true;
+        for (int it = group; it < steps; it += T::kScaleGroups) {
+            const int st = it % kStages;
+            ok = __all_sync(0xffffffffu, mbar_wait(bars->scales + st, (it / kStages) & 1, p.status));
+            if (!ok) break;
+            const uint8_t* sc = smem + st * T::kStageBytes + 2 * kCodeBytes;
+            scales_of_128(quarter + st * T::kSfCols, sc, lane);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {                    // 64-input steps 2 half, 2 half + 1: row l + 32 g in column g
+                uint32_t w[16];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(sc + kScaleBytes + (lane + 32 * g) * 16 + half * 8);
+                    w[g] = v.x; w[8 + g] = v.y;
+                }
+                tmem_store16(quarter + st * T::kSfCols + 16 + half * 16, w);
+            }
+            tmem_store_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_at(of_first_block(bars->sf_ready + st));
+        }
+    } else {
+        const int quadrant = warp & 3, half = (warp - T::kFirst) >> 2;
+        uint4* lines = reinterpret_cast<uint4*>(staging + (warp - T::kFirst) * T::kStagingBytes);
+        const float scale = p.x_global[0] * p.w_global[0];
+        bool ok = true;
+        int i = 0;
+        for (int tile = pair; tile < tiles && ok; tile += pairs, ++i) {
+            const int t0 = (tile % across) * 256 + rank * 128 + quadrant * 32, n0 = (tile / across) * 256 + half * 128;
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->ready, i & 1, p.status));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t packed[64];
+#pragma unroll
+            for (int c = 0; c < 128; c += 16) {
+                uint32_t v[16];
+                tmem_load16(tmem + ((uint32_t)(quadrant * 32) << 16) + half * 128 + c, v);
+                tmem_load_wait();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(v[2 * q]) * scale, __uint_as_float(v[2 * q + 1]) * scale);
+                    packed[c / 2 + q] = *reinterpret_cast<const uint32_t*>(&two);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_at(of_first_block(&bars->taken));
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {                    // 64 outputs: a 128-byte line, pieces q of line l at q ^ (l & 7)
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t* w = packed + part * 32 + q * 4;
+                    lines[lane * 8 + (q ^ (lane & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int row = 4 * r + (lane >> 3), q = lane & 7, n = n0 + part * 64 + q * 8;
+                    const uint4 w = lines[row * 8 + (q ^ (row & 7))];
+                    if (t0 + row < p.tokens && n < p.out_features) *reinterpret_cast<uint4*>(p.y + (size_t)(t0 + row) * p.out_features + n) = w;
+                }
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync();
+    tc_fence_after();
+    if (warp == 1) pair_tmem_dealloc(tmem, 512);
 }
 
 // ---- activation quantiser --------------------------------------------------------------
@@ -314,22 +475,23 @@ extern "C" int qd_nvfp4_matmul_w4a4(const void* x_codes, const void* x_scales, c
     Gemm4Params p = {};
     p.x_global = x_global; p.w_global = w_global; p.y = reinterpret_cast<bf16*>(y);
     p.tokens = tokens; p.out_features = out_features; p.in_features = in_features; p.status = status;
-    // 256-row weight tiles where they still give every SM a tile or more; 128-row tiles otherwise
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long token_tiles = (tokens + kTile - 1) / kTile;
-    const bool wide = wide_tiles >= 0 ? wide_tiles != 0 : (out_features % 256 == 0 && token_tiles * (out_features / 256) >= 2ll * sms);
+    const long long token_tiles = (tokens + kTile - 1) / kTile, tiles = (long long)((tokens + 255) / 256) * ((out_features + 255) / 256);
+    // a pair needs two tiles or more to hide its start (256 tiles 33 us against 38 of the small form, 128 tiles 20.0 / 20.2, 100 tiles 18 / 16)
+    const bool wide = wide_tiles >= 0 ? wide_tiles != 0 : tiles >= sms;
+    constexpr size_t smem = (size_t)kStages4 * kStage4Bytes + sizeof(Bars4) + 64 + 1024;
     static bool configured[2][64];
-    const size_t smem = wide ? (size_t)stages_of(256) * stage_bytes(256) + sizeof(Bars4) + 64 + 1024
-                             : (size_t)stages_of(128) * stage_bytes(128) + sizeof(Bars4) + 64 + 1024;
     if (!configured[wide][dev]) {
-        if ((wide ? cudaFuncSetAttribute(nvfp4_gemm_w4a4_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                  : cudaFuncSetAttribute(nvfp4_gemm_w4a4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        if ((wide ? cudaFuncSetAttribute(w4a4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pair4::kSmem)
+                  : cudaFuncSetAttribute(nvfp4_gemm_w4a4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
             return QD_ERR_LAUNCH;
         configured[wide][dev] = true;
     }
-    const dim3 grid((unsigned)(out_features / (wide ? 256 : 128)), (unsigned)token_tiles);
-    if (wide) return qd_launch(nvfp4_gemm_w4a4_kernel<256>, grid, dim3(kThreads4), smem, (cudaStream_t)stream, 3, p, xc, xs, wc, ws);
-    return qd_launch(nvfp4_gemm_w4a4_kernel<128>, grid, dim3(kThreads4), smem, (cudaStream_t)stream, 3, p, xc, xs, wc, ws);
+    if (wide)
+        return qd_launch(w4a4_pair_kernel, dim3((unsigned)(2 * std::min<long long>(tiles, sms / 2))), dim3(Pair4::kThreads), Pair4::kSmem, (cudaStream_t)stream, 3, p,
+                         xc, xs, wc, ws);
+    return qd_launch(nvfp4_gemm_w4a4_kernel, dim3((unsigned)(out_features / kTile), (unsigned)token_tiles), dim3(kThreads4), smem, (cudaStream_t)stream, 3, p, xc, xs,
+                     wc, ws);
 }

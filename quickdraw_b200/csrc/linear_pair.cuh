@@ -9,6 +9,7 @@
 // 2048 -> 8192 259 -> 185 (176) = 1.49 PFLOP/s.  What bounds it: operands come from L2 at some 40 bytes a clock and SM (tiles of 128 weight rows,
 // which ask for half as much again per product, took 305 us there), and the power limit.
 #pragma once
+#include "pair.cuh"
 
 namespace qd {
 namespace {
@@ -21,29 +22,11 @@ struct PairTile {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + (2 * kStages + 4) * 8 + 16 + 1024;
 };
 
-QD_DEVINL uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-QD_DEVINL uint32_t of_first_block(const void* p) {                    // the same place in the first block of the pair
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
-    return r;
-}
-QD_DEVINL void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-QD_DEVINL void pair_tma_tile(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
-}
 QD_DEVINL void pair_umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-QD_DEVINL void pair_commit(uint64_t* bar) {                           // arrives at this place in both blocks
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
-
 // Sixteen sums of a token, the first of them output n of the matrix, finished: eight (glu) or sixteen values into `out`.
 QD_DEVINL void finish16(const Finish& f, const uint32_t* v, int n, const float* bias, float (&out)[16]) {
     float x[16];
@@ -144,10 +127,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
         for (int s = 0; s < 2; ++s) { mbar_init(ready + s, 1); mbar_init(taken + s, 2 * Tile::kEpilogueWarps); }
         mbar_fence_init();
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(2 * TN) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
+    if (warp == 1) pair_tmem_alloc(slot, 2 * TN);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync();                            // the barriers of both blocks are there
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -231,15 +211,14 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(of_first_block(taken + buf)) : "memory");
+            if (lane == 0) arrive_at(of_first_block(taken + buf));
         }
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TN) : "memory");
+    if (warp == 1) pair_tmem_dealloc(tmem, 2 * TN);
 }
 
 }  // namespace

@@ -185,8 +185,8 @@ def matmul_w4a4(xq, proj: NVFP4Linear, *, wide_tiles: bool | None = None) -> tor
     """Quantised activations (``quantize_act``) times a packed NVFP4 matrix on the block-scaled
     FP4 tensor core: neither operand is expanded.  Differs from ``matmul`` by the activation
     rounding only (the W4A4 variant quickdraw's notes ask to validate separately from W4A16);
-    in_features a multiple of 256, out_features a multiple of 128.  ``wide_tiles``: 256 weight rows
-    per block and MMA (needs out_features % 256 == 0) instead of 128; None lets the library choose."""
+    in_features a multiple of 256, out_features a multiple of 128.  ``wide_tiles``: tiles of 256 tokens
+    and 256 weight rows on pairs of SMs instead of 128 and 128; None lets the library choose."""
     codes, scales, scale_2 = xq
     assert isinstance(proj, NVFP4Linear) and proj.weight.ndim == 2 and proj.group_size == 16
     assert codes.is_cuda and codes.dtype == torch.uint8 and codes.is_contiguous() and scales.is_contiguous()

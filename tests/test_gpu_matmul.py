@@ -180,3 +180,16 @@ def test_w4a4_matmul_matches_oracle(cuda_device, tokens, out_features, in_featur
     assert O.rel_l2(got, want) < 2e-3
     exact = O.nvfp4_matmul(x, proj)
     assert O.rel_l2(got, exact) < 0.2
+
+
+@pytest.mark.parametrize("tokens,out_features,in_features", [(1, 128, 256), (129, 384, 512), (257, 256, 1536), (600, 640, 768), (2500, 2176, 256)])
+def test_w4a4_matmul_on_pairs(cuda_device, tokens, out_features, in_features):
+    """Tiles that end inside a block's half of the tokens and inside the weight rows, fewer and more stages than there are, one tile to a
+    pair of SMs and several (90 tiles): the same sums as in the small form, in the same order of the inputs."""
+    from quickdraw_b200 import kernels
+    src = synthetic.Source(35, cuda_device)
+    proj = src.nvfp4("w", out_features, in_features, global_scale=0.75)
+    xq = kernels.quantize_act(src.normal("x", tokens, in_features))
+    got, want = (kernels.matmul_w4a4(xq, proj, wide_tiles=wide) for wide in (True, False))
+    assert kernels.matmul_status(cuda_device) == 0
+    assert torch.isfinite(got.float()).all() and O.rel_l2(got, want) < 1e-4
