@@ -25,7 +25,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
 COMMON = ("library",)
 HYBRID_SOURCES = {"hybrid": ("linear", "residual", "window_attention"), "recurrent": ("linear_recurrence", "channel_chunk"),
                   "latent": ("latent_attention",)}
-HYBRID_HEADERS = ("common.cuh", "typed.cuh", "pieces_mma.cuh", "linear_pair.cuh", "pair.cuh", "softmax_attention.cuh", "flash_umma.cuh")
+HYBRID_HEADERS = ("common.cuh", "typed.cuh", "pieces_mma.cuh", "linear_pair.cuh", "pair.cuh", "softmax_attention.cuh", "flash_umma.cuh", "attention_pieces.cuh")
 TARGETS = ("nvfp4", *HYBRID_SOURCES)
 
 

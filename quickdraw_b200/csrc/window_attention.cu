@@ -10,8 +10,8 @@
 // Prompt chunks: attn_prepare_kernel (norm, rotation, ring rows), then flash_umma.cuh for heads of 128 value and 128 or 192 key
 // columns, attn_flash_kernel for other bf16 rows (mma.sync m16n8k16;
 // 64 or 128 packed (token, head of the group) rows per block, key tiles of 64 through two cp.async buffers,
-// only the tiles a row of the block can see; probabilities as two bf16 pieces).  attn_tiles_kernel takes fp32 rows of whole
-// 16-byte pieces, attn_rows_kernel everything else.  Decode: attn_step_kernel, one launch: norm and rotation in every
+// only the tiles a row of the block can see; probabilities as two bf16 pieces).  attention_pieces.cuh takes fp32 rows of heads of 128 value and
+// 128 or 192 key columns, attn_tiles_kernel others of whole 16-byte pieces, attn_rows_kernel everything else.  Decode: attn_step_kernel, one launch: norm and rotation in every
 // block, blocks = (key/value head, split of the span), the last block of a head merges.
 #include <type_traits>
 
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const __grid_constant__ 
 // A dot product is summed in pieces of 32, so that its rounding does not grow with the head size.  Bound by the FMA pipe and
 // the shared-memory reads that feed it.  A warp per (token, head), as in attn_rows_kernel, reads every key row again for
 // every head and token, 32 rows at a time side by side: 777 tokens, 16/4
-// heads of 128, window 1024: 2902 us there, 382 us here (2.5 GFLOP).
+// heads of 128, window 1024: 2902 us there, 382 us here (2.5 GFLOP; attention_pieces.cuh 117).
 constexpr int kTileKeys = 64;
 __host__ __device__ constexpr size_t tiles_floats(int rows, int qdim, int vdim) {
     return (size_t)qdim * (rows + 4) + (size_t)qdim * (kTileKeys + 4) + (size_t)kTileKeys * vdim + (size_t)rows * (kTileKeys + 4);
@@ -397,6 +397,14 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const __grid_constant__
         }
     }
 }
+
+}  // namespace
+}  // namespace qd
+
+#include "attention_pieces.cuh"
+
+namespace qd {
+namespace {
 
 // ------------------------------------------------------------------------------- tensor cores
 constexpr int kFlashKeys = 64;
@@ -957,6 +965,13 @@ bool tiles_cover(const AttnParams& p) {
            p.ld_shared % 4 == 0 && aligned16(p.q_rows) && aligned16(p.k_cache) && aligned16(p.v_cache) && aligned16(p.k_shared) && p.vdim <= 256 &&
            4 * tiles_floats(64, p.dim + p.shared_dim, p.vdim) <= kMaxSmem;
 }
+// Heads of 128 value columns and 128 or 192 key columns, on top of what the tiles need.
+template <int QD>
+int launch_pieces(const AttnParams& p, long long rows, cudaStream_t s) {
+    constexpr size_t smem = PieceShape<QD, 128>::kSmem;
+    if (!allow_smem(attn_pieces_kernel<QD, 128>, smem)) return QD_ERR_UNSUPPORTED;
+    return qd_launch(attn_pieces_kernel<QD, 128>, dim3((unsigned)((rows + kPieceRows - 1) / kPieceRows), p.kv_heads), dim3(kPieceThreads), smem, s, 1, p);
+}
 template <typename T>
 int chunk(const AttnParams& p, cudaStream_t s) {
     if (p.q) {
@@ -987,7 +1002,11 @@ int chunk(const AttnParams& p, cudaStream_t s) {
     if (!handful && tiles_cover(p)) {
         const long long rows = (long long)p.tokens * (p.heads / p.kv_heads);
         // 64 rows share a key tile once such blocks give half the SMs one; below that more blocks count for more
-        return rows * p.kv_heads >= 32ll * device_sms() ? launch_tiles<64>(p, rows, s) : launch_tiles<16>(p, rows, s);
+        if (rows * p.kv_heads < 32ll * device_sms()) return launch_tiles<16>(p, rows, s);
+        const int qdim = p.dim + p.shared_dim;
+        if (p.vdim == 128 && qdim == 128) return launch_pieces<128>(p, rows, s);
+        if (p.vdim == 128 && qdim == 192) return launch_pieces<192>(p, rows, s);
+        return launch_tiles<64>(p, rows, s);
     }
     const dim3 grid((unsigned)(((long long)p.tokens * p.heads + 7) / 8), (p.vdim + 32 * kRowsPerLane - 1) / (32 * kRowsPerLane));
     return qd_launch(attn_rows_kernel<T>, grid, dim3(256), 0, s, 1, p);

@@ -194,3 +194,51 @@ def test_forms_of_rows_that_a_chunk_may_have(cuda_device, dim, shared, heads, kv
     call_hybrid("qd_attention", byref(args), stream_of(q))
     at, j = torch.arange(position, end, device=cuda_device)[:, None], torch.arange(end, device=cuda_device)[None]
     close(out, plain(q, torch.cat([keys, common[:, None].expand(-1, kv_heads, -1)], -1), values, scale, (j <= at) & (j > at - span)), 1.5)
+
+
+@pytest.mark.parametrize("tokens,position,heads,kv_heads,shared,span,capacity,chunked,slopes,sink,gate,bad", [
+    (300, 0, 16, 4, 0, 1024, 300, False, False, 1, 1, None), (700, 100, 8, 2, 0, 100, 900, False, False, 1, 1, None),
+    (593, 2000, 8, 8, 64, 256, 1024, False, False, 0, 2, None), (400, 700, 16, 4, 0, 256, 1024, True, True, 2, 0, None),
+    (1601, 0, 3, 1, 0, 33, 1700, True, True, 2, 0, None), (1200, 5, 4, 4, 64, 5000, 1300, False, False, 0, 2, None),
+    (600, 50, 8, 2, 64, 64, 700, False, False, 0, 0, math.inf), (500, 0, 12, 4, 0, 5000, 500, False, False, 1, 2, math.nan)])
+def test_bounded_attention_of_an_fp32_chunk(cuda_device, tokens, position, heads, kv_heads, shared, span, capacity, chunked, slopes, sink, gate, bad):
+    """Operands as three bf16 pieces: masks, rings that wrap, rows for the one and the other group of warps alone, everything that may stand
+    around the softmax, values that are not finite.  fp32 sums of some 128 and 1000 terms and scores of about ten: 2e-6."""
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call_hybrid, ptr, stream_of
+    assert tokens * heads >= 32 * 148
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    new = lambda *shape, std=1.0: torch.randn(shape, generator=gen, device=cuda_device) * std
+    first, end = max(0, position - span + 1), position + tokens
+    keys, values, common = new(end, kv_heads, 128, std=2.0), new(end, kv_heads, 128), new(end, shared)
+    spoilt = values.clone()
+    if bad is not None:
+        spoilt[position + 201, 0, 7] = bad
+    ring = lambda t: torch.full((capacity, *t.shape[1:]), float("nan"), device=cuda_device)
+    kr, vr, cr = ring(keys), ring(values), ring(common)
+    for j in range(max(first, end - capacity), end):
+        kr[j % capacity], vr[j % capacity], cr[j % capacity] = keys[j], spoilt[j], common[j]
+    q, gates = new(tokens, heads, 128 + shared), new(tokens, heads * (128 if gate == 2 else 1))
+    slope = torch.rand(heads, generator=gen, device=cuda_device) * 0.05
+    sinks, out = new(heads).to(BF16), torch.full((tokens, heads, 128), float("nan"), device=cuda_device)
+    scale = (128 + shared) ** -0.5
+    args = AttentionArgs(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, shared_dim=shared, scale=scale, ld_k=kv_heads * 128, ld_v=kv_heads * 128,
+                         ld_shared=shared, k_cache=ptr(kr), v_cache=ptr(vr), k_shared=ptr(cr) if shared else None, q_rows=ptr(q), out=ptr(out),
+                         gate=ptr(gates), ld_gate=gates.shape[1], gate_kind=gate, sink=ptr(sinks), sink_kind=sink,
+                         slopes=ptr(slope) if slopes else None, mask=int(chunked), span=min(span, capacity), capacity=capacity, position=position,
+                         tokens=tokens, dtype=1)
+    call_hybrid("qd_attention", byref(args), stream_of(q))
+    at, j = torch.arange(position, end, device=cuda_device)[:, None], torch.arange(end, device=cuda_device)[None]
+    visible = (j <= at) & (j >= (at - at % span if chunked else at - span + 1))
+    bias = -slope.double()[:, None, None] * (at - j) if slopes else None
+    with_shared = torch.cat([keys, common[:, None].expand(-1, kv_heads, -1)], -1)
+    extra = {0: None, 1: sinks, 2: torch.zeros(heads, device=cuda_device)}[sink]
+    want = plain(q, with_shared, values, scale, visible, bias, extra)
+    if gate:
+        want = want * torch.sigmoid(gates.double().view(tokens, heads, -1))
+    kept = torch.ones_like(want, dtype=torch.bool)
+    if bad is not None:
+        kept[:, :heads // kv_heads, 7] = ~visible[:, position + 201, None]
+        assert not torch.isfinite(out[~kept]).any()
+    assert float((out.double() - want)[kept].norm() / want[kept].norm()) < 2e-6
