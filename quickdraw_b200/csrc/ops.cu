@@ -351,12 +351,10 @@ QD_DEVINL void route_warp(const bf16* __restrict__ logits_bf16, const float* __r
 #pragma unroll
         for (int i = 0; i < PER; ++i)
             if (p[i] > v) { v = p[i]; idx = i * 32 + lane; }   // ascending index within the lane
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-        }
+        // as integers: probabilities are not negative, and -1 is below them
+        const int top = __reduce_max_sync(0xffffffffu, __float_as_int(v));
+        idx = __reduce_min_sync(0xffffffffu, __float_as_int(v) == top ? idx : 0x7fffffff);
+        v = __int_as_float(top);
         chosen_sum += v;
         if (lane == (s & 31)) { my_weight = v; my_id = idx; }
         if ((idx & 31) == lane) {

@@ -135,11 +135,13 @@ __global__ void seq_bf16_matmul_kernel(const bf16* __restrict__ x, const bf16* _
 // once, straight from global memory into A fragments: lane (g, t) loads the 32 bytes of rows g
 // and g + 8 at inputs 64 s + 16 t .. + 15 of step s (a quarter-warp reads two whole 128-byte
 // lines), and the 16 inputs of token 8 nt + g at the same offsets are its B fragments, so every
-// element of the 16 x 32 result is used.  fp32 accumulators, one bf16 rounding.
+// element of the 16 x 32 result is used.  fp32 accumulators, one bf16 rounding.  A second matrix of the same input
+// (w1, y1, rows1; or NULL) takes the groups of sixteen rows behind those of the first.
 constexpr int kTallTokens = 32, kTallMaxWidth = 3072, kTallUnroll = 2, kTallWarps = 16;
 __global__ void __launch_bounds__(kTallWarps * 32, 1)
 seq_bf16_matmul_tall_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
-                            int tokens, int rows, int width, int groups_per_block, int input_parts) {
+                            int tokens, int rows, int width, int groups_per_block, int input_parts, const bf16* __restrict__ w1,
+                            bf16* __restrict__ y1, int rows1) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char tall_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -161,12 +163,14 @@ seq_bf16_matmul_tall_kernel(const bf16* __restrict__ x, const bf16* __restrict__
     }
     __syncthreads();
     const unsigned char* xs = tall_smem + (size_t)g * x_row + t * 32;
-    const int steps = width / 64;
-    // sixteen weight rows (n0 ..) against the tile's tokens over steps [s_begin, s_end) of 64 inputs
-    auto rows_times_tokens = [&](int n0, int s_begin, int s_end, float (&acc)[4][4]) {
+    const int steps = width / 64, groups0 = (rows + 15) / 16, groups = groups0 + (w1 ? (rows1 + 15) / 16 : 0);
+    // sixteen weight rows (a group) against the tile's tokens over steps [s_begin, s_end) of 64 inputs
+    auto rows_times_tokens = [&](int group, int s_begin, int s_end, float (&acc)[4][4]) {
         // rows past the matrix read its last row and store nothing
-        const uint4* lo = reinterpret_cast<const uint4*>(w + (size_t)min(n0 + g, rows - 1) * width + t * 16);
-        const uint4* hi = reinterpret_cast<const uint4*>(w + (size_t)min(n0 + g + 8, rows - 1) * width + t * 16);
+        const bf16* mat = group < groups0 ? w : w1;
+        const int n0 = 16 * (group < groups0 ? group : group - groups0), last = (group < groups0 ? rows : rows1) - 1;
+        const uint4* lo = reinterpret_cast<const uint4*>(mat + (size_t)min(n0 + g, last) * width + t * 16);
+        const uint4* hi = reinterpret_cast<const uint4*>(mat + (size_t)min(n0 + g + 8, last) * width + t * 16);
         // two register buffers of kTallUnroll steps: the loads of one are in flight while the
         // other is multiplied (the warps of a block run in step, so nothing else would hide them)
         auto load = [&](uint4 (&a)[kTallUnroll][4], int s0) {
@@ -203,27 +207,29 @@ seq_bf16_matmul_tall_kernel(const bf16* __restrict__ x, const bf16* __restrict__
         }
     };
     // acc[nt][0..1] = row n0 + g, tokens 8 nt + 2 t and + 1; [2..3] = row n0 + g + 8
-    auto store = [&](int n0, const float (&acc)[4][4]) {
+    auto store = [&](int group, const float (&acc)[4][4]) {
+        bf16* to = group < groups0 ? y : y1;
+        const int n0 = 16 * (group < groups0 ? group : group - groups0), all = group < groups0 ? rows : rows1;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int token = 8 * nt + 2 * t + (c & 1), row = n0 + g + 8 * (c >> 1);
-                if (token < nt_rows && row < rows) y[(size_t)(t0 + token) * rows + row] = __float2bfloat16_rn(acc[nt][c]);
+                if (token < nt_rows && row < all) to[(size_t)(t0 + token) * all + row] = __float2bfloat16_rn(acc[nt][c]);
             }
     };
     if (input_parts > 1) {
         // few rows (one pass per block): the warps beyond the row groups take parts of the inputs, the parts'
         // sums meet in shared memory behind the tokens and are added in order
         const int slot = warp % groups_per_block, part = warp / groups_per_block;
-        const int n0 = (blockIdx.x * groups_per_block + slot) * 16;
-        const bool active = n0 < rows && part < input_parts;
+        const int group = blockIdx.x * groups_per_block + slot;
+        const bool active = group < groups && part < input_parts;
         float acc[4][4];
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[nt][c] = 0.f;
-        if (active) rows_times_tokens(n0, part * steps / input_parts, (part + 1) * steps / input_parts, acc);
+        if (active) rows_times_tokens(group, part * steps / input_parts, (part + 1) * steps / input_parts, acc);
         float4* meet = reinterpret_cast<float4*>(tall_smem + (size_t)kTallTokens * x_row);     // [part - 1][slot][nt][lane]
         if (active && part > 0) {
 #pragma unroll
@@ -238,20 +244,20 @@ seq_bf16_matmul_tall_kernel(const bf16* __restrict__ x, const bf16* __restrict__
                     const float4 v = meet[(((other - 1) * groups_per_block + slot) * 4 + nt) * 32 + lane];
                     acc[nt][0] += v.x; acc[nt][1] += v.y; acc[nt][2] += v.z; acc[nt][3] += v.w;
                 }
-            store(n0, acc);
+            store(group, acc);
         }
         return;
     }
     // many rows: only the first groups_per_block warps multiply (more blocks share the rows)
-    for (int n0 = warp < groups_per_block ? (blockIdx.x * groups_per_block + warp) * 16 : rows; n0 < rows;
-         n0 += gridDim.x * groups_per_block * 16) {
+    for (int group = warp < groups_per_block ? blockIdx.x * groups_per_block + warp : groups; group < groups;
+         group += gridDim.x * groups_per_block) {
         float acc[4][4];
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[nt][c] = 0.f;
-        rows_times_tokens(n0, 0, steps, acc);
-        store(n0, acc);
+        rows_times_tokens(group, 0, steps, acc);
+        store(group, acc);
     }
 }
 
@@ -1010,93 +1016,97 @@ __global__ void seq_route_kernel(const bf16* __restrict__ logits, int experts, i
 // --------------------------------------------------------- routes of a chunk by expert
 // The stable order of the chunk's (token, slot) routes by expert id, as the reference groups
 // them (quickdraw/kernel/triton/moe.py:60-97): order[r] = route index of sorted row r,
-// boundaries[e] = first sorted row of expert e.  One block; every warp owns a contiguous slice
-// of the routes and a private row of per-expert counters in shared memory.  Pass 1 counts the
-// slice, a scan in (expert, warp) order turns the counters into first positions, pass 2 walks the
-// slice again, 32 routes at a time: lanes with the same expert find one another with match_any, a
-// route goes to its expert's running position plus its rank among the equal lanes below it.
-// Latency-bound: 2048 tokens of eight routes 29 us, 39 with the ids fetched 32 at a time.
-__global__ void __launch_bounds__(1024)
-seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts, int32_t* __restrict__ order,
+// boundaries[e] = first sorted row of expert e.  A block owns OWN neighbouring experts and reads every id (64 KB from L2 for 16384
+// routes, whole 16-byte pieces a lane): how many are below its experts and how many each of them has in every warp's slice gives the
+// first positions, so blocks need nothing from one another.  Then the slice again, still in registers where it is 512 routes or less:
+// four ballots an expert rank the 128 routes of a step, one vote skips the steps that hold none.  Two trips to memory and a barrier:
+// 2048 tokens of eight routes 29.0 -> 7.9 us, 511 9.5 -> 5.4, 64 3.8 -> 2.7 (one block for all experts: its scattered stores and its match_any of every 32
+// routes passed through one SM).
+constexpr int kRouteWarps = 32, kRouteAhead = 4;
+template <int OWN>
+__global__ void __launch_bounds__(kRouteWarps * 32)
+seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts, int whole, int32_t* __restrict__ order,
                         int32_t* __restrict__ boundaries) {
     chain_enter();
-    extern __shared__ int32_t counters[];               // [warps][experts], then first[experts + 1]
-    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int32_t* first = counters + warps * experts;
-    for (int i = threadIdx.x; i < warps * experts; i += blockDim.x) counters[i] = 0;
-    __syncthreads();
-    const int slice = ((routes + warps - 1) / warps + 31) & ~31;
-    const int begin = min(routes, warp * slice), end = min(routes, begin + slice);
-    int32_t* mine = counters + warp * experts;
-    constexpr int kAhead = 16;                           // ids of a slice requested together: one trip to memory for 512 routes
-    int id[kAhead];
-    const auto fetch = [&](int r0) {
+    __shared__ int32_t counts[kRouteWarps][OWN + 1];               // of every warp: own experts, then the ids below them
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e0 = blockIdx.x * OWN, e1 = min(experts, e0 + OWN);
+    const int steps = (routes + 127) / 128, per_warp = (steps + kRouteWarps - 1) / kRouteWarps;
+    const int s0 = min(steps, warp * per_warp), s1 = min(steps, s0 + per_warp);
+    int4 id[kRouteAhead];                                                 // four neighbouring routes a lane and step; INT_MAX: none
+    const auto fetch = [&](int s) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            if (r0 + 32 * u >= end) break;               // (a slice of a short chunk is 32 routes, often of one warp only)
-            const int r = r0 + 32 * u + lane;
-            id[u] = r < end ? __ldg(ids + r) : -1;
+        for (int u = 0; u < kRouteAhead; ++u) {
+            const int r = (s + u) * 128 + 4 * lane;
+            id[u] = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+            if (s + u >= s1) continue;
+            if (whole && r + 3 < routes) {
+                id[u] = __ldg(reinterpret_cast<const int4*>(ids + r));
+            } else {
+                if (r < routes) id[u].x = __ldg(ids + r);
+                if (r + 1 < routes) id[u].y = __ldg(ids + r + 1);
+                if (r + 2 < routes) id[u].z = __ldg(ids + r + 2);
+                if (r + 3 < routes) id[u].w = __ldg(ids + r + 3);
+            }
         }
     };
-    for (int r0 = begin; r0 < end; r0 += 32 * kAhead) {
-        fetch(r0);
+    int below = 0, mine[OWN];
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            if (r0 + 32 * u >= end) break;
-            if (id[u] >= 0) atomicAdd(mine + id[u], 1);
+    for (int k = 0; k < OWN; ++k) mine[k] = 0;
+    for (int s = s0; s < s1; s += kRouteAhead) {
+        fetch(s);
+#pragma unroll
+        for (int u = 0; u < kRouteAhead; ++u) {
+            const int four[4] = {id[u].x, id[u].y, id[u].z, id[u].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                below += four[j] < e0;
+#pragma unroll
+                for (int k = 0; k < OWN; ++k)
+                    mine[k] += four[j] == e0 + k;
+            }
         }
     }
-    __syncthreads();
-    // totals per expert, their exclusive scan, then every warp's first position per expert
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-        int total = 0;
-        for (int w = 0; w < warps; ++w) total += counters[w * experts + e];
-        first[e + 1] = total;
-    }
-    if (threadIdx.x == 0) first[0] = 0;
-    __syncthreads();
-    if (warp == 0) {      // inclusive scan by one warp: a lane adds up its run of experts, the runs are scanned with shuffles
-        const int run = (experts + 31) / 32, lo = min(experts, lane * run), hi = min(experts, lo + run);
-        int sum = 0;
-        for (int e = lo; e < hi; ++e) sum += first[e + 1];
-        int inclusive = sum;
+    below = __reduce_add_sync(0xffffffffu, below);
+    if (lane == 0) counts[warp][OWN] = below;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int below = __shfl_up_sync(0xffffffffu, inclusive, d);
-            if (lane >= d) inclusive += below;
-        }
-        int running = inclusive - sum;
-        for (int e = lo; e < hi; ++e) { running += first[e + 1]; first[e + 1] = running; }
+    for (int k = 0; k < OWN; ++k) {
+        const int n = __reduce_add_sync(0xffffffffu, mine[k]);
+        if (lane == 0) counts[warp][k] = n;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e <= experts; e += blockDim.x) boundaries[e] = first[e];
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-        int at = first[e];
-        for (int w = 0; w < warps; ++w) {
-            const int n = counters[w * experts + e];
-            counters[w * experts + e] = at;
-            at += n;
-        }
+    int at[OWN], first = __reduce_add_sync(0xffffffffu, counts[lane][OWN]);       // this warp's next position of every own expert
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+        if (threadIdx.x == 0 && e0 + k < experts) boundaries[e0 + k] = first;
+        const int n = counts[lane][k];
+        at[k] = first + __reduce_add_sync(0xffffffffu, lane < warp ? n : 0);
+        first += __reduce_add_sync(0xffffffffu, n);
     }
-    __syncthreads();
-    for (int r0 = begin; r0 < end; r0 += 32 * kAhead) {
-        if (end - begin > 32 * kAhead) fetch(r0);        // (a single batch is still there)
-        unsigned same[kAhead];
+    if (threadIdx.x == 0 && e1 == experts) boundaries[experts] = first;
+    const unsigned lower = (1u << lane) - 1u;
+    for (int s = s0; s < s1; s += kRouteAhead) {
+        if (s1 - s0 > kRouteAhead) fetch(s);                              // (a single batch is still there)
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            if (r0 + 32 * u >= end) break;
-            same[u] = __match_any_sync(0xffffffffu, id[u]);
-        }
+        for (int u = 0; u < kRouteAhead; ++u) {
+            const int four[4] = {id[u].x, id[u].y, id[u].z, id[u].w};
+            bool some = false;
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            if (r0 + 32 * u >= end) break;
-            const int e = id[u];
-            int at = 0;
-            if (e >= 0) at = mine[e] + __popc(same[u] & ((1u << lane) - 1u));
-            __syncwarp();
-            if (e >= 0 && lane == __ffs(same[u]) - 1) mine[e] = at + __popc(same[u]);
-            __syncwarp();
-            if (e >= 0) order[at] = r0 + 32 * u + lane;
+            for (int j = 0; j < 4; ++j) some |= four[j] >= e0 && four[j] < e1;
+            if (!__any_sync(0xffffffffu, some)) continue;
+#pragma unroll
+            for (int k = 0; k < OWN; ++k) {
+                        int rank = 0, all = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const unsigned same = __ballot_sync(0xffffffffu, four[j] == e0 + k);
+                    rank += __popc(same & lower);
+                    all += __popc(same);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (four[j] == e0 + k) order[at[k] + rank++] = (s + u) * 128 + 4 * lane + j;
+                at[k] += all;
+            }
         }
     }
 }
@@ -1244,54 +1254,66 @@ extern "C" int qd_seq_add_rms_norm(const void* x, const void* residual, const fl
     return qd_launch_status();
 }
 
+// A tall matrix, or many tokens: every weight row is read once per tile of 32 tokens (tensor-core form).
+static bool tall_form(const void* x, const void* w, int tokens, int rows, int width) {
+    return (rows >= 4096 || tokens >= 64) && width % 64 == 0 && width <= kTallMaxWidth && !(((uintptr_t)x | (uintptr_t)w) & 15u) &&
+           (tokens + 31) / 32 <= 65535;
+}
+static int launch_tall(const void* x, const void* w, void* y, int rows, const void* w1, void* y1, int rows1, int tokens, int width, void* stream) {
+    const size_t smem = (size_t)kTallTokens * (width * sizeof(bf16) + 16);
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
+    static bool configured[64];
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(seq_bf16_matmul_tall_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTallTokens * (kTallMaxWidth * 2 + 16)) != cudaSuccess)
+            return QD_ERR_LAUNCH;
+        configured[dev] = true;
+    }
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 148;
+    // Sixteen row groups per block where those blocks fill the GPU.  Else what a block takes from L2 (its 32 tokens, as much as two groups,
+    // and its groups' weights) times the waves of blocks, one an SM, as few as can be: the launch is bound by it.  Then the idle warps
+    // take parts of the inputs (a power of two that divides the steps of 64 inputs), if the sums fit behind the tokens.
+    const int row_groups = (rows + 15) / 16 + (w1 ? (rows1 + 15) / 16 : 0), token_tiles = (tokens + 31) / 32;
+    int per_block = kTallWarps;
+    if ((long long)((row_groups + kTallWarps - 1) / kTallWarps) * token_tiles < sms) {
+        long long least = 0;
+        for (int n = row_groups < kTallWarps ? row_groups : kTallWarps; n >= 1; --n) {
+            const long long blocks = (long long)((row_groups + n - 1) / n) * token_tiles, cost = (blocks + sms - 1) / sms * (n + 2);
+            if (!least || cost < least) { least = cost; per_block = n; }
+        }
+    }
+    const int row_blocks = (row_groups + per_block - 1) / per_block;
+    int parts = 1;
+    if (row_blocks <= sms)
+        while (2 * parts * per_block <= kTallWarps && (width / 64) % (2 * parts) == 0) parts *= 2;
+    size_t launch_smem = smem;
+    if (parts > 1) {
+        launch_smem += (size_t)(parts - 1) * per_block * 4 * 32 * 16;
+        if (launch_smem > (size_t)kTallTokens * (kTallMaxWidth * 2 + 16)) { parts = 1; launch_smem = smem; }
+    }
+    qd_launch(seq_bf16_matmul_tall_kernel, dim3(row_blocks < sms ? row_blocks : sms, token_tiles), dim3(kTallWarps * 32), launch_smem, (cudaStream_t)stream, true,
+              (const bf16*)x, (const bf16*)w, (bf16*)y, tokens, rows, width, per_block, parts, (const bf16*)w1, (bf16*)y1, rows1);
+    return qd_launch_status();
+}
+
 extern "C" int qd_seq_bf16_matmul(const void* x, const void* w, void* y, int tokens, int rows, int width, void* stream) {
     QD_CHECK_ARG(x && w && y && tokens > 0 && rows > 0 && width > 0);
-    const uintptr_t align = (uintptr_t)x | (uintptr_t)w;
-    if ((rows >= 4096 || tokens >= 64) && width % 64 == 0 && width <= kTallMaxWidth && !(align & 15u) && (tokens + 31) / 32 <= 65535) {
-        // tall matrix or many tokens: every weight row is read once per tile of 32 tokens (tensor-core form)
-        const size_t smem = (size_t)kTallTokens * (width * sizeof(bf16) + 16);
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
-        static bool configured[64];
-        if (!configured[dev]) {
-            if (cudaFuncSetAttribute(seq_bf16_matmul_tall_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTallTokens * (kTallMaxWidth * 2 + 16)) != cudaSuccess)
-                return QD_ERR_LAUNCH;
-            configured[dev] = true;
-        }
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-        // sixteen row groups per block, fewer while the blocks do not fill the GPU; then the idle warps take
-        // parts of the inputs (a power of two that divides the steps of 64 inputs), if the sums fit behind the tokens
-        const int row_groups = (rows + 15) / 16, token_tiles = (tokens + 31) / 32;
-        int per_block = kTallWarps;
-        while (per_block > 1 && (long long)((row_groups + per_block - 1) / per_block) * token_tiles < sms &&
-               (per_block > 2 || row_groups == 1)) per_block >>= 1;
-        const int row_blocks = (row_groups + per_block - 1) / per_block;
-        int parts = 1;
-        if (row_blocks <= sms && per_block < kTallWarps) {
-            parts = kTallWarps / per_block;
-            while (parts > 1 && (width / 64) % parts != 0) parts >>= 1;
-        }
-        size_t launch_smem = smem;
-        if (parts > 1) {
-            launch_smem += (size_t)(parts - 1) * per_block * 4 * 32 * 16;
-            if (launch_smem > (size_t)kTallTokens * (kTallMaxWidth * 2 + 16)) { parts = 1; launch_smem = smem; }
-        }
-        qd_launch(seq_bf16_matmul_tall_kernel, dim3(row_blocks < sms ? row_blocks : sms, token_tiles), dim3(kTallWarps * 32), launch_smem, (cudaStream_t)stream, true, 
-            (const bf16*)x, (const bf16*)w, (bf16*)y, tokens, rows, width, per_block, parts);
-        return qd_launch_status();
-    }
+    if (tall_form(x, w, tokens, rows, width)) return launch_tall(x, w, y, rows, nullptr, nullptr, 0, tokens, width, stream);
     qd_launch(seq_bf16_matmul_kernel, dim3((rows + 7) / 8, tokens), dim3(256), 0, (cudaStream_t)stream, true,
               (const bf16*)x, (const bf16*)w, (bf16*)y, rows, width, (const bf16*)nullptr, (bf16*)nullptr, 0, 0);
     return qd_launch_status();
 }
 
 // Two small matrices of the same input in one launch (the a and b projections of a DeltaNet layer, the
-// router and the shared-expert gate: quickdraw/models/qwen.py:120-131, 165-170); shapes that
-// qd_seq_bf16_matmul gives to the tensor-core form go there one after the other.
+// router and the shared-expert gate: quickdraw/models/qwen.py:120-131, 165-170); a matrix of 4096 rows has the GPU to itself.
+// Of 2048 tokens and 2048 inputs, 32 + 32 rows 14.0 -> 7.3 us, 256 + 1
+// 24.3 -> 16.7; of 511 tokens 13.7 -> 6.3 and 12.8 -> 7.3 (before: a launch each, and blocks for two waves of the GPU).
 extern "C" int qd_seq_bf16_matmul2(const void* x, const void* w0, void* y0, int rows0, const void* w1, void* y1, int rows1,
                                    int tokens, int width, void* stream) {
     QD_CHECK_ARG(x && w0 && y0 && w1 && y1 && tokens > 0 && rows0 > 0 && rows1 > 0 && width > 0);
+    if (rows0 < 4096 && rows1 < 4096 && tall_form(x, w0, tokens, rows0, width) && tall_form(x, w1, tokens, rows1, width))
+        return launch_tall(x, w0, y0, rows0, w1, y1, rows1, tokens, width, stream);
     if (rows0 >= 4096 || rows1 >= 4096 || tokens >= 64 || tokens > 65535) {
         const int first = qd_seq_bf16_matmul(x, w0, y0, tokens, rows0, width, stream);
         return first != QD_OK ? first : qd_seq_bf16_matmul(x, w1, y1, tokens, rows1, width, stream);
@@ -1453,11 +1475,16 @@ extern "C" int qd_seq_group_routes(const int32_t* ids, int routes, int experts, 
                                    void* stream) {
     QD_CHECK_ARG(ids && order && boundaries && routes > 0 && experts > 0);
     if (experts > 1023) return QD_ERR_UNSUPPORTED;
-    // as many warps as 40 KB of counters allow (32 at 256 experts, 8 at 1023)
-    int warps = 32;
-    while (warps > 1 && (size_t)warps * experts * 4 > 40960) warps >>= 1;
-    const size_t smem = ((size_t)warps * experts + experts + 1) * sizeof(int32_t);
-    qd_launch(seq_group_routes_kernel, dim3(1), dim3(warps * 32), smem, (cudaStream_t)stream, true, ids, routes, experts, order, boundaries);
+    // one to eight experts a block: at most 128 blocks, one a multiprocessor
+    const int whole = ((uintptr_t)ids & 15u) == 0;
+    const auto launch = [&](auto kernel, int own) {
+        qd_launch(kernel, dim3((experts + own - 1) / own), dim3(kRouteWarps * 32), 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order,
+                  boundaries);
+    };
+    if (experts <= 128) launch(seq_group_routes_kernel<1>, 1);
+    else if (experts <= 256) launch(seq_group_routes_kernel<2>, 2);
+    else if (experts <= 512) launch(seq_group_routes_kernel<4>, 4);
+    else launch(seq_group_routes_kernel<8>, 8);
     return qd_launch_status();
 }
 

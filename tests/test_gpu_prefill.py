@@ -264,6 +264,37 @@ def test_group_routes_is_the_stable_sort_by_expert(cuda_device, routes, experts)
     assert torch.equal(order.long(), want_order) and torch.equal(boundaries.long(), want_boundaries)
 
 
+@pytest.mark.parametrize("routes,experts,offset", [(16384, 256, 0), (16385, 129, 0), (33000, 1023, 0), (128, 128, 0), (2047, 2, 0), (4090, 255, 1), (70001, 640, 3)])
+def test_group_routes_of_every_block_of_experts(cuda_device, routes, experts, offset):
+    """One to eight experts a block, the last block with fewer, slices beyond the registers, ids off the 16-byte grid."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator().manual_seed(routes)
+    ids = torch.randint(0, experts, (routes + offset,), generator=gen).to(torch.int32).to(cuda_device)[offset:]
+    ids[ids == experts - 1] = 0
+    order = torch.full((routes,), -1, dtype=torch.int32, device=cuda_device)
+    boundaries = torch.full((experts + 1,), -1, dtype=torch.int32, device=cuda_device)
+    call("qd_seq_group_routes", ptr(ids), routes, experts, ptr(order), ptr(boundaries), stream_of(ids))
+    sorted_ids, want_order = ids.sort(stable=True)
+    want_boundaries = torch.searchsorted(sorted_ids, torch.arange(experts + 1, device=cuda_device, dtype=torch.int32))
+    assert torch.equal(order.long(), want_order) and torch.equal(boundaries.long(), want_boundaries)
+
+
+@pytest.mark.parametrize("tokens,rows0,rows1,width", [(64, 32, 32, 2048), (511, 256, 1, 2048), (2048, 256, 1, 2048), (2048, 32, 32, 2048), (100, 7, 300, 192),
+                                                      (129, 16, 17, 3072), (1030, 1, 1, 64), (3000, 600, 31, 512), (70, 4096, 5, 256)])
+def test_two_small_products_of_many_tokens(cuda_device, tokens, rows0, rows1, width):
+    """One launch, groups of sixteen rows of either matrix, parts of the inputs.  fp32 sums in another order, one bf16 rounding (2^-9)."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens + rows0)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).to(torch.bfloat16)
+    x, w0, w1 = new(tokens, width), new(rows0, width), new(rows1, width)
+    y0, y1 = (torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device=cuda_device) for n in (rows0, rows1))
+    call("qd_seq_bf16_matmul2", ptr(x), ptr(w0), ptr(y0), rows0, ptr(w1), ptr(y1), rows1, tokens, width, stream_of(x))
+    for w, y in ((w0, y0), (w1, y1)):
+        want = x.double() @ w.double().T
+        bound = want.abs() * 2.0 ** -8 + width * 2.0 ** -22 * (x.double().abs() @ w.double().abs().T) / width ** 0.5
+        assert bool(((y.double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("tokens,hidden,topk", [(5, 2048, 8), (33, 4096, 2), (1, 520, 3)])
 def test_combine_with_the_next_norm_equals_the_two_calls(cuda_device, tokens, hidden, topk):
     """The MoE combine with the residual add + RMSNorm of the next layer in its launch: the same bits as
