@@ -162,6 +162,36 @@ QD_DEVINL bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned int* status) {
         if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, status);
 }
+// One lane of a converged warp, the same every time; the branch on it keeps the operands of tcgen05 instructions in uniform registers
+// (18 clocks an MMA; 60 in a branch on the lane's number, where each operand is moved over).
+QD_DEVINL bool elect_one() {
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+    return leader != 0;
+}
+QD_DEVINL bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+// How many of the `most` <= `ring` barriers from bars[at] on have completed their phase, one after the other (the parity turns where the
+// ring does); a whole warp asks, a lane each, because one look at a barrier beside MMAs in flight takes 150 to 300 clocks.  It waits for the first;
+// 0 if that wait runs out.  A short ring is seldom further than one stage ahead, and a look in vain in front of the wait costs it more:
+// linear_pieces_kernel (3 stages) 56 -> 61 us, fp8_gemm_kernel (4) 24.9 -> 26.1, w4a4_pair_kernel (5) 103 -> 105.
+QD_DEVINL int ring_ready(uint64_t* bars, int at, uint32_t parity, int ring, int most, unsigned int* status) {
+    if (ring < 6) {
+        const bool there = __all_sync(0xffffffffu, mbar_wait(bars + at, parity, status));
+        __syncwarp();
+        return there ? 1 : 0;
+    }
+    const int lane = threadIdx.x & 31, mine = at + lane < ring ? at + lane : at + lane - ring;
+    const bool done = lane < most && mbar_test_wait(bars + mine, parity ^ (at + lane >= ring ? 1u : 0u));
+    int n = __ffs(~__ballot_sync(0xffffffffu, done)) - 1;
+    if (n == 0) n = __all_sync(0xffffffffu, mbar_wait(bars + at, parity, status)) ? 1 : 0;
+    __syncwarp();
+    return n;
+}
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.
 // dst, src 16-byte aligned; bytes a multiple of 16.
 QD_DEVINL void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

@@ -81,11 +81,6 @@ QD_DEVINL void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uin
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
                  ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(kDescHiSw128), "r"(idesc), "r"(accumulate) : "memory");
 }
-QD_DEVINL bool elect_one() {
-    uint32_t leader;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
-    return leader != 0;
-}
 QD_DEVINL void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 QD_DEVINL void copy16_async(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -269,23 +264,27 @@ expert_tiles_kernel(const __grid_constant__ TileParams p, const __grid_constant_
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
             const uint32_t d = kColD + (turn & 1) * kSetCols;
             ok = __all_sync(0xffffffffu, mbar_wait(bars->d_empty + (turn & 1), ((turn >> 1) & 1) ^ 1, p.status));
-            for (int s = 0; s < 4 * chunks && ok; ++s) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bars->full + bs, phase, p.status));
+            for (int s = 0, m; s < 4 * chunks && ok; s += m) {
+                m = ring_ready(bars->full, bs, phase, kBStages, min(4 * chunks - s, kBStages), p.status);
+                ok = m > 0;
                 if (ok) {
                     tc_fence_after();
                     if (leader) {
-                        const uint32_t b = b0 + bs * (kBStageBytes >> 4), a = kColA + as * 64;
+                        for (int k = 0; k < m; ++k) {
+                            const int at = bs + k < kBStages ? bs + k : bs + k - kBStages;
+                            const uint32_t b = b0 + at * (kBStageBytes >> 4), a = kColA + (as + k) % kAStages * 64;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            umma_bf16_ts(d, a + j * 8, b + 2 * j, idesc, (s | j) ? 1u : 0u);
-                            umma_bf16_ts(d + kTileRoutes, a + 32 + j * 8, b + 2 * j, idesc, (s | j) ? 1u : 0u);
+                            for (int j = 0; j < 4; ++j) {
+                                umma_bf16_ts(d, a + j * 8, b + 2 * j, idesc, (s | k | j) ? 1u : 0u);
+                                umma_bf16_ts(d + kTileRoutes, a + 32 + j * 8, b + 2 * j, idesc, (s | k | j) ? 1u : 0u);
+                            }
+                            umma_commit(bars->empty + at);
                         }
-                        umma_commit(bars->empty + bs);
                     }
                     __syncwarp();
                 }
-                if (++bs == kBStages) { bs = 0; phase ^= 1; }
-                if (++as == kAStages) as = 0;
+                if ((bs += m) >= kBStages) { bs -= kBStages; phase ^= 1; }
+                as = (as + m) % kAStages;
             }
             if (ok && leader) umma_commit(bars->d_full + (turn & 1));
             __syncwarp();

@@ -44,10 +44,10 @@ __global__ void __launch_bounds__(256) fp8_quantize_rows_kernel(const uint4* __r
     q[i] = make_uint2(out[0], out[1]);
 }
 
-QD_DEVINL void umma_e4m3(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+QD_DEVINL void umma_e4m3(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128) : "memory");
 }
 
 struct F8Params { const float* w_scale; const float* in_scale; bf16* y; int tokens, rows, chunks, across, tiles; };
@@ -81,47 +81,59 @@ fp8_gemm_kernel(const __grid_constant__ F8Params p, const __grid_constant__ CUte
     const int mine = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, steps = mine * p.chunks;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0, tile = blockIdx.x;
-            bool ok = true;
-            for (int c = 0; issued < steps; ++issued, ++c) {
+        const bool leader = elect_one();
+        int issued = 0, st = 0, n = 1, c = 0, tile = blockIdx.x;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (; issued < steps; issued += n) {
+            n = ring_ready(empty, st, parity, kStages, min(steps - issued, kStages), nullptr);
+            if (n == 0) break;
+            for (int u = 0; u < n; ++u, ++c) {
                 if (c == p.chunks) { c = 0; tile += gridDim.x; }
-                const int st = issued % kStages;
-                if (issued >= kStages) ok = mbar_wait(empty + st, ((issued / kStages) - 1) & 1, nullptr);
-                if (!ok) break;
-                uint8_t* a = smem + st * Tile::kStageBytes;
-                mbar_expect_tx(full + st, Tile::kStageBytes);          // rows past a matrix's end arrive as zeros and count in full
-                tma_load_2d(a, &xmap, c * kF8Chunk, tile / p.across * kF8Tokens, full + st);
-                tma_load_2d(a + Tile::kABytes, &wmap, c * kF8Chunk, tile % p.across * TN, full + st);
-            }
-            if (!ok)            // leave no copy in flight behind
-                for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
-                    mbar_wait(full + s % kStages, (s / kStages) & 1, nullptr);
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            int s = 0;
-            for (int k = 0; k < mine && ok; ++k) {
-                if (k >= 2) ok = mbar_wait(taken + (k & 1), ((k >> 1) - 1) & 1, nullptr);
-                if (!ok) break;
-                tc_fence_after();
-                for (int c = 0; c < p.chunks; ++c, ++s) {
-                    const int st = s % kStages;
-                    ok = mbar_wait(full + st, (s / kStages) & 1, nullptr);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + Tile::kABytes;
-#pragma unroll
-                    for (int j = 0; j < kF8Chunk / 32; ++j)
-                        umma_e4m3(tmem + (k & 1) * TN, smem_desc_sw128(a + j * 32), smem_desc_sw128(b + j * 32), Tile::kDesc, (c | j) ? 1u : 0u);
-                    umma_commit(empty + st);
+                const int at = st + u < kStages ? st + u : st + u - kStages;
+                if (leader) {
+                    uint8_t* a = smem + at * Tile::kStageBytes;
+                    mbar_expect_tx(full + at, Tile::kStageBytes);          // rows past a matrix's end arrive as zeros and count in full
+                    tma_load_2d(a, &xmap, c * kF8Chunk, tile / p.across * kF8Tokens, full + at);
+                    tma_load_2d(a + Tile::kABytes, &wmap, c * kF8Chunk, tile % p.across * TN, full + at);
                 }
-                if (ok) umma_commit(ready + (k & 1));
             }
-            umma_commit(drained);             // tensor memory is given back only behind the last MMA, also where a wait ran out
-            mbar_wait(drained, 0, nullptr);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
         }
+        if (n == 0)             // leave no copy in flight behind
+            for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
+                mbar_wait(full + s % kStages, (s / kStages) & 1, nullptr);
+    } else if (warp == 1) {
+        const bool leader = elect_one();
+        const uint32_t low0 = __shfl_sync(0xffffffffu, desc_lo_sw128(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+        int st = 0, n = 1;
+        uint32_t parity = 0;
+        for (int k = 0; k < mine && n; ++k) {
+            if (k >= 2 && !__all_sync(0xffffffffu, mbar_wait(taken + (k & 1), ((k >> 1) - 1) & 1, nullptr))) break;
+            tc_fence_after();
+            for (int c = 0; c < p.chunks; c += n) {
+                n = ring_ready(full, st, parity, kStages, min(p.chunks - c, kStages), nullptr);
+                if (n == 0) break;
+                tc_fence_after();
+                if (leader) {
+                    for (int u = 0; u < n; ++u) {
+                        const int at = st + u < kStages ? st + u : st + u - kStages;
+                        const uint32_t a = low0 + at * (Tile::kStageBytes >> 4), b = a + (Tile::kABytes >> 4);
+#pragma unroll
+                        for (int j = 0; j < kF8Chunk / 32; ++j) umma_e4m3(to + (k & 1) * TN, a + 2 * j, b + 2 * j, Tile::kDesc, (c | u | j) ? 1u : 0u);
+                        umma_commit(empty + at);
+                    }
+                }
+                __syncwarp();
+                st += n;
+                if (st >= kStages) { st -= kStages; parity ^= 1u; }
+            }
+            if (n && leader) umma_commit(ready + (k & 1));
+            __syncwarp();
+        }
+        if (leader) umma_commit(drained);             // tensor memory is given back only behind the last MMA, also where a wait ran out
+        mbar_wait(drained, 0, nullptr);
     } else {
         const int quadrant = warp & 3;
         const float s_in = *p.in_scale, s_w = *p.w_scale;

@@ -19,9 +19,15 @@
 //               order, so the producers copy them with 16-byte loads into the same layout
 //   warp 0      allocates all 512 columns of tensor memory, issues 2 x 4 MMAs of 128x256x16 per
 //               stage and commits them to the stage's "empty" barrier
-// Stages: 3 x (32 KB activations + 32 KB weights) guarded by full / empty mbarriers.  Every wait
-// is bounded; a wait that runs out sets the status word, the block frees its tensor memory and
-// leaves.
+// Stages: as many as 192 KB hold (3 of 64 KB to 8 of 24 KB), guarded by full / empty mbarriers.  Every wait is bounded; a wait that runs
+// out sets the status word, the block frees its tensor memory and leaves.
+//
+// What bounds it: large tiles the expansion of the weights beside the MMAs and then the power limit; small ones, one block an SM, the hand-over from
+// stage to stage.  There the issuing warp was the chain: a look at a barrier takes it 150 to 300 clocks beside MMAs in flight, and an MMA 60 to issue
+// from one lane's branch.  Now the warp walks together, one lane chosen by elect.sync issues (18 clocks an MMA, operands in uniform registers), one
+// look serves all stages that are ready (ring_ready), and small tiles have 8 stages instead of 2.  512 rows of 2048 inputs: 64 tokens 13.8 -> 9.5 us, 2048
+// tokens 15.2 -> 10.7; 2048 rows of 4096 inputs: 511 tokens 26.7 -> 17.5, 2048 tokens 43.3 -> 35.0; 8192 rows of 2048: 511 tokens 25.0 -> 20.9, 2048
+// tokens 64.3 -> 63.3 (two rounds of blocks).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -34,10 +40,9 @@ constexpr int kTileM = 256;                 // tokens per tile: two halves of 12
 // large problems, 128 or 64 where 256 would leave most SMs without a tile
 constexpr int kTileK = 64;                  // inputs per stage
 // Tile heights: 256 tokens (two 128-token halves; the plain product and large grouped tiles) or
-// 128 (grouped product with few rows per expert: 2 stages of 48 KB and 8 producer warps, so that
-// two blocks share an SM and one block's prologue and epilogue overlap the other's K loop).
-constexpr int stages_of(int tm) { return tm == 128 ? 2 : 3; }
-constexpr int blocks_per_sm(int tm) { return tm == 128 ? 2 : 1; }
+// 128 (the plain product of few tiles, at most one block an SM; the grouped product with few rows per expert: 2 stages of 48 KB and 8 producer
+// warps, so that two blocks share an SM and one block's prologue and epilogue overlap the other's K loop).
+constexpr int blocks_per_sm(bool dense, int tm) { return !dense && tm == 128 ? 2 : 1; }
 // Producer warps: 8 for the plain product (they only expand weights), 16 for the grouped product
 // (they also gather the activation rows, and an expert's weights come from DRAM, not from L2:
 // more warps keep more loads in flight; measured 171 -> 149 us on the gate bank of a
@@ -45,19 +50,19 @@ constexpr int blocks_per_sm(int tm) { return tm == 128 ? 2 : 1; }
 constexpr int producer_warps(bool dense, int tm) { return (dense || tm == 128) ? 8 : 16; }
 constexpr int block_threads(bool dense, int tm) { return (2 + producer_warps(dense, tm)) * 32; }
 // The producer warps work in kGroups groups on alternate K steps, so that two stages fill at
-// the same time (measured: plain product 1 104 -> 1 138 TFLOP/s, grouped product unchanged).
+// the same time (measured: plain product 1 104 -> 1 138 TFLOP/s, grouped product unchanged); small plain tiles in up to four.
 #ifndef QD_GEMM_GROUPS
 #define QD_GEMM_GROUPS 2
 #endif
-constexpr int groups_of(int tm) { return tm == 128 ? 1 : QD_GEMM_GROUPS; }
-constexpr int group_threads(bool dense, int tm) { return producer_warps(dense, tm) * 32 / groups_of(tm); }
+constexpr int groups_of(bool dense, int tm, int tn) { return tm == 128 ? (dense ? (tn == 64 ? 4 : 2) : 1) : QD_GEMM_GROUPS; }
+constexpr int group_threads(bool dense, int tm, int tn) { return producer_warps(dense, tm) * 32 / groups_of(dense, tm, tn); }
 // Both operands of a stage use the 128-byte swizzled K-major layout: row r of the tile is 128
 // bytes (64 inputs) at r * 128, its 16-byte piece c stored at piece c ^ (r & 7).  The TMA load
 // writes it for the activations of the plain product; the producers write it themselves for
 // the weights (and for the gathered activation rows of the grouped product).
 constexpr int a_bytes(int tm) { return tm * kTileK * 2; }                  // 32 KB at 256 tokens
-constexpr int kBBytesMax = 256 * kTileK * 2;                                // 32 KB at 256 rows
-constexpr int stage_bytes(int tm) { return a_bytes(tm) + kBBytesMax; }
+constexpr int stage_bytes(bool dense, int tm, int tn) { return a_bytes(tm) + (dense ? tn : 256) * kTileK * 2; }
+constexpr int stages_of(bool dense, int tm, int tn) { return !dense && tm == 128 ? 2 : 196608 / stage_bytes(dense, tm, tn); }
 
 struct GemmParams {
     const bf16* x; const uint8_t* codes; const uint8_t* scales; const float* global; bf16* y;
@@ -82,10 +87,12 @@ QD_DEVINL void tmem_dealloc(uint32_t addr, uint32_t cols) {
 QD_DEVINL void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 QD_DEVINL void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 QD_DEVINL void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-QD_DEVINL void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+// a_low, b_low: the low words of the shared-memory descriptors (below); the high word is the same for every tile
+QD_DEVINL void umma_bf16(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    constexpr uint32_t high = (1024u >> 4) | (1u << 14) | (2u << 29);
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(high) : "memory");
 }
 QD_DEVINL void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -109,9 +116,7 @@ QD_DEVINL void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" 
 // 1024-byte boundary).  Bits: [0,14) address >> 4, [16,30) leading byte offset >> 4 (unused
 // here), [32,46) bytes between 8-row groups >> 4 = 64, [46,48) descriptor version 1, [61,64)
 // layout type 2.  A K step of 16 inputs advances the start address by 32 bytes inside the row.
-QD_DEVINL uint64_t smem_desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
+QD_DEVINL uint32_t smem_desc_low(uint32_t addr) { return ((addr >> 4) & 0x3fffu) | (1u << 16); }
 // Tiled 2-D TMA load global -> shared; c0 = innermost coordinate (elements; c0 * 2 bytes must be
 // a multiple of 16), c1 = row.  Completion is counted in bytes on the mbarrier.
 QD_DEVINL void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
@@ -147,24 +152,24 @@ QD_DEVINL uint4 expand8(uint32_t word, float scale) {
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-template <bool DENSE, int TM>
+template <bool DENSE, int TM, int TN>
 struct StageRegs {
-    static constexpr int kXPieces = TM * (kTileK / 8) / group_threads(DENSE, TM);   // 16-byte activation pieces per thread
-    static constexpr int kWPieces = 256 * 2 / group_threads(DENSE, TM);             // 16-byte code pieces per thread
+    static constexpr int kXPieces = TM * (kTileK / 8) / group_threads(DENSE, TM, TN);           // 16-byte activation pieces per thread
+    static constexpr int kWPieces = ((DENSE ? TN : 256) * 2 + group_threads(DENSE, TM, TN) - 1) / group_threads(DENSE, TM, TN);      // 16-byte code pieces per thread
     uint4 wc[kWPieces];               // 16-byte pieces of codes (32 weights each)
     uint16_t ws[kWPieces];            // their two block scales each
 };
 
 // DENSE: plain product (activation tiles by TMA through `xmap`); otherwise the grouped product.
 template <int TN, bool DENSE, int AHEAD, int TM>
-__global__ void __launch_bounds__(block_threads(DENSE, TM), blocks_per_sm(TM))
+__global__ void __launch_bounds__(block_threads(DENSE, TM), blocks_per_sm(DENSE, TM))
 nvfp4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap xmap) {
     chain_enter();
-    constexpr int kProducerWarps = producer_warps(DENSE, TM), kProducerThreads = group_threads(DENSE, TM);
+    constexpr int kProducerWarps = producer_warps(DENSE, TM), kProducerThreads = group_threads(DENSE, TM, TN);
     constexpr int kThreads = block_threads(DENSE, TM), kLoaderWarp = 1 + kProducerWarps;
-    constexpr int kGroups = groups_of(TM), kStages = stages_of(TM), kTileM = TM;
-    constexpr int kABytes = a_bytes(TM), kATmaBytes = kABytes, kStageBytes = stage_bytes(TM);
-    constexpr int kXPieces = StageRegs<DENSE, TM>::kXPieces, kWPiecesPerThread = StageRegs<DENSE, TM>::kWPieces;
+    constexpr int kGroups = groups_of(DENSE, TM, TN), kStages = stages_of(DENSE, TM, TN), kTileM = TM;
+    constexpr int kABytes = a_bytes(TM), kATmaBytes = kABytes, kStageBytes = stage_bytes(DENSE, TM, TN);
+    constexpr int kXPieces = StageRegs<DENSE, TM, TN>::kXPieces, kWPiecesPerThread = StageRegs<DENSE, TM, TN>::kWPieces;
     constexpr int kTileN = TN;
     constexpr int kTmemCols = (TM / 128) * TN;   // one 128 x TN fp32 accumulator per token half
     constexpr uint32_t kInstrDesc = instr_desc<TN>();
@@ -234,41 +239,62 @@ nvfp4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ 
 
     if (warp == 0) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            bool ok = true;
-            for (int s = 0; s < nk && ok; ++s) {
-                const int st = s % kStages;
-                ok = mbar_wait(full + st, (s / kStages) & 1, p.status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a = smem_u32(smem + st * kStageBytes), b = a + kABytes;
-#pragma unroll 1
-                for (int h = 0; h < halves; ++h)
+        const bool leader = elect_one();
+        const uint32_t low0 = __shfl_sync(0xffffffffu, smem_desc_low(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+        int st = 0, n = 1;
+        uint32_t parity = 0;
+        for (int s = 0; s < nk; s += n) {
+            n = ring_ready(full, st, parity, kStages, min(nk - s, kStages), p.status);
+            if (n == 0) break;
+            tc_fence_after();
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages ? st + u : st + u - kStages;
+                    const uint32_t a = low0 + at * (kStageBytes >> 4), b = a + (kABytes >> 4);
 #pragma unroll
-                    for (int j = 0; j < kTileK / 16; ++j) {
-                        umma_bf16(tmem + h * kTileN, smem_desc_sw128(a + h * (kABytes / 2) + j * 32),
-                                  smem_desc_sw128(b + j * 32), kInstrDesc, (s | j) ? 1u : 0u);
+                    for (int j = 0; j < kTileK / 16; ++j) umma_bf16(to, a + 2 * j, b + 2 * j, kInstrDesc, (s | u | j) ? 1u : 0u);
+                    if (halves > 1) {
+#pragma unroll
+                        for (int j = 0; j < kTileK / 16; ++j)
+                            umma_bf16(to + kTileN, a + (kABytes >> 5) + 2 * j, b + 2 * j, kInstrDesc, (s | u | j) ? 1u : 0u);
                     }
-                umma_commit(empty + st);          // the stage is free once these MMAs have read it
+                    umma_commit(empty + at);          // the stage is free once these MMAs have read it
+                }
             }
-            if (ok) umma_commit(done);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
+        }
+        if (leader) {
+            if (n) umma_commit(done);
             else *failed = 1;
         }
     } else if (warp == kLoaderWarp) {
         // ------------------------------------------------------- activation tiles by TMA
-        if (DENSE && lane == 0) {
-            for (int s = 0; s < nk; ++s) {
-                const int st = s % kStages;
-                if (s >= kStages && !mbar_wait(empty + st, ((s / kStages) - 1) & 1, p.status)) break;
-                mbar_expect_tx(full + st, kATmaBytes);
-                tma_load_2d(smem + st * kStageBytes, &xmap, s * kTileK, t0, full + st);
+        if (DENSE) {
+            const bool leader = elect_one();
+            int st = 0, n = 1;
+            uint32_t parity = 1;
+            for (int s = 0; s < nk; s += n) {
+                n = ring_ready(empty, st, parity, kStages, min(nk - s, kStages), p.status);      // (a new barrier's phase before the first is over)
+                if (n == 0) break;
+                if (leader) {
+                    for (int u = 0; u < n; ++u) {
+                        const int at = st + u < kStages ? st + u : st + u - kStages;
+                        mbar_expect_tx(full + at, kATmaBytes);
+                        tma_load_2d(smem + at * kStageBytes, &xmap, (s + u) * kTileK, t0, full + at);
+                    }
+                }
+                __syncwarp();
+                st += n;
+                if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
     } else {
         // ------------------------------------------------------------------- producers
         const int group = (tid - 32) / kProducerThreads;          // this warp's K steps: group, group + kGroups, ...
         const int pt = (tid - 32) % kProducerThreads;           // thread within the group
-        StageRegs<DENSE, TM> cur, nxt, far;      // K steps s, s + 1 and (AHEAD == 2) s + 2
+        StageRegs<DENSE, TM, TN> cur, nxt, far;      // K steps s, s + 1 and (AHEAD == 2) s + 2
         // the eight activation rows this thread copies pieces of (piece = (row, 8-input group))
         const bf16* xrow[DENSE ? 1 : kXPieces];
         if (!DENSE) {
@@ -293,7 +319,7 @@ nvfp4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ 
                 for (int off = 0; off < K / 16; off += 128) prefetch_l2(row_scales + off);
             }
         }
-        auto fetch = [&](int s, StageRegs<DENSE, TM>& r) {
+        auto fetch = [&](int s, StageRegs<DENSE, TM, TN>& r) {
             const int k0 = s * kTileK;
 #pragma unroll
             for (int i = 0; i < kWPiecesPerThread; ++i) {   // weights: piece = (row, 32-input half of the stage)
@@ -308,7 +334,7 @@ nvfp4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ 
                 }
             }
         };
-        auto store = [&](int st, int s, const StageRegs<DENSE, TM>& r) {
+        auto store = [&](int st, int s, const StageRegs<DENSE, TM, TN>& r) {
             uint8_t* a = smem + st * kStageBytes;
             uint8_t* b = a + kABytes;
             // rows without a token are not stored: an accumulator row depends on its own activation
@@ -439,7 +465,7 @@ static int activation_map(const GemmParams& p, CUtensorMap* map, int tile_tokens
 template <int TN, bool DENSE, int AHEAD, int TM>
 static int launch_variant(const GemmParams& p, int row_tiles, cudaStream_t stream) {
     // + 1024: the kernel moves its base up to a 1024-byte boundary
-    const size_t smem = (size_t)stages_of(TM) * stage_bytes(TM) + (2 * stages_of(TM) + 1) * 8 + 16 + 1024;
+    const size_t smem = (size_t)stages_of(DENSE, TM, TN) * stage_bytes(DENSE, TM, TN) + (2 * stages_of(DENSE, TM, TN) + 1) * 8 + 16 + 1024;
     static bool configured[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return QD_ERR_LAUNCH;
@@ -457,7 +483,7 @@ static int launch_variant(const GemmParams& p, int row_tiles, cudaStream_t strea
     return qd_launch(nvfp4_gemm_kernel<TN, DENSE, AHEAD, TM>, grid, dim3(block_threads(DENSE, TM)), smem, stream, true, p, map);
 }
 
-// The widest weight tile that still gives every SM a tile (narrower tiles expand fewer weights
+// The widest weight tile that still gives most SMs a tile (narrower tiles expand fewer weights
 // per block, so small problems finish sooner); `busy_row_tiles`: row tiles that will have rows.
 template <bool DENSE, int TM>
 static int launch_gemm(const GemmParams& p, int row_tiles, int busy_row_tiles, cudaStream_t stream) {
@@ -470,7 +496,10 @@ static int launch_gemm(const GemmParams& p, int row_tiles, int busy_row_tiles, c
     constexpr int kAhead = DENSE ? 2 : 1;
     // (narrower tiles to balance the last round of blocks do not pay: a 128-row block takes far
     // more than half the time of a 256-row block - gate bank of a 511-token chunk 143 -> 191 us)
-    if (wide >= sms) return launch_variant<256, DENSE, kAhead, TM>(p, row_tiles, stream);
+    // Plain product: the fewer rounds of blocks, a round of 128-row tiles taking 5/8 of one of 256-row tiles (2048 inputs: 20 and 32 us):
+    // 2048 tokens to 4096 rows one round of 128 wide tiles 33.2 us, two of narrow ones 39.9.
+    const bool fill = DENSE ? 8 * ((wide + sms - 1) / sms) <= 5 * ((2 * wide + sms - 1) / sms) : wide >= sms;
+    if (fill) return launch_variant<256, DENSE, kAhead, TM>(p, row_tiles, stream);
     if (4 * wide >= sms) return launch_variant<128, DENSE, kAhead, TM>(p, row_tiles, stream);
     return launch_variant<64, DENSE, kAhead, TM>(p, row_tiles, stream);
 }

@@ -87,41 +87,57 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
     auto stage = [&](int st) { return smem + (size_t)st * kStage4Bytes; };
 
     if (warp == 0) {
-        if (lane == 0) {
-            tma_prefetch_map(&x_codes); tma_prefetch_map(&x_scales); tma_prefetch_map(&w_codes); tma_prefetch_map(&w_scales);
-            for (int c = 0; c < chunks; ++c) {
-                const int st = c % kStages4;
-                if (!mbar_wait(bars->empty + st, ((c / kStages4) & 1) ^ 1, p.status)) break;
-                // rows past the end of a matrix arrive as zeros; a box always counts in full
-                mbar_expect_tx(bars->full + st, kStage4Bytes);
-                uint8_t* base = stage(st);
-                // codes: tokens, then the weight rows; scales in the same order
-                uint8_t* sc = base + 2 * kCodeBytes;
-                tma_load_2d(base, &x_codes, c * 128, t0, bars->full + st);
-                tma_load_2d(sc, &x_scales, c * 16, t0, bars->full + st);
-                tma_load_2d(base + kCodeBytes, &w_codes, c * 128, n0, bars->full + st);
-                tma_load_2d(sc + kScaleBytes, &w_scales, c * 16, n0, bars->full + st);
+        const bool leader = elect_one();
+        if (leader) { tma_prefetch_map(&x_codes); tma_prefetch_map(&x_scales); tma_prefetch_map(&w_codes); tma_prefetch_map(&w_scales); }
+        int st = 0, n = 1;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (int c = 0; c < chunks; c += n) {
+            n = ring_ready(bars->empty, st, parity, kStages4, min(chunks - c, kStages4), p.status);
+            if (n == 0) break;
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages4 ? st + u : st + u - kStages4;
+                    // rows past the end of a matrix arrive as zeros; a box always counts in full
+                    mbar_expect_tx(bars->full + at, kStage4Bytes);
+                    uint8_t* base = stage(at);
+                    // codes: tokens, then the weight rows; scales in the same order
+                    uint8_t* sc = base + 2 * kCodeBytes;
+                    tma_load_2d(base, &x_codes, (c + u) * 128, t0, bars->full + at);
+                    tma_load_2d(sc, &x_scales, (c + u) * 16, t0, bars->full + at);
+                    tma_load_2d(base + kCodeBytes, &w_codes, (c + u) * 128, n0, bars->full + at);
+                    tma_load_2d(sc + kScaleBytes, &w_scales, (c + u) * 16, n0, bars->full + at);
+                }
             }
+            __syncwarp();
+            st += n;
+            if (st >= kStages4) { st -= kStages4; parity ^= 1u; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int c = 0; c < chunks && ok; ++c) {
-                const int st = c % kStages4;
-                ok = mbar_wait(bars->full + st, (c / kStages4) & 1, p.status) &&
-                     mbar_wait(bars->sf_ready + st, (c / kStages4) & 1, p.status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a_lo = desc_lo_sw128(smem_u32(stage(st))), b_lo = desc_lo_sw128(smem_u32(stage(st) + kCodeBytes));
-                const uint32_t sfa = tmem + kColSf + st * kSfCols, sfb = sfa + 16;
+        const bool leader = elect_one();
+        const uint32_t low0 = __shfl_sync(0xffffffffu, desc_lo_sw128(smem_u32(stage(0))), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+        int st = 0, n = 1;
+        uint32_t parity = 0;
+        for (int c = 0; c < chunks; c += n) {
+            n = ring_ready(bars->full, st, parity, kStages4, min(chunks - c, kStages4), p.status);
+            if (n) n = ring_ready(bars->sf_ready, st, parity, kStages4, n, p.status);
+            if (n == 0) break;
+            tc_fence_after();
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages4 ? st + u : st + u - kStages4;
+                    const uint32_t a_lo = low0 + at * (kStage4Bytes >> 4), b_lo = a_lo + (kCodeBytes >> 4);
+                    const uint32_t sfa = to + kColSf + at * kSfCols, sfb = sfa + 16;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)       // a 64-input step: 32 bytes further in both operands
-                    umma_nvfp4_lo(tmem + kColAcc, a_lo + 2 * j, b_lo + 2 * j, desc_of(128, 128), sfa + j * 4, sfb + j * 4,
-                                  (c | j) ? 1u : 0u);
-                umma_commit(bars->empty + st);    // the stage (and its scale columns) is free once these MMAs are done
+                    for (int j = 0; j < 4; ++j)       // a 64-input step: 32 bytes further in both operands
+                        umma_nvfp4_lo(to + kColAcc, a_lo + 2 * j, b_lo + 2 * j, desc_of(128, 128), sfa + j * 4, sfb + j * 4, (c | u | j) ? 1u : 0u);
+                    umma_commit(bars->empty + at);    // the stage (and its scale columns) is free once these MMAs are done
+                }
             }
-            if (ok) umma_commit(&bars->done);
+            __syncwarp();
+            st += n;
+            if (st >= kStages4) { st -= kStages4; parity ^= 1u; }
         }
+        if (n && leader) umma_commit(&bars->done);
     } else {
         // ---- block scales of every stage into tensor memory: lane l of a quarter holds, per
         //      64-input step, the scale words of rows l, l + 32, l + 64, l + 96 in four columns
@@ -226,47 +242,65 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
 
     // A wait that runs out ends a role; everybody meets at the end, by when all copies and MMAs have long ended (the limit is 0.2 s).
     if (warp == 0) {
-        if (lane == 0) {
-            bool ok = true;
-            int it = 0;
-            for (int tile = pair; tile < tiles && ok; tile += pairs) {
-                const int t0 = (tile % across) * 256 + rank * 128, n0 = (tile / across) * 256;
-                for (int c = 0; c < chunks; ++c, ++it) {
-                    const int st = it % kStages;
-                    ok = mbar_wait(bars->empty + st, ((it / kStages) & 1) ^ 1, p.status);
-                    if (!ok) break;
-                    uint8_t* base = smem + st * T::kStageBytes;
-                    uint8_t* sc = base + 2 * kCodeBytes;
-                    const uint32_t bar = of_first_block(bars->full + st);
-                    if (rank == 0) mbar_expect_tx(bars->full + st, 4 * kCodeBytes);
-                    pair_tma_tile(base, &x_codes, c * 128, t0, bar);
-                    pair_tma_tile(base + kCodeBytes, &w_codes, c * 128, n0 + rank * 128, bar);
-                    mbar_expect_tx(bars->scales + st, 3 * kScaleBytes);
-                    tma_load_2d(sc, &x_scales, c * 16, t0, bars->scales + st);
-                    tma_load_2d(sc + kScaleBytes, &w_scales, c * 16, n0, bars->scales + st);
-                    tma_load_2d(sc + 2 * kScaleBytes, &w_scales, c * 16, n0 + 128, bars->scales + st);
+        const bool leader = elect_one();
+        int st = 0, n = 1;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (int tile = pair; tile < tiles && n; tile += pairs) {
+            const int t0 = (tile % across) * 256 + rank * 128, n0 = (tile / across) * 256;
+            for (int c = 0; c < chunks; c += n) {
+                n = ring_ready(bars->empty, st, parity, kStages, min(chunks - c, kStages), p.status);
+                if (n == 0) break;
+                if (leader) {
+                    for (int u = 0; u < n; ++u) {
+                        const int at = st + u < kStages ? st + u : st + u - kStages;
+                        uint8_t* base = smem + at * T::kStageBytes;
+                        uint8_t* sc = base + 2 * kCodeBytes;
+                        const uint32_t bar = of_first_block(bars->full + at);
+                        if (rank == 0) mbar_expect_tx(bars->full + at, 4 * kCodeBytes);
+                        pair_tma_tile(base, &x_codes, (c + u) * 128, t0, bar);
+                        pair_tma_tile(base + kCodeBytes, &w_codes, (c + u) * 128, n0 + rank * 128, bar);
+                        mbar_expect_tx(bars->scales + at, 3 * kScaleBytes);
+                        tma_load_2d(sc, &x_scales, (c + u) * 16, t0, bars->scales + at);
+                        tma_load_2d(sc + kScaleBytes, &w_scales, (c + u) * 16, n0, bars->scales + at);
+                        tma_load_2d(sc + 2 * kScaleBytes, &w_scales, (c + u) * 16, n0 + 128, bars->scales + at);
+                    }
                 }
+                __syncwarp();
+                st += n;
+                if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            bool ok = true;
-            int it = 0, i = 0;
-            for (int tile = pair; tile < tiles && ok; tile += pairs, ++i) {
-                if (i) ok = mbar_wait(&bars->taken, (i - 1) & 1, p.status);
-                for (int c = 0; c < chunks && ok; ++c, ++it) {
-                    const int st = it % kStages;
-                    ok = mbar_wait(bars->full + st, (it / kStages) & 1, p.status) && mbar_wait(bars->sf_ready + st, (it / kStages) & 1, p.status);
-                    if (!ok) break;
+        if (rank == 0) {
+            const bool leader = elect_one();
+            const uint32_t low0 = __shfl_sync(0xffffffffu, desc_lo_sw128(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+            int st = 0, n = 1, i = 0;
+            uint32_t parity = 0;
+            for (int tile = pair; tile < tiles; tile += pairs, ++i) {
+                if (i && !__all_sync(0xffffffffu, mbar_wait(&bars->taken, (i - 1) & 1, p.status))) break;
+                for (int c = 0; c < chunks; c += n) {
+                    n = ring_ready(bars->full, st, parity, kStages, min(chunks - c, kStages), p.status);
+                    if (n) n = ring_ready(bars->sf_ready, st, parity, kStages, n, p.status);
+                    if (n == 0) break;
                     tc_fence_after();
-                    const uint32_t a_lo = desc_lo_sw128(smem_u32(smem + st * T::kStageBytes)), b_lo = a_lo + (kCodeBytes >> 4);
-                    const uint32_t sfa = tmem + T::kColSf + st * T::kSfCols, sfb = sfa + 16;
+                    if (leader) {
+                        for (int u = 0; u < n; ++u) {
+                            const int at = st + u < kStages ? st + u : st + u - kStages;
+                            const uint32_t a_lo = low0 + at * (T::kStageBytes >> 4), b_lo = a_lo + (kCodeBytes >> 4);
+                            const uint32_t sfa = to + T::kColSf + at * T::kSfCols, sfb = sfa + 16;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        pair_umma_nvfp4(tmem, a_lo + 2 * j, b_lo + 2 * j, desc_of(256, 256), sfa + j * 4, sfb + j * 8, (c | j) ? 1u : 0u);
-                    pair_commit(bars->empty + st);
+                            for (int j = 0; j < 4; ++j)
+                                pair_umma_nvfp4(to, a_lo + 2 * j, b_lo + 2 * j, desc_of(256, 256), sfa + j * 4, sfb + j * 8, (c | u | j) ? 1u : 0u);
+                            pair_commit(bars->empty + at);
+                        }
+                    }
+                    __syncwarp();
+                    st += n;
+                    if (st >= kStages) { st -= kStages; parity ^= 1u; }
                 }
-                if (ok) pair_commit(&bars->ready);
+                if (n == 0) break;
+                if (leader) pair_commit(&bars->ready);
+                __syncwarp();
             }
         }
     } else if (warp < T::kFirst) {

@@ -282,17 +282,18 @@ template <int TN> struct UmmaTile {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
 };
 
-QD_DEVINL uint64_t desc_sw128(uint32_t addr) {      // K-major, 128-byte swizzle, 1024 bytes between groups of eight rows
-    return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);       // the same for every tile
+QD_DEVINL uint32_t desc_low(uint32_t addr) {      // K-major, 128-byte swizzle, 1024 bytes between groups of eight rows
+    return ((addr >> 4) & 0x3fffu) | (1u << 16);
 }
 QD_DEVINL void tma_tile(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
 }
-QD_DEVINL void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+QD_DEVINL void umma_f16(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(kDescHigh) : "memory");
 }
 QD_DEVINL void umma_commit_to(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -381,36 +382,52 @@ linear_umma_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     const uint32_t tmem = *slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0;
-            bool ok = true;
-            for (; issued < steps; ++issued) {
-                const int st = issued % kStages;
-                if (issued >= kStages) ok = mbar_wait(empty + st, ((issued / kStages) - 1) & 1, p.status);
-                if (!ok) break;
-                uint8_t* a = smem + st * Tile::kStageBytes;
-                mbar_expect_tx(full + st, Tile::kStageBytes);
-                tma_tile(a, &xmap, issued * kStepK, t0, full + st);
-                tma_tile(a + Tile::kABytes, &wmap, issued * kStepK, n0, full + st);
+        const bool leader = elect_one();
+        int issued = 0, st = 0, n = 1;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (; issued < steps; issued += n) {
+            n = ring_ready(empty, st, parity, kStages, min(steps - issued, kStages), p.status);
+            if (n == 0) break;
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages ? st + u : st + u - kStages;
+                    uint8_t* a = smem + at * Tile::kStageBytes;
+                    mbar_expect_tx(full + at, Tile::kStageBytes);
+                    tma_tile(a, &xmap, (issued + u) * kStepK, t0, full + at);
+                    tma_tile(a + Tile::kABytes, &wmap, (issued + u) * kStepK, n0, full + at);
+                }
             }
-            if (!ok)            // leave no copy in flight behind
-                for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
-                    mbar_wait(full + s % kStages, (s / kStages) & 1, p.status);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
         }
+        if (n == 0)             // leave no copy in flight behind
+            for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
+                mbar_wait(full + s % kStages, (s / kStages) & 1, p.status);
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int s = 0; s < steps; ++s) {
-                const int st = s % kStages;
-                ok = mbar_wait(full + st, (s / kStages) & 1, p.status);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + Tile::kABytes;
+        const bool leader = elect_one();
+        const uint32_t low0 = __shfl_sync(0xffffffffu, desc_low(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+        int st = 0, n = 1;
+        uint32_t parity = 0;
+        for (int s = 0; s < steps; s += n) {
+            n = ring_ready(full, st, parity, kStages, min(steps - s, kStages), p.status);
+            if (n == 0) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages ? st + u : st + u - kStages;
+                    const uint32_t a = low0 + at * (Tile::kStageBytes >> 4), b = a + (Tile::kABytes >> 4);
 #pragma unroll
-                for (int j = 0; j < kStepK / 16; ++j) umma_f16(tmem, desc_sw128(a + j * 32), desc_sw128(b + j * 32), kDesc, (s | j) ? 1u : 0u);
-                umma_commit_to(empty + st);
+                    for (int j = 0; j < kStepK / 16; ++j) umma_f16(to, a + 2 * j, b + 2 * j, kDesc, (s | u | j) ? 1u : 0u);
+                    umma_commit_to(empty + at);
+                }
             }
-            if (ok) umma_commit_to(done);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
+        }
+        if (leader) {
+            if (n) umma_commit_to(done);
             else *failed = 1;
         }
     } else {
@@ -560,44 +577,60 @@ linear_pieces_kernel(const __grid_constant__ LinearParams p, const __grid_consta
     const uint32_t tmem = *slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int issued = 0;
-            bool ok = true;
-            for (; issued < steps; ++issued) {
-                const int st = issued % kStages;
-                if (issued >= kStages) ok = mbar_wait(empty + st, ((issued / kStages) - 1) & 1, p.status);
-                if (!ok) break;
-                uint8_t* a = smem + st * Tile::kStageBytes;
-                mbar_expect_tx(full + st, Tile::kStageBytes);
-                for (int k = 0; k < 3; ++k)        // rows past a piece's last are another piece's: finite where x is, and not stored
-                    tma_tile(a + k * Tile::kABytes, &xmap, issued * kStepK, k * p.tokens + t0, full + st);
-                tma_tile(a + 3 * Tile::kABytes, &wmap, issued * kStepK, n0, full + st);
+        const bool leader = elect_one();
+        int issued = 0, st = 0, n = 1;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (; issued < steps; issued += n) {
+            n = ring_ready(empty, st, parity, kStages, min(steps - issued, kStages), p.status);
+            if (n == 0) break;
+            if (leader) {
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages ? st + u : st + u - kStages;
+                    uint8_t* a = smem + at * Tile::kStageBytes;
+                    mbar_expect_tx(full + at, Tile::kStageBytes);
+                    for (int k = 0; k < 3; ++k)        // rows past a piece's last are another piece's: finite where x is, and not stored
+                        tma_tile(a + k * Tile::kABytes, &xmap, (issued + u) * kStepK, k * p.tokens + t0, full + at);
+                    tma_tile(a + 3 * Tile::kABytes, &wmap, (issued + u) * kStepK, n0, full + at);
+                }
             }
-            if (!ok)            // leave no copy in flight behind
-                for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
-                    mbar_wait(full + s % kStages, (s / kStages) & 1, p.status);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
         }
+        if (n == 0)             // leave no copy in flight behind
+            for (int s = issued > kStages ? issued - kStages : 0; s < issued; ++s)
+                mbar_wait(full + s % kStages, (s / kStages) & 1, p.status);
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int s = 0; s < steps && ok; ++s) {
-                const int st = s % kStages, seg = s / kPerSegment, inside = s % kPerSegment;
-                if (inside == 0 && seg >= 2) ok = mbar_wait(taken + (seg & 1), ((seg >> 1) - 1) & 1, p.status);
-                ok = ok && mbar_wait(full + st, (s / kStages) & 1, p.status);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + 3 * Tile::kABytes, d = tmem + (seg & 1) * TN;
+        const bool leader = elect_one();
+        const uint32_t low0 = __shfl_sync(0xffffffffu, desc_low(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+        int st = 0, n = 1;
+        uint32_t parity = 0;
+        for (int s = 0; s < steps; s += n) {
+            const int seg = s / kPerSegment, inside0 = s % kPerSegment;
+            if (inside0 == 0 && seg >= 2 && !__all_sync(0xffffffffu, mbar_wait(taken + (seg & 1), ((seg >> 1) - 1) & 1, p.status))) break;
+            n = ring_ready(full, st, parity, kStages, min(min(steps - s, kPerSegment - inside0), kStages), p.status);       // of one segment
+            if (n == 0) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (leader) {
+                const uint32_t d = to + (seg & 1) * TN;
+                for (int u = 0; u < n; ++u) {
+                    const int at = st + u < kStages ? st + u : st + u - kStages, inside = inside0 + u;
+                    const uint32_t a = low0 + at * (Tile::kStageBytes >> 4), b = a + (3 * Tile::kABytes >> 4);
 #pragma unroll
-                for (int k = 2; k >= 0; --k)       // the small pieces first
+                    for (int k = 2; k >= 0; --k)       // the small pieces first
 #pragma unroll
-                    for (int j = 0; j < kStepK / 16; ++j)
-                        umma_f16(d, desc_sw128(a + k * Tile::kABytes + j * 32), desc_sw128(b + j * 32), kDesc, (inside || k < 2 || j) ? 1u : 0u);
-                umma_commit_to(empty + st);
-                if (inside == kPerSegment - 1 || s == steps - 1) umma_commit_to(ready + (seg & 1));
+                        for (int j = 0; j < kStepK / 16; ++j)
+                            umma_f16(d, a + k * (Tile::kABytes >> 4) + 2 * j, b + 2 * j, kDesc, (inside || k < 2 || j) ? 1u : 0u);
+                    umma_commit_to(empty + at);
+                    if (inside == kPerSegment - 1 || s + u == steps - 1) umma_commit_to(ready + (seg & 1));
+                }
             }
-            umma_commit_to(drained);          // tensor memory is given back only behind the last MMA, also where a wait ran out
-            mbar_wait(drained, 0, p.status);
+            __syncwarp();
+            st += n;
+            if (st >= kStages) { st -= kStages; parity ^= 1u; }
         }
+        if (leader) umma_commit_to(drained);          // tensor memory is given back only behind the last MMA, also where a wait ran out
+        mbar_wait(drained, 0, p.status);
     } else {
         const int half = (warp - 2) >> 2, quadrant = warp & 3;
         float acc[kHalf];

@@ -22,10 +22,10 @@ struct PairTile {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + (2 * kStages + 4) * 8 + 16 + 1024;
 };
 
-QD_DEVINL void pair_umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+QD_DEVINL void pair_umma_f16(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(kDescHigh) : "memory");
 }
 // Sixteen sums of a token, the first of them output n of the matrix, finished: eight (glu) or sixteen values into `out`.
 QD_DEVINL void finish16(const Finish& f, const uint32_t* v, int n, const float* bias, float (&out)[16]) {
@@ -135,42 +135,58 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
 
     // A wait that runs out ends a role; everybody meets at the end, by when all copies and MMAs have long ended (the limit is 0.2 s).
     if (warp == 0) {
-        if (lane == 0) {
-            bool ok = true;
-            int it = 0;
-            for (int tile = pair; tile < tiles && ok; tile += pairs) {
-                const int t0 = (tile % across) * 256 + rank * 128, n0 = (tile / across) * TN + rank * (TN / 2);
-                for (int s = 0; s < steps; ++s, ++it) {
-                    const int st = it % kStages;
-                    if (it >= kStages) ok = mbar_wait(empty + st, ((it / kStages) - 1) & 1, p.status);
-                    if (!ok) break;
-                    uint8_t* a = smem + st * Tile::kStageBytes;
-                    const uint32_t bar = of_first_block(full + st);
-                    if (rank == 0) mbar_expect_tx(full + st, 2 * Tile::kStageBytes);
-                    pair_tma_tile(a, &xmap, s * kStepK, t0, bar);
-                    pair_tma_tile(a + Tile::kHalfBytes, &wmap, s * kStepK, n0, bar);
+        const bool leader = elect_one();
+        int st = 0, n = 1;
+        uint32_t parity = 1;                       // (a new barrier's phase before the first is over)
+        for (int tile = pair; tile < tiles && n; tile += pairs) {
+            const int t0 = (tile % across) * 256 + rank * 128, n0 = (tile / across) * TN + rank * (TN / 2);
+            for (int s = 0; s < steps; s += n) {
+                n = ring_ready(empty, st, parity, kStages, min(steps - s, kStages), p.status);
+                if (n == 0) break;
+                if (leader) {
+                    for (int u = 0; u < n; ++u) {
+                        const int at = st + u < kStages ? st + u : st + u - kStages;
+                        uint8_t* a = smem + at * Tile::kStageBytes;
+                        const uint32_t bar = of_first_block(full + at);
+                        if (rank == 0) mbar_expect_tx(full + at, 2 * Tile::kStageBytes);
+                        pair_tma_tile(a, &xmap, (s + u) * kStepK, t0, bar);
+                        pair_tma_tile(a + Tile::kHalfBytes, &wmap, (s + u) * kStepK, n0, bar);
+                    }
                 }
+                __syncwarp();
+                st += n;
+                if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            bool ok = true;
-            int it = 0, i = 0;
-            for (int tile = pair; tile < tiles && ok; tile += pairs, ++i) {
+        if (rank == 0) {
+            const bool leader = elect_one();
+            const uint32_t low0 = __shfl_sync(0xffffffffu, desc_low(smem_u32(smem)), 0), to = __shfl_sync(0xffffffffu, tmem, 0);
+            int st = 0, n = 1, i = 0;
+            uint32_t parity = 0;
+            for (int tile = pair; tile < tiles; tile += pairs, ++i) {
                 const int buf = i & 1;
-                if (i >= 2) ok = mbar_wait(taken + buf, ((i >> 1) - 1) & 1, p.status);
-                for (int s = 0; s < steps && ok; ++s, ++it) {
-                    const int st = it % kStages;
-                    ok = mbar_wait(full + st, (it / kStages) & 1, p.status);
-                    if (!ok) break;
+                if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait(taken + buf, ((i >> 1) - 1) & 1, p.status))) break;
+                for (int s = 0; s < steps; s += n) {
+                    n = ring_ready(full, st, parity, kStages, min(steps - s, kStages), p.status);
+                    if (n == 0) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a = smem_u32(smem + st * Tile::kStageBytes), b = a + Tile::kHalfBytes;
+                    if (leader) {
+                        for (int u = 0; u < n; ++u) {
+                            const int at = st + u < kStages ? st + u : st + u - kStages;
+                            const uint32_t a = low0 + at * (Tile::kStageBytes >> 4), b = a + (Tile::kHalfBytes >> 4);
 #pragma unroll
-                    for (int j = 0; j < kStepK / 16; ++j)
-                        pair_umma_f16(tmem + buf * TN, desc_sw128(a + j * 32), desc_sw128(b + j * 32), kDesc, (s | j) ? 1u : 0u);
-                    pair_commit(empty + st);
+                            for (int j = 0; j < kStepK / 16; ++j) pair_umma_f16(to + buf * TN, a + 2 * j, b + 2 * j, kDesc, (s | u | j) ? 1u : 0u);
+                            pair_commit(empty + at);
+                        }
+                    }
+                    __syncwarp();
+                    st += n;
+                    if (st >= kStages) { st -= kStages; parity ^= 1u; }
                 }
-                if (ok) pair_commit(ready + buf);
+                if (n == 0) break;
+                if (leader) pair_commit(ready + buf);
+                __syncwarp();
             }
         }
     } else {

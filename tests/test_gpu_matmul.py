@@ -33,6 +33,22 @@ def test_matmul_matches_oracle(cuda_device, tokens, out_features, in_features):
     assert O.rel_l2(got, exact) < 1e-2
 
 
+@pytest.mark.parametrize("tokens,out_features,in_features", [(40, 72, 64), (130, 200, 576), (500, 4096, 448), (600, 6400, 320), (300, 8200, 256), (1025, 3080, 768)])
+def test_matmul_of_every_tile(cuda_device, tokens, out_features, in_features):
+    """Tiles of 128 and 256 tokens by 64, 128 and 256 rows, with fewer steps than stages, as many, and rings that turn.
+    Exact products, fp32 sums, one bf16 rounding: 2^-9 of each output and 2^-22 of the terms' root sum."""
+    from quickdraw_b200 import kernels
+    src = synthetic.Source(22, "cpu")
+    proj = src.nvfp4(f"w{out_features}x{in_features}", out_features, in_features, global_scale=0.75)
+    x = src.normal(f"x{tokens}", tokens, in_features)
+    got = kernels.matmul(x.to(cuda_device), to_device(proj, cuda_device)).double()
+    assert kernels.matmul_status(cuda_device) == 0
+    w, xd = O.dequantize_fp32(proj).to(cuda_device).double(), x.to(cuda_device).double()
+    want = xd @ w.T
+    bound = want.abs() * 2.0 ** -8 + 2.0 ** -20 * ((xd * xd) @ (w * w).T).sqrt()
+    assert bool(((got - want).abs() <= bound).all())
+
+
 ROWS_SHAPES = [(1, 16, 512), (7, 528, 2048), (32, 8192, 2048), (32, 2048, 4096), (19, 96, 1024), (32, 9472, 512)]
 
 
