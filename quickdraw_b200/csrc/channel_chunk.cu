@@ -300,12 +300,14 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
         for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[nt][c] = tile[(size_t)(8 * nt + 2 * t + (c & 1)) * p.vdim + 8 * (c >> 1)];
+        bool ahead = false;                    // the next chunk's terms are there: asked for under this one's products (a look takes 200 clocks)
 #pragma unroll 1
         for (int chunk = 0; chunk < chunks; ++chunk) {
             const ChannelStage<DELTA>& st = s.stage[chunk % kStages];
             const int odd = chunk & 1;
             ChannelHandover& over = s.over[slice][odd];
-            if (there) there = __all_sync(0xffffffffu, mbar_wait(s.full + chunk % kStages, (chunk / kStages) & 1, p.status));
+            if (there)
+                there = __all_sync(0xffffffffu, ahead) || __all_sync(0xffffffffu, mbar_wait(s.full + chunk % kStages, (chunk / kStages) & 1, p.status));
             if (chunk >= 2) named_barrier(bar + kBarFree + odd, 128);         // the results of two chunks ago are formed
             // ---- U = V, or (I + L)^-1 B (V - K+ S_0), transposed; the state is handed over on the way
             float u[2][4];
@@ -363,6 +365,7 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
             if (half == 0) over.u[lane] = w;
             named_arrive(bar + kBarU + odd, 128);
             // ---- S = diag(G_C) S_0 + K-^T U, transposed: four key tiles at a time
+            ahead = mbar_test_wait(s.full + (chunk + 1) % kStages, ((chunk + 1) / kStages) & 1);
             uint4 b[2][2][3];
 #pragma unroll
             for (int h = 0; h < 2; ++h)

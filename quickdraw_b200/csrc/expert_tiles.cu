@@ -295,11 +295,12 @@ expert_tiles_kernel(const __grid_constant__ TileParams p, const __grid_constant_
         const int tile = (warp >> 2) & 1, group = warp >> 3, row = (warp & 3) * 32 + lane;
         const uint32_t a = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kColA + tile * 32;
         int fill = 0, slot = group, phase = 0;                              // of the group's next step
-        bool ok = true;
+        bool ok = true, there = mbar_test_wait(bars->w_full, 0);
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             for (int c = 0; c < chunks && ok; ++c, ++fill) {
                 const int st = fill % kWStages;
-                ok = __all_sync(0xffffffffu, mbar_wait(bars->w_full + st, (fill / kWStages) & 1, p.status));
+                // (a look at a barrier takes some 200 clocks: it is asked for ahead of its use, and again only if it came too early)
+                ok = __all_sync(0xffffffffu, there) || __all_sync(0xffffffffu, mbar_wait(bars->w_full + st, (fill / kWStages) & 1, p.status));
                 if (!ok) break;
                 const uint8_t* codes = smem + st * kWStageBytes + tile * kCodeTile + row * 128;
                 const uint4 sc = lds128(smem + st * kWStageBytes + 2 * kCodeTile + tile * kScaleTile + row * 16);
@@ -311,7 +312,12 @@ expert_tiles_kernel(const __grid_constant__ TileParams p, const __grid_constant_
                     if (half == 1) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bars->w_empty + st);
+                        there = mbar_test_wait(bars->w_full + (fill + 1) % kWStages, ((fill + 1) / kWStages) & 1);
                     }
+                    // whether the step kAStages before this one has been multiplied
+                    uint64_t* const before_it = bars->empty + (slot >= kAStages ? slot - kAStages : slot + kAStages);
+                    const int its_phase = slot >= kAStages ? phase : phase ^ 1;
+                    const bool freed = mbar_test_wait(before_it, its_phase);
                     const uint32_t words[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                     uint32_t v[32];
 #pragma unroll
@@ -322,10 +328,8 @@ expert_tiles_kernel(const __grid_constant__ TileParams p, const __grid_constant_
                         decode8<1>(words[4 * q + 2], scales, v + 16 * q + 8);
                         decode8<1>(words[4 * q + 3], scales, v + 16 * q + 12);
                     }
-                    // the step kAStages before this one has been multiplied
-                    ok = slot >= kAStages ? mbar_wait(bars->empty + slot - kAStages, phase, p.status)
-                                          : mbar_wait(bars->empty + slot + kAStages, phase ^ 1, p.status);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, freed) || __all_sync(0xffffffffu, mbar_wait(before_it, its_phase, p.status));
+                    if (!ok) break;
                     tc_fence_after();
                     tmem_store32(a + (slot >= kAStages ? slot - kAStages : slot) * 64, v);
                     tmem_store_wait();
