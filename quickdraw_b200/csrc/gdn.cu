@@ -177,9 +177,54 @@ __global__ void gdn_gated_norm_kernel(const bf16* __restrict__ o, const bf16* __
     }
 }
 
+// The same for many heads of 128 on 16-byte boundaries: sixteen lanes a head, eight values a lane, four heads a warp requested at once.  Bound by
+// its SiLUs and the 50 MB of 65536 heads (7.6 us): 17.5 -> 10.3 us.
+__global__ void __launch_bounds__(128)
+gdn_gated_norm128_kernel(const bf16* __restrict__ o, const bf16* __restrict__ z, const bf16* __restrict__ gamma, bf16* __restrict__ out, int heads, float eps) {
+    chain_enter();
+    const int lane = threadIdx.x & 31, head0 = ((blockIdx.x * 4 + (threadIdx.x >> 5)) << 2) + (lane >> 4), c = 8 * (lane & 15);
+    uint4 ov[2], zv[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const size_t at = (size_t)min(head0 + 2 * i, heads - 1) * 128 + c;
+        ov[i] = *reinterpret_cast<const uint4*>(o + at);
+        zv[i] = *reinterpret_cast<const uint4*>(z + at);
+    }
+    const uint4 gv = *reinterpret_cast<const uint4*>(gamma + c);
+    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w}, zw[4] = {zv[i].x, zv[i].y, zv[i].z, zv[i].w};
+        float ss = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float a = bf16_bits_to_float(ow[q] & 0xffffu), b = bf16_bits_to_float(ow[q] >> 16);
+            ss += a * a + b * b;
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+        const float inv = rsqrtf(ss / 128.f + eps);
+        uint32_t r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float a = ((bf16_bits_to_float(ow[q] & 0xffffu) * inv) * bf16_bits_to_float(gw[q] & 0xffffu)) * silu_precise(bf16_bits_to_float(zw[q] & 0xffffu));
+            const float b = ((bf16_bits_to_float(ow[q] >> 16) * inv) * bf16_bits_to_float(gw[q] >> 16)) * silu_precise(bf16_bits_to_float(zw[q] >> 16));
+            const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
+            r[q] = *reinterpret_cast<const uint32_t*>(&two);
+        }
+        if (head0 + 2 * i < heads) *reinterpret_cast<uint4*>(out + (size_t)(head0 + 2 * i) * 128 + c) = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
 extern "C" int qd_gdn_gated_norm(const void* o, const void* z, const void* gamma, void* out, int heads,
                                  int value_dim, float eps, void* stream) {
     QD_CHECK_ARG(o && z && gamma && out && heads > 0 && value_dim > 0);
+    // (few heads, a token's 32: a warp each, so that their loads start side by side)
+    if (heads >= 2048 && value_dim == 128 && !(((uintptr_t)o | (uintptr_t)z | (uintptr_t)gamma | (uintptr_t)out) & 15u)) {
+        qd_launch(gdn_gated_norm128_kernel, dim3((heads + 15) / 16), dim3(128), 0, (cudaStream_t)stream, true,
+                  (const bf16*)o, (const bf16*)z, (const bf16*)gamma, (bf16*)out, heads, eps);
+        return qd_launch_status();
+    }
     qd_launch(gdn_gated_norm_kernel, dim3((heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, true, 
         (const bf16*)o, (const bf16*)z, (const bf16*)gamma, (bf16*)out, heads, value_dim, eps);
     return qd_launch_status();

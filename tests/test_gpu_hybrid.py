@@ -671,3 +671,52 @@ def test_recurrence_in_chunks_keeps_to_the_past(delta, bad):
     reached[21:, 1, 5] = True
     assert not torch.isfinite(out[reached]).any()
     assert error(out[~reached], want[~reached]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim,vdim,taps,position", [(1, 2, 1, 128, 128, 4, 0), (13, 3, 3, 20, 132, 4, 2), (40, 8, 2, 128, 64, 3, 1),
+                                                                          (16, 1, 1, 4, 4, 2, 5), (9, 16, 16, 128, 128, 4, 700)])
+def test_prepares_in_whole_pieces_give_the_bits_of_the_narrow_ones(cuda_device, dtype, tokens, heads, kv_heads, dim, vdim, taps, position):
+    """Inputs on the boundaries of four values, and the same one element further on (the narrow kernels): the same arithmetic, the same bits."""
+    from quickdraw_b200._lib import call_hybrid, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens + heads)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device)
+    code = 0 if dtype is torch.bfloat16 else 1
+    keys, values, kv = heads * dim, heads * vdim, kv_heads * dim
+    ld = (2 * max(kv, keys) + values + heads + 11) // 8 * 8
+    rows, z = new(tokens, ld).to(dtype), new(tokens, keys)
+    bias, a_log = new(keys).to(torch.bfloat16), new(heads).to(torch.bfloat16)
+    weights = [new(n, taps).to(torch.bfloat16) for n in (kv, kv, values)]
+    ring = new(taps, 2 * kv + values).to(dtype)
+    results = []
+    for shift in (0, 1):
+        flat = torch.zeros(tokens * ld + 8, dtype=dtype, device=cuda_device)
+        flat[shift:shift + tokens * ld] = rows.flatten()
+        size, at = flat.element_size(), flat.data_ptr() + shift * flat.element_size()
+        outs = [torch.full((tokens, n), float("nan"), device=cuda_device) for n in (kv, kv, keys, values, heads, 3 * kv_heads)]
+        history = ring.clone()
+        call_hybrid("qd_channel_delta_prepare", at, at + kv * size, at + 2 * kv * size, at + (2 * kv + values) * size, ld, ptr(z), ptr(bias), ptr(a_log),
+                    *[ptr(w) for w in weights], ptr(history), taps, None, position, *[ptr(o) for o in outs], tokens, heads, kv_heads, dim, vdim, code,
+                    stream_of(z))
+        more = [torch.full((tokens, n), float("nan"), device=cuda_device) for n in (keys, keys, keys, values)]
+        call_hybrid("qd_gla_prepare", at, at + keys * size, at + 2 * keys * size, ld, ptr(z), ptr(bias), 16.0, *[ptr(o) for o in more], tokens, heads, dim,
+                    vdim, code, stream_of(z))
+        results.append(outs + more + [history])
+    assert all(torch.equal(a, b) and torch.isfinite(a).all() for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,heads,act", [(1, 1, 0), (3, 5, 1), (130, 16, 0)])
+def test_head_norm_and_gate_of_heads_of_128(cuda_device, dtype, tokens, heads, act):
+    """Two heads a warp, also an odd number of them; fp32 sums of 128 squares (2^-20), one rounding of the result."""
+    from quickdraw_b200._lib import call_hybrid, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(tokens)
+    x, w = torch.randn(tokens, heads * 128, generator=gen, device=cuda_device) * 3, torch.randn(128, generator=gen, device=cuda_device).to(torch.bfloat16)
+    gate = torch.randn(tokens, heads * 128 + 8, generator=gen, device=cuda_device).to(dtype)
+    out = torch.full((tokens, heads * 128), float("nan"), dtype=dtype, device=cuda_device)
+    call_hybrid("qd_head_norm_gate", ptr(x), ptr(w), ptr(gate), gate.shape[1], ptr(out), tokens, heads, 128, 1e-5, act,
+                0 if dtype is torch.bfloat16 else 1, stream_of(x))
+    v, g = x.double().view(tokens, heads, 128), gate[:, :heads * 128].double().view(tokens, heads, 128)
+    want = v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(g) * (1 if act else g)
+    bound = want.abs() * (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -19)
+    assert bool(((out.double().view_as(want) - want).abs() <= bound + 1e-30).all())

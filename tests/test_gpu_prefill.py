@@ -405,3 +405,19 @@ def test_grouped_product_in_every_tile_shape(cuda_device, counts, width, rows):
         torch.testing.assert_close(plain[here].double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
         want = x[here].double() @ matrix.T * weights[at].double()[:, None]
         torch.testing.assert_close(routed[at].double(), want, rtol=3.1 * 2 ** -8, atol=1e-5 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("heads", [2048, 2049, 2063, 8192])
+def test_gated_norm_of_many_heads(cuda_device, heads):
+    """Four heads a warp from 2048 heads on, ragged ends; one rounding of fp32 arithmetic, and fewer heads with the other kernel."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(heads)
+    o, z = (torch.randn(heads, 128, generator=gen, device=cuda_device).to(torch.bfloat16) for _ in range(2))
+    gamma = torch.randn(128, generator=gen, device=cuda_device).to(torch.bfloat16)
+    out, few = torch.full_like(o, float("nan")), torch.empty_like(o[:100])
+    call("qd_gdn_gated_norm", ptr(o), ptr(z), ptr(gamma), ptr(out), heads, 128, 1e-6, stream_of(o))
+    call("qd_gdn_gated_norm", ptr(o), ptr(z), ptr(gamma), ptr(few), 100, 128, 1e-6, stream_of(o))
+    v, g = o.double(), z.double()
+    want = v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-6) * gamma.double() * g * torch.sigmoid(g)
+    assert bool(((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-30).all())
+    assert bool(((few.double() - want[:100]).abs() <= want[:100].abs() * 2.0 ** -8 + 1e-30).all())
