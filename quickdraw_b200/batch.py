@@ -64,8 +64,11 @@ class BatchDecode(ChunkPrefill):
         self._graphs = {}
 
     def _attn_splits(self, batch, context):
-        """Context splits per (sequence, KV head): the count whose blocks fill whole waves of the
-        GPU best (one block per SM; a split costs a merge, 16 at most)."""
+        """Context splits per (sequence, KV head), 16 at most.  Heads of 256, up to 256 sequences: the kernel shares the context out by the
+        sequences' own lengths and only wants to know how many parts the scratch has room for.  Else the count whose blocks
+        fill whole waves of the GPU best (one block per SM; a split costs a merge)."""
+        if self.ckpt.config.head_dim == 256 and batch <= 256:
+            return MAX_ATTN_SPLITS
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         pairs = batch * self.ckpt.config.num_key_value_heads
         cost = lambda s: -(-pairs * s // sms) * (-(-context // s) + 64)

@@ -908,7 +908,8 @@ batch_attn_lanes_kernel(const LaneAttnParams p) {
 // into the MMA fragments (no staging in shared memory): per chunk a lane loads 16 x 16 bytes of
 // its two key rows, and, once the scores are out, 16 x 16 bytes of four value rows while the
 // next chunk's keys are already on their way.  The lane-per-position kernel above spends its
-// time in scalar FMAs (28 % of the HBM bandwidth at 32 sequences x 8192 positions).
+// time in scalar FMAs (28 % of the HBM bandwidth at 32 sequences x 8192 positions).  The kernel with a block for each (KV head, split, sequence)
+// is left for what batch_attn_flat_kernel, below, does not take: tokens of one sequence over a shared cache, split count 1, more sequences.
 struct AttnKeys { uint4 a[8], b[8]; };      // bytes 64 m + 16 t .. + 15 of key rows prow and 8 + prow
 
 QD_DEVINL uint4 ld_stream16(const uint8_t* p) {
@@ -925,33 +926,19 @@ QD_DEVINL void attn_load_keys(AttnKeys& k, const uint8_t* __restrict__ base, siz
     for (int m = 0; m < 8; ++m) { k.a[m] = ld_stream16(r0 + m * 64); k.b[m] = ld_stream16(r1 + m * 64); }
 }
 
-__global__ void __launch_bounds__(kLaneAttnWarps * 32, 1)
-batch_attn_mma_kernel(const LaneAttnParams p) {
-    chain_enter();
-    extern __shared__ __align__(16) unsigned char mma_attn_smem[];
+// Positions [t0, t1) of sequence z against the query heads of KV head kvh by all warps of a block: every warp's running state into
+// red[warp][head][d + 2] (weighted values, maximum, sum).
+QD_DEVINL void lane_attn_walk(const LaneAttnParams& p, uint8_t* q_s, float* red, size_t z, int kvh, int T, int t0, int t1, int tid) {
     constexpr int D = 256;
-    const int G = p.hq / p.hk, stride = D + 2;
-    uint8_t* q_s = mma_attn_smem;                                                       // [8][kAttnQRow]
-    float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][D + 2]
-    const int kvh = blockIdx.x, split = blockIdx.y;
-    const size_t z = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int T = p.positions[z] + 1;
-    if (T < 1 || T > p.capacity) return;      // a position outside the cache: the sequence's output is left alone
-    int active = (T + kLaneAttnSplitMin - 1) / kLaneAttnSplitMin;
-    if (active > p.splits) active = p.splits;
-    const int per = ((T + active - 1) / active + 31) & ~31;
-    const int t0 = split * per, t1 = min(T, t0 + per);
-    const bool mine = split < active && t0 < t1;
+    const int G = p.hq / p.hk, stride = D + 2, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const size_t row_bytes = (size_t)p.hk * D * sizeof(bf16);
     const uint8_t* kc = reinterpret_cast<const uint8_t*>(p.k_cache + z * p.cache_stride + (size_t)kvh * D);
     const uint8_t* vc = reinterpret_cast<const uint8_t*>(p.v_cache + z * p.cache_stride + (size_t)kvh * D);
-
     AttnAcc acc;
     acc.m = -INFINITY; acc.l = 0.f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) { acc.out[i][0] = 0.f; acc.out[i][1] = 0.f; acc.out[i][2] = 0.f; acc.out[i][3] = 0.f; }
-    if (mine) {
+    if (t0 < t1) {
         AttnKeys keys;
         int c = t0 + warp * 16;
         if (c < t1) attn_load_keys(keys, kc, row_bytes, c, T - 1, lane);
@@ -981,8 +968,6 @@ batch_attn_mma_kernel(const LaneAttnParams p) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) qd::attn_value_step(acc, q, values[q][0], values[q][1], values[q][2], values[q][3], pr);
         }
-    } else {
-        __syncthreads();
     }
     // ---- the warp's state in the layout of the merge: lane (g, t) holds the statistics of head g
     // (the sum still spread over its four lanes) and out[i][c] = feature 32 g + 2 i + (c >> 1) of head 2 t + (c & 1)
@@ -1000,8 +985,145 @@ batch_attn_mma_kernel(const LaneAttnParams p) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) { dst[2 * i] = acc.out[i][cc]; dst[2 * i + 1] = acc.out[i][2 + cc]; }
     }
+}
+
+__global__ void __launch_bounds__(kLaneAttnWarps * 32, 1)
+batch_attn_mma_kernel(const LaneAttnParams p) {
+    chain_enter();
+    extern __shared__ __align__(16) unsigned char mma_attn_smem[];
+    uint8_t* q_s = mma_attn_smem;                                                       // [8][kAttnQRow]
+    float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][D + 2]
+    const int kvh = blockIdx.x, split = blockIdx.y;
+    const size_t z = blockIdx.z;
+    const int tid = threadIdx.x;
+    const int T = p.positions[z] + 1;
+    if (T < 1 || T > p.capacity) return;      // a position outside the cache: the sequence's output is left alone
+    int active = (T + kLaneAttnSplitMin - 1) / kLaneAttnSplitMin;
+    if (active > p.splits) active = p.splits;
+    const int per = ((T + active - 1) / active + 31) & ~31;
+    const int t0 = split * per, t1 = min(T, t0 + per);
+    lane_attn_walk(p, q_s, red, z, kvh, T, t0, split < active ? t1 : t0, tid);
     __syncthreads();
     lane_attn_finish(p, red, z, kvh, split, active, tid);
+}
+
+// The same with the batch's whole context shared out evenly, whatever the sequences' lengths and the cache's capacity: the 32-position units of
+// all (sequence, KV head) pairs lie one after the other and block b takes units [b share, (b + 1) share), most often parts of one or
+// two pairs.  A pair that one block holds needs no partial result; of others the last block to arrive merges at most `splits` parts.
+// With a split count from the capacity (32768 where the contexts were 8192) a block of 512 positions spent half of its 27 us on its start and
+// on merging its warps: 32 sequences of 8192 positions, 16 heads on 2 of 256, 190 -> 97 us
+// (537 MB); of 2000 103 -> 45, of 500 75 -> 22, of 64 60 -> 13.  At most kFlatBatch sequences.
+constexpr int kFlatBatch = kLaneAttnWarps * 32, kFlatMin = 8;           // units of a share at least, where a sequence has as many
+__global__ void __launch_bounds__(kLaneAttnWarps * 32, 1)
+batch_attn_flat_kernel(const LaneAttnParams p, int batch) {
+    chain_enter();
+    extern __shared__ __align__(16) unsigned char mma_attn_smem[];
+    __shared__ int before[kFlatBatch + 1], longest[kLaneAttnWarps], sums[kLaneAttnWarps], s_last;
+    __shared__ float weight[kLaneAttnGroup][16], most[kLaneAttnGroup], norm[kLaneAttnGroup];
+    constexpr int D = 256;
+    uint8_t* q_s = mma_attn_smem;                                                       // [8][kAttnQRow]
+    float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][D + 2]
+    const int G = p.hq / p.hk, stride = D + 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    {   // units of the sequences in front of each
+        const int T = tid < batch ? p.positions[tid] + 1 : 0, n = T < 1 || T > p.capacity ? 0 : (T + 31) / 32;     // (outside the cache: left alone)
+        int sum = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += up;
+        }
+        const int top = __reduce_max_sync(0xffffffffu, n);
+        if (lane == 31) { sums[warp] = sum; longest[warp] = top; }
+        __syncthreads();
+        int front = 0;
+        for (int w = 0; w < warp; ++w) front += sums[w];
+        if (tid < batch) before[tid + 1] = front + sum;
+        if (tid == 0) before[0] = 0;
+        __syncthreads();
+    }
+    int top = 0;
+    for (int w = 0; w < kLaneAttnWarps; ++w) top = max(top, longest[w]);
+    const int units = p.hk * before[batch];
+    const int share = max(max((units + (int)gridDim.x - 1) / (int)gridDim.x, min(kFlatMin, top)), (top + p.splits - 2) / (p.splits - 1));
+    const int end = min(units, ((int)blockIdx.x + 1) * share);
+    for (int u = (int)blockIdx.x * share; u < end;) {
+        int lo = 0, hi = batch;                              // hk before[lo] <= u < hk before[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (p.hk * before[mid] <= u) lo = mid; else hi = mid;
+        }
+        const size_t z = lo;
+        const int n = before[lo + 1] - before[lo], kvh = (u - p.hk * before[lo]) / n, start = p.hk * before[lo] + kvh * n, from = u - start;
+        const int count = min(end - u, n - from), T = p.positions[z] + 1, first = start / share, parts = (start + n - 1) / share - first + 1;
+        lane_attn_walk(p, q_s, red, z, kvh, T, from * 32, min(T, (from + count) * 32), tid);
+        __syncthreads();
+        if (tid < 8 * kLaneAttnGroup) {                      // a lane for each warp's state of a head
+            const int h = tid >> 3, w = tid & 7;
+            const float* src = red + ((size_t)w * G + h) * stride + D;
+            const float m = h < G ? src[0] : -INFINITY, l = h < G ? src[1] : 0.f;
+            float mm = m;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+            const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+            float den = wgt * l;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+            weight[h][w] = wgt;
+            if (w == 0) { most[h] = mm; norm[h] = den; }
+        }
+        __syncthreads();
+        const auto put = [&](int h, float num, float den) {
+            const int qh = kvh * G + h;
+            const float gate = round_bf16(sigmoid_precise(ld_bf16(p.qg + (z * p.hq + qh) * 2 * (size_t)D + D + tid)));
+            p.out[(z * p.hq + qh) * (size_t)D + tid] = __float2bfloat16_rn(round_bf16(num / den) * gate);
+        };
+        float* partial = p.partial + (z * p.hk + kvh) * (size_t)p.splits * G * stride;            // [part][G][D + 2]
+        for (int h = 0; h < G; ++h) {                        // a thread's feature of every head
+            float num = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLaneAttnWarps; ++w) num += weight[h][w] * red[((size_t)w * G + h) * stride + tid];
+            if (parts == 1) put(h, num, norm[h]);
+            else {
+                float* dst = partial + ((size_t)(blockIdx.x - first) * G + h) * stride;
+                dst[tid] = num;
+                if (tid == 0) { dst[D] = most[h]; dst[D + 1] = norm[h]; }
+            }
+        }
+        if (parts > 1) {
+            unsigned int* counter = p.counters + z * p.hk + kvh;
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)parts - 1;
+            __syncthreads();
+            if (s_last) {
+                __threadfence();
+                if (tid < 16 * kLaneAttnGroup) {             // a lane for each part's state of a head
+                    const int h = tid >> 4, s = tid & 15;
+                    const bool on = h < G && s < parts;
+                    const float* src = partial + ((size_t)s * G + h) * stride + D;
+                    const float m = on ? __ldcg(src) : -INFINITY, l = on ? __ldcg(src + 1) : 0.f;
+                    float mm = m;
+#pragma unroll
+                    for (int d = 1; d < 16; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+                    const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+                    float den = wgt * l;
+#pragma unroll
+                    for (int d = 1; d < 16; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+                    weight[h][s] = wgt;
+                    if (s == 0) norm[h] = den;
+                }
+                __syncthreads();
+                for (int h = 0; h < G; ++h) {
+                    float num = 0.f;
+                    for (int s = 0; s < parts; ++s) num += weight[h][s] * __ldcg(partial + ((size_t)s * G + h) * stride + tid);
+                    put(h, num, norm[h]);
+                }
+                if (tid == 0) *counter = 0;
+            }
+        }
+        __syncthreads();                                     // the states and weights are read
+        u += count;
+    }
 }
 
 // ----------------------------------------------------------------------------- routing
@@ -1455,6 +1577,20 @@ extern "C" int qd_batch_attention(const void* qg, const void* k_new, const void*
             if (cudaFuncSetAttribute(batch_attn_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
                 return QD_ERR_LAUNCH;
             mma_configured[dev] = true;
+        }
+        if (batch <= kFlatBatch && splits > 1 && splits <= 16 && (cache_stride || batch == 1)) {
+            int sms = 0;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (sms <= 0) sms = 148;
+            const long long most = (long long)batch * kv_heads * splits;
+            static bool flat_configured[64];
+            if (!flat_configured[dev]) {
+                if (cudaFuncSetAttribute(batch_attn_flat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
+                    return QD_ERR_LAUNCH;
+                flat_configured[dev] = true;
+            }
+            qd_launch(batch_attn_flat_kernel, dim3(most < sms ? (int)most : sms), dim3(kLaneAttnWarps * 32), mma_smem, (cudaStream_t)stream, true, p, batch);
+            return qd_launch_status();
         }
         qd_launch(batch_attn_mma_kernel, dim3(kv_heads, splits, batch), dim3(kLaneAttnWarps * 32), mma_smem, (cudaStream_t)stream, true, p);
         return qd_launch_status();

@@ -219,6 +219,35 @@ def test_batch_attention_forms_against_the_single_sequence_kernel(cuda_device, h
             assert O.rel_l2(kb[i, :n].float().cpu(), ks[i, :n].float().cpu()) < 1e-3 and torch.equal(vb[i, :n], vs[i, :n])
 
 
+@pytest.mark.parametrize("hq,hkv,lengths", [(16, 2, [1, 1024, 0, 33, 32, 1025, 31, 640]), (6, 3, [5]), (8, 1, [1000] * 40), (4, 2, list(range(1, 200))), (16, 2, [900] + [3] * 60)])
+def test_batch_attention_shares_the_context_out(cuda_device, hq, hkv, lengths):
+    """Blocks with parts of several sequences and sequences in several blocks, against the form with a block for each (sequence, KV head)
+    (split count 1).  Lengths outside the cache (0, 1025) leave the output alone.  fp32 sums in another order, two bf16 roundings: 2^-7 of the largest."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    dev, cap, d, batch = cuda_device, 1024, 256, len(lengths)
+    gen = torch.Generator(device=dev).manual_seed(batch)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=dev).to(torch.bfloat16)
+    qg, k_new, v_new, q_norm, k_norm = new(batch, hq * 2 * d), new(batch, hkv * d), new(batch, hkv * d), new(d) * 0.1, new(d) * 0.1
+    k0, v0 = new(batch, cap, hkv, d), new(batch, cap, hkv, d)
+    positions = torch.tensor(lengths, dtype=torch.int32, device=dev) - 1
+    scratch = torch.empty(batch * lib().qd_attn_scratch_floats(hq, hkv, d, 16), device=dev)
+    counters = torch.zeros(batch * hkv, dtype=torch.int32, device=dev)
+    outs = []
+    for splits in (1, 2, 3, 16):
+        kb, vb = k0.clone(), v0.clone()
+        for i, n in enumerate(lengths):
+            kb[i, max(0, n):], vb[i, max(0, n):] = float("nan"), float("nan")
+        out, q_scratch = torch.full((batch, hq * d), 7.0, dtype=torch.bfloat16, device=dev), torch.empty(batch, hq * d, dtype=torch.bfloat16, device=dev)
+        call("qd_batch_attention", ptr(qg), ptr(k_new), ptr(v_new), ptr(q_norm), ptr(k_norm), ptr(kb), ptr(vb), kb.stride(0), ptr(q_scratch), ptr(out),
+             ptr(scratch), ptr(counters), ptr(positions), batch, cap, hq, hkv, d, 64, 1e6, 1e-6, splits, stream_of(qg))
+        assert int(counters.abs().sum()) == 0
+        outs.append(out.float())
+    outside = (positions < 0) | (positions >= cap)
+    for out in outs:
+        assert bool((out[outside] == 7.0).all()) and torch.isfinite(out).all()
+        assert float((out - outs[0]).abs().max()) <= 2.0 ** -7 * float(outs[0][~outside].abs().max())
+
+
 def test_batch_decode_with_the_published_checkpoint_formats(cuda_device):
     """FP8 mixers and an NVFP4 LM head in the batched step (E4M3 x E4M3 product, NVFP4 rows form):
     the first step of two sequences from empty state against the single-sequence step (one step:
