@@ -271,3 +271,20 @@ def test_batch_decode_with_the_published_checkpoint_formats(cuda_device):
         seq = state.sequence(b)
         assert O.rel_l2(seq.rec_state.cpu(), ref.rec_state.cpu()) < 1e-2 and O.rel_l2(seq.conv_state.cpu(), ref.conv_state.cpu()) < 1e-3
     assert single.status() == 0
+
+
+@pytest.mark.parametrize("batch,hk,hv,dv", [(1, 1, 1, 128), (5, 2, 6, 128), (3, 1, 2, 20), (2, 2, 2, 260), (3, 1, 2, 18)])
+def test_batch_recurrence_equals_the_sequences_one_by_one(cuda_device, batch, hk, hv, dv):
+    """One token of every sequence (a block of whole rows of the state; 18 columns: the kernel for runs) against the run kernel on each sequence alone.
+    fp32 sums of 128 terms in another order: 2^-18 of the state, one bf16 rounding of the results."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(batch + dv)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=cuda_device).to(torch.bfloat16)
+    qkv, a, b, a_log, bias = new(batch, 2 * hk * 128 + hv * dv), new(batch, hv), new(batch, hv), new(hv), new(hv)
+    state = torch.randn(batch, hv, 128, dv, generator=gen, device=cuda_device)
+    one, out, alone = state.clone(), torch.full((batch, hv * dv), float("nan"), dtype=torch.bfloat16, device=cuda_device), torch.empty(batch, hv * dv, dtype=torch.bfloat16, device=cuda_device)
+    call("qd_batch_gdn_recurrence", ptr(qkv), ptr(a), ptr(b), ptr(a_log), ptr(bias), ptr(state), state.stride(0), ptr(out), batch, hk, hv, 128, dv, stream_of(qkv))
+    for z in range(batch):
+        call("qd_seq_gdn_recurrence", ptr(qkv[z]), ptr(a[z]), ptr(b[z]), ptr(a_log), ptr(bias), ptr(one[z]), ptr(alone[z]), 1, hk, hv, 128, dv, stream_of(qkv))
+    assert float((state - one).abs().max()) <= 2.0 ** -18 * float(one.abs().max())
+    assert float((out.double() - alone.double()).abs().max()) <= 2.0 ** -8 * float(alone.double().abs().max())
