@@ -9,7 +9,7 @@
 // warp-level tensor-core instruction, with the routes as the columns of the B operand:
 //   a first small kernel writes the input rows as f16 (a row scaled down by a power of two only if it
 //   would leave f16; optionally the SwiGLU of two inputs) into a scratch area;
-//   block = (expert, 64 to 256 weight rows: about 90 KB); its NVFP4 tile (codes and block scales, checkpoint
+//   block = (expert, 64 or 128 weight rows); its NVFP4 tile (codes and block scales, checkpoint
 //   layout) is copied to shared memory with cp.async in two halves of the inputs, rows padded
 //   against bank conflicts; two blocks share an SM, so one computes while the other loads;
 //   the expert's input rows follow eight at a time through two buffers of half a row each (cp.async
@@ -30,43 +30,39 @@ namespace {
 
 constexpr int kRowsThreads = 256;
 // Shape of a block per input width K and routes per pass (8 NT): PARTS warps share a group of
-// sixteen rows (each takes a part of the inputs), the 8 / PARTS groups take ITERS turns:
-// 16 * (8 / PARTS) * ITERS weight rows.  NT = 1 (a decode batch: one or two routes per expert):
-// about 110 KB of shared memory, two blocks per SM.  NT = 4 (a short prompt chunk: some sixteen
+// sixteen rows (each takes a part of the inputs): 16 * (8 / PARTS) weight rows.  NT = 1 (a decode batch: one or two routes per expert):
+// about 110 KB of shared memory, two blocks per SM; at 512 inputs 53 KB and four (256 rows a block in two turns and two blocks: 31.7 us for the down
+// products of 32 tokens over 256 experts, 27.8 now; 32 rows and three blocks at 2048 inputs: 60 -> 63; with the tile of a later block
+// asked into L2 60 -> 58, 27.8 -> 28.4: neither kept).  NT = 4 (a short prompt chunk: some sixteen
 // routes per expert, all multiplied with ONE decoding of the tile): the two buffers of 32 half rows
 // take up to 130 KB, one block per SM.
 template <int K, int NT> struct RowsShape {
     static constexpr int kParts = K >= 2048 ? 2 : 1;
-    static constexpr int kIters = (K <= 512 && NT == 1) ? 2 : 1;
     static constexpr int kGroups = 8 / kParts;
-    static constexpr int kTile = 16 * kGroups * kIters;
-    static constexpr int kBlocksPerSM = (NT == 1 || K <= 512) ? 2 : 1;
+    static constexpr int kTile = 16 * kGroups;
+    static constexpr int kBlocksPerSM = NT == 1 ? (K <= 512 ? 4 : 2) : (K <= 512 ? 2 : 1);
 };
 
-// The f16 input rows of a pass go through two buffers: a pass's rows in halves of the inputs (one half is
-// multiplied while the next is copied), or whole when the row groups take turns (kIters = 2: every turn
-// reads both halves).
-template <int K, int NT> constexpr int rows_units_per_pass() { return RowsShape<K, NT>::kIters == 1 ? 2 : 1; }
-template <int K, int NT> constexpr int rows_x_unit_row() { return 2 * K / rows_units_per_pass<K, NT>() + 16; }   // padded, bytes
+// The f16 input rows of a pass go through two buffers, in halves of the inputs: one half is multiplied while the next is copied.
+constexpr int kUnits = 2;
+template <int K> constexpr int rows_x_unit_row() { return 2 * K / kUnits + 16; }   // padded, bytes
 template <int K, int NT> constexpr size_t rows_smem_bytes() {
-    return (size_t)RowsShape<K, NT>::kTile * (rows_code_row<K>() + rows_scale_row<K>()) + (size_t)2 * 8 * NT * rows_x_unit_row<K, NT>();
+    return (size_t)RowsShape<K, NT>::kTile * (rows_code_row<K>() + rows_scale_row<K>()) + (size_t)2 * 8 * NT * rows_x_unit_row<K>();
 }
 
 template <int K, int NT>
 __global__ void __launch_bounds__(kRowsThreads, RowsShape<K, NT>::kBlocksPerSM) expert_rows_kernel(const RowsParams p) {
     extern __shared__ __align__(16) uint8_t rows_smem[];
     using Shape = RowsShape<K, NT>;
-    constexpr int kParts = Shape::kParts, kIters = Shape::kIters, kGroups = Shape::kGroups, kRowsTile = Shape::kTile;
+    constexpr int kParts = Shape::kParts, kGroups = Shape::kGroups, kRowsTile = Shape::kTile;
     constexpr int kTokens = 8 * NT;                         // routes per pass over the tile
-    constexpr int kUnits = rows_units_per_pass<K, NT>();    // copies of input rows per pass
-    static_assert(kParts == 1 || kIters == 1, "one meeting buffer");
     // chain_enter() in two parts: the wait follows the fetch of the weight tile.  What is read before it
     // (the boundaries) was written before the conversion kernel let this one start; read past L1.
     grid_launch_dependents();
     const int e = blockIdx.y, r0 = blockIdx.x * kRowsTile;
     const int b0 = __ldcg(p.boundaries + e), b1 = __ldcg(p.boundaries + e + 1);
     if (b1 <= b0) return;
-    constexpr int code_row = rows_code_row<K>(), scale_row = rows_scale_row<K>(), x_row = rows_x_unit_row<K, NT>();
+    constexpr int code_row = rows_code_row<K>(), scale_row = rows_scale_row<K>(), x_row = rows_x_unit_row<K>();
     constexpr int kUnitPieces = K / 8 / kUnits;             // 16-byte pieces of an f16 input row per copy
     constexpr int kUnitBytes = kTokens * x_row;
     const int R = p.out_features;
@@ -124,97 +120,87 @@ __global__ void __launch_bounds__(kRowsThreads, RowsShape<K, NT>::kBlocksPerSM) 
         const int n = min(kTokens, b1 - first), nts = (n + 7) >> 3;     // routes of this pass, groups of eight in use
         // ---- sixteen weight rows of this warp against the pass's routes, its part of either half
         constexpr int part_spans = K / 128 / (2 * kParts);
-#pragma unroll 1
-        for (int it = 0; it < kIters; ++it) {
-            const int mine = (it * kGroups + group) * 16;
-            const bool live = mine < rows;                 // a warp without rows computes on rows 0..15 and stores nothing
-            const int slot0 = live ? mine : 0;
-            float acc[NT][4];
+        const int mine = group * 16;
+        const bool live = mine < rows;                 // a warp without rows computes on rows 0..15 and stores nothing
+        const int slot0 = live ? mine : 0;
+        float acc[NT][4];
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) { acc[nt][0] = 0.f; acc[nt][1] = 0.f; acc[nt][2] = 0.f; acc[nt][3] = 0.f; }
+        for (int nt = 0; nt < NT; ++nt) { acc[nt][0] = 0.f; acc[nt][1] = 0.f; acc[nt][2] = 0.f; acc[nt][3] = 0.f; }
 #pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                if (kUnits == 2 || (it == 0 && h == 0)) {  // block-uniform: the next copy of input rows is due
-                    // this copy has landed (behind the first one the second half of the codes may be in flight) ...
-                    if (unit == 0 && !p.dependent) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    __syncthreads();      // ... for everybody, and everybody is done with the copy before (and its pass)
-                    if (unit % kUnits == 0 && tid < kTokens) {     // where a route's result goes, what multiplies it
-                        const int r = first + tid, route = tid < n ? p.order[r] : 0;
-                        route_of[tid] = p.scatter ? route : r;
-                        factor[tid] = (p.routing && tid < n) ? round_bf16(global * p.routing[route]) : global;
-                        undo[tid] = tid < n ? p.up[p.by_token ? route / p.topk : r] : 1.f;
-                    }
-                    if (unit + 1 < units) issue_x(unit + 1);
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                    if (kUnits == 1) __syncthreads();      // the epilogue of the first turn reads the route tables
-                    ++unit;
-                }
-                if (kUnits == 1 && first == b0 && it == 0 && h == 1) {       // the second half of the codes (the next rows may be in flight)
-                    asm volatile("cp.async.wait_group 1;" ::: "memory");
-                    __syncthreads();
-                }
-                const uint8_t* xs0 = xt + (size_t)((unit - 1) & 1) * kUnitBytes + (size_t)g * x_row;
+        for (int h = 0; h < 2; ++h) {
+            // this copy has landed (behind the first one the second half of the codes may be in flight) ...
+            if (unit == 0 && !p.dependent) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();      // ... for everybody, and everybody is done with the copy before (and its pass)
+            if (unit % kUnits == 0 && tid < kTokens) {     // where a route's result goes, what multiplies it
+                const int r = first + tid, route = tid < n ? p.order[r] : 0;
+                route_of[tid] = p.scatter ? route : r;
+                factor[tid] = (p.routing && tid < n) ? round_bf16(global * p.routing[route]) : global;
+                undo[tid] = tid < n ? p.up[p.by_token ? route / p.topk : r] : 1.f;
+            }
+            if (unit + 1 < units) issue_x(unit + 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            ++unit;
+            const uint8_t* xs0 = xt + (size_t)((unit - 1) & 1) * kUnitBytes + (size_t)g * x_row;
 #pragma unroll 2
-                for (int s = 0; s < part_spans; ++s) {
-                    const int span = (h * kParts + part) * part_spans + s;
-                    const uint8_t* c0 = w_codes + (size_t)(slot0 + g) * code_row + span * 64 + t * 16;
-                    const uint8_t* s0 = w_scales + (size_t)(slot0 + g) * scale_row + span * 8 + t * 2;
-                    const uint4 w0 = lds128(c0), w1 = lds128(c0 + 8 * code_row);
-                    const uint32_t p0 = e4m3x2_to_f16x2(*reinterpret_cast<const uint16_t*>(s0));
-                    const uint32_t p1 = e4m3x2_to_f16x2(*reinterpret_cast<const uint16_t*>(s0 + 8 * scale_row));
-                    const uint32_t sa0 = __byte_perm(p0, 0u, 0x1010), sb0 = __byte_perm(p0, 0u, 0x3232);
-                    const uint32_t sa1 = __byte_perm(p1, 0u, 0x1010), sb1 = __byte_perm(p1, 0u, 0x3232);
-                    const uint32_t ra[4] = {w0.x, w0.y, w0.z, w0.w}, rb[4] = {w1.x, w1.y, w1.z, w1.w};
-                    // the lane's activations of this span: route 8 nt + g is its column of group nt
-                    const int piece0 = (kUnits == 2 ? span - h * kParts * part_spans : span) * 16 + t * 4;
+            for (int s = 0; s < part_spans; ++s) {
+                const int span = (h * kParts + part) * part_spans + s;
+                const uint8_t* c0 = w_codes + (size_t)(slot0 + g) * code_row + span * 64 + t * 16;
+                const uint8_t* s0 = w_scales + (size_t)(slot0 + g) * scale_row + span * 8 + t * 2;
+                const uint4 w0 = lds128(c0), w1 = lds128(c0 + 8 * code_row);
+                const uint32_t p0 = e4m3x2_to_f16x2(*reinterpret_cast<const uint16_t*>(s0));
+                const uint32_t p1 = e4m3x2_to_f16x2(*reinterpret_cast<const uint16_t*>(s0 + 8 * scale_row));
+                const uint32_t sa0 = __byte_perm(p0, 0u, 0x1010), sb0 = __byte_perm(p0, 0u, 0x3232);
+                const uint32_t sa1 = __byte_perm(p1, 0u, 0x1010), sb1 = __byte_perm(p1, 0u, 0x3232);
+                const uint32_t ra[4] = {w0.x, w0.y, w0.z, w0.w}, rb[4] = {w1.x, w1.y, w1.z, w1.w};
+                // the lane's activations of this span: route 8 nt + g is its column of group nt
+                const int piece0 = (span - h * kParts * part_spans) * 16 + t * 4;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint32_t h0[4], h1[4];
-                        e2m1x8_to_f16x2(ra[j], h0);
-                        e2m1x8_to_f16x2(rb[j], h1);
-                        const uint32_t s_lo = j < 2 ? sa0 : sb0, s_hi = j < 2 ? sa1 : sb1;
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t h0[4], h1[4];
+                    e2m1x8_to_f16x2(ra[j], h0);
+                    e2m1x8_to_f16x2(rb[j], h1);
+                    const uint32_t s_lo = j < 2 ? sa0 : sb0, s_hi = j < 2 ? sa1 : sb1;
 #pragma unroll
-                        for (int b = 0; b < 4; ++b) { h0[b] = hmul2(h0[b], s_lo); h1[b] = hmul2(h1[b], s_hi); }
-                        const int at = x_piece(piece0 + j) * 16;
+                    for (int b = 0; b < 4; ++b) { h0[b] = hmul2(h0[b], s_lo); h1[b] = hmul2(h1[b], s_hi); }
+                    const int at = x_piece(piece0 + j) * 16;
 #pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) {
-                            if (NT == 1 || nt < nts) {
-                                const uint4 u = lds128(xs0 + (size_t)nt * 8 * x_row + at);
-                                mma_f16(acc[nt], h0[0], h1[0], h0[1], h1[1], u.x, u.y);
-                                mma_f16(acc[nt], h0[2], h1[2], h0[3], h1[3], u.z, u.w);
-                            }
+                    for (int nt = 0; nt < NT; ++nt) {
+                        if (NT == 1 || nt < nts) {
+                            const uint4 u = lds128(xs0 + (size_t)nt * 8 * x_row + at);
+                            mma_f16(acc[nt], h0[0], h1[0], h0[1], h1[1], u.x, u.y);
+                            mma_f16(acc[nt], h0[2], h1[2], h0[3], h1[3], u.z, u.w);
                         }
                     }
                 }
             }
-            // ---- the warps of a row group meet; acc[nt][0..1] = row slot0 + g, routes 8 nt + 2 t and + 1; [2..3] = row + 8
-            if (kParts == 2) {
-                if (part == 1) {
+        }
+        // ---- the warps of a row group meet; acc[nt][0..1] = row slot0 + g, routes 8 nt + 2 t and + 1; [2..3] = row + 8
+        if (kParts == 2) {
+            if (part == 1) {
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) meet[nt][group][lane] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
-                }
-                __syncthreads();
-                if (part == 0) {
+                for (int nt = 0; nt < NT; ++nt) meet[nt][group][lane] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+            }
+            __syncthreads();
+            if (part == 0) {
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) {
-                        const float4 other = meet[nt][group][lane];
-                        acc[nt][0] += other.x; acc[nt][1] += other.y; acc[nt][2] += other.z; acc[nt][3] += other.w;
-                    }
+                for (int nt = 0; nt < NT; ++nt) {
+                    const float4 other = meet[nt][group][lane];
+                    acc[nt][0] += other.x; acc[nt][1] += other.y; acc[nt][2] += other.z; acc[nt][3] += other.w;
                 }
             }
-            if (part == 0 && live) {
+        }
+        if (part == 0 && live) {
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const int j = 8 * nt + 2 * t + (c & 1), row = r0 + slot0 + g + 8 * (c >> 1);
-                        if (j >= n || row >= R) continue;
-                        const float sum = acc[nt][c] * undo[j];
-                        const float result = p.routing ? round_bf16(sum) * factor[j] : sum * factor[j];
-                        y[(size_t)route_of[j] * R + row] = __float2bfloat16_rn(result);
-                    }
-            }
+                for (int c = 0; c < 4; ++c) {
+                    const int j = 8 * nt + 2 * t + (c & 1), row = r0 + slot0 + g + 8 * (c >> 1);
+                    if (j >= n || row >= R) continue;
+                    const float sum = acc[nt][c] * undo[j];
+                    const float result = p.routing ? round_bf16(sum) * factor[j] : sum * factor[j];
+                    y[(size_t)route_of[j] * R + row] = __float2bfloat16_rn(result);
+                }
         }
     }
 }
