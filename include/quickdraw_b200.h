@@ -195,6 +195,8 @@ int qd_seq_attention(const void* qg, const void* k_new, const void* v_new, const
                      const void* k_norm, void* k_cache, void* v_cache, void* q_scratch, void* out,
                      int tokens, int position0, int capacity, int q_heads, int kv_heads, int head_dim,
                      int rotary_dim, float theta, float eps, void* stream);
+/* The largest of every row of bf16 logits [rows, columns], lowest index on ties, a NaN above all numbers: int64 tokens [rows]. */
+int qd_argmax_rows(const void* logits, int rows, int columns, void* tokens, void* stream);
 int qd_seq_route_topk(const void* logits, int tokens, int experts, int topk, int32_t* ids, float* weights,
                       void* stream);
 /* ---- Small-batch decode with per-sequence state: one token of each of `batch` independent

@@ -72,6 +72,7 @@ SIGNATURES = {
     "qd_seq_gdn_chunk_scratch_bytes": [I, I],
     "qd_seq_gdn_recurrence_chunked": [P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "qd_seq_attention": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, F, P],
+    "qd_argmax_rows": [P, I, I, P, P],
     "qd_seq_route_topk": [P, I, I, I, P, P, P],
     "qd_batch_gdn_conv": [P, P, P, L, P, I, I, I, P],
     "qd_batch_gdn_recurrence": [P, P, P, P, P, P, L, P, I, I, I, I, I, P],

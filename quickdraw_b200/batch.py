@@ -149,7 +149,9 @@ class BatchDecode(ChunkPrefill):
             dist.all_gather_into_tensor(shards, logits.contiguous(), group=self.group)
             logits = shards.permute(1, 0, 2).reshape(logits.shape[0], c.vocab_size)
         state.positions += 1
-        return logits.float().argmax(dim=-1), logits
+        picked = torch.empty(state.batch, dtype=torch.long, device=logits.device)
+        call("qd_argmax_rows", ptr(logits), state.batch, logits.shape[1], ptr(picked), stream_of(logits))
+        return picked, logits
 
     def graph_step(self, tokens: torch.Tensor, state: BatchState):
         """``step`` replayed from a CUDA graph: a step is some 1 100 launches, which the host

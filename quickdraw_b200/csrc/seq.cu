@@ -1201,6 +1201,61 @@ batch_attn_flat_kernel(const LaneAttnParams p, int batch) {
     }
 }
 
+// ----------------------------------------------------------------------------- greedy choice of a batch
+// Eight blocks a row, which meet in the first one's shared memory.  A value's key orders like the values (-0 as +0, NaN above all), the index
+// below it turns ties to the lowest.  Latency: 32 rows of 151936, in L2 behind the LM head, 8.3 us; an fp32 copy and a library reduction of it took 29.
+constexpr int kArgmaxBlocks = 8, kArgmaxThreads = 512;
+QD_DEVINL unsigned long long argmax_key(uint32_t bits, int index) {
+    if (bits == 0x8000u) bits = 0u;
+    const uint32_t order = (bits & 0x7fffu) > 0x7f80u ? 0xffffu : (bits & 0x8000u) ? 0x7fffu - (bits & 0x7fffu) : 0x8000u + bits;
+    return ((unsigned long long)order << 32) | (0xffffffffu - (uint32_t)index);
+}
+__global__ void __cluster_dims__(kArgmaxBlocks, 1, 1) __launch_bounds__(kArgmaxThreads)
+argmax_rows_kernel(const bf16* __restrict__ logits, int columns, long long* __restrict__ tokens) {
+    chain_enter();
+    __shared__ unsigned long long best[kArgmaxThreads / 32], blocks[kArgmaxBlocks];
+    const int part = blockIdx.x, tid = threadIdx.x;
+    const unsigned short* row = reinterpret_cast<const unsigned short*>(logits) + (size_t)blockIdx.y * columns;
+    unsigned long long key = 0;
+    const auto take = [&](uint32_t bits, int index) { const unsigned long long k = argmax_key(bits, index); key = k > key ? k : key; };
+    if (columns % 8 == 0 && !((uintptr_t)logits & 15u)) {
+#pragma unroll 4
+        for (int i = 8 * (part * kArgmaxThreads + tid); i < columns; i += 8 * kArgmaxBlocks * kArgmaxThreads) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + i));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { take(w[q] & 0xffffu, i + 2 * q); take(w[q] >> 16, i + 2 * q + 1); }
+        }
+    } else {
+        for (int i = part * kArgmaxThreads + tid; i < columns; i += kArgmaxBlocks * kArgmaxThreads) take(row[i], i);
+    }
+    const auto meet = [&](unsigned long long k) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, k, d);
+            k = other > k ? other : k;
+        }
+        return k;
+    };
+    key = meet(key);
+    if ((tid & 31) == 0) best[tid >> 5] = key;
+    __syncthreads();
+    if (tid < 32) {
+        key = meet(tid < kArgmaxThreads / 32 ? best[tid] : 0);
+        if (tid == 0) {
+            uint32_t at;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(smem_u32(blocks + part)));
+            asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(at), "l"(key) : "memory");
+        }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (part == 0 && tid < 32) {
+        key = meet(tid < kArgmaxBlocks ? blocks[tid] : 0);
+        if (tid == 0) tokens[blockIdx.y] = (long long)(0xffffffffu - (uint32_t)key);
+    }
+}
+
 // ----------------------------------------------------------------------------- routing
 __global__ void seq_route_kernel(const bf16* __restrict__ logits, int experts, int topk, int32_t* __restrict__ ids,
                                  float* __restrict__ weights) {
@@ -1681,6 +1736,12 @@ extern "C" int qd_batch_attention(const void* qg, const void* k_new, const void*
     return qd_launch_status();
 }
 
+extern "C" int qd_argmax_rows(const void* logits, int rows, int columns, void* tokens, void* stream) {
+    QD_CHECK_ARG(logits && tokens && rows > 0 && rows <= 65535 && columns > 0);
+    return qd_launch(argmax_rows_kernel, dim3(kArgmaxBlocks, rows), dim3(kArgmaxThreads), 0, (cudaStream_t)stream, true, (const bf16*)logits, columns,
+                     (long long*)tokens);
+}
+
 extern "C" int qd_seq_route_topk(const void* logits, int tokens, int experts, int topk, int32_t* ids, float* weights,
                                  void* stream) {
     QD_CHECK_ARG(logits && ids && weights && tokens > 0 && topk >= 1 && topk <= 32 && topk <= experts);
@@ -1695,14 +1756,16 @@ extern "C" int qd_seq_group_routes(const int32_t* ids, int routes, int experts, 
     if (experts > 1023) return QD_ERR_UNSUPPORTED;
     // one to eight experts a block: at most 128 blocks, one a multiprocessor
     const int whole = ((uintptr_t)ids & 15u) == 0;
-    const auto launch = [&](auto kernel, int own) {
-        qd_launch(kernel, dim3((experts + own - 1) / own), dim3(kRouteWarps * 32), 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order,
-                  boundaries);
-    };
-    if (experts <= 128) launch(seq_group_routes_kernel<1>, 1);
-    else if (experts <= 256) launch(seq_group_routes_kernel<2>, 2);
-    else if (experts <= 512) launch(seq_group_routes_kernel<4>, 4);
-    else launch(seq_group_routes_kernel<8>, 8);
+    const auto blocks = [&](int own) { return dim3((experts + own - 1) / own); };
+    const dim3 threads(kRouteWarps * 32);
+    if (experts <= 128)
+        qd_launch(seq_group_routes_kernel<1>, blocks(1), threads, 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order, boundaries);
+    else if (experts <= 256)
+        qd_launch(seq_group_routes_kernel<2>, blocks(2), threads, 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order, boundaries);
+    else if (experts <= 512)
+        qd_launch(seq_group_routes_kernel<4>, blocks(4), threads, 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order, boundaries);
+    else
+        qd_launch(seq_group_routes_kernel<8>, blocks(8), threads, 0, (cudaStream_t)stream, true, ids, routes, experts, whole, order, boundaries);
     return qd_launch_status();
 }
 

@@ -2,6 +2,8 @@
 reference has no batched decode; its single-sequence step, applied to every sequence on its
 own, is the oracle)."""
 
+import math
+
 import pytest
 import torch
 
@@ -288,3 +290,19 @@ def test_batch_recurrence_equals_the_sequences_one_by_one(cuda_device, batch, hk
         call("qd_seq_gdn_recurrence", ptr(qkv[z]), ptr(a[z]), ptr(b[z]), ptr(a_log), ptr(bias), ptr(one[z]), ptr(alone[z]), 1, hk, hv, 128, dv, stream_of(qkv))
     assert float((state - one).abs().max()) <= 2.0 ** -18 * float(one.abs().max())
     assert float((out.double() - alone.double()).abs().max()) <= 2.0 ** -8 * float(alone.double().abs().max())
+
+
+@pytest.mark.parametrize("rows,columns,kind", [(32, 151936, "plain"), (3, 1000, "ties"), (1, 7, "plain"), (5, 4099, "negative"), (4, 33000, "nan"), (2, 16, "zeros"), (2, 264, "lowest")])
+def test_argmax_of_rows(cuda_device, rows, columns, kind):
+    """The greedy choice as torch makes it of the same values in fp32: the first of equal ones, -0 equal to 0, NaN above infinity."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator(device=cuda_device).manual_seed(columns)
+    x = torch.randn(rows, columns, generator=gen, device=cuda_device)
+    x = {"ties": x.round(), "negative": -x.abs() - 1, "zeros": torch.zeros_like(x) * (x - 1).sign(), "lowest": torch.full_like(x, -math.inf)}.get(kind, x).to(torch.bfloat16)
+    if kind == "nan":
+        x[1, 5], x[1, 20000], x[1, 31000], x[2, 32999] = math.inf, math.nan, math.nan, math.inf
+    picked = torch.full((rows,), -1, dtype=torch.long, device=cuda_device)
+    call("qd_argmax_rows", ptr(x), rows, columns, ptr(picked), stream_of(x))
+    values = x.float().nan_to_num(nan=math.inf, posinf=3e38).cpu()
+    first = torch.where(values == values.amax(1, keepdim=True), torch.arange(columns), columns).amin(1)
+    assert picked.tolist() == first.tolist()
