@@ -424,9 +424,7 @@ def batch_attention_leg(cfg, device, batch, context, peak, reps=12):
     vn = torch.randn(batch, hkv, d, generator=gen, device=device).to(BF16)
     norm = torch.zeros(d, dtype=BF16, device=device)
     out, q_scratch = (torch.empty(batch, hq * d, dtype=BF16, device=device) for _ in range(2))
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    pairs = batch * hkv
-    splits = min(range(1, 17), key=lambda s: -(-pairs * s // sms) * (-(-context // s) + 64))
+    splits = 16                 # as BatchDecode: at most sixteen parts of a (sequence, KV head)
     scratch = torch.empty(batch * lib().qd_attn_scratch_floats(hq, hkv, d, 16), dtype=torch.float32, device=device)
     counters = torch.zeros(batch * hkv, dtype=torch.int32, device=device)
     positions = torch.full((batch,), context, dtype=torch.int32, device=device)
@@ -446,7 +444,7 @@ def batch_attention_leg(cfg, device, batch, context, peak, reps=12):
     torch.cuda.synchronize(device)
     us = e0.elapsed_time(e1) * 1e3 / reps
     nbytes = batch * 2 * (context + 1) * hkv * d * 2
-    return {"kernel": "seq_attn_prepare_kernel + batch_attn_mma_kernel (mma.sync, rows straight from the cache)", "batch": batch,
+    return {"kernel": "seq_attn_prepare_kernel + batch_attn_flat_kernel (mma.sync, rows straight from the cache)", "batch": batch,
             "context": context, "splits": splits, "launch_us": us, "bytes_per_launch": nbytes, "achieved": nbytes / us / 1e3,
             "peak": peak, "unit": "GB/s", "frac": nbytes / us / 1e3 / peak}
 

@@ -87,7 +87,7 @@ class Cases:
         like = lambda: call("qd_nvfp4_matmul", ptr(x), ptr(proj.weight), ptr(proj.weight_scale), ptr(proj.weight_scale_2), ptr(out), tokens,
                             rows, width, 16, ptr(self.status), stream_of(x))
         own = lambda: linear(x, 0, width, w, out, tokens=tokens, status=self.status)
-        self.pair(f"linear_umma_kernel {tokens} x [{rows}, {width}]", ([own] * 8, 0, flops), "nvfp4_gemm_kernel (W4A16)", ([like] * 8, 0, flops))
+        self.pair(f"qd_linear {tokens} x [{rows}, {width}]", ([own] * 8, 0, flops), "nvfp4_gemm_kernel (W4A16)", ([like] * 8, 0, flops))
 
     def matvec(self, rows, width):
         own_bytes, like_bytes = rows * width * 2, rows * width * (0.5 + 1 / 16)
@@ -270,7 +270,7 @@ class LatentCases(Cases):
         glu = lambda: linear(x, 0, width, w, half, tokens=tokens, status=self.status, glu=True)
         biased = lambda: linear(x, 0, width, w, out, tokens=tokens, status=self.status, bias=bias)
         for name, own in (("gated unit", glu), ("bias", biased)):
-            self.pair(f"linear_umma_kernel, {name}, {tokens} x [{rows}, {width}]", ([own] * 8, 0, flops), "linear_umma_kernel", ([plain] * 8, 0, flops))
+            self.pair(f"qd_linear, {name}, {tokens} x [{rows}, {width}]", ([own] * 8, 0, flops), "qd_linear", ([plain] * 8, 0, flops))
 
     def matvec_forms(self, rows, width):
         nbytes = rows * width * 2
