@@ -385,6 +385,27 @@ def test_a_wait_that_ran_out_leaves_nothing_in_flight():
     assert re.search(r"\n        if \(issued >= 0\) mbar_wait\(full, \(issued >> 1\) & 1, nullptr\);", loaders)
 
 
+def test_another_block_is_known_to_run_before_its_memory_is_used():
+    """Source check of the kernels that reach into another block's shared memory: a barrier of the whole cluster is waited for in front of
+    the first such access (until then the other block may not have started)."""
+    remote, waits = r"\bmapa\b|\bof_first_block\(|\bmap_shared_rank\(", r"\bcluster_sync\(\);|barrier\.cluster\.wait|\bbarrier_wait\(\);|\bcluster\.sync\(\);"
+    found = set()
+    for path in (ROOT / "quickdraw_b200" / "csrc").glob("*.cu*"):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for match in re.finditer(r"__global__[^{;]*?\b(\w+)\s*\((?:[^{;()]|\([^()]*\))*\)\s*\{", text, flags=re.S):
+            depth, at = 1, match.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[at], 0)
+                at += 1
+            body = text[match.end():at]
+            access = re.search(remote, body)
+            if access:
+                found.add(match.group(1))
+                wait = re.search(waits, body)
+                assert wait and wait.start() < access.start(), (path.name, match.group(1))
+    assert found >= {"argmax_rows_kernel", "linear_pair_kernel", "w4a4_pair_kernel", "recurrence_step_kernel"}, found
+
+
 def test_banks_off_a_16_byte_boundary_keep_the_form_that_takes_them():
     """The launch of gate, up and SwiGLU refuses such addresses, the grouped product does not: a chunk goes the second way then."""
     from types import SimpleNamespace
