@@ -191,7 +191,8 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
 // sums wait only for a pass of eight warps from tensor memory into registers (tensor memory holds no second set beside the scales).
 //   warp 0      TMA: codes count at the first block, scales in their own
 //   warp 1      of the first block: 4 MMAs of 256 x 256 x 64 per stage
-//   warps 2-13  scales to tensor memory, as above, every third stage each four; the weight rows' in eight columns per 64-input step
+//   warps 2-13  scales to tensor memory, as above, four warps a group, a stage of the ring always the same group's (below); the weight rows' in
+//               eight columns per 64-input step
 //   the last 8  sums, 32 tokens x 128 outputs each, as bf16 through shared memory in whole 128-byte lines
 // What bounded both forms was the way of the scales, some 1000 clocks a stage for its four warps from the wait to the hand-over: 8192 x 8192 x
 // 2048 127 us before, here 141 with one group of four warps, 111 with two, 102 with three, then the operands from L2 (1100 clocks a
@@ -204,6 +205,15 @@ struct Pair4 {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + sizeof(Bars) + 64 + 1024;
     static_assert(kColSf + kStages * kSfCols <= 512 && kStageBytes % 1024 == 0 && kSmem <= 227 * 1024, "");
 };
+// The step of the loads (one stage each) that a group of scale warps takes after step `it`; group g begins with step g.  A stage has the same
+// group in every round of the ring.  Copies end in any order, so a group that met a stage only every third round could ask for a round while the
+// copy of the one before, which another group waits for, is still on its way: the parity of a phase that is over would let it pass.  Two
+// of the groups have two of the five stages, 2.5 steps of time for each.
+constexpr int next_scale_step(int it) {
+    constexpr int S = Pair4::kStages, G = Pair4::kScaleGroups;
+    return it % S + G < S ? it + G : it / S * S + S + it % S % G;
+}
+
 QD_DEVINL void pair_umma_nvfp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %7, 0;\n\t"
                  "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
@@ -307,7 +317,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
         const uint32_t quarter = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T::kColSf;
         const int group = (warp - 2) >> 2, steps = pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0;
         bool ok = true;
-        for (int it = group; it < steps; it += T::kScaleGroups) {
+        for (int it = group; it < steps; it = next_scale_step(it)) {
             const int st = it % kStages;
             ok = __all_sync(0xffffffffu, mbar_wait(bars->scales + st, (it / kStages) & 1, p.status));
             if (!ok) break;

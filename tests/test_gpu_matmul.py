@@ -185,8 +185,6 @@ def test_w4a4_matmul_matches_oracle(cuda_device, tokens, out_features, in_featur
     src = synthetic.Source(32, "cpu")
     proj = src.nvfp4(f"w{out_features}x{in_features}", out_features, in_features, global_scale=0.75)
     x = src.normal(f"x{tokens}", tokens, in_features)
-    if wide and out_features % 256:
-        pytest.skip("256-row tiles need out_features % 256 == 0")
     xq = kernels.quantize_act(x.to(cuda_device))
     got = kernels.matmul_w4a4(xq, to_device(proj, cuda_device), wide_tiles=wide).cpu()
     assert kernels.matmul_status(cuda_device) == 0
@@ -198,10 +196,12 @@ def test_w4a4_matmul_matches_oracle(cuda_device, tokens, out_features, in_featur
     assert O.rel_l2(got, exact) < 0.2
 
 
-@pytest.mark.parametrize("tokens,out_features,in_features", [(1, 128, 256), (129, 384, 512), (257, 256, 1536), (600, 640, 768), (2500, 2176, 256)])
+@pytest.mark.parametrize("tokens,out_features,in_features", [(1, 128, 256), (129, 384, 512), (257, 256, 1536), (600, 640, 768), (2500, 2176, 256),
+                                                             (4100, 4224, 768), (4100, 4224, 1792)])
 def test_w4a4_matmul_on_pairs(cuda_device, tokens, out_features, in_features):
     """Tiles that end inside a block's half of the tokens and inside the weight rows, fewer and more stages than there are, one tile to a
-    pair of SMs and several (90 tiles): the same sums as in the small form, in the same order of the inputs."""
+    pair of SMs and several (90 and 289 tiles: up to four a pair, of three and seven stages on a ring of five, so that tiles begin anywhere in it):
+    the same sums as in the small form, in the same order of the inputs."""
     from quickdraw_b200 import kernels
     src = synthetic.Source(35, cuda_device)
     proj = src.nvfp4("w", out_features, in_features, global_scale=0.75)

@@ -406,6 +406,28 @@ def test_another_block_is_known_to_run_before_its_memory_is_used():
     assert found >= {"argmax_rows_kernel", "linear_pair_kernel", "w4a4_pair_kernel", "recurrence_step_kernel"}, found
 
 
+def test_a_stage_of_scales_belongs_to_one_group_of_warps():
+    """Source check of the FP4 product on pairs of SMs: the groups that move block scales take every step once, and whoever waits for a
+    stage of the ring has waited for each of its rounds before (the parity of a barrier tells neighbouring rounds apart, no more)."""
+    text = (ROOT / "quickdraw_b200" / "csrc" / "gemm4.cu").read_text()
+    stages, groups = (int(re.search(r"struct Pair4 \{.*?\b" + name + r" = (\d+)", text, flags=re.S).group(1)) for name in ("kStages", "kScaleGroups"))
+    step = re.search(r"for \(int it = group; it < steps; it (\+?=) ([^)]*\)?)\) \{", text)
+    if step.group(1) == "+=":
+        after = lambda it: it + groups
+    else:
+        assert step.group(2) == "next_scale_step(it)"
+        test, yes, no = re.search(r"int next_scale_step\(int it\) \{.*?return (.*?) \? (.*?) : (.*?);", text, flags=re.S).groups()
+        after = eval(f"lambda it: ({yes}) if ({test}) else ({no})".replace("/", "//"), {"S": stages, "G": groups})
+    owners, taken = {}, []
+    for group in range(groups):
+        it = group
+        while it < 20 * stages * groups:
+            owners.setdefault(it % stages, set()).add(group)
+            taken.append(it)
+            it = after(it)
+    assert sorted(taken) == list(range(20 * stages * groups)) and all(len(who) == 1 for who in owners.values()), owners
+
+
 def test_banks_off_a_16_byte_boundary_keep_the_form_that_takes_them():
     """The launch of gate, up and SwiGLU refuses such addresses, the grouped product does not: a chunk goes the second way then."""
     from types import SimpleNamespace
