@@ -77,6 +77,7 @@ class BatchDecode(ChunkPrefill):
     def _attn_scratch(self, batch):
         c = self.ckpt.config
         if self._scratch is None or self._scratch[0] < batch:
+            self._retire(self._scratch)          # a graph captured for a smaller state goes on using it
             floats = lib().qd_attn_scratch_floats(c.num_attention_heads, c.num_key_value_heads, c.head_dim,
                                                   MAX_ATTN_SPLITS)
             self._scratch = (batch, torch.empty(batch * floats, dtype=torch.float32, device=self.device),

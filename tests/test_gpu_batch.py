@@ -179,6 +179,33 @@ def test_graph_replay_equals_eager_steps(cuda_device):
         assert torch.equal(getattr(eager, name), getattr(replayed, name)), name
 
 
+def test_replay_of_a_small_state_after_a_larger_batch(cuda_device):
+    """A state of two sequences is captured, another of 24 takes a step (which needs larger scratch), tensors are made where freed
+    scratch could lie, then the first one's graph is replayed: as the eager steps of the same two sequences, bit for bit.  Contexts of 600
+    positions, so that several blocks share a sequence and the counters decide who merges."""
+    from quickdraw_b200.batch import BatchDecode, BatchState
+    cfg = synthetic.model_config(num_layers=4, vocab_size=4096, experts=16, topk=8)
+    decoder = BatchDecode(synthetic.make_checkpoint(cfg, seed=6, device="cuda"))
+    eager, replayed, large = BatchState(cfg, 2, 640, "cuda"), BatchState(cfg, 2, 640, "cuda"), BatchState(cfg, 24, 640, "cuda")
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    for name in ("kv_k", "kv_v", "rec_state", "conv_state"):
+        getattr(eager, name).normal_(generator=gen).mul_(0.1)
+        getattr(replayed, name).copy_(getattr(eager, name))
+    for state in (eager, replayed):
+        state.positions.copy_(torch.tensor([600, 517], dtype=torch.int32))
+    fed_a = fed_b = torch.tensor([5, 77], device="cuda")
+    kept = []
+    for step in range(6):
+        if step == 3:
+            assert decoder._graphs[id(replayed)]["graph"] is not None
+            decoder.step(torch.arange(24, device="cuda"), large)
+            kept = [torch.full((n,), 3, dtype=torch.int32, device="cuda") for n in [1 << 8] * 64 + [1 << 18] * 4]
+        fed_b, logits_b = (t.clone() for t in decoder.graph_step(fed_b, replayed))
+        fed_a, logits_a = BatchDecode.step(decoder, fed_a, eager)
+        assert torch.equal(fed_a, fed_b) and torch.equal(logits_a, logits_b), step
+    assert all(bool((t == 3).all()) for t in kept) and decoder.check() == 0
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(16, 2, 256), (8, 2, 128)])
 def test_batch_attention_forms_against_the_single_sequence_kernel(cuda_device, hq, hkv, d):
     """``qd_batch_attention`` (head dimension 256: tensor-core form with a full group of eight

@@ -479,6 +479,27 @@ def test_launch_modes_of_the_entry_points():
             assert re.search(r"pdl != 0|launch_mode\(pdl\)", entry.group(1)) and not re.search(r"[ (]pdl[,)] *(?!!)", entry.group(1).replace("launch_mode(pdl)", "")), name
 
 
+def test_scratch_of_a_captured_step_outlives_a_larger_batch(monkeypatch):
+    """A graph captured for a state holds the addresses of the attention's scratch and counters; a larger state's step replaces both, and
+    the old ones must not go back to the allocator."""
+    import weakref
+    from types import SimpleNamespace
+
+    from quickdraw_b200 import batch
+    monkeypatch.setattr(batch, "lib", lambda: SimpleNamespace(qd_attn_scratch_floats=lambda *sizes: 8))
+    decoder = batch.BatchDecode.__new__(batch.BatchDecode)
+    decoder.ckpt = SimpleNamespace(config=SimpleNamespace(num_attention_heads=4, num_key_value_heads=2, head_dim=256))
+    decoder.device, decoder._scratch, decoder._retired = "cpu", None, []
+    small = decoder._attn_scratch(2)
+    assert decoder._attn_scratch(1) == small and not decoder._retired
+    alive = [weakref.ref(t) for t in small]
+    addresses = [t.data_ptr() for t in small]
+    del small
+    large = decoder._attn_scratch(32)
+    assert [r() is not None and r().data_ptr() for r in alive] == addresses
+    assert [t.numel() for t in large] == [256, 64]
+
+
 def test_splits_of_the_decode_attention_follow_the_form_that_is_taken():
     from quickdraw_b200.kernels import _attn_splits
     assert [_attn_splits(256, r, 4096) for r in (0, 64, 256, 32, 96)] == [74, 74, 74, 32, 32]
