@@ -201,7 +201,7 @@ struct Pair4 {
     static constexpr int kStages = 5, kStageBytes = 2 * kCodeBytes + 3 * kScaleBytes, kEpilogueWarps = 8, kStagingBytes = 32 * 128;
     static constexpr int kScaleGroups = 3, kFirst = 2 + 4 * kScaleGroups, kThreads = 32 * (kFirst + kEpilogueWarps);
     static constexpr uint32_t kColSf = 256, kSfCols = 48;
-    struct Bars { uint64_t full[kStages], scales[kStages], sf_ready[kStages], empty[kStages], ready, taken; };
+    struct Bars { uint64_t full[kStages], scales[kStages], sf_ready[kStages], empty[kStages], ready, taken, drained; };
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + sizeof(Bars) + 64 + 1024;
     static_assert(kColSf + kStages * kSfCols <= 512 && kStageBytes % 1024 == 0 && kSmem <= 227 * 1024, "");
 };
@@ -235,6 +235,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, chunks = p.in_features / 256;
     const int across = (p.tokens + 255) / 256, tiles = across * ((p.out_features + 255) / 256);
+    const int steps = pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0;         // stages that the pair takes
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -242,6 +243,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
         }
         mbar_init(&bars->ready, 1);
         mbar_init(&bars->taken, 2 * T::kEpilogueWarps);
+        mbar_init(&bars->drained, 1);
         mbar_fence_init();
     }
     if (warp == 1) pair_tmem_alloc(tmem_slot, 512);
@@ -250,7 +252,8 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // A wait that runs out ends a role; everybody meets at the end, by when all copies and MMAs have long ended (the limit is 0.2 s).
+    // A wait that runs out ends a role; the loads end when the MMAs have taken the last of them or 0.2 s after it (the limit of a wait), the
+    // blocks when a commit of all MMAs has arrived, and both together.
     if (warp == 0) {
         const bool leader = elect_one();
         int st = 0, n = 1;
@@ -280,6 +283,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
                 if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
+        if (n) pair_loads_taken(bars->empty, kStages, steps, p.status);
     } else if (warp == 1) {
         if (rank == 0) {
             const bool leader = elect_one();
@@ -312,10 +316,11 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
                 if (leader) pair_commit(&bars->ready);
                 __syncwarp();
             }
+            if (leader) pair_commit(&bars->drained);
         }
     } else if (warp < T::kFirst) {
         const uint32_t quarter = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T::kColSf;
-        const int group = (warp - 2) >> 2, steps = pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0;
+        const int group = (warp - 2) >> 2;
         bool ok = true;
         for (int it = group; it < steps; it = next_scale_step(it)) {
             const int st = it % kStages;
@@ -382,6 +387,8 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
             }
         }
     }
+    __syncthreads();
+    if (warp == 1) mbar_wait(&bars->drained, 0, p.status);     // tensor memory is given back only behind the last MMA, also where a wait ran out
     __syncwarp();
     tc_fence_before();
     cluster_sync();

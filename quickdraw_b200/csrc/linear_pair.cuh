@@ -19,7 +19,7 @@ struct PairTile {
     static constexpr int kHalfBytes = 128 * 128, kStageBytes = 2 * kHalfBytes, kStages = 6;      // a block's rows, 64 inputs
     static constexpr int kLineBytes = 128, kStagingBytes = 32 * kLineBytes;       // of an epilogue warp
     static constexpr int kEpilogueWarps = 8, kThreads = 64 + 32 * kEpilogueWarps;
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + (2 * kStages + 4) * 8 + 16 + 1024;
+    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kEpilogueWarps * kStagingBytes + (2 * kStages + 5) * 8 + 16 + 1024;
 };
 
 QD_DEVINL void pair_umma_f16(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
@@ -117,7 +117,8 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     uint64_t* empty = full + kStages;
     uint64_t* ready = empty + kStages;         // an accumulator holds a tile
     uint64_t* taken = ready + 2;               // (the first block's:) both blocks have read it
-    uint32_t* slot = reinterpret_cast<uint32_t*>(taken + 2);
+    uint64_t* drained = taken + 2;             // every MMA has ended
+    uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int across = (p.tokens + 255) / 256, tiles = across * ((p.rows + TN - 1) / TN), steps = (p.width + kStepK - 1) / kStepK;
@@ -125,6 +126,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(ready + s, 1); mbar_init(taken + s, 2 * Tile::kEpilogueWarps); }
+        mbar_init(drained, 1);
         mbar_fence_init();
     }
     if (warp == 1) pair_tmem_alloc(slot, 2 * TN);
@@ -133,7 +135,8 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *slot;
 
-    // A wait that runs out ends a role; everybody meets at the end, by when all copies and MMAs have long ended (the limit is 0.2 s).
+    // A wait that runs out ends a role; the loads end when the MMAs have taken the last of them or 0.2 s after it (the limit of a wait), the
+    // blocks when a commit of all MMAs has arrived, and both together.
     if (warp == 0) {
         const bool leader = elect_one();
         int st = 0, n = 1;
@@ -158,6 +161,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
                 if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
+        if (n) pair_loads_taken(empty, kStages, pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * steps : 0, p.status);
     } else if (warp == 1) {
         if (rank == 0) {
             const bool leader = elect_one();
@@ -188,6 +192,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
                 if (leader) pair_commit(ready + buf);
                 __syncwarp();
             }
+            if (leader) pair_commit(drained);
         }
     } else {
         const int quadrant = warp & 3, half = (warp - 2) >> 2;        // lanes of tensor memory that the warp may read; columns that it takes
@@ -230,6 +235,8 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
             if (lane == 0) arrive_at(of_first_block(taken + buf));
         }
     }
+    __syncthreads();
+    if (warp == 1) mbar_wait(drained, 0, p.status);           // tensor memory is given back only behind the last MMA, also where a wait ran out
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync();

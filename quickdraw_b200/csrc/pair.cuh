@@ -26,6 +26,12 @@ QD_DEVINL void pair_commit(uint64_t* bar) {                           // arrives
 QD_DEVINL void arrive_at(uint32_t bar) {                              // `bar` as of of_first_block
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The end of a loading warp: the last `issued` copies (of a ring of barriers on which the MMAs release stages) have been used.  A wait
+// that runs out ends it as well: by then 0.2 s have passed since the last copy was asked for.
+QD_DEVINL void pair_loads_taken(uint64_t* empty, int ring, int issued, unsigned int* status) {
+    for (int i = issued > ring ? issued - ring : 0; i < issued; ++i)
+        if (!__all_sync(0xffffffffu, mbar_wait(empty + i % ring, (i / ring) & 1, status))) return;
+}
 QD_DEVINL void pair_tmem_alloc(uint32_t* slot, uint32_t cols) {       // a warp of each block
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");

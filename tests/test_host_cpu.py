@@ -381,6 +381,13 @@ def test_a_wait_that_ran_out_leaves_nothing_in_flight():
         body = text[re.search(r"\b" + kernel + r"\(const", text).start():]
         body = body[:min(body.index(word) for word in ("tmem_dealloc", "tcgen05.dealloc") if word in body)]
         assert re.search(r"commit\w*\(&?(?:bars->)?drained\);[^\n]*\n\s*mbar_wait\(&?(?:bars->)?drained, 0", body), name
+    for name, kernel in (("gemm4.cu", "w4a4_pair_kernel"), ("linear_pair.cuh", "linear_pair_kernel")):      # pairs of blocks: the first one issues
+        text = (csrc / name).read_text()
+        body = text[re.search(r"\b" + kernel + r"\(const", text).start():]
+        body = body[:body.index("pair_tmem_dealloc")]
+        assert re.search(r"\n            if \(leader\) pair_commit\(&?(?:bars->)?drained\);\n        \}", body), name
+        assert re.search(r"__syncthreads\(\);\n    if \(warp == 1\) mbar_wait\(&?(?:bars->)?drained, 0, p\.status\);[^;]*\n    __syncwarp\(\);[^}]*\bcluster_sync\(\);", body), name
+        assert "\n        if (n) pair_loads_taken(" in body, name
     loaders = (csrc / "flash_umma.cuh").read_text()
     assert re.search(r"\n        if \(issued >= 0\) mbar_wait\(full, \(issued >> 1\) & 1, nullptr\);", loaders)
 
