@@ -14,6 +14,7 @@
 namespace qd {
 namespace {
 
+constexpr float kNoPieces = 3.3961775292304e38f;                    // 2^128 (1 - 2^-9): from here on the first piece rounds up to infinity
 constexpr int kPieceRows = 64, kPieceKeys = 32, kPieceThreads = 256;
 template <int QD, int DV> struct PieceShape {
     static constexpr int kQRow = QD + 8, kVRow = DV + 8;               // bf16 to a row: an odd number of 16-byte pieces
@@ -36,6 +37,23 @@ QD_DEVINL void put_planes(bf16* to, int plane, const float4& x) {
     split_three(x.z, x.w, v[0].y, v[1].y, v[2].y);
 #pragma unroll
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * plane) = v[i];
+}
+
+// The score of a query and a key whose pieces give no number (one of them has an infinity or a magnitude that rounds up to one, or the sum passes
+// the largest number), without them and in the order of attn_tiles_kernel: an infinity that a key of weight zero may have, or NaN.
+template <int QD> QD_DEVINL float plain_score(const float* q, const float* k, const float* common, int dim) {
+    float sum = 0.f;
+#pragma unroll 1
+    for (int d0 = 0; d0 < QD; d0 += 32) {
+        float part = 0.f;
+#pragma unroll 1
+        for (int d = d0; d < d0 + 32; d += 4) {
+            const float4 a = load4(q + d), b = d < dim ? load4(k + d) : load4(common + (d - dim));
+            part = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, part))));
+        }
+        sum += part;
+    }
+    return sum;
 }
 
 template <int QD, int DV>
@@ -100,10 +118,10 @@ __global__ void __launch_bounds__(kPieceThreads, 1) attn_pieces_kernel(const __g
         for (int i = tid; i < kPieceKeys * DV / 4; i += 128) {
             const int r = i / (DV / 4), c = i % (DV / 4) * 4;
             const float4 x = j0 + r <= pos_last ? load4(vc + slot_of(j0 + r) * p.ld_v + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            odd |= !(fabsf(x.x) < INFINITY && fabsf(x.y) < INFINITY && fabsf(x.z) < INFINITY && fabsf(x.w) < INFINITY);
+            odd |= !(fabsf(x.x) < kNoPieces && fabsf(x.y) < kNoPieces && fabsf(x.z) < kNoPieces && fabsf(x.w) < kNoPieces);
             put_planes(vs + r * S::kVRow + c, S::kVPlane, x);
         }
-        odd = group_any(3 + group, odd);               // values that a product with a masked key's zero must not reach
+        odd = group_any(3 + group, odd);               // values without pieces, or that a product with a masked key's zero must not reach
         // ---- scores
         float s[4][4];
         {
@@ -132,6 +150,26 @@ __global__ void __launch_bounds__(kPieceThreads, 1) attn_pieces_kernel(const __g
             for (int n = 0; n < 4; ++n)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) s[n][c] = (large[0][n][c] + large[1][n][c]) + small[n][c];
+        }
+        bool unbounded = false;
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) unbounded |= !(fabsf(s[n][c]) < INFINITY);
+        if (__any_sync(0xffffffffu, unbounded)) {
+#pragma unroll 1
+            for (int e = 0; e < 16; ++e) {
+                const int i = (e >> 1) & 1, key = j0 + 8 * (e >> 2) + 2 * t4 + (e & 1), row = min(r0 + warp * 16 + g4 + 8 * i, total - 1);
+                if (key > (i ? pos[1] : pos[0]) || key < (i ? low[1] : low[0])) continue;
+                const int slot = slot_of(key);
+                const float x = plain_score<QD>(q + ((size_t)(row / share) * p.heads + g * share + row % share) * QD, kc + slot * p.ld_k,
+                                                common + slot * p.ld_shared, p.dim);
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (e == 4 * n + c && !(fabsf(s[n][c]) < INFINITY)) s[n][c] = x;
+            }
         }
         // ---- softmax
 #pragma unroll

@@ -242,3 +242,50 @@ def test_bounded_attention_of_an_fp32_chunk(cuda_device, tokens, position, heads
         kept[:, :heads // kv_heads, 7] = ~visible[:, position + 201, None]
         assert not torch.isfinite(out[~kept]).any()
     assert float((out.double() - want)[kept].norm() / want[kept].norm()) < 2e-6
+
+
+@pytest.mark.parametrize("heads,kv_heads,shared", [(16, 4, 0), (16, 16, 64)])
+def test_bounded_attention_of_an_fp32_chunk_at_the_end_of_the_range(cuda_device, heads, kv_heads, shared):
+    """Keys and queries with infinities and with the largest number, products that pass it, values of the largest number: what plain fp32 sums
+    give.  A key whose score is minus infinity has weight zero and touches nothing, one of plus infinity or NaN spoils the rows that see it, a
+    masked one none.  fp32 sums as in the test above: 2e-6; a row that weighs one huge value: as an fp32 product."""
+    from ctypes import byref
+
+    from quickdraw_b200._lib import AttentionArgs, call_hybrid, ptr, stream_of
+    tokens, span, largest = 320, 150, torch.finfo(torch.float32).max
+    gen = torch.Generator(device=cuda_device).manual_seed(heads)
+    new = lambda *shape, std=1.0: torch.randn(shape, generator=gen, device=cuda_device) * std
+    keys, values, common, q = new(tokens, kv_heads, 128, std=2.0), new(tokens, kv_heads, 128), new(tokens, shared), new(tokens, heads, 128 + shared)
+    q[..., 0] = q[..., 0].abs() + 0.1
+    q[..., 1] = 0.0
+    keys[..., 0], keys[..., 1] = keys[..., 0] * 0.01, 0.0
+    keys[20, 0, 0] = -math.inf                     # weight zero for all that see it
+    keys[40, 0, 0] = -largest                      # a product of it and 4 passes the largest number: weight zero too
+    q[40:190, :heads // kv_heads, 0] += 4.0
+    keys[60, 1, 0] = math.inf                      # plus infinity: rows 60 .. 209 of key/value head 1
+    q[250, 2 * heads // kv_heads, 1] = math.inf    # a query: infinity times zero is NaN
+    keys[301, 3, 1] = -largest                     # times zero: nothing
+    values[5, 0, 9], values[310, 2, 3] = -largest, largest
+    args = dict(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, shared_dim=shared, scale=(128 + shared) ** -0.5, ld_k=kv_heads * 128, ld_v=kv_heads * 128,
+                ld_shared=shared, k_cache=ptr(keys), v_cache=ptr(values), k_shared=ptr(common) if shared else None, gate=None, ld_gate=8, gate_kind=0,
+                sink_kind=0, mask=0, span=span, capacity=tokens, position=0, tokens=tokens, dtype=1)
+    out = torch.full((tokens, heads, 128), float("nan"), device=cuda_device)
+    call_hybrid("qd_attention", byref(AttentionArgs(q_rows=ptr(q), out=ptr(out), **args)), stream_of(q))
+    at, j = torch.arange(tokens, device=cuda_device)[:, None], torch.arange(tokens, device=cuda_device)[None]
+    share = heads // kv_heads
+    k = torch.cat([keys, common[:, None].expand(-1, kv_heads, -1)], -1).repeat_interleave(share, 1).double()
+    v = values.repeat_interleave(share, 1).double()
+    terms = torch.einsum("thd,jhd->htj", q.double(), k)
+    terms = torch.where(terms.abs() > largest, terms.sign() * math.inf, terms)
+    scores = (terms * (128 + shared) ** -0.5).masked_fill(~((j <= at) & (j > at - span)), -math.inf)
+    weights = torch.softmax(scores, -1)
+    want = torch.einsum("htj,jhd->thd", weights, v)
+    spoilt = weights.isnan().any(-1).T
+    assert int(spoilt.sum()) == 150 * share + 1
+    assert bool(out[spoilt].isnan().all()) and bool(out[~spoilt].isfinite().all())
+    huge = torch.zeros_like(want, dtype=torch.bool)
+    huge[5:5 + span, :share, 9] = True
+    huge[310:, 2 * share:3 * share, 3] = True
+    plain_ones = ~huge & ~spoilt[..., None]
+    assert float((out.double() - want)[plain_ones].norm() / want[plain_ones].norm()) < 2e-6
+    assert float(((out.double() - want)[huge & ~spoilt[..., None]] / largest).abs().max()) < 1e-6
