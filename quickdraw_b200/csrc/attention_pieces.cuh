@@ -33,8 +33,8 @@ QD_DEVINL bool group_any(int id, bool found) {
 // four values as pieces into three planes
 QD_DEVINL void put_planes(bf16* to, int plane, const float4& x) {
     uint2 v[3];
-    split_three(x.x, x.y, v[0].x, v[1].x, v[2].x);
-    split_three(x.z, x.w, v[0].y, v[1].y, v[2].y);
+    split_three<false>(x.x, x.y, v[0].x, v[1].x, v[2].x);
+    split_three<false>(x.z, x.w, v[0].y, v[1].y, v[2].y);
 #pragma unroll
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * plane) = v[i];
 }

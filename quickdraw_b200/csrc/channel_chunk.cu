@@ -11,6 +11,8 @@
 // What enters a recurrence is fp32.  So every operand is three bf16 pieces, each rounded, and a product six of theirs (what is left
 // out is below 2^-26 of it).  The tensor core does not round sums to nearest, which would pull a state that lives long towards zero: what
 // a chunk adds to the state is summed from zero and added in fp32, large and small products have accumulators of their own.
+// The walk holds half of the state and of the values (exact, and everything is linear in the two), so that no piece rounds up to infinity; to
+// stop each one at the largest bf16 instead cost the chain 5 %.
 // The walk is a chain: 1.2 us a chunk (0.8 without the delta rule), of which the MMAs of a warp, at eight clocks, are 0.45 (0.2); before, it was
 // 285 ns a token on the FMA pipe.  2048 tokens, both kernels: delta rule of 32 / 16 heads of 128 583 / 581 -> 272 / 192 us (the prepare kernel 72 / 35
 // of them), gated linear attention of 16 heads 224 -> 126 us.  Error against 64 bits 1.4e-7 (1.4e-7 before), with decays near one 1.7e-7 (4.0e-7).
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(128) channel_prepare_kernel(const __grid_const
         const float2 a = *reinterpret_cast<const float2*>(m + g * ld + 2 * t), b = *reinterpret_cast<const float2*>(m + g * ld + 2 * t + 8);
         const float2 c = *reinterpret_cast<const float2*>(m + (g + 8) * ld + 2 * t), d = *reinterpret_cast<const float2*>(m + (g + 8) * ld + 2 * t + 8);
         const float x[2][4] = {{a.x, a.y, b.x, b.y}, {c.x, c.y, d.x, d.y}};
-        const Pieces v = split_tiles3(x[0], x[1]);
+        const Pieces v = split_tiles3<true>(x[0], x[1]);
         dst[0][lane] = v.p[0]; dst[1][lane] = v.p[1]; dst[2][lane] = v.p[2];
     };
 #pragma unroll
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(128) channel_prepare_kernel(const __grid_const
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int c = 0; c < 4; ++c) x[n][c] = m[(2 * t + (c & 1) + 8 * (c >> 1)) * kPad + 8 * n];
-        const Pieces v = split_tiles3(x[0], x[1]);
+        const Pieces v = split_tiles3<true>(x[0], x[1]);
 #pragma unroll
         for (int j = 0; j < 3; ++j) out->minus[kk][j][lane] = v.p[j];
     }
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[nt][c] = tile[(size_t)(8 * nt + 2 * t + (c & 1)) * p.vdim + 8 * (c >> 1)];
+            for (int c = 0; c < 4; ++c) acc[nt][c] = 0.5f * tile[(size_t)(8 * nt + 2 * t + (c & 1)) * p.vdim + 8 * (c >> 1)];
         bool ahead = false;                    // the next chunk's terms are there: asked for under this one's products (a look takes 200 clocks)
 #pragma unroll 1
         for (int chunk = 0; chunk < chunks; ++chunk) {
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
 #pragma unroll
             for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) u[n][c] = st.v[8 * n + 2 * t + (c & 1)][16 * slice + g + 8 * (c >> 1)];
+                for (int c = 0; c < 4; ++c) u[n][c] = 0.5f * st.v[8 * n + 2 * t + (c & 1)][16 * slice + g + 8 * (c >> 1)];
             if constexpr (DELTA) {
                 Sums sum[2] = {};
                 uint2 b[2][2][3];
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) tile[(size_t)(8 * nt + 2 * t + (c & 1)) * p.vdim + 8 * (c >> 1)] = acc[nt][c];
+            for (int c = 0; c < 4; ++c) tile[(size_t)(8 * nt + 2 * t + (c & 1)) * p.vdim + 8 * (c >> 1)] = 2.f * acc[nt][c];
         return;
     }
     // ---- results of tokens 8 half .. + 7 of a chunk
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__(walk_threads<SLICES>(), 1) channel_walk_kernel
         const int left = p.tokens - (p.first + chunk * kTok + 8 * half + 2 * t);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-            if ((c & 1) < left) to[(c & 1) * stride + 8 * (c >> 1)] = o[c];
+            if ((c & 1) < left) to[(c & 1) * stride + 8 * (c >> 1)] = 2.f * o[c];
     }
 }
 

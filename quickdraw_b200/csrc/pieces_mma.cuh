@@ -26,11 +26,13 @@ QD_DEVINL void split_tiles(const float (&l)[4], const float (&r)[4], uint4& hi, 
     split_pair(r[2], r[3], hi.w, lo.w);
 }
 QD_DEVINL float rounded_up(float x) { return __uint_as_float(__float_as_uint(x) + 0x8000u); }
+QD_DEVINL float kept_finite(float x) { return fminf(fmaxf(x, -3.38953139e38f), 3.38953139e38f); }      // to the largest bf16, 2^128 (1 - 2^-8)
 // x0, x1 as three bf16 pieces each, the first two rounded (half away from zero; in integer instructions, because the conversion of a pair
 // takes longer: 64 values of a lane 281 against 124 clocks): together they are x to its last bit or the one before.  Where x is an
-// infinity or NaN the third is NaN (the others need not be: a NaN's bits can run over).
-QD_DEVINL void split_three(float x0, float x1, uint32_t& a, uint32_t& b, uint32_t& c) {
-    float u = rounded_up(x0), v = rounded_up(x1);
+// infinity or NaN the third is NaN (the others need not be: a NaN's bits can run over).  From 2^128 (1 - 2^-9) on the first piece would round up to
+// infinity: with BOUND it stops at the largest bf16, else these magnitudes count as infinite.
+template <bool BOUND> QD_DEVINL void split_three(float x0, float x1, uint32_t& a, uint32_t& b, uint32_t& c) {
+    float u = rounded_up(BOUND ? kept_finite(x0) : x0), v = rounded_up(BOUND ? kept_finite(x1) : x1);
     a = upper_halves(u, v);
     x0 -= upper_half(u); x1 -= upper_half(v);
     u = rounded_up(x0); v = rounded_up(x1);
@@ -38,12 +40,12 @@ QD_DEVINL void split_three(float x0, float x1, uint32_t& a, uint32_t& b, uint32_
     c = upper_halves(x0 - upper_half(u), x1 - upper_half(v));
 }
 struct Pieces { uint4 p[3]; };
-QD_DEVINL Pieces split_tiles3(const float (&l)[4], const float (&r)[4]) {
+template <bool BOUND = false> QD_DEVINL Pieces split_tiles3(const float (&l)[4], const float (&r)[4]) {
     Pieces v;
-    split_three(l[0], l[1], v.p[0].x, v.p[1].x, v.p[2].x);
-    split_three(l[2], l[3], v.p[0].y, v.p[1].y, v.p[2].y);
-    split_three(r[0], r[1], v.p[0].z, v.p[1].z, v.p[2].z);
-    split_three(r[2], r[3], v.p[0].w, v.p[1].w, v.p[2].w);
+    split_three<BOUND>(l[0], l[1], v.p[0].x, v.p[1].x, v.p[2].x);
+    split_three<BOUND>(l[2], l[3], v.p[0].y, v.p[1].y, v.p[2].y);
+    split_three<BOUND>(r[0], r[1], v.p[0].z, v.p[1].z, v.p[2].z);
+    split_three<BOUND>(r[2], r[3], v.p[0].w, v.p[1].w, v.p[2].w);
     return v;
 }
 

@@ -660,6 +660,30 @@ def test_recurrence_in_chunks(delta, tokens, heads, kv_heads, vdim):
 
 
 @pytest.mark.parametrize("delta", [False, True])
+def test_recurrence_in_chunks_up_to_the_largest_number(delta):
+    """Values of the largest fp32 number, which two bf16 roundings of a piece would carry to infinity: their column against 64 bits, 1e-6 as above."""
+    tokens, heads, vdim, column = 40, 2, 32, 5
+    inputs, _, _ = recurrence_inputs(tokens, heads, heads, vdim, delta)
+    q, k, g, v, beta, scales, state = inputs
+    if not delta:
+        q *= 0.01; k *= 0.1                        # so that no sum passes the largest number either
+    v[7, 1, column], v[21, 1, column] = torch.finfo(torch.float32).max, -torch.finfo(torch.float32).max
+    out, last = run_chunked(inputs, tokens, heads, heads, vdim, delta)
+    s, want = state[1, :, column].to(F64), torch.empty(tokens, dtype=F64)
+    for t in range(tokens):
+        kt, qt, u = k[t, 1].to(F64), q[t, 1].to(F64), v[t, 1, column].to(F64)
+        s = s + s * g[t, 1].to(F64)
+        if delta:
+            kt, qt = kt * scales[t, 1, 0].to(F64), qt * scales[t, 1, 1].to(F64)
+            u = beta[t, 1].to(F64) * (u - kt @ s)
+        s = s + kt * u
+        want[t] = qt @ s
+    assert torch.isfinite(out).all() and torch.isfinite(last).all()
+    for a, b in ((out[:, 1, column], want), (last[1, :, column], s)):
+        assert float((a.to(F64) - b).norm() / b.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("delta", [False, True])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 def test_recurrence_in_chunks_keeps_to_the_past(delta, bad):
     """A value that is not finite reaches its column from its token on and nothing else."""
