@@ -64,8 +64,8 @@ class BatchDecode(ChunkPrefill):
         self._graphs = {}
 
     def _attn_splits(self, batch, context):
-        """Context splits per (sequence, KV head), 16 at most.  Heads of 256, up to 256 sequences: the kernel shares the context out by the
-        sequences' own lengths and only wants to know how many parts the scratch has room for.  Else the count whose blocks
+        """Context splits per (sequence, KV head), 16 at most.  Heads of 256, up to 256 sequences: the kernel cuts a sequence by its own
+        length (a neighbour's changes nothing) and only wants to know how many parts the scratch has room for.  Else the count whose blocks
         fill whole waves of the GPU best (one block per SM; a split costs a merge)."""
         if self.ckpt.config.head_dim == 256 and batch <= 256:
             return MAX_ATTN_SPLITS

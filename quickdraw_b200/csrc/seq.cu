@@ -1082,122 +1082,137 @@ batch_attn_mma_kernel(const LaneAttnParams p) {
     lane_attn_finish(p, red, z, kvh, split, active, tid);
 }
 
-// The same with the batch's whole context shared out evenly, whatever the sequences' lengths and the cache's capacity: the 32-position units of
-// all (sequence, KV head) pairs lie one after the other and block b takes units [b share, (b + 1) share), most often parts of one or
-// two pairs.  A pair that one block holds needs no partial result; of others the last block to arrive merges at most `splits` parts.
-// With a split count from the capacity (32768 where the contexts were 8192) a block of 512 positions spent half of its 27 us on its start and
-// on merging its warps: 32 sequences of 8192 positions, 16 heads on 2 of 256, 190 -> 97 us
-// (537 MB); of 2000 103 -> 45, of 500 75 -> 22, of 64 60 -> 13.  At most kFlatBatch sequences.
-constexpr int kFlatBatch = kLaneAttnWarps * 32, kFlatMin = 8;           // units of a share at least, where a sequence has as many
+// The same for a batch of sequences of their own lengths.  A (sequence, KV head) pair is cut into parts by its own length and the number of pairs
+// alone, so that a sequence's result does not depend on its neighbours: as many parts as fill the GPU, none above kFlatMost units of 32 positions
+// where the scratch has room for as many, none below kFlatMin.  The parts of all pairs lie one after the other, and block b takes
+// those that begin in its share of the work.  A pair of one part needs no partial result; of others the last block to arrive merges.
+// Before, a block for each (pair, split) with a split count from the capacity (a block of 512 positions spent half of its 27 us on its
+// start and on merging its warps); then the units of all pairs shared out evenly, which cut a sequence where its neighbours' lengths happened to; now.  With
+// the preparation, 16 heads on 2 of 256, weights and caches from HBM, us: 32 sequences of 8192 positions 202 / 114 / 122 (537 MB), of 2000 112 / 52 /
+// 50, of 500 85 / 32 / 36, of 64 68 / 21 / 23; 8 of 8192 87 / 58 / 56, one 64 / 52 / 46; 32 of 30 to 8192 157 / 89 / 108; one of 8192 beside 31 of 64
+// 71 / 99 / 62.  kFlatMost of 32 / 48 / 96: 148 / 132 / 155 for the first, 105 / 105 / 97 for the mixed ones, 50 / 56 / 77 for the last.  Parts of less
+// than kFlatMin units are not worth their merge.  At most kFlatBatch sequences.
+constexpr int kFlatBatch = kLaneAttnWarps * 32, kFlatMin = 8, kFlatMost = 64;
+constexpr int kFlatFixed = 8;                                // what a part costs beside its units, in units (6 us)
+QD_DEVINL int flat_part(int n, int pairs, int blocks, int splits) {               // units of a part of a sequence of n
+    const int parts = min(splits, max(blocks / pairs, (n + kFlatMost - 1) / kFlatMost));
+    return parts > 1 ? max((n + parts - 1) / parts, min(n, kFlatMin)) : n;
+}
 __global__ void __launch_bounds__(kLaneAttnWarps * 32, 1)
 batch_attn_flat_kernel(const LaneAttnParams p, int batch) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char mma_attn_smem[];
-    __shared__ int before[kFlatBatch + 1], longest[kLaneAttnWarps], sums[kLaneAttnWarps], s_last;
+    __shared__ long long before[kFlatBatch + 1], sums[kLaneAttnWarps];
+    __shared__ int s_last;
     __shared__ float weight[kLaneAttnGroup][16], most[kLaneAttnGroup], norm[kLaneAttnGroup];
     constexpr int D = 256;
     uint8_t* q_s = mma_attn_smem;                                                       // [8][kAttnQRow]
     float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][D + 2]
-    const int G = p.hq / p.hk, stride = D + 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    {   // units of the sequences in front of each
-        const int T = tid < batch ? p.positions[tid] + 1 : 0, n = T < 1 || T > p.capacity ? 0 : (T + 31) / 32;     // (outside the cache: left alone)
-        int sum = n;
+    const int G = p.hq / p.hk, stride = D + 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = batch * p.hk;
+    const auto units_of = [&](int z) {
+        const int T = p.positions[z] + 1;
+        return T < 1 || T > p.capacity ? 0 : (T + 31) / 32;                             // (outside the cache: left alone)
+    };
+    {   // work of the sequences in front of each
+        const int n = tid < batch ? units_of(tid) : 0, per = n ? flat_part(n, pairs, (int)gridDim.x, p.splits) : 1;
+        long long sum = (long long)p.hk * ((n + per - 1) / per) * (per + kFlatFixed);
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int up = __shfl_up_sync(0xffffffffu, sum, d);
+            const long long up = __shfl_up_sync(0xffffffffu, sum, d);
             if (lane >= d) sum += up;
         }
-        const int top = __reduce_max_sync(0xffffffffu, n);
-        if (lane == 31) { sums[warp] = sum; longest[warp] = top; }
+        if (lane == 31) sums[warp] = sum;
         __syncthreads();
-        int front = 0;
+        long long front = 0;
         for (int w = 0; w < warp; ++w) front += sums[w];
         if (tid < batch) before[tid + 1] = front + sum;
         if (tid == 0) before[0] = 0;
         __syncthreads();
     }
-    int top = 0;
-    for (int w = 0; w < kLaneAttnWarps; ++w) top = max(top, longest[w]);
-    const int units = p.hk * before[batch];
-    const int share = max(max((units + (int)gridDim.x - 1) / (int)gridDim.x, min(kFlatMin, top)), (top + p.splits - 2) / (p.splits - 1));
-    const int end = min(units, ((int)blockIdx.x + 1) * share);
-    for (int u = (int)blockIdx.x * share; u < end;) {
-        int lo = 0, hi = batch;                              // hk before[lo] <= u < hk before[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (p.hk * before[mid] <= u) lo = mid; else hi = mid;
-        }
-        const size_t z = lo;
-        const int n = before[lo + 1] - before[lo], kvh = (u - p.hk * before[lo]) / n, start = p.hk * before[lo] + kvh * n, from = u - start;
-        const int count = min(end - u, n - from), T = p.positions[z] + 1, first = start / share, parts = (start + n - 1) / share - first + 1;
-        lane_attn_walk(p, q_s, red, z, kvh, T, from * 32, min(T, (from + count) * 32), tid);
-        __syncthreads();
-        if (tid < 8 * kLaneAttnGroup) {                      // a lane for each warp's state of a head
-            const int h = tid >> 3, w = tid & 7;
-            const float* src = red + ((size_t)w * G + h) * stride + D;
-            const float m = h < G ? src[0] : -INFINITY, l = h < G ? src[1] : 0.f;
-            float mm = m;
+    const long long all = before[batch], begin = all * blockIdx.x / gridDim.x, end = all * (blockIdx.x + 1) / gridDim.x;
+    int first = 0;                                           // the sequence in which the share begins
+    for (int hi = batch; hi - first > 1;) {
+        const int mid = (first + hi) >> 1;
+        if (before[mid] <= begin) first = mid; else hi = mid;
+    }
+    int part = -1;                                           // of a sequence's, all KV heads; the share's first one is still to be found
+    for (int seq = first; seq < batch; ++seq, part = 0) {
+        const int n = units_of(seq);
+        if (n == 0) continue;
+        const size_t z = seq;
+        const int per = flat_part(n, pairs, (int)gridDim.x, p.splits), parts = (n + per - 1) / per, cost = per + kFlatFixed, T = p.positions[seq] + 1;
+        if (part < 0) part = (int)((begin - before[seq] + cost - 1) / cost);
+        for (; part < p.hk * parts; ++part) {
+            if (before[seq] + (long long)part * cost >= end) return;
+            const int kvh = part / parts, at = part - kvh * parts;
+            lane_attn_walk(p, q_s, red, z, kvh, T, at * per * 32, min(T, (at + 1) * per * 32), tid);
+            __syncthreads();
+            if (tid < 8 * kLaneAttnGroup) {                      // a lane for each warp's state of a head
+                const int h = tid >> 3, w = tid & 7;
+                const float* src = red + ((size_t)w * G + h) * stride + D;
+                const float m = h < G ? src[0] : -INFINITY, l = h < G ? src[1] : 0.f;
+                float mm = m;
 #pragma unroll
-            for (int d = 1; d < 8; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
-            const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
-            float den = wgt * l;
+                for (int d = 1; d < 8; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+                const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+                float den = wgt * l;
 #pragma unroll
-            for (int d = 1; d < 8; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-            weight[h][w] = wgt;
-            if (w == 0) { most[h] = mm; norm[h] = den; }
-        }
-        __syncthreads();
-        const auto put = [&](int h, float num, float den) {
-            const int qh = kvh * G + h;
-            const float gate = round_bf16(sigmoid_precise(ld_bf16(p.qg + (z * p.hq + qh) * 2 * (size_t)D + D + tid)));
-            p.out[(z * p.hq + qh) * (size_t)D + tid] = __float2bfloat16_rn(round_bf16(num / den) * gate);
-        };
-        float* partial = p.partial + (z * p.hk + kvh) * (size_t)p.splits * G * stride;            // [part][G][D + 2]
-        for (int h = 0; h < G; ++h) {                        // a thread's feature of every head
-            float num = 0.f;
-#pragma unroll
-            for (int w = 0; w < kLaneAttnWarps; ++w) num += weight[h][w] * red[((size_t)w * G + h) * stride + tid];
-            if (parts == 1) put(h, num, norm[h]);
-            else {
-                float* dst = partial + ((size_t)(blockIdx.x - first) * G + h) * stride;
-                dst[tid] = num;
-                if (tid == 0) { dst[D] = most[h]; dst[D + 1] = norm[h]; }
+                for (int d = 1; d < 8; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+                weight[h][w] = wgt;
+                if (w == 0) { most[h] = mm; norm[h] = den; }
             }
-        }
-        if (parts > 1) {
-            unsigned int* counter = p.counters + z * p.hk + kvh;
-            __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)parts - 1;
-            __syncthreads();
-            if (s_last) {
+            const auto put = [&](int h, float num, float den) {
+                const int qh = kvh * G + h;
+                const float gate = round_bf16(sigmoid_precise(ld_bf16(p.qg + (z * p.hq + qh) * 2 * (size_t)D + D + tid)));
+                p.out[(z * p.hq + qh) * (size_t)D + tid] = __float2bfloat16_rn(round_bf16(num / den) * gate);
+            };
+            float* partial = p.partial + (z * p.hk + kvh) * (size_t)p.splits * G * stride;            // [part][G][D + 2]
+            for (int h = 0; h < G; ++h) {                        // a thread's feature of every head
+                float num = 0.f;
+#pragma unroll
+                for (int w = 0; w < kLaneAttnWarps; ++w) num += weight[h][w] * red[((size_t)w * G + h) * stride + tid];
+                if (parts == 1) put(h, num, norm[h]);
+                else {
+                    float* dst = partial + ((size_t)at * G + h) * stride;
+                    dst[tid] = num;
+                    if (tid == 0) { dst[D] = most[h]; dst[D + 1] = norm[h]; }
+                }
+            }
+            if (parts > 1) {
+                unsigned int* counter = p.counters + z * p.hk + kvh;
                 __threadfence();
-                if (tid < 16 * kLaneAttnGroup) {             // a lane for each part's state of a head
-                    const int h = tid >> 4, s = tid & 15;
-                    const bool on = h < G && s < parts;
-                    const float* src = partial + ((size_t)s * G + h) * stride + D;
-                    const float m = on ? __ldcg(src) : -INFINITY, l = on ? __ldcg(src + 1) : 0.f;
-                    float mm = m;
-#pragma unroll
-                    for (int d = 1; d < 16; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
-                    const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
-                    float den = wgt * l;
-#pragma unroll
-                    for (int d = 1; d < 16; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-                    weight[h][s] = wgt;
-                    if (s == 0) norm[h] = den;
-                }
                 __syncthreads();
-                for (int h = 0; h < G; ++h) {
-                    float num = 0.f;
-                    for (int s = 0; s < parts; ++s) num += weight[h][s] * __ldcg(partial + ((size_t)s * G + h) * stride + tid);
-                    put(h, num, norm[h]);
+                if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)parts - 1;
+                __syncthreads();
+                if (s_last) {
+                    __threadfence();
+                    if (tid < 16 * kLaneAttnGroup) {             // a lane for each part's state of a head
+                        const int h = tid >> 4, s = tid & 15;
+                        const bool on = h < G && s < parts;
+                        const float* src = partial + ((size_t)s * G + h) * stride + D;
+                        const float m = on ? __ldcg(src) : -INFINITY, l = on ? __ldcg(src + 1) : 0.f;
+                        float mm = m;
+#pragma unroll
+                        for (int d = 1; d < 16; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+                        const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+                        float den = wgt * l;
+#pragma unroll
+                        for (int d = 1; d < 16; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+                        weight[h][s] = wgt;
+                        if (s == 0) norm[h] = den;
+                    }
+                    __syncthreads();
+                    for (int h = 0; h < G; ++h) {
+                        float num = 0.f;
+                        for (int s = 0; s < parts; ++s) num += weight[h][s] * __ldcg(partial + ((size_t)s * G + h) * stride + tid);
+                        put(h, num, norm[h]);
+                    }
+                    if (tid == 0) *counter = 0;
                 }
-                if (tid == 0) *counter = 0;
             }
+            __syncthreads();                                     // the states and weights are read
         }
-        __syncthreads();                                     // the states and weights are read
-        u += count;
     }
 }
 

@@ -277,6 +277,35 @@ def test_batch_attention_shares_the_context_out(cuda_device, hq, hkv, lengths):
         assert float((out - outs[0]).abs().max()) <= 2.0 ** -7 * float(outs[0][~outside].abs().max())
 
 
+@pytest.mark.parametrize("hq,hkv,batch,length", [(16, 2, 8, 1000), (16, 2, 32, 1024), (4, 2, 60, 700), (8, 1, 3, 513), (8, 1, 200, 70)])
+def test_batch_attention_of_a_sequence_does_not_depend_on_its_neighbours(cuda_device, hq, hkv, batch, length):
+    """The same sequence in every place of a batch, beside neighbours of other lengths, some outside the cache: the same bits."""
+    from quickdraw_b200._lib import call, lib, ptr, stream_of
+    dev, cap, d = cuda_device, 1024, 256
+    gen = torch.Generator(device=dev).manual_seed(length)
+    new = lambda *shape: torch.randn(shape, generator=gen, device=dev).to(torch.bfloat16)
+    qg, k_new, v_new, q_norm, k_norm = (new(1, n).expand(batch, n).contiguous() for n in (hq * 2 * d, hkv * d, hkv * d, d, d))
+    k0, v0 = new(1, cap, hkv, d), new(1, cap, hkv, d)
+    scratch = torch.empty(batch * lib().qd_attn_scratch_floats(hq, hkv, d, 16), device=dev)
+    counters = torch.zeros(batch * hkv, dtype=torch.int32, device=dev)
+    mine = torch.zeros(batch, dtype=torch.bool, device=dev)
+    mine[0] = mine[batch // 2] = mine[-1] = True
+    outs = []
+    for others in ("same", 0, 1, 40, cap, cap + 1, "mixed"):
+        lengths = torch.full((batch,), length, dtype=torch.int32, device=dev)
+        if others == "mixed":
+            lengths = torch.where(mine, lengths, torch.randint(0, cap + 2, (batch,), generator=gen, device=dev, dtype=torch.int32))
+        elif others != "same":
+            lengths[~mine] = others
+        kb, vb = k0.expand(batch, -1, -1, -1).clone(), v0.expand(batch, -1, -1, -1).clone()
+        out, q_scratch = (torch.full((batch, hq * d), 7.0, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        call("qd_batch_attention", ptr(qg), ptr(k_new), ptr(v_new), ptr(q_norm[0]), ptr(k_norm[0]), ptr(kb), ptr(vb), kb.stride(0), ptr(q_scratch),
+             ptr(out), ptr(scratch), ptr(counters), ptr(lengths - 1), batch, cap, hq, hkv, d, 64, 1e6, 1e-6, 16, stream_of(qg))
+        assert int(counters.abs().sum()) == 0
+        outs += [out[i] for i in range(batch) if mine[i]]
+    assert torch.isfinite(outs[0]).all() and all(torch.equal(o, outs[0]) for o in outs)
+
+
 def test_batch_decode_with_the_published_checkpoint_formats(cuda_device):
     """FP8 mixers and an NVFP4 LM head in the batched step (E4M3 x E4M3 product, NVFP4 rows form):
     the first step of two sequences from empty state against the single-sequence step (one step:
