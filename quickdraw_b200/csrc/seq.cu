@@ -1316,6 +1316,8 @@ seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts
                 if (r + 2 < routes) id[u].z = __ldg(ids + r + 2);
                 if (r + 3 < routes) id[u].w = __ldg(ids + r + 3);
             }
+            const auto known = [&](int e) { return (unsigned)e < (unsigned)experts ? e : INT_MAX; };      // others are in nobody's run
+            id[u] = make_int4(known(id[u].x), known(id[u].y), known(id[u].z), known(id[u].w));
         }
     };
     int below = 0, mine[OWN];
@@ -1364,7 +1366,7 @@ seq_group_routes_kernel(const int32_t* __restrict__ ids, int routes, int experts
             if (!__any_sync(0xffffffffu, some)) continue;
 #pragma unroll
             for (int k = 0; k < OWN; ++k) {
-                        int rank = 0, all = 0;
+                int rank = 0, all = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const unsigned same = __ballot_sync(0xffffffffu, four[j] == e0 + k);

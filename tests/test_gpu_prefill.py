@@ -279,6 +279,22 @@ def test_group_routes_of_every_block_of_experts(cuda_device, routes, experts, of
     assert torch.equal(order.long(), want_order) and torch.equal(boundaries.long(), want_boundaries)
 
 
+@pytest.mark.parametrize("routes,experts", [(200, 5), (16385, 129), (9000, 257), (20000, 641)])
+def test_group_routes_leaves_out_ids_of_no_expert(cuda_device, routes, experts):
+    """Negative ids and ids from ``experts`` on (also those that the last block would own) are in no expert's run, and the first run begins at 0."""
+    from quickdraw_b200._lib import call, ptr, stream_of
+    gen = torch.Generator().manual_seed(routes)
+    ids = torch.randint(-3, experts + 8, (routes,), generator=gen).to(torch.int32).to(cuda_device)
+    order = torch.full((routes,), -1, dtype=torch.int32, device=cuda_device)
+    boundaries = torch.full((experts + 1,), -1, dtype=torch.int32, device=cuda_device)
+    call("qd_seq_group_routes", ptr(ids), routes, experts, ptr(order), ptr(boundaries), stream_of(ids))
+    known = ((ids >= 0) & (ids < experts)).nonzero()[:, 0]
+    sorted_ids, at = ids[known].sort(stable=True)
+    want_boundaries = torch.searchsorted(sorted_ids, torch.arange(experts + 1, device=cuda_device, dtype=torch.int32))
+    assert torch.equal(order[:known.numel()].long(), known[at]) and bool((order[known.numel():] == -1).all())
+    assert torch.equal(boundaries.long(), want_boundaries)
+
+
 @pytest.mark.parametrize("tokens,rows0,rows1,width", [(64, 32, 32, 2048), (511, 256, 1, 2048), (2048, 256, 1, 2048), (2048, 32, 32, 2048), (100, 7, 300, 192),
                                                       (129, 16, 17, 3072), (1030, 1, 1, 64), (3000, 600, 31, 512), (70, 4096, 5, 256)])
 def test_two_small_products_of_many_tokens(cuda_device, tokens, rows0, rows1, width):
