@@ -235,7 +235,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, chunks = p.in_features / 256;
     const int across = (p.tokens + 255) / 256, tiles = across * ((p.out_features + 255) / 256);
-    const int steps = pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0;         // stages that the pair takes
+    const auto steps_of_pair = [&] { return pair < tiles ? ((tiles - 1 - pair) / pairs + 1) * chunks : 0; };       // (its value held throughout costs spills)
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -253,7 +253,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
     const uint32_t tmem = *tmem_slot;
 
     // A wait that runs out ends a role; the loads end when the MMAs have taken the last of them or 0.2 s after it (the limit of a wait), the
-    // blocks when a commit of all MMAs has arrived, and both together.
+    // issuing warp when a commit of all MMAs has arrived, and both blocks together.
     if (warp == 0) {
         const bool leader = elect_one();
         int st = 0, n = 1;
@@ -283,7 +283,7 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
                 if (st >= kStages) { st -= kStages; parity ^= 1u; }
             }
         }
-        if (n) pair_loads_taken(bars->empty, kStages, steps, p.status);
+        if (n) pair_loads_taken(bars->empty, kStages, steps_of_pair(), p.status);
     } else if (warp == 1) {
         if (rank == 0) {
             const bool leader = elect_one();
@@ -316,11 +316,12 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
                 if (leader) pair_commit(&bars->ready);
                 __syncwarp();
             }
-            if (leader) pair_commit(&bars->drained);
+            if (leader) pair_commit_here(&bars->drained);     // tensor memory is given back only behind the last MMA, also where a wait ran out
+            mbar_wait(&bars->drained, 0, p.status);
         }
     } else if (warp < T::kFirst) {
         const uint32_t quarter = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T::kColSf;
-        const int group = (warp - 2) >> 2;
+        const int group = (warp - 2) >> 2, steps = steps_of_pair();
         bool ok = true;
         for (int it = group; it < steps; it = next_scale_step(it)) {
             const int st = it % kStages;
@@ -387,8 +388,6 @@ w4a4_pair_kernel(const __grid_constant__ Gemm4Params p, const __grid_constant__ 
             }
         }
     }
-    __syncthreads();
-    if (warp == 1) mbar_wait(&bars->drained, 0, p.status);     // tensor memory is given back only behind the last MMA, also where a wait ran out
     __syncwarp();
     tc_fence_before();
     cluster_sync();

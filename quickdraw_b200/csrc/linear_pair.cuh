@@ -117,7 +117,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     uint64_t* empty = full + kStages;
     uint64_t* ready = empty + kStages;         // an accumulator holds a tile
     uint64_t* taken = ready + 2;               // (the first block's:) both blocks have read it
-    uint64_t* drained = taken + 2;             // every MMA has ended
+    uint64_t* drained = taken + 2;             // (the first block's:) every MMA has ended
     uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -136,7 +136,7 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
     const uint32_t tmem = *slot;
 
     // A wait that runs out ends a role; the loads end when the MMAs have taken the last of them or 0.2 s after it (the limit of a wait), the
-    // blocks when a commit of all MMAs has arrived, and both together.
+    // issuing warp when a commit of all MMAs has arrived, and both blocks together.
     if (warp == 0) {
         const bool leader = elect_one();
         int st = 0, n = 1;
@@ -192,7 +192,8 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
                 if (leader) pair_commit(ready + buf);
                 __syncwarp();
             }
-            if (leader) pair_commit(drained);
+            if (leader) pair_commit_here(drained);            // tensor memory is given back only behind the last MMA, also where a wait ran out
+            mbar_wait(drained, 0, p.status);
         }
     } else {
         const int quadrant = warp & 3, half = (warp - 2) >> 2;        // lanes of tensor memory that the warp may read; columns that it takes
@@ -235,8 +236,6 @@ linear_pair_kernel(const __grid_constant__ LinearParams p, const __grid_constant
             if (lane == 0) arrive_at(of_first_block(taken + buf));
         }
     }
-    __syncthreads();
-    if (warp == 1) mbar_wait(drained, 0, p.status);           // tensor memory is given back only behind the last MMA, also where a wait ran out
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync();

@@ -23,6 +23,9 @@ QD_DEVINL void pair_commit(uint64_t* bar) {                           // arrives
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
+QD_DEVINL void pair_commit_here(uint64_t* bar) {                      // arrives in this block alone
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 QD_DEVINL void arrive_at(uint32_t bar) {                              // `bar` as of of_first_block
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
