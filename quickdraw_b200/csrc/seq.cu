@@ -1003,9 +1003,10 @@ QD_DEVINL void attn_load_keys(AttnKeys& k, const uint8_t* __restrict__ base, siz
 
 // Positions [t0, t1) of sequence z against the query heads of KV head kvh by all warps of a block: every warp's running state into
 // red[warp][head][d + 2] (weighted values, maximum, sum).
+template <int PAD>
 QD_DEVINL void lane_attn_walk(const LaneAttnParams& p, uint8_t* q_s, float* red, size_t z, int kvh, int T, int t0, int t1, int tid) {
     constexpr int D = 256;
-    const int G = p.hq / p.hk, stride = D + 2, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int G = p.hq / p.hk, stride = D + 8 * PAD + 2, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const size_t row_bytes = (size_t)p.hk * D * sizeof(bf16);
     const uint8_t* kc = reinterpret_cast<const uint8_t*>(p.k_cache + z * p.cache_stride + (size_t)kvh * D);
     const uint8_t* vc = reinterpret_cast<const uint8_t*>(p.v_cache + z * p.cache_stride + (size_t)kvh * D);
@@ -1050,15 +1051,15 @@ QD_DEVINL void lane_attn_walk(const LaneAttnParams& p, uint8_t* q_s, float* red,
     acc.l += __shfl_xor_sync(0xffffffffu, acc.l, 2);
     if (t == 0 && g < G) {
         float* dst = red + ((size_t)warp * G + g) * stride;
-        dst[D] = acc.m; dst[D + 1] = acc.l;
+        dst[D + 8 * PAD] = acc.m; dst[D + 8 * PAD + 1] = acc.l;
     }
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
         const int h = 2 * t + cc;
         if (h >= G) continue;
-        float* dst = red + ((size_t)warp * G + h) * stride + 32 * g;
+        float* dst = red + ((size_t)warp * G + h) * stride + (32 + PAD) * g;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { dst[2 * i] = acc.out[i][cc]; dst[2 * i + 1] = acc.out[i][2 + cc]; }
+        for (int i = 0; i < 16; ++i) *reinterpret_cast<float2*>(dst + 2 * i) = make_float2(acc.out[i][cc], acc.out[i][2 + cc]);
     }
 }
 
@@ -1077,142 +1078,171 @@ batch_attn_mma_kernel(const LaneAttnParams p) {
     if (active > p.splits) active = p.splits;
     const int per = ((T + active - 1) / active + 31) & ~31;
     const int t0 = split * per, t1 = min(T, t0 + per);
-    lane_attn_walk(p, q_s, red, z, kvh, T, t0, split < active ? t1 : t0, tid);
+    lane_attn_walk<0>(p, q_s, red, z, kvh, T, t0, split < active ? t1 : t0, tid);
     __syncthreads();
     lane_attn_finish(p, red, z, kvh, split, active, tid);
 }
 
-// The same for a batch of sequences of their own lengths.  A (sequence, KV head) pair is cut into parts by its own length and the number of pairs
-// alone, so that a sequence's result does not depend on its neighbours: as many parts as fill the GPU, none above kFlatMost units of 32 positions
-// where the scratch has room for as many, none below kFlatMin.  The parts of all pairs lie one after the other, and block b takes
-// those that begin in its share of the work.  A pair of one part needs no partial result; of others the last block to arrive merges.
-// Before, a block for each (pair, split) with a split count from the capacity (a block of 512 positions spent half of its 27 us on its
-// start and on merging its warps); then the units of all pairs shared out evenly, which cut a sequence where its neighbours' lengths happened to; now.  With
-// the preparation, 16 heads on 2 of 256, weights and caches from HBM, us: 32 sequences of 8192 positions 202 / 114 / 122 (537 MB), of 2000 112 / 52 /
-// 50, of 500 85 / 32 / 36, of 64 68 / 21 / 23; 8 of 8192 87 / 58 / 56, one 64 / 52 / 46; 32 of 30 to 8192 157 / 89 / 108; one of 8192 beside 31 of 64
-// 71 / 99 / 62.  kFlatMost of 32 / 48 / 96: 148 / 132 / 155 for the first, 105 / 105 / 97 for the mixed ones, 50 / 56 / 77 for the last.  Parts of less
-// than kFlatMin units are not worth their merge.  At most kFlatBatch sequences.
-constexpr int kFlatBatch = kLaneAttnWarps * 32, kFlatMin = 8, kFlatMost = 64;
-constexpr int kFlatFixed = 8;                                // what a part costs beside its units, in units (6 us)
-QD_DEVINL int flat_part(int n, int pairs, int blocks, int splits) {               // units of a part of a sequence of n
-    const int parts = min(splits, max(blocks / pairs, (n + kFlatMost - 1) / kFlatMost));
-    return parts > 1 ? max((n + parts - 1) / parts, min(n, kFlatMin)) : n;
+// The same for a batch of sequences of their own lengths.  A (sequence, KV head) pair is cut into parts by its own length, the number of pairs and that of
+// blocks alone, so that a sequence's result does not depend on its neighbours.  The parts, largest first, go to the blocks in rounds, to and
+// fro.  A pair of one part needs no partial result; of others the last block to arrive merges.  Before, a block for each (pair, split)
+// with a split count from the capacity (a block of 512 positions spent half of its 27 us on its start and on merging its warps); then the
+// units of all pairs shared out evenly, which cut a sequence where its neighbours' lengths happened to; now.  With the preparation, 16
+// heads on 2 of 256, caches from HBM, us: 32 sequences of 8192 positions 202 / 112 / 112 (537 MB), of 5000 - / 82 / 79, of 2000 112 / 54 / 50, of 500
+// 85 / 32 / 32, of 64 68 / 22 / 23; 8 of 8192 87 / 58 / 52, one 64 / 52 / 40; 100 of 1000 216 / 69 / 77; 32 of 30 to 8192 157 / 91 / 98, 16 - / 73 /
+// 60, 64 249 / 134 / 142; one of 8192 beside 31 of 64 71 / 99 / 95.  Parts of at most 64 units whatever the batch: 122 for the first, and 40 more
+// for 32 of 8193, whose five parts make three rounds.
+// A part's fixed cost is 6 to 7 us (a unit 0.75); kFlatMin of 4 / 8 / 16, us: 32 of 256 positions 21.3 / 18.2 / 18.2, 8 of 1000 24 / 23.5 / 28,
+// one of 300 20.2 / 20.6 / 16.2.  At most kFlatBatch sequences.
+constexpr int kFlatBatch = kLaneAttnWarps * 32, kFlatMin = 8, kFlatLarge = 64;
+constexpr int kFlatFixed = 9, kFlatAlone = 5;                // what a part costs beside its units, in units; where a sequence is not cut
+constexpr int kFlatPad = 2, kFlatRow = 256 + 8 * kFlatPad + 2;     // floats of a warp's state of a head: 32 features and a bank offset, eight times; maximum, sum
+// Units of a part of a sequence of n: into 1 .. splits parts as a batch of such sequences would take least time, rounds[k - 1] rounds of k parts
+// each; within 1 / 16 of that smaller ones, down to kFlatLarge, because beside other lengths the largest parts decide.
+QD_DEVINL int flat_part(int n, const int* rounds, int splits) {
+    long long cost[16], least = LLONG_MAX;
+    int best = n;
+#pragma unroll
+    for (int k = 1; k <= 16; ++k) {
+        const int per = max((n + k - 1) / k, min(n, kFlatMin));
+        cost[k - 1] = k <= splits ? (long long)rounds[k - 1] * (per + (k > 1 ? kFlatFixed : kFlatAlone)) : LLONG_MAX;
+        if (cost[k - 1] < least) { least = cost[k - 1]; best = per; }
+    }
+    least += least / 16;
+#pragma unroll
+    for (int k = 2; k <= 16; ++k) {
+        const int per = (n + k - 1) / k;
+        if (per >= kFlatLarge && per < best && cost[k - 1] <= least) best = per;
+    }
+    return best;
 }
 __global__ void __launch_bounds__(kLaneAttnWarps * 32, 1)
 batch_attn_flat_kernel(const LaneAttnParams p, int batch) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char mma_attn_smem[];
-    __shared__ long long before[kFlatBatch + 1], sums[kLaneAttnWarps];
-    __shared__ int s_last;
+    __shared__ int rounds[16], per_of[kFlatBatch], order[kFlatBatch], before[kFlatBatch + 1], sums[kLaneAttnWarps], s_last;
     __shared__ float weight[kLaneAttnGroup][16], most[kLaneAttnGroup], norm[kLaneAttnGroup];
     constexpr int D = 256;
     uint8_t* q_s = mma_attn_smem;                                                       // [8][kAttnQRow]
-    float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][D + 2]
-    const int G = p.hq / p.hk, stride = D + 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = batch * p.hk;
+    float* red = reinterpret_cast<float*>(mma_attn_smem + 8 * kAttnQRow);               // [warps][G][kFlatRow]
+    const int G = p.hq / p.hk, stride = D + 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, feature = tid + tid / 32 * kFlatPad;
     const auto units_of = [&](int z) {
         const int T = p.positions[z] + 1;
         return T < 1 || T > p.capacity ? 0 : (T + 31) / 32;                             // (outside the cache: left alone)
     };
-    {   // work of the sequences in front of each
-        const int n = tid < batch ? units_of(tid) : 0, per = n ? flat_part(n, pairs, (int)gridDim.x, p.splits) : 1;
-        long long sum = (long long)p.hk * ((n + per - 1) / per) * (per + kFlatFixed);
+    {   // the sequences by the size of their parts, largest first, and how many parts are in front of each
+        if (tid < 16) rounds[tid] = (int)(((long long)batch * p.hk * (tid + 1) + gridDim.x - 1) / gridDim.x);
+        __syncthreads();
+        const int n = tid < batch ? units_of(tid) : 0, per = n ? flat_part(n, rounds, p.splits) : 0;
+        per_of[tid] = per;
+        __syncthreads();
+        if (tid < batch) {
+            int rank = 0;
+            for (int z = 0; z < batch; ++z) rank += per_of[z] > per || (per_of[z] == per && z < tid);
+            order[rank] = tid;
+            before[rank + 1] = n ? p.hk * ((n + per - 1) / per) : 0;
+        }
+        if (tid == 0) before[0] = 0;
+        __syncthreads();
+        int sum = tid < batch ? before[tid + 1] : 0;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const long long up = __shfl_up_sync(0xffffffffu, sum, d);
+            const int up = __shfl_up_sync(0xffffffffu, sum, d);
             if (lane >= d) sum += up;
         }
         if (lane == 31) sums[warp] = sum;
         __syncthreads();
-        long long front = 0;
-        for (int w = 0; w < warp; ++w) front += sums[w];
-        if (tid < batch) before[tid + 1] = front + sum;
-        if (tid == 0) before[0] = 0;
+        for (int w = 0; w < warp; ++w) sum += sums[w];
+        if (tid < batch) before[tid + 1] = sum;
         __syncthreads();
     }
-    const long long all = before[batch], begin = all * blockIdx.x / gridDim.x, end = all * (blockIdx.x + 1) / gridDim.x;
-    int first = 0;                                           // the sequence in which the share begins
-    for (int hi = batch; hi - first > 1;) {
-        const int mid = (first + hi) >> 1;
-        if (before[mid] <= begin) first = mid; else hi = mid;
-    }
-    int part = -1;                                           // of a sequence's, all KV heads; the share's first one is still to be found
-    for (int seq = first; seq < batch; ++seq, part = 0) {
-        const int n = units_of(seq);
-        if (n == 0) continue;
-        const size_t z = seq;
-        const int per = flat_part(n, pairs, (int)gridDim.x, p.splits), parts = (n + per - 1) / per, cost = per + kFlatFixed, T = p.positions[seq] + 1;
-        if (part < 0) part = (int)((begin - before[seq] + cost - 1) / cost);
-        for (; part < p.hk * parts; ++part) {
-            if (before[seq] + (long long)part * cost >= end) return;
-            const int kvh = part / parts, at = part - kvh * parts;
-            lane_attn_walk(p, q_s, red, z, kvh, T, at * per * 32, min(T, (at + 1) * per * 32), tid);
-            __syncthreads();
-            if (tid < 8 * kLaneAttnGroup) {                      // a lane for each warp's state of a head
-                const int h = tid >> 3, w = tid & 7;
-                const float* src = red + ((size_t)w * G + h) * stride + D;
-                const float m = h < G ? src[0] : -INFINITY, l = h < G ? src[1] : 0.f;
-                float mm = m;
-#pragma unroll
-                for (int d = 1; d < 8; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
-                const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
-                float den = wgt * l;
-#pragma unroll
-                for (int d = 1; d < 8; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-                weight[h][w] = wgt;
-                if (w == 0) { most[h] = mm; norm[h] = den; }
-            }
-            __syncthreads();
-            const auto put = [&](int h, float num, float den) {
-                const int qh = kvh * G + h;
-                const float gate = round_bf16(sigmoid_precise(ld_bf16(p.qg + (z * p.hq + qh) * 2 * (size_t)D + D + tid)));
-                p.out[(z * p.hq + qh) * (size_t)D + tid] = __float2bfloat16_rn(round_bf16(num / den) * gate);
-            };
-            float* partial = p.partial + (z * p.hk + kvh) * (size_t)p.splits * G * stride;            // [part][G][D + 2]
-            for (int h = 0; h < G; ++h) {                        // a thread's feature of every head
-                float num = 0.f;
-#pragma unroll
-                for (int w = 0; w < kLaneAttnWarps; ++w) num += weight[h][w] * red[((size_t)w * G + h) * stride + tid];
-                if (parts == 1) put(h, num, norm[h]);
-                else {
-                    float* dst = partial + ((size_t)at * G + h) * stride;
-                    dst[tid] = num;
-                    if (tid == 0) { dst[D] = most[h]; dst[D + 1] = norm[h]; }
-                }
-            }
-            if (parts > 1) {
-                unsigned int* counter = p.counters + z * p.hk + kvh;
-                __threadfence();
-                __syncthreads();
-                if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)parts - 1;
-                __syncthreads();
-                if (s_last) {
-                    __threadfence();
-                    if (tid < 16 * kLaneAttnGroup) {             // a lane for each part's state of a head
-                        const int h = tid >> 4, s = tid & 15;
-                        const bool on = h < G && s < parts;
-                        const float* src = partial + ((size_t)s * G + h) * stride + D;
-                        const float m = on ? __ldcg(src) : -INFINITY, l = on ? __ldcg(src + 1) : 0.f;
-                        float mm = m;
-#pragma unroll
-                        for (int d = 1; d < 16; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
-                        const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
-                        float den = wgt * l;
-#pragma unroll
-                        for (int d = 1; d < 16; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-                        weight[h][s] = wgt;
-                        if (s == 0) norm[h] = den;
-                    }
-                    __syncthreads();
-                    for (int h = 0; h < G; ++h) {
-                        float num = 0.f;
-                        for (int s = 0; s < parts; ++s) num += weight[h][s] * __ldcg(partial + ((size_t)s * G + h) * stride + tid);
-                        put(h, num, norm[h]);
-                    }
-                    if (tid == 0) *counter = 0;
-                }
-            }
-            __syncthreads();                                     // the states and weights are read
+    const int all = before[batch], blocks = (int)gridDim.x;
+    // rounds of parts, one a block, to and fro, so that who had a larger one takes a smaller one next
+    for (int round = 0; round * blocks < all; ++round) {
+        const int r = round * blocks + (round & 1 ? blocks - 1 - (int)blockIdx.x : (int)blockIdx.x);
+        if (r >= all) continue;
+        int lo = 0;
+        for (int hi = batch; hi - lo > 1;) {
+            const int mid = (lo + hi) >> 1;
+            if (before[mid] <= r) lo = mid; else hi = mid;
         }
+        const size_t z = order[lo];
+        const int per = per_of[z], n = units_of((int)z), T = p.positions[z] + 1, parts = (n + per - 1) / per, part = r - before[lo];
+        const int kvh = part / parts, at = part - kvh * parts;
+        lane_attn_walk<kFlatPad>(p, q_s, red, z, kvh, T, at * per * 32, min(T, (at + 1) * per * 32), tid);
+        __syncthreads();
+        if (tid < 8 * kLaneAttnGroup) {                      // a lane for each warp's state of a head
+            const int h = tid >> 3, w = tid & 7;
+            const float* src = red + ((size_t)w * G + h) * kFlatRow + D + 8 * kFlatPad;
+            const float m = h < G ? src[0] : -INFINITY, l = h < G ? src[1] : 0.f;
+            float mm = m;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+            const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+            float den = wgt * l;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+            weight[h][w] = wgt;
+            if (w == 0) { most[h] = mm; norm[h] = den; }
+        }
+        __syncthreads();
+        const auto put = [&](int h, float num, float den) {
+            const int qh = kvh * G + h;
+            const float gate = round_bf16(sigmoid_precise(ld_bf16(p.qg + (z * p.hq + qh) * 2 * (size_t)D + D + tid)));
+            p.out[(z * p.hq + qh) * (size_t)D + tid] = __float2bfloat16_rn(round_bf16(num / den) * gate);
+        };
+        float* partial = p.partial + (z * p.hk + kvh) * (size_t)p.splits * G * stride;            // [part][G][D + 2]
+        for (int h = 0; h < G; ++h) {                        // a thread's feature of every head
+            float num = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLaneAttnWarps; ++w) num += weight[h][w] * red[((size_t)w * G + h) * kFlatRow + feature];
+            if (parts == 1) put(h, num, norm[h]);
+            else {
+                float* dst = partial + ((size_t)at * G + h) * stride;
+                dst[tid] = num;
+                if (tid == 0) { dst[D] = most[h]; dst[D + 1] = norm[h]; }
+            }
+        }
+        if (parts > 1) {
+            unsigned int* counter = p.counters + z * p.hk + kvh;
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(counter, 1u) == (unsigned int)parts - 1;
+            __syncthreads();
+            if (s_last) {
+                __threadfence();
+                if (tid < 16 * kLaneAttnGroup) {             // a lane for each part's state of a head
+                    const int h = tid >> 4, s = tid & 15;
+                    const bool on = h < G && s < parts;
+                    const float* src = partial + ((size_t)s * G + h) * stride + D;
+                    const float m = on ? __ldcg(src) : -INFINITY, l = on ? __ldcg(src + 1) : 0.f;
+                    float mm = m;
+#pragma unroll
+                    for (int d = 1; d < 16; d <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, d));
+                    const float wgt = m == -INFINITY ? 0.f : expf(m - mm);
+                    float den = wgt * l;
+#pragma unroll
+                    for (int d = 1; d < 16; d <<= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+                    weight[h][s] = wgt;
+                    if (s == 0) norm[h] = den;
+                }
+                __syncthreads();
+                float num[kLaneAttnGroup] = {};          // all heads of a part requested at once
+#pragma unroll 2
+                for (int s = 0; s < parts; ++s) {
+                    float v[kLaneAttnGroup];
+#pragma unroll
+                    for (int h = 0; h < kLaneAttnGroup; ++h) v[h] = h < G ? __ldcg(partial + ((size_t)s * G + h) * stride + tid) : 0.f;
+#pragma unroll
+                    for (int h = 0; h < kLaneAttnGroup; ++h) num[h] += weight[h][s] * v[h];
+                }
+#pragma unroll
+                for (int h = 0; h < kLaneAttnGroup; ++h)
+                    if (h < G) put(h, num[h], norm[h]);
+                if (tid == 0) *counter = 0;
+            }
+        }
+        __syncthreads();                                     // the states and weights are read
     }
 }
 
@@ -1745,7 +1775,8 @@ extern "C" int qd_batch_attention(const void* qg, const void* k_new, const void*
                     return QD_ERR_LAUNCH;
                 flat_configured[dev] = true;
             }
-            qd_launch(batch_attn_flat_kernel, dim3(most < sms ? (int)most : sms), dim3(kLaneAttnWarps * 32), mma_smem, (cudaStream_t)stream, true, p, batch);
+            qd_launch(batch_attn_flat_kernel, dim3(most < sms ? (int)most : sms), dim3(kLaneAttnWarps * 32),
+                      8 * kAttnQRow + sizeof(float) * (size_t)kLaneAttnWarps * G * kFlatRow, (cudaStream_t)stream, true, p, batch);
             return qd_launch_status();
         }
         qd_launch(batch_attn_mma_kernel, dim3(kv_heads, splits, batch), dim3(kLaneAttnWarps * 32), mma_smem, (cudaStream_t)stream, true, p);
