@@ -695,7 +695,7 @@ def run_gpu(args):
         # both operands NVFP4 (activations quantised per chunk): no measured FP4 peak exists on this
         # pool, so the fraction is given against the measured bf16 burst (the nominal FP4 dense
         # rate is four times the bf16 one) and against the nominal 9 PFLOP/s
-        "w4a4_gemm_roofline": {"bound": "tensor", "kernel": "nvfp4_gemm_w4a4_kernel (tcgen05 kind::mxf4nvf4, 8192 tokens x [8192, 2048])",
+        "w4a4_gemm_roofline": {"bound": "tensor", "kernel": "w4a4_pair_kernel (tcgen05 kind::mxf4nvf4, 8192 tokens x [8192, 2048])",
                                "achieved": w4a4_tflops, "peak": tensor_peak, "unit": "TFLOP/s",
                                "frac": w4a4_tflops / tensor_peak, "peak_source": f"{tensor_peak_kind} cuBLAS bf16",
                                "frac_of_nominal_fp4": w4a4_tflops / 9000.0, "launch_us": w4a4_launch_s * 1e6,

@@ -1,5 +1,7 @@
 // Gated linear recurrences with one decay per head and key channel over a long run of tokens, sixteen tokens at a time on the tensor
-// cores (linear_recurrence.cu has the definitions and the walk of a token at a time).  With G_t the products of the decays
+// cores (linear_recurrence.cu has the definitions and the walk of a token at a time).  The chunked forms are published: gated linear attention with
+// Gated Linear Attention Transformers (Yang et al., 2023), the delta rule with Parallelizing Linear Transformers with the Delta Rule (Yang et al.,
+// 2024).  With G_t the products of the decays
 // of tokens 0 .. t of a chunk, per key channel, S_0 the state in front of it and G_C the product of all sixteen:
 //   K+ = k_t G_t,  Q+ = q_t G_t,  K- = k_t G_C / G_t                                    (formed as products, never as quotients: all <= 1)
 //   L[t][i] = beta_t sum_c k_t[c] k_i[c] (decays of i + 1 .. t)[c]  for i < t,  A[t][i] the same with q_t, for i <= t
@@ -12,7 +14,7 @@
 // out is below 2^-26 of it).  The tensor core does not round sums to nearest, which would pull a state that lives long towards zero: what
 // a chunk adds to the state is summed from zero and added in fp32, large and small products have accumulators of their own.
 // The walk holds half of the state and of the values (exact, and everything is linear in the two), so that no piece rounds up to infinity; to
-// stop each one at the largest bf16 instead cost the chain 5 %.
+// stop each one at the largest bf16 instead cost the chain 4 %.
 // The walk is a chain: 1.2 us a chunk (0.8 without the delta rule), of which the MMAs of a warp, at eight clocks, are 0.45 (0.2); before, it was
 // 285 ns a token on the FMA pipe.  2048 tokens, both kernels: delta rule of 32 / 16 heads of 128 583 / 581 -> 272 / 192 us (the prepare kernel 72 / 35
 // of them), gated linear attention of 16 heads 224 -> 126 us.  Error against 64 bits 1.4e-7 (1.4e-7 before), with decays near one 1.7e-7 (4.0e-7).

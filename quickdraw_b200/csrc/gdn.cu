@@ -219,7 +219,8 @@ gdn_gated_norm128_kernel(const bf16* __restrict__ o, const bf16* __restrict__ z,
 extern "C" int qd_gdn_gated_norm(const void* o, const void* z, const void* gamma, void* out, int heads,
                                  int value_dim, float eps, void* stream) {
     QD_CHECK_ARG(o && z && gamma && out && heads > 0 && value_dim > 0);
-    // (few heads, a token's 32: a warp each, so that their loads start side by side)
+    // Below, a warp each: the two differ by 0.3 us there (32 / 1024 heads 2.0 / 2.1 us in whole pieces, 2.3 / 2.4 a warp a head; 2048 2.1 | 2.6, 4096 2.6 |
+    // 3.4, 16384 4.6 | 6.4), and the sums of a decode step keep their order.
     if (heads >= 2048 && value_dim == 128 && !(((uintptr_t)o | (uintptr_t)z | (uintptr_t)gamma | (uintptr_t)out) & 15u)) {
         qd_launch(gdn_gated_norm128_kernel, dim3((heads + 15) / 16), dim3(128), 0, (cudaStream_t)stream, true,
                   (const bf16*)o, (const bf16*)z, (const bf16*)gamma, (bf16*)out, heads, eps);

@@ -494,10 +494,11 @@ static int launch_gemm(const GemmParams& p, int row_tiles, int busy_row_tiles, c
     const long long wide = (long long)busy_row_tiles * ((p.out_features + 255) / 256);
     // weight codes are fetched two K steps ahead where the registers allow it (plain product)
     constexpr int kAhead = DENSE ? 2 : 1;
-    // (narrower tiles to balance the last round of blocks do not pay: a 128-row block takes far
-    // more than half the time of a 256-row block - gate bank of a 511-token chunk 143 -> 191 us)
-    // Plain product: the fewer rounds of blocks, a round of 128-row tiles taking 5/8 of one of 256-row tiles (2048 inputs: 20 and 32 us):
-    // 2048 tokens to 4096 rows one round of 128 wide tiles 33.2 us, two of narrow ones 39.9.
+    // Grouped product: narrower tiles to balance the last round of blocks do not pay, a 128-row block takes far
+    // more than half the time of a 256-row block (gate bank of a 511-token chunk 143 -> 191 us).
+    // Plain product: the fewer rounds of blocks, a round of 128-row tiles counted as 5/8 of one of 256-row tiles.  Wide against narrow, us, of 512 /
+    // 2048 / 4096 inputs: one round against two 14.9 | 18.0, 33.2 | 39.2, 55 | 66, two against four 27.9 | 34.9, 62.8 | 75.7, 107 | 128; two against three
+    // 27.2 | 26.4 and 105.9 | 97.6 (512, 4096), one against one 54.6 | 34.4 (4096).
     const bool fill = DENSE ? 8 * ((wide + sms - 1) / sms) <= 5 * ((2 * wide + sms - 1) / sms) : wide >= sms;
     if (fill) return launch_variant<256, DENSE, kAhead, TM>(p, row_tiles, stream);
     if (4 * wide >= sms) return launch_variant<128, DENSE, kAhead, TM>(p, row_tiles, stream);
@@ -516,8 +517,8 @@ extern "C" int qd_nvfp4_matmul(const void* x, const void* codes, const void* sca
     p.x = (const bf16*)x; p.codes = (const uint8_t*)codes; p.scales = (const uint8_t*)scales; p.global = global;
     p.y = (bf16*)y; p.tokens = tokens; p.out_features = out_features; p.in_features = in_features; p.status = status;
     const int row_tiles = (tokens + kTileM - 1) / kTileM;
-    // so few 256-token tiles that even 64-row weight tiles leave SMs idle: 128-token tiles, two
-    // blocks per SM (measured on a 511-token chunk: better for the projections up to 4096 rows,
+    // so few 256-token tiles that even 64-row weight tiles leave SMs idle: 128-token tiles
+    // (measured on a 511-token chunk: better for the projections up to 4096 rows,
     // worse for 8192 rows, where 128-row weight tiles already fill the GPU)
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);

@@ -195,8 +195,8 @@ nvfp4_gemm_w4a4_kernel(const __grid_constant__ Gemm4Params p, const __grid_const
 //               eight columns per 64-input step
 //   the last 8  sums, 32 tokens x 128 outputs each, as bf16 through shared memory in whole 128-byte lines
 // What bounded both forms was the way of the scales, some 1000 clocks a stage for its four warps from the wait to the hand-over: 8192 x 8192 x
-// 2048 127 us before, here 141 with one group of four warps, 111 with two, 102 with three, then the operands from L2 (1100 clocks a
-// stage).  2048 x 8192 x 2048 37 -> 33 us.
+// 2048 127 us before, here 141 with one group of four warps, 111 with two, 105 with three (102 before a stage had a group of its own).  Its
+// counters there: L2 40 % busy, tensor pipe 32 %, issue 20 %.  2048 x 8192 x 2048 37 -> 33 us.
 struct Pair4 {
     static constexpr int kStages = 5, kStageBytes = 2 * kCodeBytes + 3 * kScaleBytes, kEpilogueWarps = 8, kStagingBytes = 32 * 128;
     static constexpr int kScaleGroups = 3, kFirst = 2 + 4 * kScaleGroups, kThreads = 32 * (kFirst + kEpilogueWarps);

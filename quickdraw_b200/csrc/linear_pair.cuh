@@ -6,8 +6,8 @@
 // and the accumulators of its tokens twice, so that one tile is read out while the next is multiplied; rows leave through shared
 // memory in whole 128-byte lines.  Inputs and outputs, bf16, before and now (cuBLAS): 2048 tokens 2048 -> 4160 39.1 -> 30.3 us (29.9), 2048 -> 12416
 // 114 -> 77 (73), 2048 -> 16384 with gated pairs 116 -> 93, 576 -> 4096 for 3071 tokens 35.8 -> 18.2, 8192 -> 2048 56 -> 51 (48); 8192 tokens
-// 2048 -> 8192 259 -> 185 (176) = 1.49 PFLOP/s.  What bounds it: operands come from L2 at some 40 bytes a clock and SM (tiles of 128 weight rows,
-// which ask for half as much again per product, took 305 us there), and the power limit.
+// 2048 -> 8192 259 -> 185 (176) = 1.49 PFLOP/s.  What bounds that one is the tensor pipe, active in 90 % of the cycles (L2 49 % busy), at the clock that
+// the power limit leaves.  (Tiles of 128 weight rows, which ask L2 for half as much again per product, took 305 us.)
 #pragma once
 #include "pair.cuh"
 

@@ -744,3 +744,22 @@ def test_head_norm_and_gate_of_heads_of_128(cuda_device, dtype, tokens, heads, a
     want = v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(g) * (1 if act else g)
     bound = want.abs() * (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -19)
     assert bool(((out.double().view_as(want) - want).abs() <= bound + 1e-30).all())
+
+
+@pytest.mark.parametrize("cuts", [[512], [256, 640]])
+def test_portions_at_multiples_of_a_chunk_change_no_bit(cuda_device, cuts):
+    """A bf16 prompt in portions that end where chunks of the recurrences (16 tokens) and blocks of the attention (64) end: the logits and the
+    history of the whole prompt.  (Other portions move both by some bf16 roundings.)"""
+    config = synthetic.fezopel_config(6, hidden=1024, heads=8, kv_heads=2, window=256)
+    engine = Engine(synthetic.make_fezopel(config, 5, "cuda"), max_context=900, device="cuda", dtype=torch.bfloat16)
+    tokens = torch.randint(0, config.vocab_size, (900,), generator=torch.Generator().manual_seed(5)).tolist()
+    results = []
+    for places in (cuts, []):
+        engine.reset()
+        at = 0
+        for cut in places:
+            engine.extend(tokens[at:cut])
+            at = cut
+        logits = engine.extend(tokens[at:], [len(tokens) - at - 1])
+        results.append([logits, *(t.clone() for t in engine.state.history())])
+    assert all(torch.equal(a, b) for a, b in zip(*results)) and torch.isfinite(results[0][0]).all()

@@ -353,7 +353,7 @@ def test_operator_table_kernels_read_nothing_before_their_wait():
     assert body.index("if (p.ids_in || p.wait_first) grid_dependency_wait();") < body.index("bulk_load(")
     entry = sources["stream.cu"][sources["stream.cu"].index("int qd_stream_matvec_try("):]
     assert entry.index("p.prologue = PRO_NONE;") < entry.index("p.wait_first = 1;") < entry.index("return stream_launch(p, 0, stream, 3);")
-    for name in ("act_quantize_kernel", "nvfp4_gemm_w4a4_kernel", "rms_norm_kernel", "gdn_conv_kernel"):
+    for name in ("act_quantize_kernel", "nvfp4_gemm_w4a4_kernel", "w4a4_pair_kernel", "rms_norm_kernel", "gdn_conv_kernel"):
         body = kernel(name)[1]
         assert "chain_enter" not in body and "grid_launch_dependents" not in body, name
 
